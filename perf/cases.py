@@ -51,38 +51,38 @@ PRESET = {"bits": 2, "group": 64}
 def listed():
     return [
         # one layer of one request, as a serving engine's attention backend calls it per layer and token
-        {"name": "call, 3000 tokens", "kind": "call", "tokens": 3000, "block": 64, "heads": 8, "q_heads": 32},
+        {"name": "call 3000", "kind": "call", "tokens": 3000, "block": 64, "heads": 8, "q_heads": 32},
         # a short conversation: the step's fixed costs weigh as much as its bytes (odd length, fp16)
-        {"name": "step, 28 x 1999", "kind": "step", "layers": 28, "tokens": 1999, "block": 256, "heads": 4, "q_heads": 28,
+        {"name": "step 28x1999", "kind": "step", "layers": 28, "tokens": 1999, "block": 256, "heads": 4, "q_heads": 28,
          "dtype": "fp16", "graph": True, **PRESET},
         # the benchmark's decode step: one request of 32768 tokens, replayed from a graph
-        {"name": "step, 28 x 32768", "kind": "step", "layers": 28, "tokens": 32768, "block": 256, "heads": 4, "q_heads": 28,
+        {"name": "step 28x32768", "kind": "step", "layers": 28, "tokens": 32768, "block": 256, "heads": 4, "q_heads": 28,
          "dtype": "bf16", "graph": True, **PRESET},
         # the longest context: one request of 131072 tokens on one GPU
-        {"name": "step, 28 x 131072", "kind": "step", "layers": 28, "tokens": 131072, "block": 256, "heads": 4, "q_heads": 28,
+        {"name": "step 28x131072", "kind": "step", "layers": 28, "tokens": 131072, "block": 256, "heads": 4, "q_heads": 28,
          "dtype": "bf16", "graph": False, **PRESET},
         # the cache's default value codec (values coded like the keys)
-        {"name": "step, 28 x 16384, coded values", "kind": "step", "layers": 28, "tokens": 16384, "block": 256, "heads": 4,
+        {"name": "step 28x16384 coded values", "kind": "step", "layers": 28, "tokens": 16384, "block": 256, "heads": 4,
          "q_heads": 28, "dtype": "bf16", "graph": False, "bits": 0, "group": 64},
         # a model's own decode loop: append and attention layer by layer through the cache
-        {"name": "loop, 28 x 4096", "kind": "loop", "layers": 28, "tokens": 4096, "block": 256, "heads": 4, "q_heads": 28,
+        {"name": "loop 28x4096", "kind": "loop", "layers": 28, "tokens": 4096, "block": 256, "heads": 4, "q_heads": 28,
          "dtype": "bf16", **PRESET},
         # batched serving, 16 requests with contexts of 4096 to 32768 tokens: pages of 64 and of 16 tokens
-        {"name": "paged, 16 requests, pages of 64", "kind": "paged", "requests": 16, "layers": 32, "low": 4096, "high": 32768,
+        {"name": "paged 16 requests by 64", "kind": "paged", "requests": 16, "layers": 32, "low": 4096, "high": 32768,
          "block": 64, "heads": 8, "q_heads": 32},
-        {"name": "paged, 16 requests, pages of 16", "kind": "paged", "requests": 16, "layers": 32, "low": 4096, "high": 32768,
+        {"name": "paged 16 requests by 16", "kind": "paged", "requests": 16, "layers": 32, "low": 4096, "high": 32768,
          "block": 16, "heads": 8, "q_heads": 32},
         # a long prompt in chunks of 2048 tokens, one layer
-        {"name": "prompt, 32768 by 2048", "kind": "prompt", "tokens": 32768, "chunk": 2048, "block": 256, "heads": 4,
+        {"name": "prompt 32768 by 2048", "kind": "prompt", "tokens": 32768, "chunk": 2048, "block": 256, "heads": 4,
          "q_heads": 28, "dtype": "bf16", **PRESET},
         # a fresh prompt of a serving engine (ragged, fp16)
-        {"name": "prefill, 1500 of 1500", "kind": "prefill", "queries": 1500, "tokens": 1500, "heads": 8, "q_heads": 32,
+        {"name": "prefill 1500", "kind": "prefill", "queries": 1500, "tokens": 1500, "heads": 8, "q_heads": 32,
          "dtype": "fp16"},
         # a prompt and a following chunk through the cache alone, one layer
-        {"name": "update, 32000 and 700", "kind": "update", "tokens": 32000, "chunk": 700, "block": 256, "heads": 4,
+        {"name": "update 32000 and 700", "kind": "update", "tokens": 32000, "chunk": 700, "block": 256, "heads": 4,
          "dtype": "bf16", **PRESET},
         # the pages of a prompt, one layer
-        {"name": "pages, 12000 tokens by 64", "kind": "pages", "tokens": 12000, "block": 64, "heads": 8, "dtype": "bf16"},
+        {"name": "pages 12000 by 64", "kind": "pages", "tokens": 12000, "block": 64, "heads": 8, "dtype": "bf16"},
     ]
 
 
