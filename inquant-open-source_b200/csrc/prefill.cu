@@ -6,7 +6,8 @@
 //     row of S from tensor memory (tcgen05.ld) once, takes base-2 probabilities against a lazily
 //     raised reference maximum (the pass is repeated in the rare case that the maximum has to
 //     rise) and writes P in the model dtype back to tensor memory (tcgen05.st) over S.
-//   * warp 8 (one lane): issues the contractions.  S = Q K^T (tcgen05.mma 128 x 128 x 128, both
+//   * warp 8 (an elected lane of the converged warp, see tc_elect: issued from a branch on the lane index the
+//     same MMAs took the 2048 x 32768 chunk 1185 instead of 1033 us): issues the contractions.  S = Q K^T (tcgen05.mma 128 x 128 x 128, both
 //     operands in shared memory) and O += P V (128 x 128 x 128, P from tensor memory, V as an
 //     MN-major shared-memory operand), fp32 accumulators in tensor memory.  The order S_A, S_B,
 //     PV_A, S_A', PV_B, S_B', ... keeps the tensor core busy with one tile while the other
@@ -27,7 +28,7 @@
 #include <algorithm>
 #include <type_traits>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace inq {
 
@@ -56,40 +57,10 @@ struct PrefillParams {
   int* status;
 };
 
-__device__ __forceinline__ unsigned pf_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-// 64-bit shared-memory matrix descriptor, 128-byte swizzle: start address, leading and stride
-// byte offsets in 16-byte units, descriptor version 1, layout type 2.
-__device__ __forceinline__ unsigned long long pf_desc(unsigned saddr, unsigned lbo_bytes, unsigned sbo_bytes) {
-  unsigned long long d = 0;
-  d |= (unsigned long long)((saddr & 0x3FFFFu) >> 4);
-  d |= (unsigned long long)(lbo_bytes >> 4) << 16;
-  d |= (unsigned long long)(sbo_bytes >> 4) << 32;
-  d |= 1ull << 46;
-  d |= 2ull << 61;
-  return d;
-}
-
-__device__ __forceinline__ void pf_mma(unsigned tmem_d, unsigned long long da, unsigned long long db, unsigned idesc,
-                                       unsigned accumulate) {
-  asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }"
-               ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void pf_mma_ta(unsigned tmem_d, unsigned tmem_a, unsigned long long db, unsigned idesc,
-                                          unsigned accumulate) {
-  asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
-               ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void pf_commit(unsigned mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
-}
 // Bounded wait; gives up early when another role has raised the abort flag.
 __device__ __forceinline__ bool pf_wait(unsigned mbar, unsigned parity, volatile int* abort_flag) {
   for (int it = 0; it < kPfSpinLimit; ++it) {
-    unsigned done;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                 : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
-    if (done) return true;
+    if (tc_try_wait(mbar, parity)) return true;
     if ((it & 255) == 255 && *abort_flag) return false;
   }
   *abort_flag = 1;
@@ -97,27 +68,6 @@ __device__ __forceinline__ bool pf_wait(unsigned mbar, unsigned parity, volatile
 }
 __device__ __forceinline__ void pf_arrive(unsigned mbar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
-}
-__device__ __forceinline__ void pf_tmem_ld32(unsigned taddr, unsigned (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
-      "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr) : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void pf_tmem_st32(unsigned taddr, const unsigned (&v)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
-      "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
-        "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
-        "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-      : "memory");
 }
 __device__ __forceinline__ float pf_exp2(float x) {
   float y;
@@ -151,7 +101,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
   // no static shared memory: the dynamic region starts the CTA's window, 1024-byte aligned as the
   // 128-byte swizzle needs (checked below)
   extern __shared__ __align__(1024) unsigned char pf_raw[];
-  const unsigned smem0 = pf_smem(pf_raw);
+  const unsigned smem0 = tc_smem(pf_raw);
   const unsigned sQ = smem0;                                  // tile A, then tile B
   const unsigned sKb = smem0 + 2 * kPfTileBytes;              // K stages
   const unsigned sVb = sKb + kPfStages * kPfTileBytes;        // V stages
@@ -160,7 +110,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
   const unsigned bars = smem0 + kPfTiles + 16;
   const unsigned bar_q = bars, bar_k = bars + 8 /* per stage */, bar_v = bar_k + 8 * kPfStages /* per stage */;
   const unsigned bar_s = bar_v + 8 * kPfStages /* A, B */, bar_p = bar_s + 16 /* A, B */, bar_o = bar_p + 16 /* A, B */;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   if (smem0 & 1023u) {
     if (tid == 0) atomicOr(P.status, INQ_STATUS_BAD_INDEX);
     return;
@@ -185,28 +135,28 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
 
   if (tid == 0) {
     *abort_flag = 0;
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_q) : "memory");
+    tc_bar_init(bar_q, 1);
 #pragma unroll
     for (int i = 0; i < kPfStages; ++i) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_k + 8 * i) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_v + 8 * i) : "memory");
+      tc_bar_init(bar_k + 8 * i, 1);
+      tc_bar_init(bar_v + 8 * i, 1);
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_s + 8 * i) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_p + 8 * i), "r"(kPfTile) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_o + 8 * i) : "memory");
+      tc_bar_init(bar_s + 8 * i, 1);
+      tc_bar_init(bar_p + 8 * i, kPfTile);
+      tc_bar_init(bar_o + 8 * i, 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 8) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 ::"r"(pf_smem(tmem_base_p)), "r"(kPfTmemCols) : "memory");
+                 ::"r"(tc_smem(tmem_base_p)), "r"(kPfTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  tc_fence_before();
   __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  tc_fence_after();
   const unsigned tmem = *tmem_base_p;
 
   if (warp == 9) {
@@ -245,32 +195,35 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
     }
   } else if (warp == 8) {
     // ================================================================ MMA warp
-    if (lane == 0 && n_b > 0) {
+    if (n_b > 0) {
       // instruction descriptors: fp32 accumulate, A/B in the model dtype, M = N = 128; the value
       // tile is an MN-major B operand (tokens are its K dimension, stored row by row)
-      const unsigned fmt = std::is_same<QT, __half>::value ? 0u : 1u;
-      const unsigned idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
-      const unsigned idesc_o = idesc_s | (1u << 16);
+      constexpr bool kBf16 = !std::is_same<QT, __half>::value;
+      constexpr unsigned idesc_s = tc_idesc<kBf16, 128, 128, false>(), idesc_o = tc_idesc<kBf16, 128, 128, true>();
       auto issue_s = [&](int x, int t) {      // S_x = Q_x K(t)^T
         const unsigned q = sQ + x * kPfTileBytes, k = sKb + (t % kPfStages) * kPfTileBytes;
+        if (tc_elect()) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const unsigned off = (kk >> 2) * kPfSlab + (kk & 3) * 32;
-          pf_mma(tmem + x * kPfTile, pf_desc(q + off, 16, 1024), pf_desc(k + off, 16, 1024), idesc_s, kk > 0);
+          for (int kk = 0; kk < 8; ++kk) {
+            const unsigned off = (kk >> 2) * kPfSlab + (kk & 3) * 32;
+            tc_mma(tmem + x * kPfTile, tc_desc(q + off, 16, 1024), tc_desc(k + off, 16, 1024), idesc_s, kk > 0);
+          }
+          tc_commit(bar_s + 8 * x);
         }
-        pf_commit(bar_s + 8 * x);
       };
       auto issue_o = [&](int x, int t) {      // O_x += P_x V(t): 16 tokens per step = 8 columns of packed P
         const unsigned v = sVb + (t % kPfStages) * kPfTileBytes;
+        if (tc_elect()) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          pf_mma_ta(tmem + 2 * kPfTile + x * kPfTile, tmem + x * kPfTile + kk * 8, pf_desc(v + kk * 2048, kPfSlab, 1024), idesc_o,
-                    (t > 0 || kk > 0) ? 1u : 0u);
-        pf_commit(bar_o + 8 * x);
+          for (int kk = 0; kk < 8; ++kk)
+            tc_mma_ta(tmem + 2 * kPfTile + x * kPfTile, tmem + x * kPfTile + kk * 8, tc_desc(v + kk * 2048, kPfSlab, 1024), idesc_o,
+                      (t > 0 || kk > 0) ? 1u : 0u);
+          tc_commit(bar_o + 8 * x);
+        }
       };
       bool ok = pf_wait(bar_q, 0, abort_flag) && pf_wait(bar_k, 0, abort_flag);
       if (ok) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tc_fence_after();
         if (n_a > 0) issue_s(0, 0);
         issue_s(1, 0);
       }
@@ -279,7 +232,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
         if (a_live) ok = ok && pf_wait(bar_p, (unsigned)t & 1u, abort_flag);       // P_A(t) written, S_A(t) read
         ok = ok && pf_wait(bar_v + 8 * (t % kPfStages), (unsigned)(t / kPfStages) & 1u, abort_flag);
         if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tc_fence_after();
         if (a_live) issue_o(0, t);
         if (t + 1 < n_b) {
           ok = pf_wait(bar_k + 8 * ((t + 1) % kPfStages), (unsigned)((t + 1) / kPfStages) & 1u, abort_flag);
@@ -288,7 +241,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
         }
         ok = pf_wait(bar_p + 8, (unsigned)t & 1u, abort_flag);                     // P_B(t) written, S_B(t) read
         if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tc_fence_after();
         issue_o(1, t);
         if (t + 1 < n_b) issue_s(1, t + 1);
       }
@@ -312,7 +265,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
       // S(t) is complete; the contractions run in issue order, so PV(t-1) is complete as well:
       // the columns of P may be overwritten by S and O may be rescaled
       if (!pf_wait(my_s, (unsigned)t & 1u, abort_flag)) { ok = false; break; }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      tc_fence_after();
       const bool masked = kv0 + kPfTile - 1 > diag0;
       // ---- one pass over S: probabilities against the running reference maximum are packed
       //      into registers while the row maximum is tracked; P is stored over S only afterwards,
@@ -326,7 +279,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
 #pragma unroll
         for (int c0 = 0; c0 < kPfTile; c0 += 32) {
           unsigned v[32];
-          pf_tmem_ld32(tS + c0, v);
+          tc_ld32(tS + c0, v);
+          tc_wait_ld();
 #pragma unroll
           for (int c = 0; c < 32; c += 2) {
             const float s0 = __uint_as_float(v[c]), s1 = __uint_as_float(v[c + 1]);
@@ -357,10 +311,11 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
 #pragma unroll 1
           for (int c0 = 0; c0 < kPfTile; c0 += 32) {
             unsigned v[32];
-            pf_tmem_ld32(tO + c0, v);
+            tc_ld32(tO + c0, v);
+            tc_wait_ld();
 #pragma unroll
             for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) * factor);
-            pf_tmem_st32(tO + c0, v);
+            tc_st32(tO + c0, v);
           }
         }
         if (masked) pass(std::true_type{}); else pass(std::false_type{});
@@ -373,16 +328,16 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
           lo[c] = packed[c];
           hi[c] = packed[32 + c];
         }
-        pf_tmem_st32(tS, lo);
-        pf_tmem_st32(tS + 32, hi);
+        tc_st32(tS, lo);
+        tc_st32(tS + 32, hi);
       }
       // P is in tensor memory, S has been read: hand both to the MMA warp
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      tc_wait_st();
+      tc_fence_before();
       pf_arrive(my_p);
     }
     if (n_x > 0) ok = ok && pf_wait(my_o, (unsigned)(n_x - 1) & 1u, abort_flag);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    tc_fence_after();
 
     if (P.splits == 1) {
       // ---- normalise and store this thread's row
@@ -392,7 +347,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
 #pragma unroll 1
       for (int c0 = 0; c0 < kPfTile; c0 += 32) {
         unsigned v[32];
-        pf_tmem_ld32(tO + c0, v);
+        tc_ld32(tO + c0, v);
+        tc_wait_ld();
         if (live) {
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
@@ -413,7 +369,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
       for (int c0 = 0; c0 < kPfTile; c0 += 32) {
         unsigned v[32];
         if (n_x > 0) {
-          pf_tmem_ld32(tO + c0, v);
+          tc_ld32(tO + c0, v);
+          tc_wait_ld();
         }
 #pragma unroll
         for (int q4 = 0; q4 < 8; ++q4) {
@@ -428,7 +385,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
       rec[129] = have ? l_sum : 0.f;
     }
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  tc_fence_before();
   __syncthreads();
   if (tid == 0 && *abort_flag) atomicOr(P.status, INQ_STATUS_WAIT_TIMEOUT);
   if (warp == 8)

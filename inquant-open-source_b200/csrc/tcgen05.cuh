@@ -1,0 +1,111 @@
+// Helpers for the 5th-generation tensor cores: descriptors, MMA issue, barriers, tensor-memory moves.
+#pragma once
+
+#include "common.cuh"
+
+namespace inq {
+
+__device__ __forceinline__ unsigned tc_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+// One lane of a converged warp.  MMAs and commits are issued as `if (tc_elect())` inside a branch that is
+// uniform over the warp: the compiler then keeps descriptors and addresses in uniform registers.  Issued
+// from a branch on the thread index instead, each tcgen05.mma costs about 50 cycles of issue (measured, eight
+// 128 x 16 x 16 MMAs with their commit and wait: 590 against 200 cycles).
+__device__ __forceinline__ unsigned tc_elect() {
+  unsigned chosen;
+  asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(chosen));
+  return chosen;
+}
+
+// 64-bit shared-memory matrix descriptor: start address, leading and stride byte offsets in 16-byte
+// units, descriptor version 1, layout type (0: no swizzle, 2: 128-byte swizzle).
+template <int LAYOUT = 2>
+__device__ __forceinline__ unsigned long long tc_desc(unsigned saddr, unsigned lbo_bytes, unsigned sbo_bytes) {
+  unsigned long long d = 0;
+  d |= (unsigned long long)((saddr & 0x3FFFFu) >> 4);
+  d |= (unsigned long long)(lbo_bytes >> 4) << 16;
+  d |= (unsigned long long)(sbo_bytes >> 4) << 32;
+  d |= 1ull << 46;
+  d |= (unsigned long long)LAYOUT << 61;
+  return d;
+}
+
+// Instruction descriptor of kind::f16 with fp32 accumulation: operand type, M, N; B_MN: B is MN-major.
+template <bool BF16, int M, int N, bool B_MN>
+__device__ __forceinline__ constexpr unsigned tc_idesc() {
+  return (1u << 4) | (BF16 ? (1u << 7) | (1u << 10) : 0u) | (B_MN ? 1u << 16 : 0u) | ((unsigned)(N >> 3) << 17) | ((unsigned)(M >> 4) << 24);
+}
+
+// D (tensor memory) = or += A B; A from shared memory or from tensor memory, B from shared memory.
+__device__ __forceinline__ void tc_mma(unsigned tmem_d, unsigned long long da, unsigned long long db, unsigned idesc, unsigned accumulate) {
+  asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }"
+               ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tc_mma_ta(unsigned tmem_d, unsigned tmem_a, unsigned long long db, unsigned idesc, unsigned accumulate) {
+  asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
+               ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tc_commit(unsigned mbar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void tc_bar_init(unsigned mbar, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
+}
+__device__ __forceinline__ bool tc_try_wait(unsigned mbar, unsigned parity) {
+  unsigned done;
+  asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+               : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
+  return done != 0;
+}
+
+#define TC_R4(v, o) "r"((v)[o]), "r"((v)[(o) + 1]), "r"((v)[(o) + 2]), "r"((v)[(o) + 3])
+#define TC_R16(v, o) TC_R4(v, o), TC_R4(v, (o) + 4), TC_R4(v, (o) + 8), TC_R4(v, (o) + 12)
+#define TC_W4(v, o) "=r"((v)[o]), "=r"((v)[(o) + 1]), "=r"((v)[(o) + 2]), "=r"((v)[(o) + 3])
+#define TC_W16(v, o) TC_W4(v, o), TC_W4(v, (o) + 4), TC_W4(v, (o) + 8), TC_W4(v, (o) + 12)
+// 32x32b: lane i of warp w moves TMEM lane 32 (w % 4) + i, register k column k.
+__device__ __forceinline__ void tc_st32(unsigned taddr, const unsigned (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
+      "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), TC_R16(v, 0), TC_R16(v, 16) : "memory");
+}
+__device__ __forceinline__ void tc_st16(unsigned taddr, const unsigned (&v)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(taddr), TC_R16(v, 0) : "memory");
+}
+__device__ __forceinline__ void tc_st8(unsigned taddr, const unsigned (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), TC_R4(v, 0), TC_R4(v, 4) : "memory");
+}
+// 16x128b: lane (r = lane / 4, j = lane % 4) supplies column 4 g + j of TMEM lane r (register 2 g) and
+// of TMEM lane r + 8 (register 2 g + 1) -- the fragment order of ldmatrix.
+__device__ __forceinline__ void tc_st_frag16(unsigned taddr, const unsigned (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x128b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
+      "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), TC_R16(v, 0), TC_R16(v, 16) : "memory");
+}
+__device__ __forceinline__ void tc_st_frag8(unsigned taddr, const unsigned (&v)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(taddr), TC_R16(v, 0) : "memory");
+}
+// The loads do not wait: tc_wait_ld() stands between a load and the first use of its registers.
+__device__ __forceinline__ void tc_ld32(unsigned taddr, unsigned (&v)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
+      "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : TC_W16(v, 0), TC_W16(v, 16) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tc_ld16(unsigned taddr, unsigned (&v)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : TC_W16(v, 0) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tc_ld8(unsigned taddr, unsigned (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" : TC_W4(v, 0), TC_W4(v, 4) : "r"(taddr) : "memory");
+}
+
+}  // namespace inq
