@@ -2,17 +2,23 @@
 //
 // One CTA owns 256 query tokens of one query head as two tiles of 128 rows (A and B) and walks
 // the visible keys and values in tiles of 128 tokens.  Ten warps, three roles:
-//   * warps 0-3 / 4-7: softmax of tile A / tile B, one thread per query row.  A thread reads its
-//     row of S from tensor memory (tcgen05.ld) once, takes base-2 probabilities against a lazily
-//     raised reference maximum (the pass is repeated in the rare case that the maximum has to
-//     rise) and writes P in the model dtype back to tensor memory (tcgen05.st) over S.
+//   * warps 0-3 / 4-7: softmax of tile A / tile B, one thread per query row.  A thread loads its whole
+//     row of S from tensor memory into registers (four tcgen05.ld in flight, waited for once), takes
+//     the maximum, raises the lagging reference maximum in the rare case that it has to, and stores the
+//     base-2 probabilities in the model dtype over S a quarter at a time, scaling and summing pairs in
+//     the packed fp32 units.  The chain S -> P bounds the kernel (per tile 1024 cycles of the exponential
+//     unit beside 2 x 512 of the tensor core), so what counts is its length: with quarters loaded and
+//     waited for one by one, the maximum tracked beside the exponentials and P stored at the end (the pass
+//     repeated when the maximum rose) the 1500-token causal prompt of 32 heads took 46.1 instead of
+//     34.2 us, a 32768-token prompt of one layer in chunks of 2048 11.9 instead of 10.4 ms.  A row in
+//     registers needs 216 of them: setmaxnreg moves registers from the issuing warps (168 -> 72).
 //   * warp 8 (an elected lane of the converged warp, see tc_elect: issued from a branch on the lane index the
 //     same MMAs took the 2048 x 32768 chunk 1185 instead of 1033 us): issues the contractions.  S = Q K^T (tcgen05.mma 128 x 128 x 128, both
 //     operands in shared memory) and O += P V (128 x 128 x 128, P from tensor memory, V as an
 //     MN-major shared-memory operand), fp32 accumulators in tensor memory.  The order S_A, S_B,
 //     PV_A, S_A', PV_B, S_B', ... keeps the tensor core busy with one tile while the other
 //     tile's softmax runs.
-//   * warp 9 (one lane): TMA (cp.async.bulk.tensor, 128-byte swizzle, no multicast) for Q once and
+//   * warp 9 (one lane, warps 10 and 11 complete the warpgroup): TMA (cp.async.bulk.tensor, 128-byte swizzle, no multicast) for Q once and
 //     for the double-buffered K and V tiles.
 // All hand-overs are mbarriers; every wait is bounded and a wait that gives up raises an abort
 // flag that ends the other loops.  One CTA per SM (tensor-memory kernels are scheduled that way),
@@ -32,7 +38,9 @@
 
 namespace inq {
 
-constexpr int kPfThreads = 320;              // 8 softmax warps, the MMA warp, the TMA warp
+constexpr int kPfThreads = 384;              // 8 softmax warps, the MMA warp, the TMA warp, two idle ones (whole warpgroups)
+// registers per thread: launched with, the MMA / TMA warpgroup, the two softmax warpgroups
+constexpr int kPfLaunchRegs = 168, kPfIssueRegs = 72, kPfSoftmaxRegs = (3 * kPfLaunchRegs - kPfIssueRegs) / 2;
 constexpr int kPfTile = 128;                 // query rows per tile, KV tokens per tile, head dimension
 constexpr int kPfRows = 2 * kPfTile;         // query rows per CTA (tiles A and B)
 constexpr int kPfSlab = kPfTile * 128;       // 128 rows x 128 bytes
@@ -73,6 +81,25 @@ __device__ __forceinline__ float pf_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// two fp32 values in one 64-bit register, for the packed units
+__device__ __forceinline__ unsigned long long pf_pair(float lo, float hi) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ void pf_unpair(unsigned long long d, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(d));
+}
+__device__ __forceinline__ unsigned long long pf_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long pf_add2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
 }
 template <typename QT>
 __device__ __forceinline__ unsigned pf_pack2(float lo, float hi) {
@@ -159,6 +186,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
   tc_fence_after();
   const unsigned tmem = *tmem_base_p;
 
+  if (warp >= 8) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPfIssueRegs));
   if (warp == 9) {
     // ================================================================ TMA warp
     if (lane == 0 && n_b > 0) {
@@ -246,7 +275,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
         if (t + 1 < n_b) issue_s(1, t + 1);
       }
     }
+  }
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPfSoftmaxRegs));
     // ================================================================ softmax warps
     const int x = warp >> 2;                       // 0: tile A, 1: tile B
     const int row = tid & (kPfTile - 1);           // query row inside the tile = TMEM lane
@@ -267,69 +298,68 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
       if (!pf_wait(my_s, (unsigned)t & 1u, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const bool masked = kv0 + kPfTile - 1 > diag0;
-      // ---- one pass over S: probabilities against the running reference maximum are packed
-      //      into registers while the row maximum is tracked; P is stored over S only afterwards,
-      //      so the rare case of a maximum that has to be raised can simply take the pass again
-      unsigned packed[64];
-      float smax, l_tile;
-      auto pass = [&](auto masked_tag) {
-        constexpr bool kMasked = decltype(masked_tag)::value;
-        smax = kPfNegBig;
-        l_tile = 0.f;
+      // ---- the row of S in registers, its maximum, then probabilities a quarter at a time, each stored
+      //      over S as soon as it is packed
+      unsigned v[4][32];
 #pragma unroll
-        for (int c0 = 0; c0 < kPfTile; c0 += 32) {
-          unsigned v[32];
-          tc_ld32(tS + c0, v);
-          tc_wait_ld();
+      for (int q = 0; q < 4; ++q) tc_ld32(tS + 32 * q, v[q]);
 #pragma unroll
-          for (int c = 0; c < 32; c += 2) {
-            const float s0 = __uint_as_float(v[c]), s1 = __uint_as_float(v[c + 1]);
-            float e0 = pf_exp2(fmaf(s0, P.scale_log2e, -m_ref));
-            float e1 = pf_exp2(fmaf(s1, P.scale_log2e, -m_ref));
-            if (kMasked) {
-              const bool vis0 = kv0 + c0 + c <= q_pos, vis1 = kv0 + c0 + c + 1 <= q_pos;
-              if (vis0) smax = fmaxf(smax, s0); else e0 = 0.f;
-              if (vis1) smax = fmaxf(smax, s1); else e1 = 0.f;
-            } else {
-              smax = fmaxf(smax, fmaxf(s0, s1));
-            }
-            l_tile += e0 + e1;
-            packed[(c0 + c) >> 1] = pf_pack2<QT>(e0, e1);
-          }
-        }
-      };
-      if (masked) pass(std::true_type{}); else pass(std::false_type{});
+      for (int q = 0; q < 4; ++q) tc_wait_ld32(v[q]);
+      if (masked) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int c = 0; c < 32; ++c)
+            if (kv0 + 32 * q + c > q_pos) v[q][c] = 0xff800000u;
+      }
+      float top[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        top[q] = __uint_as_float(v[q][0]);
+#pragma unroll
+        for (int c = 1; c < 32; ++c) top[q] = fmaxf(top[q], __uint_as_float(v[q][c]));
+      }
+      const float smax = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
       const bool raise = smax * P.scale_log2e > m_ref + kPfSlack;
       if (__any_sync(0xffffffffu, raise)) {
         // rare after the first tile: bring the running sum and the output accumulator to the new
-        // reference maximum, then take the probabilities again
+        // reference maximum
         const float m_new = raise ? smax * P.scale_log2e : m_ref;
         const float factor = pf_exp2(m_ref - m_new);
         l_sum *= factor;
         m_ref = m_new;
         if (t > 0) {
 #pragma unroll 1
-          for (int c0 = 0; c0 < kPfTile; c0 += 32) {
-            unsigned v[32];
-            tc_ld32(tO + c0, v);
+          for (int c0 = 0; c0 < kPfTile; c0 += 16) {
+            unsigned o[16];
+            tc_ld16(tO + c0, o);
             tc_wait_ld();
 #pragma unroll
-            for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) * factor);
-            tc_st32(tO + c0, v);
+            for (int c = 0; c < 16; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * factor);
+            tc_st16(tO + c0, o);
           }
         }
-        if (masked) pass(std::true_type{}); else pass(std::false_type{});
       }
-      l_sum += l_tile;
       {
-        unsigned lo[32], hi[32];
+        const unsigned long long scale2 = pf_pair(P.scale_log2e, P.scale_log2e), minus_ref2 = pf_pair(-m_ref, -m_ref);
+        unsigned long long sum2 = pf_pair(0.f, 0.f);
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          lo[c] = packed[c];
-          hi[c] = packed[32 + c];
+        for (int q = 0; q < 4; ++q) {
+          unsigned packed[16];
+#pragma unroll
+          for (int c = 0; c < 32; c += 2) {
+            float e0, e1;
+            pf_unpair(pf_fma2(pf_pair(__uint_as_float(v[q][c]), __uint_as_float(v[q][c + 1])), scale2, minus_ref2), e0, e1);
+            e0 = pf_exp2(e0);
+            e1 = pf_exp2(e1);
+            sum2 = pf_add2(sum2, pf_pair(e0, e1));
+            packed[c >> 1] = pf_pack2<QT>(e0, e1);
+          }
+          tc_st16(tS + 16 * q, packed);
         }
-        tc_st32(tS, lo);
-        tc_st32(tS + 32, hi);
+        float sum_even, sum_odd;
+        pf_unpair(sum2, sum_even, sum_odd);
+        l_sum += sum_even + sum_odd;
       }
       // P is in tensor memory, S has been read: hand both to the MMA warp
       tc_wait_st();
@@ -540,6 +570,14 @@ extern "C" int inq_prefill_attention(const inq_prefill_args_t* a, inq_stream_t s
       !make_map(&map_k, a->k, a->dtype, a->kv_tokens, a->kv_heads, a->k_stride_t, a->k_stride_h, kPfTile) ||
       !make_map(&map_v, a->v, a->dtype, a->kv_tokens, a->kv_heads, a->v_stride_t, a->v_stride_h, kPfTile))
     return INQ_ERR_ARGUMENT;
+  // the shares that setmaxnreg hands out must not exceed what the kernel is launched with
+  static const bool registers_fit = [] {
+    cudaFuncAttributes half, bfloat;
+    return cudaFuncGetAttributes(&half, prefill_kernel<__half>) == cudaSuccess &&
+           cudaFuncGetAttributes(&bfloat, prefill_kernel<__nv_bfloat16>) == cudaSuccess &&
+           half.numRegs >= kPfLaunchRegs && bfloat.numRegs >= kPfLaunchRegs;
+  }();
+  if (!registers_fit) return INQ_ERR_UNSUPPORTED;
   if (a->dtype == INQ_F16) {
     INQ_CUDA_CHECK(cudaFuncSetAttribute(prefill_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem));
     prefill_kernel<__half><<<(unsigned)ctas, kPfThreads, kPfSmem, stream>>>(P, map_q, map_k, map_v);

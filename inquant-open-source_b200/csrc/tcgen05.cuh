@@ -107,5 +107,13 @@ __device__ __forceinline__ void tc_ld16(unsigned taddr, unsigned (&v)[16]) {
 __device__ __forceinline__ void tc_ld8(unsigned taddr, unsigned (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" : TC_W4(v, 0), TC_W4(v, 4) : "r"(taddr) : "memory");
 }
+// tc_wait_ld() that also holds back every use of these registers
+__device__ __forceinline__ void tc_wait_ld32(unsigned (&v)[32]) {
+#define TC_RW4(v, o) "+r"((v)[o]), "+r"((v)[(o) + 1]), "+r"((v)[(o) + 2]), "+r"((v)[(o) + 3])
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : TC_RW4(v, 0), TC_RW4(v, 4), TC_RW4(v, 8), TC_RW4(v, 12), TC_RW4(v, 16), TC_RW4(v, 20), TC_RW4(v, 24), TC_RW4(v, 28)
+               :: "memory");
+#undef TC_RW4
+}
 
 }  // namespace inq

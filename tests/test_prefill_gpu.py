@@ -48,6 +48,21 @@ def test_prefill_attention_matches_fp32_causal_attention(q_heads, kv_heads, q_to
     attention_close(to_numpy(out.float())[0], to_numpy(expected)[0])
 
 
+@pytest.mark.parametrize("q_tokens,history,dtype", [(129, 0, torch.bfloat16), (200, 700, torch.float16), (256, 5000, torch.bfloat16)])
+def test_prefill_attention_when_the_maximum_rises_tile_after_tile(q_tokens, history, dtype):
+    """Keys that grow from KV tile to KV tile: for about half of the rows every tile raises the reference
+    maximum by more than the slack, the others keep an early one.  Bound: that of bf16 outputs."""
+    from inquant.prefill import prefill_attention
+    gen = torch.Generator(device="cuda").manual_seed(q_tokens)
+    q = torch.randn((1, 4, q_tokens, 128), device="cuda", generator=gen).to(dtype)
+    k = torch.randn((1, 2, history + q_tokens, 128), device="cuda", generator=gen) * 0.1
+    v = torch.randn((1, 2, history + q_tokens, 128), device="cuda", generator=gen).to(dtype)
+    k[..., 7] += 10.0 * torch.arange(1, history + q_tokens + 1, device="cuda") / 128   # times q[7] of either sign
+    k = k.to(dtype)
+    out = prefill_attention(q, k, v, 128 ** -0.5)
+    attention_close(to_numpy(out.float())[0], to_numpy(_reference(q, k, v, 128 ** -0.5))[0])
+
+
 def test_prefill_attention_accepts_strided_views_and_rejects_bad_arguments():
     from inquant.prefill import prefill_attention
     gen = torch.Generator(device="cuda").manual_seed(3)
