@@ -12,6 +12,8 @@
 //     repeated when the maximum rose) the 1500-token causal prompt of 32 heads took 46.1 instead of
 //     34.2 us, a 32768-token prompt of one layer in chunks of 2048 11.9 instead of 10.4 ms.  A row in
 //     registers needs 216 of them: setmaxnreg moves registers from the issuing warps (168 -> 72).
+//     P is handed over in two halves, so that the contraction with the first 64 tokens of V runs under
+//     the exponentials of the second (32768-token prompt of one layer: 10.38 -> 10.04 ms).
 //   * warp 8 (an elected lane of the converged warp, see tc_elect: issued from a branch on the lane index the
 //     same MMAs took the 2048 x 32768 chunk 1185 instead of 1033 us): issues the contractions.  S = Q K^T (tcgen05.mma 128 x 128 x 128, both
 //     operands in shared memory) and O += P V (128 x 128 x 128, P from tensor memory, V as an
@@ -47,7 +49,7 @@ constexpr int kPfSlab = kPfTile * 128;       // 128 rows x 128 bytes
 constexpr int kPfTileBytes = 2 * kPfSlab;    // one operand tile: two slabs (64-column halves)
 constexpr int kPfStages = 2;                 // K and V tiles in flight
 constexpr int kPfTiles = (2 + 2 * kPfStages) * kPfTileBytes;   // Q x2, K and V stages
-constexpr int kPfSmem = kPfTiles + 160;      // then the TMEM base address, the abort flag and 11 mbarriers
+constexpr int kPfSmem = kPfTiles + 160;      // then the TMEM base address, the abort flag and 13 mbarriers
 constexpr int kPfTmemCols = 512;             // S_A 0..127, S_B 128..255 (P over their first 64), O_A 256..383, O_B 384..511
 constexpr float kPfNegBig = -1.0e30f;
 constexpr float kPfSlack = 8.f;              // the reference maximum may lag the true one by 2^8 (P stays below 256)
@@ -137,6 +139,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
   const unsigned bars = smem0 + kPfTiles + 16;
   const unsigned bar_q = bars, bar_k = bars + 8 /* per stage */, bar_v = bar_k + 8 * kPfStages /* per stage */;
   const unsigned bar_s = bar_v + 8 * kPfStages /* A, B */, bar_p = bar_s + 16 /* A, B */, bar_o = bar_p + 16 /* A, B */;
+  const unsigned bar_h = bar_o + 16 /* A, B: first half of P */;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   if (smem0 & 1023u) {
     if (tid == 0) atomicOr(P.status, INQ_STATUS_BAD_INDEX);
@@ -173,6 +176,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
       tc_bar_init(bar_s + 8 * i, 1);
       tc_bar_init(bar_p + 8 * i, kPfTile);
       tc_bar_init(bar_o + 8 * i, 1);
+      tc_bar_init(bar_h + 8 * i, kPfTile);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -240,14 +244,17 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
           tc_commit(bar_s + 8 * x);
         }
       };
-      auto issue_o = [&](int x, int t) {      // O_x += P_x V(t): 16 tokens per step = 8 columns of packed P
+      // O_x += P_x V(t), half a tile of tokens at a time: 16 tokens per step = 8 columns of packed P
+      auto issue_o = [&](int x, int t, int half) {
         const unsigned v = sVb + (t % kPfStages) * kPfTileBytes;
         if (tc_elect()) {
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
+          for (int k = 0; k < 4; ++k) {
+            const int kk = 4 * half + k;
             tc_mma_ta(tmem + 2 * kPfTile + x * kPfTile, tmem + x * kPfTile + kk * 8, tc_desc(v + kk * 2048, kPfSlab, 1024), idesc_o,
                       (t > 0 || kk > 0) ? 1u : 0u);
-          tc_commit(bar_o + 8 * x);
+          }
+          if (half) tc_commit(bar_o + 8 * x);
         }
       };
       bool ok = pf_wait(bar_q, 0, abort_flag) && pf_wait(bar_k, 0, abort_flag);
@@ -258,20 +265,31 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
       }
       for (int t = 0; ok && t < n_b; ++t) {
         const bool a_live = t < n_a;
-        if (a_live) ok = ok && pf_wait(bar_p, (unsigned)t & 1u, abort_flag);       // P_A(t) written, S_A(t) read
-        ok = ok && pf_wait(bar_v + 8 * (t % kPfStages), (unsigned)(t / kPfStages) & 1u, abort_flag);
+        ok = pf_wait(bar_v + 8 * (t % kPfStages), (unsigned)(t / kPfStages) & 1u, abort_flag);
+        if (a_live) {
+          ok = ok && pf_wait(bar_h, (unsigned)t & 1u, abort_flag);     // S_A(t) read, the first half of P_A(t) written
+          if (!ok) break;
+          tc_fence_after();
+          issue_o(0, t, 0);
+          ok = pf_wait(bar_p, (unsigned)t & 1u, abort_flag);           // the second half
+          if (!ok) break;
+          tc_fence_after();
+          issue_o(0, t, 1);
+        }
         if (!ok) break;
-        tc_fence_after();
-        if (a_live) issue_o(0, t);
         if (t + 1 < n_b) {
           ok = pf_wait(bar_k + 8 * ((t + 1) % kPfStages), (unsigned)((t + 1) / kPfStages) & 1u, abort_flag);
           if (!ok) break;
           if (t + 1 < n_a) issue_s(0, t + 1);
         }
-        ok = pf_wait(bar_p + 8, (unsigned)t & 1u, abort_flag);                     // P_B(t) written, S_B(t) read
+        ok = pf_wait(bar_h + 8, (unsigned)t & 1u, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        issue_o(1, t);
+        issue_o(1, t, 0);
+        ok = pf_wait(bar_p + 8, (unsigned)t & 1u, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        issue_o(1, t, 1);
         if (t + 1 < n_b) issue_s(1, t + 1);
       }
     }
@@ -356,6 +374,11 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
             packed[c >> 1] = pf_pack2<QT>(e0, e1);
           }
           tc_st16(tS + 16 * q, packed);
+          if (q == 1) {   // S has been read, the first half of P is in tensor memory: the contraction with V starts
+            tc_wait_st();
+            tc_fence_before();
+            pf_arrive(bar_h + 8 * x);
+          }
         }
         float sum_even, sum_odd;
         pf_unpair(sum2, sum_even, sum_odd);
