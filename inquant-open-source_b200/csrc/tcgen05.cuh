@@ -52,7 +52,6 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_bar_init(unsigned mbar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
 }
@@ -68,29 +67,8 @@ __device__ __forceinline__ bool tc_try_wait(unsigned mbar, unsigned parity) {
 #define TC_W4(v, o) "=r"((v)[o]), "=r"((v)[(o) + 1]), "=r"((v)[(o) + 2]), "=r"((v)[(o) + 3])
 #define TC_W16(v, o) TC_W4(v, o), TC_W4(v, (o) + 4), TC_W4(v, (o) + 8), TC_W4(v, (o) + 12)
 // 32x32b: lane i of warp w moves TMEM lane 32 (w % 4) + i, register k column k.
-__device__ __forceinline__ void tc_st32(unsigned taddr, const unsigned (&v)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
-      "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), TC_R16(v, 0), TC_R16(v, 16) : "memory");
-}
 __device__ __forceinline__ void tc_st16(unsigned taddr, const unsigned (&v)[16]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-               ::"r"(taddr), TC_R16(v, 0) : "memory");
-}
-__device__ __forceinline__ void tc_st8(unsigned taddr, const unsigned (&v)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), TC_R4(v, 0), TC_R4(v, 4) : "memory");
-}
-// 16x128b: lane (r = lane / 4, j = lane % 4) supplies column 4 g + j of TMEM lane r (register 2 g) and
-// of TMEM lane r + 8 (register 2 g + 1) -- the fragment order of ldmatrix.
-__device__ __forceinline__ void tc_st_frag16(unsigned taddr, const unsigned (&v)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.16x128b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
-      "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), TC_R16(v, 0), TC_R16(v, 16) : "memory");
-}
-__device__ __forceinline__ void tc_st_frag8(unsigned taddr, const unsigned (&v)[16]) {
-  asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
                ::"r"(taddr), TC_R16(v, 0) : "memory");
 }
 // The loads do not wait: tc_wait_ld() stands between a load and the first use of its registers.
@@ -103,9 +81,6 @@ __device__ __forceinline__ void tc_ld32(unsigned taddr, unsigned (&v)[32]) {
 __device__ __forceinline__ void tc_ld16(unsigned taddr, unsigned (&v)[16]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                : TC_W16(v, 0) : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tc_ld8(unsigned taddr, unsigned (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" : TC_W4(v, 0), TC_W4(v, 4) : "r"(taddr) : "memory");
 }
 // tc_wait_ld() that also holds back every use of these registers
 __device__ __forceinline__ void tc_wait_ld32(unsigned (&v)[32]) {

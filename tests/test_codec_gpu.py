@@ -68,6 +68,24 @@ def test_k4_ring_staged_rows_match_strided_rows_and_oracle(tokens, dtype):
         assert_same_bytes(staged.tensors[name], ref.fields()[name], name)
 
 
+@pytest.mark.parametrize("runs", [((0, 16),), ((112, 128),), ((56, 72),), ((0, 8), (120, 128)), ((10, 26), (28, 44), (46, 62), (64, 80))])
+@pytest.mark.parametrize("policy", ["neighbors", "min_error"])
+@pytest.mark.parametrize("tokens", [64, 40])
+def test_k4_donors_when_sources_compete(runs, policy, tokens):
+    """Salient channels in runs at the edges and in the middle, up to 64 of them: many sources want the
+    same donor, so the common choice is repeated from conflict to conflict, over two batches of 32."""
+    CodecConfig, quantize, _ = _codec()
+    x32 = k4_input(dict(seed=tokens, shape=(3, 2, tokens, 128), dtype="bfloat16"))
+    for lo, hi in runs:
+        x32[..., lo:hi] = x32[..., lo:hi] * 16 + 8
+    x32 = oracle.round_to_dtype(x32, "bfloat16")
+    fraction = sum(hi - lo for lo, hi in runs) / 128
+    packed = quantize(to_device(x32, "bfloat16"), CodecConfig(salient_fraction=fraction, donor_policy=policy))
+    ref = oracle.quantize_k4(x32, "bfloat16", 8, fraction, policy)
+    for field, tensor in packed.tensors.items():
+        assert_same_bytes(tensor, ref.fields()[field], field)
+
+
 def test_block_axis_in_batch_and_token_major_strides_match_contiguous():
     CodecConfig, quantize, _ = _codec()
     cfg = CodecConfig(donor_policy="min_error")
