@@ -971,6 +971,30 @@ __global__ void __launch_bounds__(1024) select_kernel(const float* saliency, con
 }
 
 // ------------------------------------------------------------------------------------------
+// Eight channels of one token from the thread's word of the payload row.  The row's 16 words lie in 16
+// neighbouring lanes, so the low half of a salient code comes from its donor's lane by a shuffle (with a
+// load of that byte in a divergent branch per slot the keys of 496 rows of 256 tokens took 30.4 instead of
+// 21.6 us); `salient` names the slots where any lane of the warp needs one.  A whole
+// number below 2^23 becomes a float by its bits under those of 2^23.  All lanes of the warp call.
+template <typename T>
+__device__ __forceinline__ uint4 k4_decode8(unsigned word, const int (&role)[8], const float (&scale)[8], const float (&constant)[8],
+                                            unsigned salient) {
+  uint4 packed;
+  T* const vals = (T*)&packed;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const unsigned slot = (word >> (4 * k)) & 15u;
+    float code = __uint_as_float(0x4B000000u | slot) - 8388616.f;   // slot - 8
+    if ((salient >> k) & 1u) {
+      const unsigned other = __shfl_sync(0xffffffffu, word, (threadIdx.x & 16) | ((role[k] >> 3) & 15));
+      const unsigned both = (slot << 4) | ((other >> (4 * (role[k] & 7))) & 15u);
+      if (role[k] >= 0) code = __uint_as_float(0x4B000000u | both) - 8388736.f;   // code - 128
+    }
+    vals[k] = from_float<T>(role[k] < -1 ? constant[k] : code * scale[k]);
+  }
+  return packed;
+}
+
 // 128-channel rows, 16-bit output: a thread owns 8 consecutive channels of one token (4 payload bytes
 // in, 16 bytes out); 16 threads cover a token, a CTA of 256 threads covers 16 tokens per step.
 template <typename T>
@@ -1005,27 +1029,21 @@ __global__ void __launch_bounds__(256) k4_dequantize128_kernel(const unsigned ch
     sc[k] = scale[c0 + k];
     pd[k] = pad[c0 + k];
   }
+  unsigned any_salient = 0u;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) any_salient |= __any_sync(0xffffffffu, r[k] >= 0) ? 1u << k : 0u;
   const int per_cta = (tokens + gridDim.y - 1) / gridDim.y;
   const int t_begin = blockIdx.y * per_cta, t_end = min(tokens, t_begin + per_cta);
-  for (int t = t_begin + (threadIdx.x >> 4); t < t_end; t += 16) {
-    const unsigned char* line = bytes + (long long)t * 64;
-    const unsigned word = *(const unsigned*)(line + (c0 >> 1));
-    T vals[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int slot = (word >> (4 * k)) & 15;
-      float value;
-      if (r[k] >= 0) {
-        const int partner = (line[r[k] >> 1] >> ((r[k] & 1) * 4)) & 15;
-        value = (float)(((slot << 4) | partner) - 128) * sc[k];
-      } else if (r[k] == -1) {
-        value = (float)(slot - 8) * sc[k];
-      } else {
-        value = pd[k];
-      }
-      vals[k] = from_float<T>(value);
-    }
-    *(uint4*)(dst + (long long)t * 128 + c0) = *(const uint4*)vals;
+  // (whole warps walk the tokens; a lane past the end decodes the last token again and stores nothing)
+  const int mine = (threadIdx.x >> 4) & 1;
+  auto fetch = [&](int t) { return __ldg((const unsigned*)(bytes + (long long)min(t, t_end - 1) * 64 + (c0 >> 1))); };
+  int t = t_begin + 2 * (int)(threadIdx.x >> 5);
+  unsigned next = t < t_end ? fetch(t + mine) : 0u;
+  for (; t < t_end; t += 16) {
+    const unsigned word = next;
+    if (t + 16 < t_end) next = fetch(t + 16 + mine);
+    const uint4 vals = k4_decode8<T>(word, r, sc, pd, any_salient);
+    if (t + mine < t_end) *(uint4*)(dst + (long long)(t + mine) * 128 + c0) = vals;
   }
 }
 
@@ -1320,37 +1338,44 @@ __global__ void __launch_bounds__(256) restore_table_kernel(const long long* tab
     pd[k] = pad[c0 + k];
   }
   const long long base = (long long)h * stride_h + (position + (long long)b * tokens) * 128;
+  unsigned any_salient = 0u;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) any_salient |= __any_sync(0xffffffffu, r[k] >= 0) ? 1u << k : 0u;
   const int per_cta = (tokens + gridDim.y - 1) / gridDim.y;
   const int t_begin = blockIdx.y * per_cta, t_end = min(tokens, t_begin + per_cta);
-  for (int t = t_begin + (threadIdx.x >> 4); t < t_end; t += 16) {
-    const unsigned char* line = kp + (long long)t * 64;
-    const unsigned word = *(const unsigned*)(line + (c0 >> 1));
-    T vals[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int slot = (word >> (4 * k)) & 15;
-      float value;
-      if (r[k] >= 0) {
-        const int partner = (line[r[k] >> 1] >> ((r[k] & 1) * 4)) & 15;
-        value = (float)(((slot << 4) | partner) - 128) * sc[k];
-      } else if (r[k] == -1) {
-        value = (float)(slot - 8) * sc[k];
-      } else {
-        value = pd[k];
-      }
-      vals[k] = from_float<T>(value);
-    }
-    *(uint4*)(out_k + base + (long long)t * 128 + c0) = *(const uint4*)vals;
+  // (whole warps walk the tokens, a lane past the end decodes the last token again and stores nothing;
+  // the next step's bytes are requested before this one's are used)
+  struct Step {
+    unsigned word;
+    unsigned short codes;
+    __half scale, offset;
+  };
+  const int mine = (threadIdx.x >> 4) & 1, group = c0 >> 6;
+  auto fetch = [&](int t) {
+    t = min(t, t_end - 1);
+    return Step{__ldg((const unsigned*)(kp + (long long)t * 64 + (c0 >> 1))), __ldg((const unsigned short*)(vp + (long long)t * 32 + (c0 >> 2))),
+                __ldg(vs + t * 2 + group), __ldg(vo + t * 2 + group)};
+  };
+  int t = t_begin + 2 * (int)(threadIdx.x >> 5);
+  Step next = {};
+  if (t < t_end) next = fetch(t + mine);
+  for (; t < t_end; t += 16) {
+    const Step now = next;
+    if (t + 16 < t_end) next = fetch(t + 16 + mine);
+    const uint4 keys = k4_decode8<T>(now.word, r, sc, pd, any_salient);
     // values: 8 channels are two bytes of 2-bit codes and share a group of 64
-    const unsigned short codes = *(const unsigned short*)(vp + (long long)t * 32 + (c0 >> 2));
-    const float vsc = __half2float(vs[t * 2 + (c0 >> 6)]), vof = __half2float(vo[t * 2 + (c0 >> 6)]);
+    const float vsc = __half2float(now.scale), vof = __half2float(now.offset);
+    uint4 values;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      float value = (float)((codes >> (2 * k)) & 3u) * vsc;
+      float value = (__uint_as_float(0x4B000000u | ((now.codes >> (2 * k)) & 3u)) - 8388608.f) * vsc;
       value = value + vof;
-      vals[k] = from_float<T>(value);
+      ((T*)&values)[k] = from_float<T>(value);
     }
-    *(uint4*)(out_v + base + (long long)t * 128 + c0) = *(const uint4*)vals;
+    if (t + mine < t_end) {
+      *(uint4*)(out_k + base + (long long)(t + mine) * 128 + c0) = keys;
+      *(uint4*)(out_v + base + (long long)(t + mine) * 128 + c0) = values;
+    }
   }
 }
 
