@@ -60,13 +60,20 @@ struct SliceCfg {
 };
 constexpr int kPlanSliceTokens = 32;                // the unit of the flat work list (equal for both SUB when a block has <= 16 tokens)
 constexpr int kCtasPerSm = 3;                       // register budget: 168 per thread
+// Blocks of at most 16 tokens: every slice pays for a whole block's fold, a chain of dependent steps, and
+// a fourth CTA per SM (128 registers per thread, two ring stages to fit its shared memory) hides more of
+// it than the third stage did: 16 requests of 4096 to 32768 tokens in 32 layers, 16-token pages, 7915 ->
+// 7384 us; 8445 with three stages (shared memory for three CTAs only), 8750 with five CTAs (96 registers).
+constexpr int kCtasSmall = 4, kStagesSmall = 2;
+__host__ __device__ constexpr int ring_stages(int sub) { return sub == 1 ? kStagesSmall : kStages; }
+// per-warp scratch before the per-group parts; the metadata slots only where it does not ride in the stages
+__host__ __device__ constexpr int warp_fixed(int sub) { return 2048 + 256 + 64 + 64 + 256 + (sub == 1 ? 0 : 2048); }
 constexpr int kRecordStride = 132;                  // floats per query head: acc[128], m, l, pad
 constexpr int kRecordFloats = 8 * kRecordStride;    // one partial record (8 query heads)
 constexpr int kQChunk = 36;                         // padded 32-float chunk of the staged query
 constexpr int kQFragBytes = 8 * 32 * 8;              // the staged query as fp16 B fragments of the 8 K steps
 constexpr int kQBytes = 8 * 4 * kQChunk * 4 + 64 + kQFragBytes;   // staged query, two factors per head, fragments
 constexpr float kNegBig = -1.0e30f;
-constexpr int kWarpFixed = 2048 + 256 + 64 + 64 + 2048 + 256;  // per-warp scratch before the per-group parts
 constexpr float kRescaleSlack = 4.f;   // the running reference maximum may lag the true one by 2^4
 // start value of a gather accumulator: -(128 + 128/512) in units of 2^-13, so that it ends as
 // (code'_n - 128) + (code'_{n+8} - 128) / 512 (the fraction stays within +-1/4 even for a column
@@ -78,8 +85,8 @@ constexpr float kGatherInit = -128.25f / 8192.f;
 // channels, their kinds) and the exchange area of the donor slots' sums
 constexpr int kValueMeta = 768, kValueTables = 32 * (64 + 64 + 16), kValueXchg = 16 * 8 * 4;
 constexpr int kValueScratch = 2 * kValueMeta + kValueTables + kValueXchg;   // two metadata slots, as for the keys
-__host__ __device__ constexpr int warp_smem_bytes(int groups, int stage_bytes, int vk = 0) {
-  return kWarpFixed + groups * (256 + 2048 + 64) + (vk ? kValueScratch : 0) + kStages * stage_bytes;
+__host__ __device__ constexpr int warp_smem_bytes(int groups, int stage_bytes, int vk, int sub) {
+  return warp_fixed(sub) + groups * (256 + 2048 + 64) + (vk ? kValueScratch : 0) + ring_stages(sub) * stage_bytes;
 }
 
 struct SeqDesc {
@@ -487,11 +494,12 @@ __device__ __noinline__ void exchange_pair(const ExchangeView* X, int pair, long
 // values; a 16-byte chunk of a value row (8 words of four nibbles) is 32 channels, so every MMA lies
 // inside one group.  Their stages are 4.1 to 4.5 KB, so two CTAs fit an SM here as well.
 template <int MODE, typename QT, bool SAL, int SUB, bool FAST, int VK = 0, int VG = 2>
-__global__ void __launch_bounds__(kThreads, VK ? 2 : kCtasPerSm) decode_kernel(const DecodeParams P) {
+__global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 ? kCtasSmall : kCtasPerSm) decode_kernel(const DecodeParams P) {
   static_assert(!VK || (FAST && MODE == 0 && SAL && SUB == 2), "coded and 4-bit values: whole-slice path of the table layout only");
   static_assert(VK == 2 ? (VG == 1 || VG == 2 || VG == 4) : VK == 0 ? (VG == 2 || ((VG == 1 || VG == 4) && FAST && MODE == 0)) : VG == 2,
                 "4-bit values: groups of 32, 64 or 128 channels; 2-bit values: 64, or 32 and 128 on the whole-slice path");
   constexpr int kSub = SUB;
+  constexpr int kRing = ring_stages(SUB);
   constexpr int kSliceTokens = SliceCfg<SUB, VK, VG>::kSliceTokens;
   constexpr int kStageK = SliceCfg<SUB, VK, VG>::kStageK, kStageV = SliceCfg<SUB, VK, VG>::kStageV, kStageP = SliceCfg<SUB, VK, VG>::kStageP;
   constexpr int kStageBytes = SliceCfg<SUB, VK, VG>::kStageBytes;
@@ -509,7 +517,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : kCtasPerSm) decode_kernel(c
   const int r = lane >> 2, j = lane & 3;
   const int n_pad = FAST ? 16 : P.n_pad;                                // salient channels per head
   const int groups = FAST ? 1 : (n_pad + 15) >> 4;                      // ... in groups of 16
-  const int warp_bytes = warp_smem_bytes(groups, kStageBytes, VK == 1);
+  const int warp_bytes = warp_smem_bytes(groups, kStageBytes, VK == 1, SUB);
   unsigned char* const wb = warp_base + warp * warp_bytes;
   // folded-query B fragments of the 8 K steps ([step][lane] x 8 bytes); while a block's weights
   // are being derived the same 2 KB hold the per-channel slot weights and additive constants
@@ -521,8 +529,8 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : kCtasPerSm) decode_kernel(c
   // path stages block b into slot b % 2, so the block after the one being consumed can be requested
   // while this one's slot is still to be read
   unsigned char* wmeta = wdon + 64;
-  unsigned char* wfrag = wmeta + 2048;    // a block's channel weights as fp16 pairs in B-fragment order: [K step][chunk] x 8 B
-  unsigned char* wqsal = wb + kWarpFixed;                               // B fragments: query at salient channels
+  unsigned char* wfrag = wmeta + (SUB == 1 ? 0 : 2048);    // a block's channel weights as fp16 pairs in B-fragment order: [K step][chunk] x 8 B
+  unsigned char* wqsal = wb + warp_fixed(SUB);                               // B fragments: query at salient channels
   unsigned char* wsel = wqsal + groups * 256;                           // B fragments: nibble selection
   unsigned short* wcell = (unsigned short*)(wsel + groups * 2048);      // selection cells written by the last fold (offsets into wsel)
   // InQuant-coded values: staged value metadata of a block, the lane's flush tables, the donor sums
@@ -830,7 +838,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : kCtasPerSm) decode_kernel(c
     constexpr int kParamLane = VK != 1 && VG == 4 ? 8 : 4;   // bytes of a parameter array one lane copies per slice
     const unsigned char* fs = pf_ptrs.vs + pf_slice * (kStageP / 2) + lane * kParamLane;
     const unsigned char* fo = pf_ptrs.vo + pf_slice * (kStageP / 2) + lane * kParamLane;
-    const unsigned ring_lo = smem_addr(ring), ring_hi = ring_lo + kStages * kStageBytes;
+    const unsigned ring_lo = smem_addr(ring), ring_hi = ring_lo + kRing * kStageBytes;
     unsigned issue_addr = ring_lo;
     int pf_left = spb - pf_slice;
     // value rows in a stage.  2-bit values: 32 B per token, the halves of tokens 4..7 (mod 8) swapped.
@@ -903,7 +911,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : kCtasPerSm) decode_kernel(c
         }
         stage_slice<kSub>(stage_ptr, pf_ptrs.kp, pf_ptrs.vp, pf_ptrs.vs, pf_ptrs.vo, pf_slice * kSliceTokens, T, lane);
         --to_issue;
-        if (++issue_stage == kStages) issue_stage = 0;
+        if (++issue_stage == kRing) issue_stage = 0;
         if (++pf_slice == spb) {
           pf_slice = 0;
           ++pf_block;
@@ -913,7 +921,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : kCtasPerSm) decode_kernel(c
       cp_async_commit();
     };
 #pragma unroll
-    for (int s = 0; s < kStages - 1; ++s) issue();
+    for (int s = 0; s < kRing - 1; ++s) issue();
     // the dense slices of this warp hide behind the DRAM latency of the first packed slices;
     // their contribution is brought into the packed loop's per-row units (powers of two)
     dense_part();
@@ -1013,7 +1021,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : kCtasPerSm) decode_kernel(c
     };
 
     for (int it = 0; it < n_my; ++it) {
-      cp_async_wait<kStages - 2>();
+      cp_async_wait<kRing - 2>();
       __syncwarp();
       // With fewer than three slices per block the next block's metadata can only be staged once
       // this block's fold has released the staging area: there the copies are issued after the
@@ -1241,7 +1249,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : kCtasPerSm) decode_kernel(c
       if (FAST) {
         consume_addr += kStageBytes;
         if (consume_addr == ring_hi) consume_addr = ring_lo;
-      } else if (++stage_index == kStages) {
+      } else if (++stage_index == kRing) {
         stage_index = 0;
       }
       // ---- scores of two 16-token sub-slices (tokens 0..15 and 16..31 of the stage): K nibbles
@@ -1836,7 +1844,7 @@ static int smem_bytes(int groups, int sub, int vk = 0, int vg = 2) {
                   : vk == 0 && vg == 4 ? SliceCfg<2, 0, 4>::kStageBytes
                   : vk == 2 ? (vg == 1 ? SliceCfg<2, 2, 1>::kStageBytes : vg == 2 ? SliceCfg<2, 2, 2>::kStageBytes : SliceCfg<2, 2, 4>::kStageBytes)
                   : vk ? SliceCfg<2, 1>::kStageBytes : (sub == 1 ? SliceCfg<1>::kStageBytes : SliceCfg<2>::kStageBytes);
-  return kQBytes + kWarps * warp_smem_bytes(groups, stage, vk == 1);
+  return kQBytes + kWarps * warp_smem_bytes(groups, stage, vk == 1, sub);
 }
 
 }  // namespace inq
