@@ -1170,11 +1170,14 @@ __global__ void __launch_bounds__(256) v_encode_kernel(VParams p) {
 }
 
 // 128-channel fast path of the value encoder: a warp owns 8 consecutive tokens, issues all its
-// loads first (2 KB in flight per warp), then quantises token by token.  A lane owns 4 channels.
+// loads first (2 KB in flight per warp), then quantises two tokens at a time.  A lane owns 8 channels, so
+// a group of 64 is reduced in registers and by three shuffles per bound, for two tokens at once.  The kernel
+// is bound by issue: with 4 channels per lane and one token per warp 496 rows of 256 tokens took 25.4
+// instead of 18.5 us (38.5 MB moved: 5.8 us at 6.65 TB/s).
 template <typename T, int BITS, int GROUP>
 __global__ void __launch_bounds__(256) v_encode128_kernel(VParams p) {
   constexpr int kRows = 8;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = lane & 15;
   const long long outer = blockIdx.x / p.in.n_inner, inner = blockIdx.x % p.in.n_inner;
   const long long slot = p.in.slot(outer);
   if (!p.in.slot_ok(slot)) {   // uniform over the CTA: nothing of this row is written
@@ -1183,36 +1186,35 @@ __global__ void __launch_bounds__(256) v_encode128_kernel(VParams p) {
   }
   const int t0 = (blockIdx.y * 8 + warp) * kRows;
   if (t0 >= p.in.tokens) return;
-  const T* base = (const T*)p.in.x + outer * p.in.s_outer + inner * p.in.s_inner + lane * 4;
-  float v[kRows][4];
+  const T* base = (const T*)p.in.x + outer * p.in.s_outer + inner * p.in.s_inner + i * 8;
+  constexpr int kVec = sizeof(T) == 2 ? 1 : 2;   // 16-byte vectors per 8 channels
+  uint4 raw[kRows / 2][kVec];
 #pragma unroll
-  for (int k = 0; k < kRows; ++k) {
-    const int t = min(t0 + k, p.in.tokens - 1);
-    const T* src = base + (long long)t * p.in.s_token;
-    if (sizeof(T) == 2) {
-      const uint2 bits = *(const uint2*)src;
-      const T* hv = (const T*)&bits;
+  for (int k = 0; k < kRows / 2; ++k) {
+    const int t = min(t0 + 2 * k + (lane >> 4), p.in.tokens - 1);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) v[k][j] = to_float<T>(hv[j]);
-    } else {
-      const float4 f = *(const float4*)src;
-      v[k][0] = f.x; v[k][1] = f.y; v[k][2] = f.z; v[k][3] = f.w;
-    }
+    for (int q = 0; q < kVec; ++q) raw[k][q] = ((const uint4*)(base + (long long)t * p.in.s_token))[q];
   }
-  constexpr int lanes_per_group = GROUP / 4, groups = 128 / GROUP, bits = BITS;
+  constexpr int lanes_per_group = GROUP / 8, groups = 128 / GROUP, bits = BITS;
   constexpr float levels = (float)((1 << BITS) - 1);
   unsigned nonfinite = 0u;
   unsigned char* payload = (unsigned char*)p.payload.at(slot, inner);
   __half* scales = (__half*)p.scales.at(slot, inner);
   __half* offsets = (__half*)p.offsets.at(slot, inner);
 #pragma unroll
-  for (int k = 0; k < kRows; ++k) {
-    const int t = t0 + k;
-    if (t >= p.in.tokens) break;
-    float lo = fminf(fminf(v[k][0], v[k][1]), fminf(v[k][2], v[k][3]));
-    float hi = fmaxf(fmaxf(v[k][0], v[k][1]), fmaxf(v[k][2], v[k][3]));
-    unsigned top = max(max(__float_as_uint(v[k][0]) & 0x7fffffffu, __float_as_uint(v[k][1]) & 0x7fffffffu),
-                       max(__float_as_uint(v[k][2]) & 0x7fffffffu, __float_as_uint(v[k][3]) & 0x7fffffffu));
+  for (int k = 0; k < kRows / 2; ++k) {
+    const int t = t0 + 2 * k + (lane >> 4);
+    const bool live = t < p.in.tokens;   // (a lane past the end repeats the last token and stores nothing)
+    const T* hv = (const T*)raw[k];
+    float v[8];
+    unsigned top = 0u;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] = to_float<T>(hv[j]);
+      top = max(top, __float_as_uint(v[j]) & 0x7fffffffu);
+    }
+    float lo = fminf(fminf(fminf(v[0], v[1]), fminf(v[2], v[3])), fminf(fminf(v[4], v[5]), fminf(v[6], v[7])));
+    float hi = fmaxf(fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3])), fmaxf(fmaxf(v[4], v[5]), fmaxf(v[6], v[7])));
 #pragma unroll
     for (int off = 1; off < lanes_per_group; off <<= 1) {
       lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, off));
@@ -1223,8 +1225,8 @@ __global__ void __launch_bounds__(256) v_encode128_kernel(VParams p) {
     const float offset = __half2float(offset16), scale = __half2float(scale16);
     top = max(top, max(__float_as_uint(offset) & 0x7fffffffu, __float_as_uint(scale) & 0x7fffffffu));
     nonfinite |= top >= 0x7f800000u;
-    if (lane % lanes_per_group == 0) {
-      const int g = lane / lanes_per_group;
+    if (live && i % lanes_per_group == 0) {
+      const int g = i / lanes_per_group;
       scales[(long long)t * groups + g] = scale16;
       offsets[(long long)t * groups + g] = offset16;
     }
@@ -1232,22 +1234,18 @@ __global__ void __launch_bounds__(256) v_encode128_kernel(VParams p) {
     const float rcp = __frcp_rn(scale);
     unsigned word = 0u;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float q = exact_quotient(v[k][j] - offset, scale, rcp, false);
+    for (int j = 0; j < 8; ++j) {
+      const float q = exact_quotient(v[j] - offset, scale, rcp, false);
       // rounded to a whole code by the addition (1.5 * 2^23), which leaves it in the low bits
       const unsigned code = __float_as_uint(fminf(fmaxf(q, 0.f), levels) + 12582912.f);
       word |= (code & ((1u << bits) - 1u)) << (j * bits);
     }
     if (bits == 2) {
-      // 8 bits per lane, four lanes per 32-bit word
-      word <<= 8 * (lane & 3);
-      word |= __shfl_xor_sync(0xffffffffu, word, 1);
-      word |= __shfl_xor_sync(0xffffffffu, word, 2);
-      if ((lane & 3) == 0) ((unsigned*)(payload + (long long)t * 32))[lane >> 2] = word;
-    } else {
-      word <<= 16 * (lane & 1);
-      word |= __shfl_xor_sync(0xffffffffu, word, 1);
-      if ((lane & 1) == 0) ((unsigned*)(payload + (long long)t * 64))[lane >> 1] = word;
+      // 16 bits per lane, two lanes per 32-bit word
+      word |= __shfl_xor_sync(0xffffffffu, word, 1) << 16;
+      if (live && (lane & 1) == 0) ((unsigned*)(payload + (long long)t * 32))[i >> 1] = word;
+    } else if (live) {
+      ((unsigned*)(payload + (long long)t * 64))[i] = word;
     }
   }
   if (nonfinite) atomicOr(p.status, INQ_STATUS_NONFINITE);
