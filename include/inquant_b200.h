@@ -419,6 +419,17 @@ int64_t inq_decode_units(int32_t n_blocks, int32_t block_tokens);
 /* Scratch floats that suffice for a launch with n_pairs pairs and total_units work units on
  * the current device. */
 int64_t inq_decode_workspace_floats(int32_t n_pairs, int64_t total_units);
+/* The launch that inq_decode_attention makes for such a batch with `ctas_per_sm` resident CTAs per SM (it
+ * asks the runtime for that number): the list of total_units + n_pairs * ramp_units positions is cut into
+ * n_ctas ranges of per_cta, and shared_bytes of dynamic shared memory hold the merge of a pair that is
+ * cut into up to merge_parts parts.  INQ_ERR_CAPACITY as the launch itself would answer.  Host only. */
+typedef struct {
+  int32_t n_ctas, shared_bytes;
+  int64_t per_cta, ramp_units;
+  int32_t merge_parts, reserved;
+} inq_decode_shape_t;
+int inq_decode_launch_shape(int32_t n_pairs, int64_t total_units, int32_t block_tokens, int32_t n_pad, int32_t value_kind,
+                            int32_t value_groups, int32_t ctas_per_sm, inq_decode_shape_t* shape);
 
 /* ---------------------------------------------------------------- incremental append
  * Writes the key and value rows of ONE new token (all KV heads) at `tail_position` of the

@@ -33,6 +33,7 @@
 //   * contractions use mma.sync.m16n8k16 with 16 tokens as M and the (up to 8) query heads
 //     of the KV head as N, so one pass serves the whole GQA group; base-2 online softmax with
 //     a lazily raised reference maximum.
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -1839,6 +1840,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 ? kCtasSmall : kCt
 }
 
 #undef SEQ
+// Scratch of a whole CTA: the staged query and the four warps' parts.
 static int smem_bytes(int groups, int sub, int vk = 0, int vg = 2) {
   const int stage = vk == 0 && vg == 1 ? SliceCfg<2, 0, 1>::kStageBytes
                   : vk == 0 && vg == 4 ? SliceCfg<2, 0, 4>::kStageBytes
@@ -1846,6 +1848,9 @@ static int smem_bytes(int groups, int sub, int vk = 0, int vg = 2) {
                   : vk ? SliceCfg<2, 1>::kStageBytes : (sub == 1 ? SliceCfg<1>::kStageBytes : SliceCfg<2>::kStageBytes);
   return kQBytes + kWarps * warp_smem_bytes(groups, stage, vk == 1, sub);
 }
+// What the merge of a pair cut into `parts` parts lays over the warps' scratch: a weight and a normaliser
+// per part and query head, then two sums per query head.
+static long long merge_bytes(long long parts) { return kQBytes + (2 * 8 * parts + 2 * 8) * (long long)sizeof(float); }
 
 }  // namespace inq
 
@@ -1923,6 +1928,16 @@ static Plan make_plan(long long total_units, int n_pairs, long long uniform_unit
   return p;
 }
 
+// Dynamic shared memory of a launch.  Nothing ties the parts of ONE pair to the scratch of the warps: in a
+// batch where one sequence holds nearly all slices its pair is cut into nearly every CTA's range (556 of
+// 565 for 80000 tokens beside fifteen short requests at one KV head and 16-token blocks, 35 KB of merge
+// scratch against 32 KB for warps without salient channels).  A pair has at most n_ctas parts.
+// Negative: more than `limit` would be needed.
+static int launch_smem(int scratch, int limit, int n_ctas) {
+  const long long need = std::max<long long>(scratch, merge_bytes(n_ctas));
+  return need <= limit ? (int)need : -1;
+}
+
 extern "C" int64_t inq_decode_units(int32_t n_blocks, int32_t block_tokens) {
   const long long u = (long long)n_blocks * spb_of(block_tokens);
   return u > 0 ? u : 1;
@@ -1931,6 +1946,24 @@ extern "C" int64_t inq_decode_units(int32_t n_blocks, int32_t block_tokens) {
 extern "C" int64_t inq_decode_workspace_floats(int32_t n_pairs, int64_t total_units) {
   const Plan p = make_plan(total_units > n_pairs ? total_units : n_pairs, n_pairs, 0, 8);
   return ((int64_t)p.n_ctas + n_pairs) * kRecordFloats;
+}
+
+extern "C" int inq_decode_launch_shape(int32_t n_pairs, int64_t total_units, int32_t block_tokens, int32_t n_pad, int32_t value_kind,
+                                       int32_t value_groups, int32_t ctas_per_sm, inq_decode_shape_t* shape) {
+  if (!shape || n_pairs < 1 || total_units < n_pairs || block_tokens < 1 || n_pad < 0 || n_pad > 64 || ctas_per_sm < 1)
+    return INQ_ERR_ARGUMENT;
+  const int sub = block_tokens <= 16 ? 1 : 2, groups = (n_pad + 15) / 16;
+  const Plan plan = make_plan(total_units, n_pairs, 0, ctas_per_sm);
+  const int shared = launch_smem(smem_bytes(groups, sub, value_kind, value_groups), smem_bytes(value_kind ? 1 : 4, sub, value_kind, value_groups),
+                                 plan.n_ctas);
+  if (shared < 0) return INQ_ERR_CAPACITY;
+  shape->n_ctas = plan.n_ctas;
+  shape->shared_bytes = shared;
+  shape->per_cta = plan.per_cta;
+  shape->ramp_units = plan.ramp_units;
+  shape->merge_parts = (int32_t)((shared - merge_bytes(0)) / (merge_bytes(1) - merge_bytes(0)));
+  shape->reserved = 0;
+  return INQ_OK;
 }
 
 extern "C" int inq_decode_attention(const inq_decode_args_t* a, inq_stream_t stream_) {
@@ -1997,10 +2030,11 @@ extern "C" int inq_decode_attention(const inq_decode_args_t* a, inq_stream_t str
                   : fast ? 16 + a->layout * 2 + (a->dtype == INQ_F16 ? 0 : 1)
                          : (sub == 1 ? 8 : 0) + a->layout * 4 + (a->dtype == INQ_F16 ? 0 : 2) + (groups > 0 ? 1 : 0);
   const kernel_t kernel = kernels[which];
-  const int shared = smem_bytes(groups, sub, vk, vg);
+  const int scratch = smem_bytes(groups, sub, vk, vg);
   const int shared_limit = smem_bytes(vk ? 1 : 4, sub, vk, vg);
   const int device = current_device();
   if (device < 0) return INQ_ERR_UNSUPPORTED;   // device ordinals above 63 are not tracked
+  const int n_sm = sm_count();
   int resident = 0;
   {
     std::lock_guard<std::mutex> guard(g_devices_mutex);
@@ -2011,13 +2045,18 @@ extern "C" int inq_decode_attention(const inq_decode_args_t* a, inq_stream_t str
     }
     if (!d.per_sm[which][groups]) {
       int n = 0;
-      INQ_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kThreads, shared));
+      INQ_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kThreads, scratch));
+      // the grid stays resident as a whole with the shared memory of its largest merge as well
+      const int merge = launch_smem(scratch, shared_limit, n_sm * std::max(n, 1));
+      if (merge > scratch) INQ_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kThreads, merge));
       d.per_sm[which][groups] = n > 0 ? n : 1;
     }
     resident = d.per_sm[which][groups];
   }
   const Plan plan = make_plan(total, (int)n_pairs, uniform, resident);
   if (((long long)plan.n_ctas + n_pairs) * kRecordFloats > a->partials_floats) return INQ_ERR_CAPACITY;
+  const int shared = launch_smem(scratch, shared_limit, plan.n_ctas);
+  if (shared < 0) return INQ_ERR_CAPACITY;
   DecodeParams P;
   P.seqs = (const SeqDesc*)a->seqs_device;
   if (!a->seqs_device) P.one = *(const SeqDesc*)a->seq_host;

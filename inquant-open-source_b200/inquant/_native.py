@@ -75,6 +75,11 @@ class DecodeExchange(ctypes.Structure):
                 ("world", c_int32), ("rank", c_int32), ("spin_limit", c_int32), ("reserved", c_int32)]
 
 
+class DecodeShape(ctypes.Structure):
+    _fields_ = [("n_ctas", c_int32), ("shared_bytes", c_int32), ("per_cta", c_int64), ("ramp_units", c_int64),
+                ("merge_parts", c_int32), ("reserved", c_int32)]
+
+
 class WritePagesArgs(ctypes.Structure):
     _fields_ = [("key_payload", c_void_p), ("key_scales", c_void_p), ("salient", c_void_p), ("donors", c_void_p),
                 ("key_padding", c_void_p), ("value_payload", c_void_p), ("value_scales", c_void_p), ("value_offsets", c_void_p),
@@ -177,7 +182,7 @@ EXPORTS = (
     "inq_last_error", "inq_version", "inq_k4_encode", "inq_select_donors", "inq_k4_statistics",
     "inq_k4_dequantize", "inq_k4_dequantize_strided", "inq_v_encode", "inq_v_dequantize", "inq_v_dequantize_strided",
     "inq_build_roles", "inq_write_codec_pages",
-    "inq_decode_attention", "inq_decode_attention_noalloc", "inq_decode_units", "inq_merge_partials", "inq_decode_workspace_floats", "inq_append_token", "inq_append_token_batch", "inq_seal_blocks",
+    "inq_decode_attention", "inq_decode_attention_noalloc", "inq_decode_units", "inq_merge_partials", "inq_decode_workspace_floats", "inq_decode_launch_shape", "inq_append_token", "inq_append_token_batch", "inq_seal_blocks",
     "inq_prefill_attention", "inq_decode_generic", "inq_decode_generic_workspace_floats",
     "inq_prefill_workspace_bytes",
     "inq_exchange_merge", "inq_exchange_inbox_bytes", "inq_decode_exchange_inbox_bytes", "inq_restore_blocks_table", "inq_peer_buffer_create", "inq_peer_buffer_open",
@@ -198,6 +203,7 @@ SIGNATURES = {
     "inq_build_roles": [_P, _P, _I, _L, _I, _I, _P, _I, _P],
     "inq_restore_blocks_table": [_P, _P, _I, _I, _I, _I, _P, _P, _L, _L, _I, _P],
     "inq_decode_attention": [_P, _P],
+    "inq_decode_launch_shape": [_I, _L, _I, _I, _I, _I, _I, _P],
     "inq_write_codec_pages": [_P, _P],
     "inq_decode_attention_noalloc": [_P, _P],
     "inq_merge_partials": [_P, _I, _L, _P, _I, _P],

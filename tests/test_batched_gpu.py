@@ -163,3 +163,33 @@ def test_paged_batch_of_requests_with_different_lengths(block, heads, q_heads):
         attention_close(to_numpy(out[i].float()), expected[i])
     from inquant import _native as N
     assert N.take_status(batch.device) == 0
+
+
+@pytest.mark.parametrize("fraction", [0.0, 0.125])
+def test_a_long_request_beside_short_ones_at_one_kv_head(fraction):
+    """16-token blocks: the long request's pair is cut into nearly every CTA's range (tests/test_decode_plan_cpu.py),
+    so the merge of its parts needs more shared memory than the warps' own scratch.  Against float64
+    attention over the restored caches."""
+    from inquant.batched import DecodeBatch, SequenceState
+    from inquant.cache import CacheConfig, InQuantCache
+    from inquant.codec import CodecConfig
+    from inquant import _native as N
+    config = CacheConfig(CodecConfig(salient_fraction=fraction, donor_policy="min_error"), block_size=16, residual_length=32,
+                         sink_tokens=4, value_bits=2, validate_positions=False)
+    caches = []
+    for i in range(16):
+        cache = InQuantCache(config)
+        # (outlier channels only where salient channels keep them: the kernel folds the other channels' scales
+        # into the query unrounded, and the bf16 keys of the comparison are off by up to 0.25 in an outlier)
+        k, v = workloads.make_kv_torch(60 + i, 1, 80000 if i == 5 else 60 + i, "cuda", **({} if fraction else {"scale_range": (1.0, 1.0)}))
+        cache.update(k, v, 0)
+        caches.append(cache)
+    batch = DecodeBatch([SequenceState.from_cache_layer(c, 0) for c in caches], 8, torch.bfloat16)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    batch.queries.copy_(torch.randn(batch.queries.shape, device="cuda", generator=gen))
+    out = batch.attend()
+    for i, cache in enumerate(caches):
+        k, v = (t[0, 0].double() for t in cache.materialize(0))
+        p = torch.softmax(batch.queries[i].double() @ k.T * 128 ** -0.5, -1)
+        attention_close(to_numpy(out[i].float()), to_numpy(p @ v))
+    assert N.take_status(batch.device) == 0

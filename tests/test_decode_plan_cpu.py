@@ -1,0 +1,72 @@
+"""Host side of a decode launch: the work list of uneven batches against the merge scratch (no GPU)."""
+import ctypes
+
+import pytest
+
+from inquant import _native as N
+
+
+def _shape(starts, block_tokens, n_pad, ctas_per_sm, value_kind=0, value_groups=2):
+    shape = N.DecodeShape()
+    rc = N.library().inq_decode_launch_shape(len(starts) - 1, starts[-1], block_tokens, n_pad, value_kind, value_groups, ctas_per_sm,
+                                             ctypes.byref(shape))
+    assert rc == N.OK
+    return shape
+
+
+def _most_parts(starts, shape):
+    """Largest number of CTA ranges that hold slices of one pair, by the kernel's own arithmetic."""
+    most = 0
+    for pair in range(len(starts) - 1):
+        lo, hi = (starts[pair + k] + (pair + 1) * shape.ramp_units for k in (0, 1))
+        most = max(most, (hi - 1) // shape.per_cta - lo // shape.per_cta + 1)
+    return most
+
+
+def _batches(block_tokens):
+    """Slices per pair: even batches, one long sequence among short ones, one pair alone, heads of a layer."""
+    per_block = max(1, block_tokens // 32)
+    for heads in (1, 2, 8):
+        for long, others in ((5000, 15), (8000, 15), (40000, 63), (600, 3), (5000, 0), (1, 300)):
+            for position in {0, others // 2, others}:
+                units = [long * per_block if i == position else per_block for i in range(others + 1)]
+                starts = [0]
+                for u in units:
+                    for _ in range(heads):
+                        starts.append(starts[-1] + u)
+                yield starts
+
+
+@pytest.mark.parametrize("block_tokens", [16, 64, 256])
+@pytest.mark.parametrize("n_pad", [0, 1, 16, 17, 32, 48, 64])
+def test_merge_of_the_most_divided_pair_fits_the_shared_memory_of_the_launch(block_tokens, n_pad):
+    for ctas_per_sm in (1, 2, 3, 4):
+        for starts in _batches(block_tokens):
+            shape = _shape(starts, block_tokens, n_pad, ctas_per_sm)
+            total = starts[-1] + (len(starts) - 1) * shape.ramp_units
+            assert (shape.n_ctas - 1) * shape.per_cta < total <= shape.n_ctas * shape.per_cta
+            assert _most_parts(starts, shape) <= shape.merge_parts, (starts[-1], len(starts) - 1, ctas_per_sm)
+            assert shape.shared_bytes <= 227 * 1024
+
+
+@pytest.mark.parametrize("value_kind,value_groups", [(1, 0), (2, 1), (2, 2), (2, 4), (0, 1), (0, 4)])
+def test_merge_fits_with_the_other_value_codecs(value_kind, value_groups):
+    for starts in _batches(64):
+        shape = _shape(starts, 64, 16, 3, value_kind, value_groups)
+        assert _most_parts(starts, shape) <= shape.merge_parts
+
+
+def test_a_long_request_beside_short_ones_takes_more_parts_than_the_warps_scratch_holds():
+    """16-token blocks without salient channels, one KV head, 80000 tokens beside fifteen requests of one
+    block: four CTAs per SM give the long pair 556 parts, and the four warps' own 32256 bytes hold 503."""
+    starts = [0, 5000] + [5000 + i for i in range(1, 16)]
+    shape = _shape(starts, 16, 0, 4)
+    assert _most_parts(starts, shape) > 503
+    assert shape.merge_parts >= shape.n_ctas
+
+
+def test_launch_shape_refuses_what_no_launch_could_have():
+    lib, shape = N.library(), N.DecodeShape()
+    assert lib.inq_decode_launch_shape(1, 1, 16, 0, 0, 2, 4, None) == N.ERR_ARGUMENT
+    for bad in ((0, 1, 16, 0, 0, 2, 4), (2, 1, 16, 0, 0, 2, 4), (1, 1, 0, 0, 0, 2, 4), (1, 1, 16, 65, 0, 2, 4), (1, 1, 16, 0, 0, 2, 0)):
+        assert lib.inq_decode_launch_shape(*bad, ctypes.byref(shape)) == N.ERR_ARGUMENT
