@@ -23,7 +23,8 @@
 //   * warp 9 (one lane, warps 10 and 11 complete the warpgroup): TMA (cp.async.bulk.tensor, 128-byte swizzle, no multicast) for Q once and
 //     for the double-buffered K and V tiles.
 // All hand-overs are mbarriers; every wait is bounded and a wait that gives up raises an abort
-// flag that ends the other loops.  One CTA per SM (tensor-memory kernels are scheduled that way),
+// flag that ends the other loops, whole warps at a time; copies and contractions in flight are then
+// waited for (again bounded) before tensor memory is freed and the CTA ends.  One CTA per SM (tensor-memory kernels are scheduled that way),
 // 192 KB of shared memory, all 512 TMEM columns.  Keys and values are dense tensors in the model
 // dtype: the dequantised packed history followed by the chunk's own tokens; query i sees
 // positions <= history + i.
@@ -49,7 +50,7 @@ constexpr int kPfSlab = kPfTile * 128;       // 128 rows x 128 bytes
 constexpr int kPfTileBytes = 2 * kPfSlab;    // one operand tile: two slabs (64-column halves)
 constexpr int kPfStages = 2;                 // K and V tiles in flight
 constexpr int kPfTiles = (2 + 2 * kPfStages) * kPfTileBytes;   // Q x2, K and V stages
-constexpr int kPfSmem = kPfTiles + 160;      // then the TMEM base address, the abort flag and 13 mbarriers
+constexpr int kPfSmem = kPfTiles + 160;      // then the TMEM base address, the abort flag, two counts and 14 mbarriers
 constexpr int kPfTmemCols = 512;             // S_A 0..127, S_B 128..255 (P over their first 64), O_A 256..383, O_B 384..511
 constexpr float kPfNegBig = -1.0e30f;
 constexpr float kPfSlack = 8.f;              // the reference maximum may lag the true one by 2^8 (P stays below 256)
@@ -67,15 +68,6 @@ struct PrefillParams {
   int* status;
 };
 
-// Bounded wait; gives up early when another role has raised the abort flag.
-__device__ __forceinline__ bool pf_wait(unsigned mbar, unsigned parity, volatile int* abort_flag) {
-  for (int it = 0; it < kPfSpinLimit; ++it) {
-    if (tc_try_wait(mbar, parity)) return true;
-    if ((it & 255) == 255 && *abort_flag) return false;
-  }
-  *abort_flag = 1;
-  return false;
-}
 __device__ __forceinline__ void pf_arrive(unsigned mbar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }
@@ -136,10 +128,11 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
   const unsigned sVb = sKb + kPfStages * kPfTileBytes;        // V stages
   unsigned* const tmem_base_p = (unsigned*)(pf_raw + kPfTiles);
   volatile int* const abort_flag = (volatile int*)(pf_raw + kPfTiles + 4);
+  volatile int* const requested = abort_flag + 1;             // K and V tiles that the TMA warp asked for in all
   const unsigned bars = smem0 + kPfTiles + 16;
   const unsigned bar_q = bars, bar_k = bars + 8 /* per stage */, bar_v = bar_k + 8 * kPfStages /* per stage */;
   const unsigned bar_s = bar_v + 8 * kPfStages /* A, B */, bar_p = bar_s + 16 /* A, B */, bar_o = bar_p + 16 /* A, B */;
-  const unsigned bar_h = bar_o + 16 /* A, B: first half of P */;
+  const unsigned bar_h = bar_o + 16 /* A, B: first half of P */, bar_e = bar_h + 16 /* end of a launch that gave up */;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   if (smem0 & 1023u) {
     if (tid == 0) atomicOr(P.status, INQ_STATUS_BAD_INDEX);
@@ -164,8 +157,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
   const int n_a = max(0, min(all_a, t_hi) - t_lo);
 
   if (tid == 0) {
-    *abort_flag = 0;
+    *abort_flag = requested[0] = requested[1] = 0;
     tc_bar_init(bar_q, 1);
+    tc_bar_init(bar_e, 1);
 #pragma unroll
     for (int i = 0; i < kPfStages; ++i) {
       tc_bar_init(bar_k + 8 * i, 1);
@@ -189,6 +183,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
   __syncthreads();
   tc_fence_after();
   const unsigned tmem = *tmem_base_p;
+  auto wait = [&](unsigned mbar, unsigned parity) { return tc_wait_warp(mbar, parity, abort_flag, kPfSpinLimit); };
 
   if (warp >= 8) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPfIssueRegs));
@@ -196,12 +191,14 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
     // ================================================================ TMA warp
     if (lane == 0 && n_b > 0) {
       auto request_k = [&](int t) {
+        requested[0] = t + 1;
         const unsigned bar = bar_k + 8 * (t % kPfStages), dst = sKb + (t % kPfStages) * kPfTileBytes;
         pf_expect(bar, kPfTileBytes);
         pf_tma(dst, &map_k, 0, (t_lo + t) * kPfTile, kvh, bar);
         pf_tma(dst + kPfSlab, &map_k, 64, (t_lo + t) * kPfTile, kvh, bar);
       };
       auto request_v = [&](int t) {
+        requested[1] = t + 1;
         const unsigned bar = bar_v + 8 * (t % kPfStages), dst = sVb + (t % kPfStages) * kPfTileBytes;
         pf_expect(bar, kPfTileBytes);
         pf_tma(dst, &map_v, 0, (t_lo + t) * kPfTile, kvh, bar);
@@ -220,9 +217,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
       for (int t = 0; t + kPfStages < n_b; ++t) {
         // K(t) is free once both score contractions of tile t are done, V(t) once both output
         // contractions are (the commits are ordered, so tile B's barrier covers tile A's)
-        if (!pf_wait(bar_s + 8, (unsigned)t & 1u, abort_flag)) break;
+        if (!tc_wait(bar_s + 8, (unsigned)t & 1u, abort_flag, kPfSpinLimit)) break;
         request_k(t + kPfStages);
-        if (!pf_wait(bar_o + 8, (unsigned)t & 1u, abort_flag)) break;
+        if (!tc_wait(bar_o + 8, (unsigned)t & 1u, abort_flag, kPfSpinLimit)) break;
         request_v(t + kPfStages);
       }
     }
@@ -257,7 +254,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
           if (half) tc_commit(bar_o + 8 * x);
         }
       };
-      bool ok = pf_wait(bar_q, 0, abort_flag) && pf_wait(bar_k, 0, abort_flag);
+      bool ok = wait(bar_q, 0) && wait(bar_k, 0);
       if (ok) {
         tc_fence_after();
         if (n_a > 0) issue_s(0, 0);
@@ -265,28 +262,28 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
       }
       for (int t = 0; ok && t < n_b; ++t) {
         const bool a_live = t < n_a;
-        ok = pf_wait(bar_v + 8 * (t % kPfStages), (unsigned)(t / kPfStages) & 1u, abort_flag);
+        ok = wait(bar_v + 8 * (t % kPfStages), (unsigned)(t / kPfStages) & 1u);
         if (a_live) {
-          ok = ok && pf_wait(bar_h, (unsigned)t & 1u, abort_flag);     // S_A(t) read, the first half of P_A(t) written
+          ok = ok && wait(bar_h, (unsigned)t & 1u);     // S_A(t) read, the first half of P_A(t) written
           if (!ok) break;
           tc_fence_after();
           issue_o(0, t, 0);
-          ok = pf_wait(bar_p, (unsigned)t & 1u, abort_flag);           // the second half
+          ok = wait(bar_p, (unsigned)t & 1u);           // the second half
           if (!ok) break;
           tc_fence_after();
           issue_o(0, t, 1);
         }
         if (!ok) break;
         if (t + 1 < n_b) {
-          ok = pf_wait(bar_k + 8 * ((t + 1) % kPfStages), (unsigned)((t + 1) / kPfStages) & 1u, abort_flag);
+          ok = wait(bar_k + 8 * ((t + 1) % kPfStages), (unsigned)((t + 1) / kPfStages) & 1u);
           if (!ok) break;
           if (t + 1 < n_a) issue_s(0, t + 1);
         }
-        ok = pf_wait(bar_h + 8, (unsigned)t & 1u, abort_flag);
+        ok = wait(bar_h + 8, (unsigned)t & 1u);
         if (!ok) break;
         tc_fence_after();
         issue_o(1, t, 0);
-        ok = pf_wait(bar_p + 8, (unsigned)t & 1u, abort_flag);
+        ok = wait(bar_p + 8, (unsigned)t & 1u);
         if (!ok) break;
         tc_fence_after();
         issue_o(1, t, 1);
@@ -313,7 +310,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
       const int kv0 = (t_lo + t) * kPfTile;
       // S(t) is complete; the contractions run in issue order, so PV(t-1) is complete as well:
       // the columns of P may be overwritten by S and O may be rescaled
-      if (!pf_wait(my_s, (unsigned)t & 1u, abort_flag)) { ok = false; break; }
+      if (!wait(my_s, (unsigned)t & 1u)) { ok = false; break; }
       tc_fence_after();
       const bool masked = kv0 + kPfTile - 1 > diag0;
       // ---- the row of S in registers, its maximum, then probabilities a quarter at a time, each stored
@@ -389,7 +386,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
       tc_fence_before();
       pf_arrive(my_p);
     }
-    if (n_x > 0) ok = ok && pf_wait(my_o, (unsigned)(n_x - 1) & 1u, abort_flag);
+    if (n_x > 0) ok = ok && wait(my_o, (unsigned)(n_x - 1) & 1u);
     tc_fence_after();
 
     if (P.splits == 1) {
@@ -441,8 +438,23 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && *abort_flag) atomicOr(P.status, INQ_STATUS_WAIT_TIMEOUT);
-  if (warp == 8)
+  if (warp == 8) {
+    __syncwarp();
+    if (__any_sync(0xffffffffu, *abort_flag != 0)) {
+      // contractions and copies may be in flight: they end before tensor memory is freed and the CTA leaves
+      if (tc_elect()) tc_commit(bar_e);
+      tc_drain(bar_e, 0, kPfSpinLimit);
+      if (requested[1] > 0) tc_drain(bar_q, 0, kPfSpinLimit);
+#pragma unroll 1
+      for (int back = kPfStages; back > 0; --back) {
+        const int k = requested[0] - back, v = requested[1] - back;
+        if (k >= 0) tc_drain(bar_k + 8 * (k % kPfStages), (unsigned)(k / kPfStages) & 1u, kPfSpinLimit);
+        if (v >= 0) tc_drain(bar_v + 8 * (v % kPfStages), (unsigned)(v / kPfStages) & 1u, kPfSpinLimit);
+      }
+      __syncwarp();
+    }
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kPfTmemCols) : "memory");
+  }
 }
 
 // Merges the KV segments of every item: out = sum_s O_s 2^(m_s - m) / sum_s l_s 2^(m_s - m).
