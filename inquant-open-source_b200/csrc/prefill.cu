@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
           for (int c0 = 0; c0 < kPfTile; c0 += 16) {
             unsigned o[16];
             tc_ld16(tO + c0, o);
-            tc_wait_ld();
+            tc_wait_ld16(o);
 #pragma unroll
             for (int c = 0; c < 16; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * factor);
             tc_st16(tO + c0, o);
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
       for (int c0 = 0; c0 < kPfTile; c0 += 32) {
         unsigned v[32];
         tc_ld32(tO + c0, v);
-        tc_wait_ld();
+        tc_wait_ld32(v);
         if (live) {
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
         unsigned v[32];
         if (n_x > 0) {
           tc_ld32(tO + c0, v);
-          tc_wait_ld();
+          tc_wait_ld32(v);
         }
 #pragma unroll
         for (int q4 = 0; q4 < 8; ++q4) {

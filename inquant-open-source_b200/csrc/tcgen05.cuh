@@ -50,7 +50,6 @@ __device__ __forceinline__ void tc_commit(unsigned mbar) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_bar_init(unsigned mbar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
@@ -92,7 +91,8 @@ __device__ __forceinline__ void tc_st16(unsigned taddr, const unsigned (&v)[16])
   asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
                ::"r"(taddr), TC_R16(v, 0) : "memory");
 }
-// The loads do not wait: tc_wait_ld() stands between a load and the first use of its registers.
+// The loads do not wait: tc_wait_ld32 / tc_wait_ld16 of the loaded registers stands between a load and their first
+// use.  The registers are operands of the wait, because nothing else holds arithmetic on them back behind it.
 __device__ __forceinline__ void tc_ld32(unsigned taddr, unsigned (&v)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
@@ -103,13 +103,13 @@ __device__ __forceinline__ void tc_ld16(unsigned taddr, unsigned (&v)[16]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                : TC_W16(v, 0) : "r"(taddr) : "memory");
 }
-// tc_wait_ld() that also holds back every use of these registers
-__device__ __forceinline__ void tc_wait_ld32(unsigned (&v)[32]) {
 #define TC_RW4(v, o) "+r"((v)[o]), "+r"((v)[(o) + 1]), "+r"((v)[(o) + 2]), "+r"((v)[(o) + 3])
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : TC_RW4(v, 0), TC_RW4(v, 4), TC_RW4(v, 8), TC_RW4(v, 12), TC_RW4(v, 16), TC_RW4(v, 20), TC_RW4(v, 24), TC_RW4(v, 28)
-               :: "memory");
-#undef TC_RW4
+#define TC_RW16(v, o) TC_RW4(v, o), TC_RW4(v, (o) + 4), TC_RW4(v, (o) + 8), TC_RW4(v, (o) + 12)
+__device__ __forceinline__ void tc_wait_ld32(unsigned (&v)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : TC_RW16(v, 0), TC_RW16(v, 16) :: "memory");
+}
+__device__ __forceinline__ void tc_wait_ld16(unsigned (&v)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : TC_RW16(v, 0) :: "memory");
 }
 
 }  // namespace inq
