@@ -35,6 +35,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "tcgen05.cuh"
@@ -534,6 +535,19 @@ bool make_map(CUtensorMap* map, const void* base, int dtype, long long tokens, l
             strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+// The shares that setmaxnreg hands out must not exceed what the kernel is launched with.  The library holds one
+// binary of the kernel for one architecture, so a yes is kept for the process; a query that fails is
+// reported like every other runtime error and asked again by the next call.
+template <typename QT>
+int registers_fit() {
+  static std::atomic<bool> known{false};
+  if (known.load(std::memory_order_relaxed)) return INQ_OK;
+  cudaFuncAttributes attributes;
+  INQ_CUDA_CHECK(cudaFuncGetAttributes(&attributes, prefill_kernel<QT>));
+  if (attributes.numRegs < kPfLaunchRegs) return INQ_ERR_UNSUPPORTED;
+  known.store(true, std::memory_order_relaxed);
+  return INQ_OK;
+}
 }  // namespace
 
 
@@ -605,14 +619,8 @@ extern "C" int inq_prefill_attention(const inq_prefill_args_t* a, inq_stream_t s
       !make_map(&map_k, a->k, a->dtype, a->kv_tokens, a->kv_heads, a->k_stride_t, a->k_stride_h, kPfTile) ||
       !make_map(&map_v, a->v, a->dtype, a->kv_tokens, a->kv_heads, a->v_stride_t, a->v_stride_h, kPfTile))
     return INQ_ERR_ARGUMENT;
-  // the shares that setmaxnreg hands out must not exceed what the kernel is launched with
-  static const bool registers_fit = [] {
-    cudaFuncAttributes half, bfloat;
-    return cudaFuncGetAttributes(&half, prefill_kernel<__half>) == cudaSuccess &&
-           cudaFuncGetAttributes(&bfloat, prefill_kernel<__nv_bfloat16>) == cudaSuccess &&
-           half.numRegs >= kPfLaunchRegs && bfloat.numRegs >= kPfLaunchRegs;
-  }();
-  if (!registers_fit) return INQ_ERR_UNSUPPORTED;
+  const int fit = a->dtype == INQ_F16 ? registers_fit<__half>() : registers_fit<__nv_bfloat16>();
+  if (fit != INQ_OK) return fit;
   if (a->dtype == INQ_F16) {
     INQ_CUDA_CHECK(cudaFuncSetAttribute(prefill_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem));
     prefill_kernel<__half><<<(unsigned)ctas, kPfThreads, kPfSmem, stream>>>(P, map_q, map_k, map_v);
