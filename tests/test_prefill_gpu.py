@@ -48,19 +48,31 @@ def test_prefill_attention_matches_fp32_causal_attention(q_heads, kv_heads, q_to
     attention_close(to_numpy(out.float())[0], to_numpy(expected)[0])
 
 
-@pytest.mark.parametrize("q_tokens,history,dtype", [(129, 0, torch.bfloat16), (200, 700, torch.float16), (256, 5000, torch.bfloat16)])
+@pytest.mark.parametrize("q_tokens,history,dtype", [(129, 256, torch.bfloat16), (200, 700, torch.float16), (256, 5000, torch.bfloat16)])
 def test_prefill_attention_when_the_maximum_rises_tile_after_tile(q_tokens, history, dtype):
-    """Keys that grow from KV tile to KV tile: for about half of the rows every tile raises the reference
-    maximum by more than the slack, the others keep an early one.  Bound: that of bf16 outputs."""
+    """Keys with a ramp in one channel, queries of +-8 there, the sign at random from row to row: for about
+    half of the rows of every warp each KV tile raises the reference maximum by more than the slack, the
+    others keep that of their first tile (both asserted below on the scores).  900 keys are one segment of
+    eight tiles, 5256 eight segments of five or six.  Bound: that of bf16 outputs."""
     from inquant.prefill import prefill_attention
+    from inquant import _native as N
+    tile, slack = 128, 8.0                                      # csrc/prefill.cu: kPfTile, kPfSlack
     gen = torch.Generator(device="cuda").manual_seed(q_tokens)
-    q = torch.randn((1, 4, q_tokens, 128), device="cuda", generator=gen).to(dtype)
+    q = torch.randn((1, 4, q_tokens, 128), device="cuda", generator=gen)
+    q[..., 7] = torch.where(q[..., 7] > 0, 8.0, -8.0)
+    q = q.to(dtype)
     k = torch.randn((1, 2, history + q_tokens, 128), device="cuda", generator=gen) * 0.1
     v = torch.randn((1, 2, history + q_tokens, 128), device="cuda", generator=gen).to(dtype)
-    k[..., 7] += 10.0 * torch.arange(1, history + q_tokens + 1, device="cuda") / 128   # times q[7] of either sign
+    k[..., 7] += 16.0 * torch.arange(1, history + q_tokens + 1, device="cuda") / tile   # base-2 scores rise by 16.3 a tile
     k = k.to(dtype)
+    scores = q[0].double() @ k[0].double().repeat_interleave(2, 0).transpose(1, 2) * 128 ** -0.5 * 1.4426950408889634
+    tops = torch.stack([tile_scores.amax(-1) for tile_scores in scores.split(tile, -1)[:history // tile]], -1)   # tiles that every row sees
+    rising = tops.diff(dim=-1).min(-1).values > slack
+    assert 0.4 < rising.double().mean() < 0.6 and torch.equal(tops.diff(dim=-1).max(-1).values < 0, ~rising)
+    assert all((rows.any(-1) & ~rows.all(-1)).all() for rows in rising[:, :128].split(32, -1))   # both kinds in a warp
     out = prefill_attention(q, k, v, 128 ** -0.5)
     attention_close(to_numpy(out.float())[0], to_numpy(_reference(q, k, v, 128 ** -0.5))[0])
+    assert N.take_status(q.device) == 0
 
 
 def test_prefill_attention_accepts_strided_views_and_rejects_bad_arguments():
