@@ -450,9 +450,6 @@ __global__ void __launch_bounds__(kMaxThreads) k4_encode_kernel(K4Params p) {
 struct Mask128 {
   unsigned long long lo, hi;
   __device__ __forceinline__ bool test(int i) const { return i >= 0 && i < 128 && (((i < 64 ? lo : hi) >> (i & 63)) & 1ull); }
-  __device__ __forceinline__ void clear(int i) {
-    if (i < 64) lo &= ~(1ull << i); else hi &= ~(1ull << (i - 64));
-  }
   __device__ __forceinline__ int below(int pos) const {   // largest member < pos, or -1
     if (pos > 64) {
       unsigned long long m = pos >= 128 ? hi : (hi & ((1ull << (pos - 64)) - 1ull));
@@ -480,13 +477,6 @@ __device__ __forceinline__ float exact_quotient(float x, float s, float r, bool 
   const float q0 = x * r;
   const float rem = fmaf(-q0, s, x);
   return fmaf(rem, r, q0);
-}
-
-__device__ __forceinline__ unsigned encode_slot_fast(float x, float scale, float rcp, bool plain, int kind) {
-  const float q = rintf(exact_quotient(x, scale, rcp, plain));
-  if (kind == 0) return (unsigned)(int)(fminf(fmaxf(q, -7.f), 7.f) + 8.f);
-  const unsigned code = (unsigned)(int)(fminf(fmaxf(q, -127.f), 127.f) + 128.f);
-  return kind == 1 ? (code >> 4) : (code & 15u);
 }
 
 template <typename T>
@@ -530,8 +520,9 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
   constexpr int kGroupBytes = kGroupTokens * kRowBytes;
   constexpr int kWarpStage = kGroupBytes / 4;   // a warp's share of a stage
   __shared__ __align__(16) unsigned char s_ring[STAGED ? kRing * kGroupBytes : 16];
-  __shared__ float s_sal[C], s_err[C], s_mean[C], s_scale[C], s_rcp[C];
-  __shared__ unsigned s_key[C];
+  __shared__ __align__(16) float s_sal[C];      // read four at a time, like s_key
+  __shared__ float s_mean[C], s_scale[C], s_rcp[C];
+  __shared__ __align__(16) unsigned s_key[C];
   __shared__ unsigned char s_kind[C], s_from[C], s_plain[C];
   __shared__ int s_src[64], s_don[64];
   __shared__ unsigned s_sel[4], s_avail[4];
@@ -703,7 +694,6 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
   const float absmax = __uint_as_float(top_bits);
   s_sal[c] = saliency;
   s_mean[c] = sampled_mean;
-  s_err[c] = donor_error;
   __syncthreads();
 
   // ---- top-`count` channels by saliency (ties: lower channel), optional least-error pool
@@ -1173,7 +1163,7 @@ __global__ void __launch_bounds__(256) v_encode_kernel(VParams p) {
 // loads first (2 KB in flight per warp), then quantises two tokens at a time.  A lane owns 8 channels, so
 // a group of 64 is reduced in registers and by three shuffles per bound, for two tokens at once.  The kernel
 // is bound by issue: with 4 channels per lane and one token per warp 496 rows of 256 tokens took 25.4
-// instead of 18.5 us (38.5 MB moved: 5.8 us at 6.65 TB/s).
+// instead of 18.5 us (37.6 MB moved: 5.7 us at the measured 6557 GB/s).
 template <typename T, int BITS, int GROUP>
 __global__ void __launch_bounds__(256) v_encode128_kernel(VParams p) {
   constexpr int kRows = 8;
