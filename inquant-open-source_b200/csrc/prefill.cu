@@ -23,8 +23,9 @@
 //   * warp 9 (one lane, warps 10 and 11 complete the warpgroup): TMA (cp.async.bulk.tensor, 128-byte swizzle, no multicast) for Q once and
 //     for the double-buffered K and V tiles.
 // All hand-overs are mbarriers; every wait is bounded and a wait that gives up raises an abort
-// flag that ends the other loops, whole warps at a time; copies and contractions in flight are then
-// waited for (again bounded) before tensor memory is freed and the CTA ends.  One CTA per SM (tensor-memory kernels are scheduled that way),
+// flag after which no other wait waits, so that every role runs through its loop (see tc_wait); copies and
+// contractions in flight are then waited for (again bounded) before tensor memory is freed and the CTA ends.
+// One CTA per SM (tensor-memory kernels are scheduled that way),
 // 192 KB of shared memory, all 512 TMEM columns.  Keys and values are dense tensors in the model
 // dtype: the dequantised packed history followed by the chunk's own tokens; query i sees
 // positions <= history + i.
@@ -55,7 +56,6 @@ constexpr int kPfSmem = kPfTiles + 160;      // then the TMEM base address, the 
 constexpr int kPfTmemCols = 512;             // S_A 0..127, S_B 128..255 (P over their first 64), O_A 256..383, O_B 384..511
 constexpr float kPfNegBig = -1.0e30f;
 constexpr float kPfSlack = 8.f;              // the reference maximum may lag the true one by 2^8 (P stays below 256)
-constexpr int kPfSpinLimit = 1 << 22;
 constexpr int kPfMaxSplits = 8;              // KV segments per item at most
 
 struct PrefillParams {
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
   __syncthreads();
   tc_fence_after();
   const unsigned tmem = *tmem_base_p;
-  auto wait = [&](unsigned mbar, unsigned parity) { return tc_wait_warp(mbar, parity, abort_flag, kPfSpinLimit); };
+  auto wait = [&](unsigned mbar, unsigned parity) { tc_wait(mbar, parity, abort_flag); };   // goes on in either case
 
   if (warp >= 8) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPfIssueRegs));
@@ -218,9 +218,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
       for (int t = 0; t + kPfStages < n_b; ++t) {
         // K(t) is free once both score contractions of tile t are done, V(t) once both output
         // contractions are (the commits are ordered, so tile B's barrier covers tile A's)
-        if (!tc_wait(bar_s + 8, (unsigned)t & 1u, abort_flag, kPfSpinLimit)) break;
+        if (!tc_wait(bar_s + 8, (unsigned)t & 1u, abort_flag)) break;
         request_k(t + kPfStages);
-        if (!tc_wait(bar_o + 8, (unsigned)t & 1u, abort_flag, kPfSpinLimit)) break;
+        if (!tc_wait(bar_o + 8, (unsigned)t & 1u, abort_flag)) break;
         request_v(t + kPfStages);
       }
     }
@@ -255,37 +255,29 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
           if (half) tc_commit(bar_o + 8 * x);
         }
       };
-      bool ok = wait(bar_q, 0) && wait(bar_k, 0);
-      if (ok) {
-        tc_fence_after();
-        if (n_a > 0) issue_s(0, 0);
-        issue_s(1, 0);
-      }
-      for (int t = 0; ok && t < n_b; ++t) {
-        const bool a_live = t < n_a;
-        ok = wait(bar_v + 8 * (t % kPfStages), (unsigned)(t / kPfStages) & 1u);
-        if (a_live) {
-          ok = ok && wait(bar_h, (unsigned)t & 1u);     // S_A(t) read, the first half of P_A(t) written
-          if (!ok) break;
+      wait(bar_q, 0);
+      wait(bar_k, 0);
+      tc_fence_after();
+      if (n_a > 0) issue_s(0, 0);
+      issue_s(1, 0);
+      for (int t = 0; t < n_b; ++t) {
+        wait(bar_v + 8 * (t % kPfStages), (unsigned)(t / kPfStages) & 1u);
+        if (t < n_a) {
+          wait(bar_h, (unsigned)t & 1u);     // S_A(t) read, the first half of P_A(t) written
           tc_fence_after();
           issue_o(0, t, 0);
-          ok = wait(bar_p, (unsigned)t & 1u);           // the second half
-          if (!ok) break;
+          wait(bar_p, (unsigned)t & 1u);     // the second half
           tc_fence_after();
           issue_o(0, t, 1);
         }
-        if (!ok) break;
         if (t + 1 < n_b) {
-          ok = wait(bar_k + 8 * ((t + 1) % kPfStages), (unsigned)((t + 1) / kPfStages) & 1u);
-          if (!ok) break;
+          wait(bar_k + 8 * ((t + 1) % kPfStages), (unsigned)((t + 1) / kPfStages) & 1u);
           if (t + 1 < n_a) issue_s(0, t + 1);
         }
-        ok = wait(bar_h + 8, (unsigned)t & 1u);
-        if (!ok) break;
+        wait(bar_h + 8, (unsigned)t & 1u);
         tc_fence_after();
         issue_o(1, t, 0);
-        ok = wait(bar_p + 8, (unsigned)t & 1u);
-        if (!ok) break;
+        wait(bar_p + 8, (unsigned)t & 1u);
         tc_fence_after();
         issue_o(1, t, 1);
         if (t + 1 < n_b) issue_s(1, t + 1);
@@ -305,13 +297,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
     const unsigned tS = tmem + lane_field + x * kPfTile, tO = tmem + lane_field + 2 * kPfTile + x * kPfTile;
     const unsigned my_s = bar_s + 8 * x, my_p = bar_p + 8 * x, my_o = bar_o + 8 * x;
     float m_ref = kPfNegBig, l_sum = 0.f;
-    bool ok = true;
 
     for (int t = 0; t < n_x; ++t) {
       const int kv0 = (t_lo + t) * kPfTile;
       // S(t) is complete; the contractions run in issue order, so PV(t-1) is complete as well:
       // the columns of P may be overwritten by S and O may be rescaled
-      if (!wait(my_s, (unsigned)t & 1u)) { ok = false; break; }
+      wait(my_s, (unsigned)t & 1u);
       tc_fence_after();
       const bool masked = kv0 + kPfTile - 1 > diag0;
       // ---- the row of S in registers, its maximum, then probabilities a quarter at a time, each stored
@@ -387,8 +378,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
       tc_fence_before();
       pf_arrive(my_p);
     }
-    if (n_x > 0) ok = ok && wait(my_o, (unsigned)(n_x - 1) & 1u);
+    if (n_x > 0) wait(my_o, (unsigned)(n_x - 1) & 1u);
     tc_fence_after();
+    const bool ok = *abort_flag == 0;
 
     if (P.splits == 1) {
       // ---- normalise and store this thread's row
@@ -444,13 +436,13 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
     if (__any_sync(0xffffffffu, *abort_flag != 0)) {
       // contractions and copies may be in flight: they end before tensor memory is freed and the CTA leaves
       if (tc_elect()) tc_commit(bar_e);
-      tc_drain(bar_e, 0, kPfSpinLimit);
-      if (requested[1] > 0) tc_drain(bar_q, 0, kPfSpinLimit);
+      tc_drain(bar_e, 0);
+      if (requested[1] > 0) tc_drain(bar_q, 0);
 #pragma unroll 1
       for (int back = kPfStages; back > 0; --back) {
         const int k = requested[0] - back, v = requested[1] - back;
-        if (k >= 0) tc_drain(bar_k + 8 * (k % kPfStages), (unsigned)(k / kPfStages) & 1u, kPfSpinLimit);
-        if (v >= 0) tc_drain(bar_v + 8 * (v % kPfStages), (unsigned)(v / kPfStages) & 1u, kPfSpinLimit);
+        if (k >= 0) tc_drain(bar_k + 8 * (k % kPfStages), (unsigned)(k / kPfStages) & 1u);
+        if (v >= 0) tc_drain(bar_v + 8 * (v % kPfStages), (unsigned)(v / kPfStages) & 1u);
       }
       __syncwarp();
     }

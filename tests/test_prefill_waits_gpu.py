@@ -15,7 +15,7 @@ SOURCE = r"""
 using namespace inq;
 // Lanes below `cut` wait for a phase that is complete (the one before a new barrier's first), the others for
 // one that nobody completes.
-__global__ void wait_kernel(int cut, int limit, int* result, int* flag_out, long long* nanoseconds) {
+__global__ void wait_kernel(int cut, int tries, int* result, int* flag_out, long long* nanoseconds) {
   __shared__ __align__(8) unsigned long long barrier;
   __shared__ int flag;
   if (threadIdx.x == 0) {
@@ -23,22 +23,24 @@ __global__ void wait_kernel(int cut, int limit, int* result, int* flag_out, long
     flag = 0;
   }
   __syncthreads();
-  long long begin, end;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(begin));
-  const bool ok = tc_wait_warp(tc_smem(&barrier), threadIdx.x < cut ? 1u : 0u, &flag, limit);
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(end));
-  result[threadIdx.x] = ok;
-  if (ok == (cut == 32)) {   // what the kernels do next needs the whole warp
-    const unsigned chosen = tc_elect();
-    result[32 + threadIdx.x] = __popc(__ballot_sync(0xffffffffu, chosen != 0u));
-  }
+  long long times[3];
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(times[0]));
+  result[threadIdx.x] = tc_wait(tc_smem(&barrier), threadIdx.x < cut ? 1u : 0u, &flag, tries);
+  // what the kernels do next needs the whole warp
+  const unsigned chosen = tc_elect();
+  result[32 + threadIdx.x] = __popc(__ballot_sync(0xffffffffu, chosen != 0u));
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(times[1]));
+  if (flag) tc_wait(tc_smem(&barrier), 0u, &flag);   // the flag is raised: this does not wait for a second
+  __syncwarp();
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(times[2]));
   if (threadIdx.x == 0) {
     *flag_out = flag;
-    *nanoseconds = end - begin;
+    nanoseconds[0] = times[1] - times[0];
+    nanoseconds[1] = times[2] - times[1];
   }
 }
-extern "C" int run_wait(int cut, int limit, int* result, int* flag, long long* nanoseconds) {
-  wait_kernel<<<1, 32>>>(cut, limit, result, flag, nanoseconds);
+extern "C" int run_wait(int cut, int tries, int* result, int* flag, long long* nanoseconds) {
+  wait_kernel<<<1, 32>>>(cut, tries, result, flag, nanoseconds);
   return cudaDeviceSynchronize();
 }
 """
@@ -55,12 +57,14 @@ def library(tmp_path_factory):
 
 
 @pytest.mark.parametrize("cut", [0, 1, 16, 31, 32])
-def test_lanes_of_a_warp_leave_a_wait_together(library, cut):
+def test_lanes_whose_wait_gives_up_go_on_with_the_others(library, cut):
     result = torch.full((64,), -1, dtype=torch.int32, device="cuda")
-    flag, time = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int64, device="cuda")
+    flag, times = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(2, dtype=torch.int64, device="cuda")
     torch.cuda.synchronize()
-    assert library.run_wait(cut, 4096, *(ctypes.c_void_p(t.data_ptr()) for t in (result, flag, time))) == 0
-    assert result[:32].tolist() == [int(cut == 32)] * 32
+    assert library.run_wait(cut, 4096, *(ctypes.c_void_p(t.data_ptr()) for t in (result, flag, times))) == 0
+    assert result[:32].tolist() == [1] * cut + [0] * (32 - cut)
     assert result[32:].tolist() == [1] * 32            # one lane is elected, by all of them
     assert flag.item() == int(cut < 32)                # a wait that gave up says so to the other roles
-    assert time.item() < 4096 * 20e3                   # 4096 tries end within 80 ms: 20 us per try at most
+    first, second = times.tolist()
+    assert first < 4096 * 20e3                         # 4 us per try were measured: 2^18 tries are about a second
+    assert second < 1e6                                # with the flag raised a wait ends after one try
