@@ -14,8 +14,8 @@
 // slices on its own:
 //
 //   * staging: each lane issues 16-byte cp.async copies of the slice's K nibbles (2 KB),
-//     V codes (1 KB) and V scale/offset pairs (256 B) into a per-warp ring of three stages in
-//     shared memory; a block's scales, role map and padding ride with its first slice;
+//     V codes (1 KB) and V scale/offset pairs (256 B) into a per-warp ring of three stages (two for
+//     16-token slices) in shared memory; a block's scales, role map and padding ride with its first slice;
 //   * dequantisation never materialises K or V.  The descriptor-guided K decode is linear
 //     in the stored nibbles, so once per block it is folded into the query:
 //         score = sum_c w_c * nibble_c + const,
@@ -62,9 +62,15 @@ struct SliceCfg {
 constexpr int kPlanSliceTokens = 32;                // the unit of the flat work list (equal for both SUB when a block has <= 16 tokens)
 constexpr int kCtasPerSm = 3;                       // register budget: 168 per thread
 // Blocks of at most 16 tokens: every slice pays for a whole block's fold, a chain of dependent steps, and
-// a fourth CTA per SM (128 registers per thread, two ring stages to fit its shared memory) hides more of
-// it than the third stage did: 16 requests of 4096 to 32768 tokens in 32 layers, 16-token pages, 7915 ->
-// 7384 us; 8445 with three stages (shared memory for three CTAs only), 8750 with five CTAs (96 registers).
+// a fourth CTA per SM (128 registers per thread, which costs 24 to 36 bytes of spills, and two ring stages to
+// fit its shared memory) hides more of it than the third stage did: 16 requests of 4096 to 32768 tokens in
+// 32 layers, 16-token pages, 7927 -> 7262 us; one layer's blocks of 8192 tokens in 28 layers 118.8 -> 110.6 us,
+// without salient channels 81.9 -> 75.8; 8445 us of the first with three stages (shared memory for three CTAs
+// only), 8750 with five CTAs (96 registers).
+// With more than 16 salient channels (WIDE) the larger scratch holds three CTAs at most, so these keep 168
+// registers, and two stages, whose space is what lets the third CTA in at 33 to 48: the same 28 layers at
+// 32 / 48 / 64 salient channels 139.3 / 159.7 / 215.0 us (with 128 registers 145.4 / 169.9 / 227.4, with 168
+// and three stages 139.3 / 200.7 / 215.0).
 constexpr int kCtasSmall = 4, kStagesSmall = 2;
 __host__ __device__ constexpr int ring_stages(int sub) { return sub == 1 ? kStagesSmall : kStages; }
 // per-warp scratch before the per-group parts; the metadata slots only where it does not ride in the stages
@@ -494,8 +500,8 @@ __device__ __noinline__ void exchange_pair(const ExchangeView* X, int pair, long
 // multiplied into the probabilities and the offsets are contracted by one more MMA as for the 2-bit
 // values; a 16-byte chunk of a value row (8 words of four nibbles) is 32 channels, so every MMA lies
 // inside one group.  Their stages are 4.1 to 4.5 KB, so two CTAs fit an SM here as well.
-template <int MODE, typename QT, bool SAL, int SUB, bool FAST, int VK = 0, int VG = 2>
-__global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 ? kCtasSmall : kCtasPerSm) decode_kernel(const DecodeParams P) {
+template <int MODE, typename QT, bool SAL, int SUB, bool FAST, int VK = 0, int VG = 2, bool WIDE = false>
+__global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSmall : kCtasPerSm) decode_kernel(const DecodeParams P) {
   static_assert(!VK || (FAST && MODE == 0 && SAL && SUB == 2), "coded and 4-bit values: whole-slice path of the table layout only");
   static_assert(VK == 2 ? (VG == 1 || VG == 2 || VG == 4) : VK == 0 ? (VG == 2 || ((VG == 1 || VG == 4) && FAST && MODE == 0)) : VG == 2,
                 "4-bit values: groups of 32, 64 or 128 channels; 2-bit values: 64, or 32 and 128 on the whole-slice path");
@@ -1860,7 +1866,7 @@ using namespace inq;
 // device, not to the process: a process that drives several GPUs (or several host threads) gets
 // one record per device ordinal, filled under a mutex on first use.
 constexpr int kMaxDevices = 64;
-constexpr int kKernelVariants = 32;   // 16 general, 4 whole-slice, 2 coded values, 6 4-bit values, 4 2-bit values in one or four groups
+constexpr int kKernelVariants = 36;   // 16 general, 4 whole-slice, 2 coded values, 6 4-bit values, 4 2-bit values in one or four groups, 4 of 16-token slices with more than 16 salient channels
 struct DeviceState {
   int sm_count = 0;
   bool raised[kKernelVariants] = {};
@@ -2012,7 +2018,10 @@ extern "C" int inq_decode_attention(const inq_decode_args_t* a, inq_stream_t str
       decode_kernel<0, __half, true, 2, true, 2, 4>, decode_kernel<0, __nv_bfloat16, true, 2, true, 2, 4>,
       // 2-bit values in one group of 128 channels, in four groups of 32
       decode_kernel<0, __half, true, 2, true, 0, 1>, decode_kernel<0, __nv_bfloat16, true, 2, true, 0, 1>,
-      decode_kernel<0, __half, true, 2, true, 0, 4>, decode_kernel<0, __nv_bfloat16, true, 2, true, 0, 4>};
+      decode_kernel<0, __half, true, 2, true, 0, 4>, decode_kernel<0, __nv_bfloat16, true, 2, true, 0, 4>,
+      // 16-token slices with more than 16 salient channels
+      decode_kernel<0, __half, true, 1, false, 0, 2, true>, decode_kernel<0, __nv_bfloat16, true, 1, false, 0, 2, true>,
+      decode_kernel<1, __half, true, 1, false, 0, 2, true>, decode_kernel<1, __nv_bfloat16, true, 1, false, 0, 2, true>};
   const bool fast = a->n_pad == 16 && a->block_tokens % 32 == 0 && a->block_tokens >= 64;
   const int vk = a->value_kind, vg = a->value_groups;
   if (vk < 0 || vk > 2 || (vk == 2 && vg != 1 && vg != 2 && vg != 4) || (vk == 0 && vg != 0 && vg != 1 && vg != 2 && vg != 4))
@@ -2028,6 +2037,7 @@ extern "C" int inq_decode_attention(const inq_decode_args_t* a, inq_stream_t str
                   : vk == 2 ? 22 + (vg == 1 ? 0 : vg == 2 ? 2 : 4) + (a->dtype == INQ_F16 ? 0 : 1)
                   : vk ? 20 + (a->dtype == INQ_F16 ? 0 : 1)
                   : fast ? 16 + a->layout * 2 + (a->dtype == INQ_F16 ? 0 : 1)
+                  : sub == 1 && groups > 1 ? 32 + a->layout * 2 + (a->dtype == INQ_F16 ? 0 : 1)
                          : (sub == 1 ? 8 : 0) + a->layout * 4 + (a->dtype == INQ_F16 ? 0 : 2) + (groups > 0 ? 1 : 0);
   const kernel_t kernel = kernels[which];
   const int scratch = smem_bytes(groups, sub, vk, vg);

@@ -165,7 +165,7 @@ def test_paged_batch_of_requests_with_different_lengths(block, heads, q_heads):
     assert N.take_status(batch.device) == 0
 
 
-@pytest.mark.parametrize("fraction", [0.0, 0.125])
+@pytest.mark.parametrize("fraction", [0.0, 0.125, 0.25, 0.375, 0.5])
 def test_a_long_request_beside_short_ones_at_one_kv_head(fraction):
     """16-token blocks: the long request's pair is cut into nearly every CTA's range (tests/test_decode_plan_cpu.py),
     so the merge of its parts needs more shared memory than the warps' own scratch.  Against float64

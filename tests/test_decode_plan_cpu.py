@@ -47,6 +47,7 @@ def test_merge_of_the_most_divided_pair_fits_the_shared_memory_of_the_launch(blo
             assert (shape.n_ctas - 1) * shape.per_cta < total <= shape.n_ctas * shape.per_cta
             assert _most_parts(starts, shape) <= shape.merge_parts, (starts[-1], len(starts) - 1, ctas_per_sm)
             assert shape.shared_bytes <= 227 * 1024
+            assert (shape.n_ctas + len(starts) - 1) * N.RECORD_FLOATS <= N.library().inq_decode_workspace_floats(len(starts) - 1, starts[-1])
 
 
 @pytest.mark.parametrize("value_kind,value_groups", [(1, 0), (2, 1), (2, 2), (2, 4), (0, 1), (0, 4)])
