@@ -1923,6 +1923,11 @@ static Plan make_plan(long long total_units, int n_pairs, long long uniform_unit
   const long long by_pairs = 64ll * n_pairs;
   long long n = slots < by_work ? slots : by_work;
   if (n > by_pairs) n = by_pairs;
+  // 16-token blocks at four CTAs per SM: a grid that leaves some SMs with three equal ranges and some with four
+  // lasts as long as one with four everywhere and has the longer merges, so such a launch takes three per SM
+  // (one layer of 8 heads, 444 instead of 512 CTAs: 8192 tokens 22.5 instead of 23.8 us, 16384 29.6 / 31.3, 32768
+  // 44.6 / 46.1; two layers of 4 heads, 8192 tokens 24.4 / 27.7)
+  if (ctas_per_sm == kCtasSmall && n < slots && n > slots - sm_count()) n = slots - sm_count();
   // the ramp charge never exceeds half of an even share of slices
   long long ramp = kRampUnits;
   const long long share = total_units / n;

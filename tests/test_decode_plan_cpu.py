@@ -66,6 +66,16 @@ def test_a_long_request_beside_short_ones_takes_more_parts_than_the_warps_scratc
     assert shape.merge_parts >= shape.n_ctas
 
 
+@pytest.mark.parametrize("pairs,units", [(8, 512), (8, 2048), (8, 1024), (16, 4096 // 16)])
+def test_four_ctas_per_sm_fill_every_sm_or_leave_the_fourth_out(pairs, units):
+    """16-token blocks, a batch whose pairs or work do not give four ranges to all of 148 SMs."""
+    starts = [p * units for p in range(pairs + 1)]
+    four, three = _shape(starts, 16, 16, 4), _shape(starts, 16, 16, 3)
+    assert four.n_ctas == three.n_ctas <= 444 and four.per_cta == three.per_cta
+    long = [p * 4096 for p in range(65)]
+    assert 444 < _shape(long, 16, 16, 4).n_ctas <= 592
+
+
 def test_launch_shape_refuses_what_no_launch_could_have():
     lib, shape = N.library(), N.DecodeShape()
     assert lib.inq_decode_launch_shape(1, 1, 16, 0, 0, 2, 4, None) == N.ERR_ARGUMENT
