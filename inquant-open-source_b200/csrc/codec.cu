@@ -446,10 +446,9 @@ __global__ void __launch_bounds__(kMaxThreads) k4_encode_kernel(K4Params p) {
 //     (NaN and Inf sort above every finite value);
 //   * x / s uses a correctly rounded reciprocal and two fused corrections, which returns the
 //     IEEE quotient (Markstein); scales below 2^-100 keep the plain division;
-//   * the selected / available sets are two 64-bit masks in registers.
+//   * the sets of channels are masks in registers.
 struct Mask128 {
   unsigned long long lo, hi;
-  __device__ __forceinline__ bool test(int i) const { return i >= 0 && i < 128 && (((i < 64 ? lo : hi) >> (i & 63)) & 1ull); }
   __device__ __forceinline__ int below(int pos) const {   // largest member < pos, or -1
     if (pos > 64) {
       unsigned long long m = pos >= 128 ? hi : (hi & ((1ull << (pos - 64)) - 1ull));
@@ -471,6 +470,9 @@ struct Mask128 {
     return m ? 63 + __ffsll((long long)m) : 128;
   }
 };
+
+// the n lowest bits, for any n
+__device__ __forceinline__ unsigned bits_below(int n) { return n <= 0 ? 0u : n >= 32 ? ~0u : (1u << n) - 1u; }
 
 __device__ __forceinline__ float exact_quotient(float x, float s, float r, bool plain) {
   if (plain) return x / s;
@@ -729,51 +731,55 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
   }
   __syncthreads();
   if (c < 32 && count > 0) {
-    // Donors are taken by the sources in ascending order, each from what the earlier ones left.  One lane
-    // per source: all choose at once, and as far as no source wants what an earlier one chose, the choices
-    // are those of the sequence -- a donor that is gone but was not this source's choice changes neither
-    // which of its candidates is nearer nor the tie between them.  From the first conflict on, the rest
-    // choose again.  (One thread walking the list took 15000 to 23000 cycles: the 12 rows of three blocks of
-    // 256 tokens 38 instead of 30 us, 496 rows 57 instead of 49.)
-    Mask128 sel{(unsigned long long)s_sel[0] | ((unsigned long long)s_sel[1] << 32),
-                (unsigned long long)s_sel[2] | ((unsigned long long)s_sel[3] << 32)};
-    const Mask128 others{~sel.lo, ~sel.hi};
-    unsigned word[4] = {s_avail[0], s_avail[1], s_avail[2], s_avail[3]};
+    // Donors are taken by the sources in ascending order, each from what the earlier ones left.  One lane per
+    // source: all choose at once, then the choices are settled one by one (a shuffle, a vote), and only when the
+    // donor just taken was the choice of a later source do the later ones choose again -- a donor that is gone
+    // but was not a source's choice changes neither which of its candidates is nearer nor the tie between
+    // them.  (All of them choosing again from conflict to conflict, with a match and four reductions a round, took
+    // 400 rows of 16 tokens 19.3 instead of 11.2 us with least-error donors, 64 rows of 64 19.5 / 11.8, 12 rows of
+    // 256 29.0 / 21.8, 496 of 256 46.8 / 39.8; one thread walking the list with branches 18.0, 19.2, 37.1 and
+    // 53.7; a walk without branches but with no choice ahead of it 11.4, 12.0, 22.4 and 40.1.)
+    const Mask128 others{~((unsigned long long)s_sel[0] | ((unsigned long long)s_sel[1] << 32)),
+                         ~((unsigned long long)s_sel[2] | ((unsigned long long)s_sel[3] << 32))};
+    unsigned free_[4] = {s_avail[0], s_avail[1], s_avail[2], s_avail[3]};
     for (int first = 0; first < count; first += 32) {
-      const bool mine = first + c < count;
-      const int source = mine ? s_src[first + c] : 0;
+      const int n = min(32, count - first);
+      const int source = c < n ? s_src[first + c] : 0;
       const int left = others.below(source) + 1, right = others.above(source) - 1;   // the run of sources around this one
-      unsigned todo = __ballot_sync(0xffffffffu, mine);
-      while (todo) {
-        const Mask128 avail{(unsigned long long)word[0] | ((unsigned long long)word[1] << 32),
-                            (unsigned long long)word[2] | ((unsigned long long)word[3] << 32)};
-        int donor = -1;
-        if ((todo >> c) & 1u) {
-          int low = avail.test(source - 1) ? source - 1 : -1;
-          int high = avail.test(source + 1) ? source + 1 : -1;
-          if (low < 0 && high < 0) {
-            const int below = avail.below(left), above = avail.above(right);
-            const int d_below = below >= 0 ? left - below : 0x7fffffff;
-            const int d_above = above < 128 ? above - right : 0x7fffffff;
-            if (d_below <= d_above) low = below;
-            if (d_above <= d_below && above < 128) high = above;
-          }
-          if (low >= 0 && high >= 0)
-            donor = s_sal[low] <= s_sal[high] ? low : high;
-          else
-            donor = low >= 0 ? low : high;
-        }
-        // (no donor is left for a source only when none is left at all)
-        const unsigned same = __match_any_sync(0xffffffffu, donor >= 0 ? donor : C + c);
-        const unsigned conflicts = __ballot_sync(0xffffffffu, (same & ((1u << c) - 1u)) != 0u);
-        const unsigned settled = todo & (conflicts ? (conflicts & (0u - conflicts)) - 1u : 0xffffffffu);
-        const bool settles = (settled >> c) & 1u;
-        if (settles) s_don[first + c] = max(donor, 0);
+      unsigned below[4], above[4];
 #pragma unroll
-        for (int w = 0; w < 4; ++w)
-          word[w] &= ~__reduce_or_sync(0xffffffffu, settles && donor >= 0 && (donor >> 5) == w ? 1u << (donor & 31) : 0u);
-        todo &= ~settled;
+      for (int w = 0; w < 4; ++w) {
+        below[w] = bits_below(left - 32 * w);
+        above[w] = ~bits_below(right + 1 - 32 * w);
       }
+      int choice = 0, i = 0;
+      while (true) {
+        // nearest free channel on either side of the run: -1 and 128 where there is none
+        int low = -1, high = C;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const unsigned b = free_[w] & below[w], h = free_[3 - w] & above[3 - w];
+          low = b ? 32 * w + 31 - __clz(b) : low;
+          high = h ? 32 * (3 - w) + __ffs(h) - 1 : high;
+        }
+        // one next to the source itself wins over any other, else the nearer one; of two the less salient, then the lower
+        const bool has_low = low >= 0, has_high = high < C;
+        const int d_low = has_low ? left - low : C, d_high = has_high ? high - right : C;
+        const bool by_low = has_low && low == source - 1, by_high = has_high && high == source + 1, beside = by_low || by_high;
+        const bool take_low = beside ? by_low : has_low && d_low <= d_high, take_high = beside ? by_high : has_high && d_high <= d_low;
+        const bool lower = s_sal[max(low, 0)] <= s_sal[min(high, C - 1)];
+        const int donor = take_low && (lower || !take_high) ? low : take_high ? high : 0;   // (one is free for every source)
+        if (c >= i) choice = donor;
+        int taken;
+        do {
+          taken = __shfl_sync(0xffffffffu, choice, i);
+#pragma unroll
+          for (int w = 0; w < 4; ++w) free_[w] &= (taken >> 5) == w ? ~(1u << (taken & 31)) : ~0u;
+          ++i;
+        } while (i < n && !__any_sync(0xffffffffu, c >= i && c < n && choice == taken));
+        if (i >= n) break;
+      }
+      if (c < n) s_don[first + c] = choice;
     }
   }
   // ---- scales and per-slot encoding parameters
