@@ -23,7 +23,7 @@
 //   * warp 9 (one lane, warps 10 and 11 complete the warpgroup): TMA (cp.async.bulk.tensor, 128-byte swizzle, no multicast) for Q once and
 //     for the double-buffered K and V tiles.
 // All hand-overs are mbarriers; every wait is bounded and a wait that gives up raises an abort
-// flag after which no other wait waits, so that every role runs through its loop (see tc_wait); copies and
+// flag after which no other wait waits for long, so that every role runs through its loop (see tc_wait); copies and
 // contractions in flight are then waited for (again bounded) before tensor memory is freed and the CTA ends.
 // One CTA per SM (tensor-memory kernels are scheduled that way),
 // 192 KB of shared memory, all 512 TMEM columns.  Keys and values are dense tensors in the model

@@ -62,16 +62,17 @@ __device__ __forceinline__ bool tc_try_wait(unsigned mbar, unsigned parity) {
 }
 // Bounded wait of a thread for a phase of a barrier.  A try sleeps for up to 4 us (measured), so 2^18 of them are
 // about a second.  A wait that runs out raises the abort flag, and once the flag is raised every wait of the
-// CTA ends after one try.  The lanes of a warp wait by themselves and need not agree on the outcome, but what
+// CTA ends after 16 tries (most tries that fail come back early, and reading the flag after each of them held
+// up the next: 1500-token prompt of 32 heads 29.3 instead of 27.9 us,
+// 2048 queries over 4096 keys of 28 heads 94.2 instead of 91.1).  The lanes of a warp wait by themselves and need not agree on the outcome, but what
 // follows a wait -- elect.sync over the full mask, the .sync.aligned tensor-memory instructions -- needs all
 // of them.  So a warp does not leave its loop where a wait gives up: it runs through its remaining turns,
-// whose waits no longer wait, on data that nobody will use.  (Voting on the outcome of every wait
-// instead took a 1500-token prompt 32.0 instead of 31.4 us.)
+// whose waits no longer wait, on data that nobody will use.
 constexpr int kTcTries = 1 << 18;
 __device__ __forceinline__ bool tc_wait(unsigned mbar, unsigned parity, volatile int* abort_flag, int tries = kTcTries) {
   for (int it = 0; it < tries; ++it) {
     if (tc_try_wait(mbar, parity)) return true;
-    if (*abort_flag) return false;
+    if ((it & 15) == 15 && *abort_flag) return false;
   }
   *abort_flag = 1;
   return false;

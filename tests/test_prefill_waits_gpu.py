@@ -67,4 +67,4 @@ def test_lanes_whose_wait_gives_up_go_on_with_the_others(library, cut):
     assert flag.item() == int(cut < 32)                # a wait that gave up says so to the other roles
     first, second = times.tolist()
     assert first < 4096 * 20e3                         # 4 us per try were measured: 2^18 tries are about a second
-    assert second < 1e6                                # with the flag raised a wait ends after one try
+    assert second < 1e6                                # with the flag raised a wait ends after 16 tries
