@@ -1,7 +1,7 @@
 // Chunked-prefill attention on the 5th-generation tensor cores (tcgen05, accumulators in TMEM).
 //
 // One CTA owns 256 query tokens of one query head as two tiles of 128 rows (A and B) and walks
-// the visible keys and values in tiles of 128 tokens.  Ten warps, three roles:
+// the visible keys and values in tiles of 128 tokens.  Twelve warps, ten of them in three roles:
 //   * warps 0-3 / 4-7: softmax of tile A / tile B, one thread per query row.  A thread loads its whole
 //     row of S from tensor memory into registers (four tcgen05.ld in flight, waited for once), takes
 //     the maximum, raises the lagging reference maximum in the rare case that it has to, and stores the
@@ -583,7 +583,9 @@ extern "C" int inq_prefill_attention(const inq_prefill_args_t* a, inq_stream_t s
     const int lightest = (int)((std::min<long long>(a->kv_tokens, (long long)a->kv_tokens - a->q_tokens + kPfRows) + kPfTile - 1) / kPfTile);
     // cost of a cut into sp segments, in KV-tile times: rounds of CTAs over the SMs, each as long
     // as one segment plus, when cut, the fixed price of a segment (pipeline fill, writing and
-    // merging a 133 KB partial record), measured at about six tile times
+    // merging a 133 KB partial record): six tile times when a tile took 30 % longer, eight to thirteen
+    // of the present ones (256 queries over 2048 keys, 28 heads, 1 / 3 / 4 / 5 segments: 38.9 / 35.8 / 33.7 /
+    // 37.6 us; 2048 over 16384, 1 / 3: 435 / 460; 2048 over 32768, 1 / 3: 883 / 857)
     const double tiles = ((double)a->kv_tokens - 0.5 * a->q_tokens) / kPfTile;
     double best = 1e30;
     for (int sp = 1; sp <= max_splits(items); ++sp) {
