@@ -1916,7 +1916,7 @@ static Plan make_plan(long long total_units, int n_pairs, long long uniform_unit
   Plan p;
   p.n_pairs = n_pairs;
   p.uniform_units = uniform_units;
-  long long slots = (long long)sm_count() * ctas_per_sm;
+  const long long n_sm = sm_count(), slots = n_sm * ctas_per_sm;
   long long by_work = total_units / 8 > 1 ? total_units / 8 : 1;   // at least 2 slices per warp
   // a pair cut into more than ~64 parts pays more for the merge of its partial records than the
   // shorter ranges save (single-layer launches: 38 instead of 44 us at 32768 tokens)
@@ -1927,7 +1927,7 @@ static Plan make_plan(long long total_units, int n_pairs, long long uniform_unit
   // lasts as long as one with four everywhere and has the longer merges, so such a launch takes three per SM
   // (one layer of 8 heads, 444 instead of 512 CTAs: 8192 tokens 22.5 instead of 23.8 us, 16384 29.6 / 31.3, 32768
   // 44.6 / 46.1; two layers of 4 heads, 8192 tokens 24.4 / 27.7)
-  if (ctas_per_sm == kCtasSmall && n < slots && n > slots - sm_count()) n = slots - sm_count();
+  if (ctas_per_sm == kCtasSmall && n < slots && n > slots - n_sm) n = slots - n_sm;
   // the ramp charge never exceeds half of an even share of slices
   long long ramp = kRampUnits;
   const long long share = total_units / n;
@@ -2049,7 +2049,6 @@ extern "C" int inq_decode_attention(const inq_decode_args_t* a, inq_stream_t str
   const int shared_limit = smem_bytes(vk ? 1 : 4, sub, vk, vg);
   const int device = current_device();
   if (device < 0) return INQ_ERR_UNSUPPORTED;   // device ordinals above 63 are not tracked
-  const int n_sm = sm_count();
   int resident = 0;
   {
     std::lock_guard<std::mutex> guard(g_devices_mutex);
@@ -2059,7 +2058,8 @@ extern "C" int inq_decode_attention(const inq_decode_args_t* a, inq_stream_t str
       d.raised[which] = true;
     }
     if (!d.per_sm[which][groups]) {
-      int n = 0;
+      int n = 0, n_sm = 0;
+      INQ_CUDA_CHECK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device));
       INQ_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kThreads, scratch));
       // the grid stays resident as a whole with the shared memory of its largest merge as well
       const int merge = launch_smem(scratch, shared_limit, n_sm * std::max(n, 1));
