@@ -64,7 +64,7 @@ constexpr int kCtasPerSm = 3;                       // register budget: 168 per 
 // Blocks of at most 16 tokens: every slice pays for a whole block's fold, a chain of dependent steps, and
 // a fourth CTA per SM (128 registers per thread, which costs 24 to 36 bytes of spills, and two ring stages to
 // fit its shared memory) hides more of it than the third stage did: 16 requests of 4096 to 32768 tokens in
-// 32 layers, 16-token pages, 7946 -> 7260 us; one layer's blocks of 8192 tokens in 28 layers 118.8 -> 110.6 us,
+// 32 layers, 16-token pages, 7946 -> 7260 us; one request of 8192 tokens in 28 layers 118.8 -> 110.6 us,
 // without salient channels 81.9 -> 75.8; 8445 us of the first with three stages (shared memory for three CTAs
 // only), 8750 with five CTAs (96 registers).
 // With more than 16 salient channels (WIDE) the larger scratch holds three CTAs at most, so these keep 168
