@@ -14,8 +14,8 @@
 // slices on its own:
 //
 //   * staging: each lane issues 16-byte cp.async copies of the slice's K nibbles (2 KB),
-//     V codes (1 KB) and V scale/offset pairs (256 B) into a per-warp ring of three stages (two for
-//     16-token slices) in shared memory; a block's scales, role map and padding ride with its first slice;
+//     V codes (1 KB) and V scale/offset pairs (256 B) into a per-warp ring of three stages in
+//     shared memory; a block's scales, role map and padding ride with its first slice;
 //   * dequantisation never materialises K or V.  The descriptor-guided K decode is linear
 //     in the stored nibbles, so once per block it is folded into the query:
 //         score = sum_c w_c * nibble_c + const,
@@ -61,24 +61,24 @@ struct SliceCfg {
 };
 constexpr int kPlanSliceTokens = 32;                // the unit of the flat work list (equal for both SUB when a block has <= 16 tokens)
 constexpr int kCtasPerSm = 3;                       // register budget: 168 per thread
-// Blocks of at most 16 tokens: every slice pays for a whole block's fold, a chain of dependent steps, and
-// a fourth CTA per SM (128 registers per thread, which costs 24 to 36 bytes of spills, and two ring stages to
-// fit its shared memory) hides more of it than the third stage did: 16 requests of 4096 to 32768 tokens in
-// 32 layers, 16-token pages, 7946 -> 7260 us; one request of 8192 tokens in 28 layers 118.8 -> 110.6 us,
-// without salient channels 81.9 -> 75.8; 8445 us of the first with three stages (shared memory for three CTAs
-// only), 8750 with five CTAs (96 registers).
-// With more than 16 salient channels (WIDE) the larger scratch holds three CTAs at most, so these keep 168
-// registers, and two stages, whose space is what lets the third CTA in at 33 to 48: the same 28 layers at
+// Blocks of at most 16 tokens: every slice pays for a whole block's fold, a chain of dependent steps, and a
+// fourth CTA per SM (128 registers per thread) hides more of it than 168 registers save.  With more than 16
+// salient channels (WIDE) the larger scratch holds three CTAs at most, so these keep 168 registers, and two
+// ring stages, whose space is what lets the third CTA in at 33 to 48 channels: 28 layers of 8192 tokens at
 // 32 / 48 / 64 salient channels 139.3 / 159.7 / 215.0 us (with 128 registers 145.4 / 169.9 / 227.4, with 168
 // and three stages 139.3 / 200.7 / 215.0).
 constexpr int kCtasSmall = 4, kStagesSmall = 2;
-__host__ __device__ constexpr int ring_stages(int sub) { return sub == 1 ? kStagesSmall : kStages; }
+__host__ __device__ constexpr int ring_stages(int sub, bool wide) { return sub == 1 && wide ? kStagesSmall : kStages; }
+// two slots for a block's row of the pointer table, requested one block ahead (whole-slice path)
+constexpr int kRowSlots = 2 * 64;
 // per-warp scratch before the per-group parts; the metadata slots only where it does not ride in the stages
-__host__ __device__ constexpr int warp_fixed(int sub) { return 2048 + 256 + 64 + 64 + 256 + (sub == 1 ? 0 : 2048); }
+__host__ __device__ constexpr int warp_fixed(int sub, bool wide) { return (sub == 1 && !wide ? 0 : 2048) + 256 + 64 + 64 + 256 + (sub == 1 ? 0 : 2048) + kRowSlots; }
 constexpr int kRecordStride = 132;                  // floats per query head: acc[128], m, l, pad
 constexpr int kRecordFloats = 8 * kRecordStride;    // one partial record (8 query heads)
 constexpr int kQChunk = 36;                         // padded 32-float chunk of the staged query
 constexpr int kQFragBytes = 8 * 32 * 8;              // the staged query as fp16 B fragments of the 8 K steps
+constexpr int kQRow = 136;                          // padded row of the query staged in the model dtype (at most 16 salient channels)
+static_assert(8 * kQRow * 2 <= 8 * 4 * kQChunk * 4 && kQRow % 8 == 0, "the 16-bit query takes the place of the fp32 one");
 constexpr int kQBytes = 8 * 4 * kQChunk * 4 + 64 + kQFragBytes;   // staged query, two factors per head, fragments
 constexpr float kNegBig = -1.0e30f;
 constexpr float kRescaleSlack = 4.f;   // the running reference maximum may lag the true one by 2^4
@@ -93,7 +93,7 @@ constexpr float kGatherInit = -128.25f / 8192.f;
 constexpr int kValueMeta = 768, kValueTables = 32 * (64 + 64 + 16), kValueXchg = 16 * 8 * 4;
 constexpr int kValueScratch = 2 * kValueMeta + kValueTables + kValueXchg;   // two metadata slots, as for the keys
 __host__ __device__ constexpr int warp_smem_bytes(int groups, int stage_bytes, int vk, int sub) {
-  return warp_fixed(sub) + groups * (256 + 2048 + 64) + (vk ? kValueScratch : 0) + ring_stages(sub) * stage_bytes;
+  return warp_fixed(sub, groups > 1) + groups * (256 + 2048 + 64) + (vk ? kValueScratch : 0) + ring_stages(sub, groups > 1) * stage_bytes;
 }
 
 struct SeqDesc {
@@ -262,15 +262,14 @@ __device__ __forceinline__ float2 half2_bits_to_float2(unsigned bits) {
 }
 
 // ------------------------------------------------------------------------------------------ block lookup
+// `row`: the block's six pointers (table layout); `id`: its physical page (paged layout)
 template <int MODE, int VK = 0, int VG = 2>
-__device__ __forceinline__ BlockPtrs locate_block(const DecodeParams& P, const long long* table,
-                                                  const signed char* roles, const unsigned char* pool,
-                                                  const int* page_table, int pool_pages, int b, int h,
+__device__ __forceinline__ BlockPtrs locate_block(const DecodeParams& P, const long long* row, const signed char* roles,
+                                                  const unsigned char* pool, int id, int pool_pages, int b, int h,
                                                   const signed char* value_roles = nullptr) {
   BlockPtrs out;
   out.vr = nullptr;
   if (MODE == 0) {
-    const long long* row = table + (long long)b * 6;
     const long long T = P.T;
     out.kp = (const unsigned char*)row[0] + (long long)h * T * 64;
     out.ks = (const unsigned char*)row[1] + (long long)h * 512;
@@ -292,7 +291,6 @@ __device__ __forceinline__ BlockPtrs locate_block(const DecodeParams& P, const l
     }
     out.kr = (const unsigned char*)roles + ((long long)b * P.H + h) * 128;
   } else {
-    int id = page_table[b];
     if (pool_pages > 0 && (unsigned)id >= (unsigned)pool_pages) {
       // never dereferenced: the first page stands in and the caller learns of it from the status word
       atomicOr(P.status, INQ_STATUS_BAD_INDEX);
@@ -506,19 +504,30 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   static_assert(VK == 2 ? (VG == 1 || VG == 2 || VG == 4) : VK == 0 ? (VG == 2 || ((VG == 1 || VG == 4) && FAST && MODE == 0)) : VG == 2,
                 "4-bit values: groups of 32, 64 or 128 channels; 2-bit values: 64, or 32 and 128 on the whole-slice path");
   constexpr int kSub = SUB;
-  constexpr int kRing = ring_stages(SUB);
+  constexpr int kRing = ring_stages(SUB, WIDE);
   constexpr int kSliceTokens = SliceCfg<SUB, VK, VG>::kSliceTokens;
   constexpr int kStageK = SliceCfg<SUB, VK, VG>::kStageK, kStageV = SliceCfg<SUB, VK, VG>::kStageV, kStageP = SliceCfg<SUB, VK, VG>::kStageP;
   constexpr int kStageBytes = SliceCfg<SUB, VK, VG>::kStageBytes;
+  // At most 16 salient channels, known at compile time: a block's fold is straight-line code over one record
+  // per salient channel; otherwise (up to 64) it loops over lists.  With the loops' branches a fold was a chain
+  // of 3500 to 4700 cycles, and the look-up of the next block (table row or page id) another 1300 to 3200: per
+  // 32-token slice of 256-token blocks 985 of 2993 cycles, per 16-token page 5000 of 6700.  Straight-line, with the
+  // look-up one block ahead, they are 630 and 1740, and a launch takes (us, before -> after, L2 warm) 129 -> 120
+  // (28 layers x 4 heads x 32768 tokens), 93.5 -> 86.5 (16384 tokens, values coded like the keys), 3084 -> 2668
+  // (16 requests x 32 layers x 8 heads, pages of 64) and 7272 -> 4201 (pages of 16).
+  constexpr bool kNarrow = FAST || (SUB == 1 && !WIDE);
+  // every slice is a block of its own: its weights are multiplied out where the score MMAs read them
+  constexpr bool kDirect = SUB == 1 && kNarrow;
   constexpr bool kMetaInStage = SliceCfg<SUB, VK, VG>::kStageMeta > 0;   // host guarantees one slice per block
   constexpr int kMetaOffset = kStageK + kStageV + kStageP;
   extern __shared__ __align__(16) unsigned char smem[];
   float* qs = (float*)smem;                                             // 8 heads x 4 chunks x kQChunk
+  // kNarrow: the staged query times 2^-12 in the model dtype, 8 heads x kQRow, in the place of qs
+  QT* q16 = (QT*)smem;
   float* qinv = qs + 8 * 4 * kQChunk;   // per head: softmax scale * log2(e) * 2^(exponent of max|q| - 12)
-  float* qunscale = qinv + 8;           // per head: the power of two that restores the staged query
   // the staged query once more as fp16 pairs in B-fragment order: entry [K step][lane (head r, chunk j)]
   // holds channels (c, c+4 | c+1, c+5), c = 32j + 8 (step / 2) + 2 (step % 2), of query head r
-  unsigned char* qfrag = (unsigned char*)(qunscale + 8);
+  unsigned char* qfrag = (unsigned char*)(qinv + 16);
   unsigned char* warp_base = smem + kQBytes;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int r = lane >> 2, j = lane & 3;
@@ -529,7 +538,10 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   // folded-query B fragments of the 8 K steps ([step][lane] x 8 bytes); while a block's weights
   // are being derived the same 2 KB hold the per-channel slot weights and additive constants
   unsigned char* wW = wb;
-  float* wssc = (float*)(wb + 2048);                                    // scale of salient channel i
+  float* wssc = (float*)(wb + (kDirect ? 0 : 2048));                                    // scale of salient channel i
+  // kNarrow: record i = {scale, source channel | donor slot << 8} of salient channel i; record 16 takes
+  // what the regular channels write
+  uint2* wrec = (uint2*)wssc;
   unsigned char* wsrc = (unsigned char*)(wssc + 64);                    // channel of salient i
   unsigned char* wdon = wsrc + 64;                                      // its donor slot
   // staged block metadata: K scales 512 B | role map 256 B | padding 256 B.  Two slots: the whole-slice
@@ -537,7 +549,8 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   // while this one's slot is still to be read
   unsigned char* wmeta = wdon + 64;
   unsigned char* wfrag = wmeta + (SUB == 1 ? 0 : 2048);    // a block's channel weights as fp16 pairs in B-fragment order: [K step][chunk] x 8 B
-  unsigned char* wqsal = wb + warp_fixed(SUB);                               // B fragments: query at salient channels
+  long long* wrow = (long long*)(wfrag + 256);             // whole-slice path, table layout: row of block b in slot b % 2
+  unsigned char* wqsal = wb + warp_fixed(SUB, WIDE);                               // B fragments: query at salient channels
   unsigned char* wsel = wqsal + groups * 256;                           // B fragments: nibble selection
   unsigned short* wcell = (unsigned short*)(wsel + groups * 2048);      // selection cells written by the last fold (offsets into wsel)
   // InQuant-coded values: staged value metadata of a block, the lane's flush tables, the donor sums
@@ -599,8 +612,8 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   }
   const int first_visible = SEQ(first_visible);
   // (loaded here, ahead of the barriers of the query staging, so that their latency overlaps it)
-  const int T = P.T;
-  const int spb = (T + kSliceTokens - 1) / kSliceTokens;   // packed slices per block
+  const int T = FAST && SUB == 1 ? 16 : P.T;
+  const int spb = SUB == 1 ? 1 : (T + kSliceTokens - 1) / kSliceTokens;   // packed slices per block
   const int n_blocks = SEQ(n_blocks);
   const int sink_tokens = SEQ(sink_tokens);
   const int* const tail_dev = SEQ(tail_tokens_dev);
@@ -614,48 +627,55 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   // matrix and an empty list of written cells
   for (int v = lane; v < groups * 128; v += 32) ((uint4*)wsel)[v] = make_uint4(0u, 0u, 0u, 0u);
   for (int v = lane; v < 64; v += 32) wssc[v] = 0.f;   // scales of unused salient slots must be finite
-  for (int v = lane; v < groups * 32; v += 32) wcell[v] = 0;
-  // query as fp32, chunked so that lanes (head, chunk) read distinct banks, then scaled per head by
-  // a power of two that brings its largest magnitude into [2^12, 2^13): every folded weight is
-  // then a product below 2^14 that fp16 holds without overflow and with full precision
-  if ((((unsigned long long)qptr | (unsigned long long)(q_stride * (long long)sizeof(QT))) & 15ull) == 0) {
-    // one 16-byte load per thread: head g = thread / 16, channels 8 * (thread % 16) .. + 7
+  if (!kNarrow)
+    for (int v = lane; v < groups * 32; v += 32) wcell[v] = 0;
+  // The query, scaled per head by a power of two that brings its largest magnitude into [2^12, 2^13): every
+  // folded weight is then a product below 2^14 that fp16 holds without overflow and with full precision.
+  // A head belongs to 16 threads with 8 channels each, so its maximum stays inside a half-warp; the eight
+  // channels are two B-fragment entries: (c, c+4 | c+1, c+5) and (c+2, c+6 | c+3, c+7).
+  {
     const int g = threadIdx.x >> 4, c0 = (threadIdx.x & 15) * 8;
     uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-    if (g < g_valid) raw = *(const uint4*)(qptr + (q_head0 + g) * q_stride + c0);
-    const QT* e = (const QT*)&raw;
-    float* dst = qs + (g * 4 + (c0 >> 5)) * kQChunk + (c0 & 31);
-    *(float4*)dst = make_float4(to_float<QT>(e[0]), to_float<QT>(e[1]), to_float<QT>(e[2]), to_float<QT>(e[3]));
-    *(float4*)(dst + 4) = make_float4(to_float<QT>(e[4]), to_float<QT>(e[5]), to_float<QT>(e[6]), to_float<QT>(e[7]));
-  } else {
-    for (int idx = threadIdx.x; idx < 8 * 128; idx += kThreads) {
-      int g = idx >> 7, c = idx & 127;
-      float v = g < g_valid ? to_float<QT>(qptr[(q_head0 + g) * q_stride + c]) : 0.f;
-      qs[(g * 4 + (c >> 5)) * kQChunk + (c & 31)] = v;
-    }
-  }
-  __syncthreads();
+    QT* const e = (QT*)&raw;
+    if (g < g_valid) {
+      const QT* const src = qptr + (q_head0 + g) * q_stride + c0;
+      if ((((unsigned long long)qptr | (unsigned long long)(q_stride * (long long)sizeof(QT))) & 15ull) == 0) {
+        raw = *(const uint4*)src;
+      } else {
 #pragma unroll
-  for (int hh = 0; hh < 8 / kWarps; ++hh) {
-    const int head = warp * (8 / kWarps) + hh;
-    float* row = qs + head * 4 * kQChunk + lane;
-    const float v0 = row[0], v1 = row[kQChunk], v2 = row[2 * kQChunk], v3 = row[3 * kQChunk];
-    unsigned top = __float_as_uint(fmaxf(fmaxf(fabsf(v0), fabsf(v1)), fmaxf(fabsf(v2), fabsf(v3))));
-    top = __reduce_max_sync(0xffffffffu, top);
+        for (int k = 0; k < 8; ++k) e[k] = src[k];
+      }
+    }
+    float v[8];
+    unsigned top = 0u;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      v[k] = to_float<QT>(e[k]);
+      top = max(top, __float_as_uint(fabsf(v[k])));
+    }
+#pragma unroll
+    for (int off = 1; off < 16; off <<= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, off));
     int ex = (int)(top >> 23) - 127;
     ex = top == 0u ? 0 : max(-60, min(60, ex));
     const float mul = __uint_as_float((unsigned)(127 + 12 - ex) << 23);
-    row[0] = v0 * mul; row[kQChunk] = v1 * mul; row[2 * kQChunk] = v2 * mul; row[3 * kQChunk] = v3 * mul;
-    if (lane == 0) {
-      qunscale[head] = __uint_as_float((unsigned)(127 + ex - 12) << 23);
-      qinv[head] = P.scale_log2e * qunscale[head];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] *= mul;
+    unsigned char* const entry = qfrag + (2 * ((c0 >> 3) & 3) * 32 + g * 4 + (c0 >> 5)) * 8;
+    *(uint2*)entry = make_uint2(pack_half2(v[0], v[4]), pack_half2(v[1], v[5]));
+    *(uint2*)(entry + 256) = make_uint2(pack_half2(v[2], v[6]), pack_half2(v[3], v[7]));
+    if constexpr (kNarrow) {
+      uint4 w;
+      w.x = pack_qt2<QT>(v[0] * (1.f / 4096.f), v[1] * (1.f / 4096.f));
+      w.y = pack_qt2<QT>(v[2] * (1.f / 4096.f), v[3] * (1.f / 4096.f));
+      w.z = pack_qt2<QT>(v[4] * (1.f / 4096.f), v[5] * (1.f / 4096.f));
+      w.w = pack_qt2<QT>(v[6] * (1.f / 4096.f), v[7] * (1.f / 4096.f));
+      *(uint4*)(q16 + g * kQRow + c0) = w;
+    } else {
+      float* const dst = qs + (g * 4 + (c0 >> 5)) * kQChunk + (c0 & 31);
+      *(float4*)dst = make_float4(v[0], v[1], v[2], v[3]);
+      *(float4*)(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
     }
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < 8 * 32; e += kThreads) {
-    const int ks = e >> 5, fr = (e & 31) >> 2, fj = e & 3;
-    const float* src = qs + (fr * 4 + fj) * kQChunk + 8 * (ks >> 1) + 2 * (ks & 1);
-    *(uint2*)(qfrag + e * 8) = make_uint2(pack_half2(src[0], src[4]), pack_half2(src[1], src[5]));
+    if ((threadIdx.x & 15) == 0) qinv[g] = P.scale_log2e * __uint_as_float((unsigned)(127 + ex - 12) << 23);
   }
   __syncthreads();
   const long long n_packed = (long long)n_blocks * spb;
@@ -823,7 +843,18 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   if (pb > pa) {
     const int n_my = (int)(pb - pa);
     int pf_block = (int)(pa / spb), pf_slice = (int)(pa % spb);   // prefetch cursor
-    BlockPtrs pf_ptrs = locate_block<MODE, VK, VG>(P, d_table, d_roles, d_pool, d_pages, d_pool_pages, pf_block, h, d_vroles);
+    auto locate = [&](int b) {
+      return locate_block<MODE, VK, VG>(P, d_table + (long long)b * 6, d_roles, d_pool, MODE == 1 ? d_pages[b] : 0, d_pool_pages, b, h, d_vroles);
+    };
+    BlockPtrs pf_ptrs = {};
+    if (!(FAST && SUB == 1)) pf_ptrs = locate(pf_block);
+    auto page_base = [&](int id) {
+      if (d_pool_pages > 0 && (unsigned)id >= (unsigned)d_pool_pages) {   // as in locate_block
+        atomicOr(P.status, INQ_STATUS_BAD_INDEX);
+        id = 0;
+      }
+      return d_pool + (long long)id * P.page_bytes;
+    };
     int to_issue = n_my, issue_stage = 0;
     int meta_block = -1;        // block whose metadata is staged (or in flight) in wmeta
     int folded_block = -2;      // last block whose weights were derived from wmeta
@@ -853,8 +884,50 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
     // the later ldmatrix reads of eight tokens' chunks fall into distinct banks.
     const unsigned fast_v_dst = VK ? (unsigned)(kStageK + (lane >> 2) * 64 + (((lane & 3) ^ ((lane >> 3) & 3)) << 4))
                                    : (unsigned)(kStageK + (((lane >> 1) * 2 + ((lane & 1) ^ ((lane >> 3) & 1))) << 4));
-    if (FAST) stage_meta(pf_ptrs, wmeta + (pf_block & 1) * 1024, pf_block & 1);   // the first block's metadata rides with its first slice
-    auto issue = [&]() {
+    // Whole-slice path: where the next block lies is asked for one block ahead, its table row by a copy into
+    // slot block % 2 (which lands with the slice requested next) or its page id by a load into a register,
+    // so that a request that enters a block waits for neither.
+    int next_page = 0;
+    auto request_row = [&](int b) {
+      if (MODE == 0) {
+        if (lane < 6) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(wrow + (b & 1) * 8 + lane)), "l"(d_table + (long long)b * 6 + lane));
+      } else {
+        next_page = d_pages[b];
+      }
+    };
+    if (FAST && SUB == 1) {
+      next_page = d_pages[pf_block];
+    } else if (FAST) {
+      stage_meta(pf_ptrs, wmeta + (pf_block & 1) * 1024, pf_block & 1);   // the first block's metadata rides with its first slice
+      if (to_issue > pf_left) request_row(pf_block + 1);
+    }
+    // FAST with 16-token slices (paged layout): where this lane's copies start inside a page
+    const int page_k = h * 1024 + lane * 16, page_v = P.off_vp + h * 512 + lane * 16;
+    const int page_p = (lane < 16 ? P.off_vs : P.off_vo) + h * 64 + (lane & 15) * 4;
+    const int page_s = P.off_ks + h * 512 + lane * 16, page_r = P.off_km + h * 256 + (lane & 15) * 16, page_c = P.off_kp + h * 64 + (lane & 15) * 4;
+    auto issue = [&](bool ahead) {   // ahead: one of the requests before the loop
+      if (FAST && SUB == 1) {
+        if (to_issue > 0) {
+          const unsigned char* const page = page_base(next_page);
+          const unsigned dk = issue_addr + lane * 16, dv = issue_addr + fast_v_dst;
+          const unsigned dm = issue_addr + kMetaOffset;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dm + lane * 16), "l"(page + page_s));
+          if (lane < 16) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dm + 512 + lane * 16), "l"(page + page_r));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dm + 768 + lane * 4), "l"(page + page_c));
+          }
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dk), "l"(page + page_k));
+          asm volatile("cp.async.cg.shared.global [%0+512], [%1+512], 16;" ::"r"(dk), "l"(page + page_k));
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dv), "l"(page + page_v));
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(issue_addr + kStageK + kStageV + lane * 4), "l"(page + page_p));
+          --to_issue;
+          issue_addr += kStageBytes;
+          if (issue_addr == ring_hi) issue_addr = ring_lo;
+          if (to_issue > 0) next_page = d_pages[++pf_block];   // needed by the next request only
+        }
+        cp_async_commit();
+        return;
+      }
       if (FAST) {
         if (to_issue > 0) {
           const unsigned dk = issue_addr + lane * 16, dv = issue_addr + fast_v_dst;
@@ -892,8 +965,12 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
               // the cursor enters a new block: its rows, and its metadata at once into slot block % 2.
               // The cursor runs at most three slices ahead of the slice being consumed and a block has
               // at least two, so the slot's previous block lies behind the consumed one or is the
-              // consumed one, whose fold precedes this request (the copies are issued after it).
-              pf_ptrs = locate_block<MODE, VK, VG>(P, d_table, d_roles, d_pool, d_pages, d_pool_pages, pf_block, h, d_vroles);
+              // consumed one, whose fold precedes this request (see issue_late).
+              // Its row was requested a block ago, at least two requests back, so the wait at the top of this
+              // iteration covered it; the two requests ahead of the loop had no such wait.
+              pf_ptrs = ahead ? locate(pf_block)
+                              : locate_block<MODE, VK, VG>(P, wrow + (pf_block & 1) * 8, d_roles, d_pool, next_page, d_pool_pages, pf_block, h, d_vroles);
+              if (to_issue > spb) request_row(pf_block + 1);
               fk = pf_ptrs.kp + lane * 16; fv = pf_ptrs.vp + lane * 16; fs = pf_ptrs.vs + lane * kParamLane; fo = pf_ptrs.vo + lane * kParamLane;
               stage_meta(pf_ptrs, wmeta + (pf_block & 1) * 1024, pf_block & 1);
             }
@@ -922,13 +999,13 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
         if (++pf_slice == spb) {
           pf_slice = 0;
           ++pf_block;
-          if (to_issue > 0) pf_ptrs = locate_block<MODE, VK, VG>(P, d_table, d_roles, d_pool, d_pages, d_pool_pages, pf_block, h, d_vroles);
+          if (to_issue > 0) pf_ptrs = locate(pf_block);
         }
       }
       cp_async_commit();
     };
 #pragma unroll
-    for (int s = 0; s < kRing - 1; ++s) issue();
+    for (int s = 0; s < kRing - 1; ++s) issue(true);
     // the dense slices of this warp hide behind the DRAM latency of the first packed slices;
     // their contribution is brought into the packed loop's per-row units (powers of two)
     dense_part();
@@ -966,6 +1043,8 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
     const unsigned ww_addr = smem_addr(wW) + lane * 8, sel_addr = smem_addr(wsel) + lane * 8;
     int stage_index = 0;
     unsigned consume_addr = ring_lo;
+    int my_cell = 0;                         // kNarrow: offset of the selection cell this lane wrote last
+    uint2 qsal = make_uint2(0u, 0u);         // kNarrow: B fragment of the salient step of the current block
     // coded values: sums of the current block alone (in subnormal units) and of its probabilities
     float bacc[8][4], l_blk[2] = {0.f, 0.f};
 #pragma unroll
@@ -978,6 +1057,36 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
     const int vk_tok = (lane & 7) + 8 * ((lane >> 3) & 1), vk_sw = (vk_tok >> 1) & 3;
     const unsigned vk_ldsm_a = (unsigned)(vk_tok * 64 + (((lane >> 4) ^ vk_sw) << 4));
     const unsigned vk_ldsm_b = (unsigned)(vk_tok * 64 + ((((lane >> 4) + 2) ^ vk_sw) << 4));
+    // Flush tables of a value block: lane (r, j) derives entries 4j .. 4j+3 of row r
+    auto fold_values = [&]() {
+      const unsigned char* const vmeta = wvmeta + (cur_block & 1) * kValueMeta;
+      const float* const vscale = (const float*)vmeta;
+      const signed char* const vroles = (const signed char*)(vmeta + 512);
+      const float* const vpads = (const float*)(vmeta + 640);
+      const float4 sc4 = *(const float4*)(vscale + 32 * j + 4 * r);
+      const int ro4 = *(const int*)(vroles + 32 * j + 4 * r);
+      const float sc[4] = {sc4.x, sc4.y, sc4.z, sc4.w};
+      float w[4], k[4];
+      int kinds = 0;
+      bool vbad = false;
+#pragma unroll
+      for (int ii = 0; ii < 4; ++ii) {
+        const float unit = (ii & 1) ? 1048576.f : 16777216.f;
+        const int role = (int)(signed char)(ro4 >> (8 * ii));
+        const int idx = -(int)vroles[max(role, 0)] - 2;
+        const bool salient = role >= 0, donor = role < -1 && role >= -17, regular = role == -1;
+        const bool listed = salient && (unsigned)idx < 16u;
+        vbad |= !(listed || donor || regular);
+        const float mean = to_float<QT>(from_float<QT>(vpads[donor ? -role - 2 : 0]));
+        w[ii] = regular ? sc[ii] * unit : listed ? 16.f * sc[ii] * unit : 0.f;
+        k[ii] = regular ? -8.f * sc[ii] : listed ? -128.f * sc[ii] : donor ? mean : 0.f;
+        kinds |= ((listed ? idx : donor ? 14 - role : -1) & 0xff) << (8 * ii);   // donor: 16 + list index
+      }
+      if (vbad) atomicOr(P.status, INQ_STATUS_BAD_INDEX);
+      *(float4*)(wvw + r * 16 + 4 * j) = make_float4(w[0], w[1], w[2], w[3]);
+      *(float4*)(wvk + r * 16 + 4 * j) = make_float4(k[0], k[1], k[2], k[3]);
+      *(int*)(wvkind + r * 16 + 4 * j) = kinds;
+    };
     // End of a block (or of this warp's range): the block's sums enter the running output with the
     // block's per-channel scales.  Entry i of a lane's tables is channel 32 (i / 4) + 4 r + i % 4.
     auto flush_values = [&]() {
@@ -1033,21 +1142,171 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
       // With fewer than three slices per block the next block's metadata can only be staged once
       // this block's fold has released the staging area: there the copies are issued after the
       // fold.  Otherwise they go out first.
-      // FAST: a request that enters a new block also requests that block's metadata, possibly into
-      // the slot of this slice's block, so the fold of this block (it reads that slot) comes first
-      const bool issue_late = FAST ? need_weights : (!kMetaInStage && spb < 3 && need_weights);
-      if (!issue_late) issue();
+      // FAST: a request that enters a new block also requests that block's metadata into slot block % 2.  It
+      // runs two slices ahead, so the slot can be the one this iteration's fold reads only when the warp's
+      // range begins with the last slice of a block of two: in the first iteration the fold comes first
+      const bool issue_late = FAST ? SUB == 2 && it == 0 : (!kMetaInStage && spb < 3 && need_weights);
+      if (!issue_late) issue(false);
 
-      if (need_weights) {
+      float wsum[4] = {0.f, 0.f, 0.f, 0.f}, dsum[4] = {0.f, 0.f, 0.f, 0.f};
+      unsigned ff_it = 0u, qf_it = 0u;   // kDirect: channel weights and query of this block's fragments
+      if (kNarrow && (kDirect || need_weights)) {
+        // ---- fold this block's descriptor, scales and padding into the query: no branches, so that the
+        //      loads of each step are in flight together (the chain of a block is what a 16-token page costs)
+        const unsigned char* const meta = kMetaInStage ? (FAST ? smem + (consume_addr - smem_addr(smem)) : ring + stage_index * kStageBytes) + kMetaOffset
+                                                       : wmeta + (cur_block & 1) * 1024;
+        // the selection cell this lane wrote for the last block
+        if (SAL) *(unsigned short*)(wsel + my_cell) = 0;
+        // this lane owns the four channels c0, c0+1, c0+4, c0+5 (c0 = 8 (lane / 2) + 2 (lane % 2)): exactly the
+        // channels of one B-fragment entry (K step 2 ((lane / 2) % 4) + lane % 2, chunk lane / 8)
+        const int c0 = 8 * (lane >> 1) + 2 * (lane & 1);
+        const signed char* const roles8 = (const signed char*)(meta + 512);
+        const short* const roles16 = (const short*)(meta + 512);
+        const float2 sa = *(const float2*)(meta + c0 * 4), sb = *(const float2*)(meta + c0 * 4 + 16);
+        const float scv[4] = {sa.x, sa.y, sb.x, sb.y};
+        int role[4], partner[4];
+        if (MODE == 0) {
+          const int ra = *(const short*)(roles8 + c0), rb = *(const short*)(roles8 + c0 + 4);
+          role[0] = (int)(signed char)ra; role[1] = ra >> 8; role[2] = (int)(signed char)rb; role[3] = rb >> 8;
+        } else {
+          const int ra = *(const int*)(roles16 + c0), rb = *(const int*)(roles16 + c0 + 4);
+          role[0] = (int)(short)ra; role[1] = ra >> 16; role[2] = (int)(short)rb; role[3] = rb >> 16;
+        }
+        float pad[4] = {0.f, 0.f, 0.f, 0.f};   // padding list entries 2j, 2j+1, 2j+8, 2j+9
+        if (SAL) {
+          const float2 pa2 = *(const float2*)(meta + 768 + 8 * j), pb2 = *(const float2*)(meta + 800 + 8 * j);
+          pad[0] = pa2.x; pad[1] = pa2.y; pad[2] = pb2.x; pad[3] = pb2.y;
+          if (!FAST) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) pad[k] = 2 * j + (k & 1) + 8 * (k >> 1) < n_pad ? pad[k] : 0.f;
+          }
+        }
+        bool bad = false;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const bool wrong = role[i] > 127 || role[i] < -1 - n_pad;
+          bad |= wrong;
+          role[i] = wrong ? -1 : role[i];
+          // a salient channel's role is its donor slot, whose own role tells the index in the lists
+          partner[i] = MODE == 0 ? (int)roles8[max(role[i], 0)] : (int)roles16[max(role[i], 0)];
+        }
+        // the block's scales are brought into [0, 2) by a power of two
+        unsigned top = __float_as_uint(fmaxf(fmaxf(fabsf(scv[0]), fabsf(scv[1])), fmaxf(fabsf(scv[2]), fabsf(scv[3]))));
+        top = __reduce_max_sync(0xffffffffu, top);
+        const int ex_f = max(-60, min(60, (int)(top >> 23) - 127));
+        const float down = __uint_as_float((unsigned)(127 - ex_f) << 23);
+        float fv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          // a regular channel; the odd channel of a byte is its high nibble: 16 times the code as an fp16
+          // subnormal.  Salient channels are rebuilt exactly below, donor slots hold their low nibbles
+          fv[i] = role[i] == -1 ? scv[i] * ((i & 1) ? 0.0625f * down : down) : 0.f;
+          if (SAL) {
+            const bool salient = role[i] >= 0;
+            const int idx = -partner[i] - 2;
+            const bool listed = salient && (unsigned)idx < (unsigned)n_pad;
+            bad |= salient && !listed;
+            // the scale in the units of the score accumulator (see below); the second code of a gather column
+            // carries a factor 1/512
+            wrec[listed ? idx : 16] = make_uint2(__float_as_uint(scv[i] * (down * ((idx & 8) ? 0.125f : (1.f / 4096.f)))),
+                                                 (unsigned)(c0 + (i & 1) + 4 * (i >> 1)) | ((unsigned)role[i] << 8));
+          } else {
+            bad |= role[i] >= 0;
+          }
+        }
+        if (bad) atomicOr(P.status, INQ_STATUS_BAD_INDEX);
+        *(uint2*)(wfrag + ((2 * ((lane >> 1) & 3) + (lane & 1)) * 4 + (lane >> 3)) * 8) =
+            make_uint2(pack_half2(fv[0], fv[2]), pack_half2(fv[1], fv[3]));
+        __syncwarp();
+        if (SAL) {
+          // selection matrix: column (idx & 7) gathers the codes of TWO salient channels into one fp32
+          // accumulator, code' = 16 * (high nibble of the source) + (low nibble in the donor slot) of
+          // salient idx with weight 2^-13 when idx & 8 is clear and with weight 2^-22 when it is set;
+          // every entry and every partial sum is exact.  One cell per lane: the source (even lane) or the
+          // donor slot (odd lane) of salient lane / 2.
+          {
+            const unsigned m = wrec[lane >> 1].y;
+            const int idx = lane >> 1, which = lane & 1;
+            const int c = (which ? m >> 8 : m) & 127;
+            const int jj = c >> 5, u = c & 31;
+            const int ks = 2 * (u >> 3) + ((u >> 1) & 1), half = u & 1, e = (u >> 2) & 1;
+            // fp16 bits of 32768 (source), 2048 (donor), each divided by 16 for the high nibble of a
+            // byte and by 512 for the second salient channel of the column
+            if (FAST || idx < n_pad) {
+              my_cell = (ks * 32 + (((idx & 7) << 2) | jj)) * 8 + half * 4 + e * 2;
+              *(unsigned short*)(wsel + my_cell) = (unsigned short)(0x7800 - (which + half) * 0x1000 - ((idx >> 3) & 1) * 0x2400);
+            }
+          }
+          // B fragments of the salient step (query at the salient channels) and of the donors' step (query at
+          // the donor slots): entries 2j, 2j+1 | 2j+8, 2j+9 of head r.  The salient step adds straight into the
+          // score accumulator, whose unit is alpha = qinv * 2^(24 + ex_f): the staged query times 2^-12 and
+          // the salient value times 2^-(12 + ex_f) give exactly that unit, and both factors are powers of
+          // two, so the rounding to the model dtype is the reference's
+          const uint4 ra = *(const uint4*)(wrec + 2 * j), rb = *(const uint4*)(wrec + 2 * j + 8);
+          const unsigned short* const qrow = (const unsigned short*)(q16 + r * kQRow);
+          const unsigned m4[4] = {ra.y, ra.w, rb.y, rb.w};
+          unsigned qa[4], qd[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            qa[k] = qrow[m4[k] & 127];
+            qd[k] = qrow[(m4[k] >> 8) & 127];
+          }
+          qsal = make_uint2(__byte_perm(qa[0], qa[1], 0x5410u), __byte_perm(qa[2], qa[3], 0x5410u));
+          // the donors' constant values (the reference stores the sampled mean as the donor channel's own
+          // value and rounds it to the model dtype) times the query, the same in all 16 rows
+          const unsigned p_lo = pack_qt2<QT>(pad[0], pad[1]), p_hi = pack_qt2<QT>(pad[2], pad[3]);
+          mma_qt<QT>(dsum, p_lo, p_lo, p_hi, p_hi, __byte_perm(qd[0], qd[1], 0x5410u), __byte_perm(qd[2], qd[3], 0x5410u));
+        }
+        // The B fragments of the eight K steps are the staged query (fp16 pairs in fragment order) times the
+        // block's channel weights, one HMUL2 per register; the same fragments against an A operand of ones
+        // (1 for a low nibble, 16 for a high one) give the sum of the weights per query head, i.e. the
+        // contribution of the codes' zero point 8.
+        qf_it = launder(smem_addr(qfrag) + lane * 8);
+        ff_it = launder(smem_addr(wfrag) + j * 8);
+        if (!kDirect) {
+          float wsum2[4] = {0.f, 0.f, 0.f, 0.f};   // two chains
+#define INQ_FOLD(KS, SUM)                                                                                  \
+  {                                                                                                        \
+    const uint2 qq = lds64<(KS) * 256>(qf_it), ff2 = lds64<(KS) * 32>(ff_it);                              \
+    const uint2 ww = make_uint2(hmul2_bits(qq.x, ff2.x), hmul2_bits(qq.y, ff2.y));                         \
+    *(uint2*)(wW + ((KS) * 32 + lane) * 8) = ww;                                                           \
+    mma_f16(SUM, 0x00010001u, 0x00010001u, 0x00100010u, 0x00100010u, ww.x, ww.y);                          \
+  }
+          INQ_FOLD(0, wsum) INQ_FOLD(1, wsum2) INQ_FOLD(2, wsum) INQ_FOLD(3, wsum2)
+          INQ_FOLD(4, wsum) INQ_FOLD(5, wsum2) INQ_FOLD(6, wsum) INQ_FOLD(7, wsum2)
+#undef INQ_FOLD
+          wsum[0] += wsum2[0];
+          wsum[1] += wsum2[1];
+        }
+        // raw score -> base-2 score: undo 2^-24 (subnormal nibbles), the scale exponent and the query
+        // factor; score columns of this thread are query heads 2j and 2j+1
+        {
+          const float2 qf = *(const float2*)(qinv + 2 * j);
+          const float up = __uint_as_float((unsigned)(127 + 24 + ex_f) << 23);
+          alpha[0] = qf.x * up;
+          alpha[1] = qf.y * up;
+          dsum[0] *= qf.x * 4096.f;
+          dsum[1] *= qf.y * 4096.f;
+        }
+        if (!kDirect) {
+          beta[0] = fmaf(-8.f * alpha[0], wsum[0], dsum[0]);
+          beta[1] = fmaf(-8.f * alpha[1], wsum[1], dsum[1]);
+          bm[0] = beta[0] - m_run[0];
+          bm[1] = beta[1] - m_run[1];
+        }
+        if (VK == 1) fold_values();
+        need_weights = false;
+        __syncwarp();   // the selection cells
+        if (issue_late) issue(false);
+      }
+      if (!kNarrow && need_weights) {
         // ---- fold this block's descriptor, scales and padding into the query
         unsigned char* meta = wmeta;
-        if (FAST) {
-          meta = wmeta + (cur_block & 1) * 1024;
-        } else if (kMetaInStage) {
+        if (kMetaInStage) {
           meta = ring + stage_index * kStageBytes + kMetaOffset;
         } else if (meta_block != cur_block) {
           // not prefetched (very short blocks): fetch now and wait for it alone
-          BlockPtrs cb = locate_block<MODE, VK, VG>(P, d_table, d_roles, d_pool, d_pages, d_pool_pages, cur_block, h, d_vroles);
+          BlockPtrs cb = locate(cur_block);
           __syncwarp();
           stage_meta(cb, wmeta);
           cp_async_commit();
@@ -1180,7 +1439,6 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
         // order) times the block's channel weights, one HMUL2 per register; the same fragments
         // against an A operand of ones (1 for a low nibble, 16 for a high one) give the sum of the
         // weights per query head, i.e. the contribution of the codes' zero point 8
-        float wsum[4] = {0.f, 0.f, 0.f, 0.f};
         {
           const unsigned qf_addr = launder(smem_addr(qfrag) + lane * 8), ff_addr = launder(smem_addr(wfrag) + j * 8);
 #define INQ_FOLD(KS)                                                                                       \
@@ -1205,54 +1463,15 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
         }
         bm[0] = beta[0] - m_run[0];
         bm[1] = beta[1] - m_run[1];
-        if (VK == 1) {
-          // flush tables of the value block: lane (r, j) derives entries 4j .. 4j+3 of row r
-          const unsigned char* const vmeta = wvmeta + (cur_block & 1) * kValueMeta;
-          const float* const vscale = (const float*)vmeta;
-          const signed char* const vroles = (const signed char*)(vmeta + 512);
-          const float* const vpads = (const float*)(vmeta + 640);
-          bool vbad = false;
-#pragma unroll
-          for (int ii = 0; ii < 4; ++ii) {
-            const int c = 32 * j + 4 * r + ii;
-            const float sc = vscale[c];
-            const float unit = (ii & 1) ? 1048576.f : 16777216.f;
-            int role = vroles[c];
-            float w = sc * unit, k = -8.f * sc;
-            int kind = -1;
-            if (role > 127 || role < -17) {
-              vbad = true;
-              w = 0.f; k = 0.f;
-            } else if (role >= 0) {
-              const int idx = -(int)vroles[role] - 2;
-              if (idx >= 0 && idx < 16) {
-                kind = idx;
-                w = 16.f * sc * unit;
-                k = -128.f * sc;
-              } else {
-                vbad = true;
-                w = 0.f; k = 0.f;
-              }
-            } else if (role < -1) {
-              kind = 16 + (-role - 2);
-              w = 0.f;
-              k = to_float<QT>(from_float<QT>(vpads[-role - 2]));
-            }
-            wvw[r * 16 + 4 * j + ii] = w;
-            wvk[r * 16 + 4 * j + ii] = k;
-            wvkind[r * 16 + 4 * j + ii] = (signed char)kind;
-          }
-          if (vbad) atomicOr(P.status, INQ_STATUS_BAD_INDEX);
-        }
         need_weights = false;
         if (issue_late) {
           __syncwarp();   // every lane has read the per-channel terms: the staging area is free
-          issue();
+          issue(false);
         }
       }
 
       const unsigned stage = launder(FAST ? consume_addr : ring_addr + stage_index * kStageBytes);
-      const unsigned ww_it = launder(ww_addr), sel_it = launder(sel_addr);
+      const unsigned ww_it = launder(ww_addr), sel_it = launder(sel_addr), rec_it = launder(smem_addr(wrec) + 16 * j);
       if (FAST) {
         consume_addr += kStageBytes;
         if (consume_addr == ring_hi) consume_addr = ring_lo;
@@ -1280,19 +1499,30 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
       else mma_f16(C[U], a0, a1, a2, a3, F.x, F.y);                                                       \
     }                                                                                                     \
   }
+#define INQ_WEIGHTS(KS, WQ)                                                                               \
+  {                                                                                                       \
+    if (kDirect) {                                                                                        \
+      const uint2 qq = lds64<(KS) * 256>(qf_it), ff2 = lds64<(KS) * 32>(ff_it);                           \
+      WQ = make_uint2(hmul2_bits(qq.x, ff2.x), hmul2_bits(qq.y, ff2.y));                                  \
+    } else {                                                                                              \
+      WQ = lds64<(KS) * 256>(ww_it);                                                                      \
+    }                                                                                                     \
+  }
 #define INQ_KSTEP(KS, M, SH, FIRST, WQ, F, WQN, FN)                                                       \
   {                                                                                                       \
     if ((KS) < 7) {                                                                                       \
-      WQN = lds64<(((KS) + 1) & 7) * 256>(ww_it);                                                         \
+      INQ_WEIGHTS(((KS) + 1) & 7, WQN)                                                                    \
       if (SAL) FN = lds64<(((KS) + 1) & 7) * 256>(sel_it);                                                \
     }                                                                                                     \
+    if (kDirect) mma_f16(wsum, 0x00010001u, 0x00010001u, 0x00100010u, 0x00100010u, WQ.x, WQ.y);           \
     INQ_KMMA(0, kx0.M >> SH, ky0.M >> SH, FIRST, WQ, F)                                                   \
     if (kSub > 1) INQ_KMMA(kSub - 1, kx1.M >> SH, ky1.M >> SH, FIRST, WQ, F)                              \
   }
         {
           const uint4 kx0 = lds128<0>(stage + lane16), ky0 = lds128<512>(stage + lane16);
           const uint4 kx1 = lds128<(kSub > 1 ? 1024 : 0)>(stage + lane16), ky1 = lds128<(kSub > 1 ? 1536 : 512)>(stage + lane16);
-          uint2 wa = lds64<0>(ww_it), wb_;
+          uint2 wa, wb_;
+          INQ_WEIGHTS(0, wa)
           uint2 fa = make_uint2(0u, 0u), fb = fa;
           if (SAL) fa = lds64<0>(sel_it);
           INQ_KSTEP(0, x, 0, true, wa, fa, wb_, fb)
@@ -1306,9 +1536,10 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
         }
 #undef INQ_KMMA
 #undef INQ_KSTEP
+#undef INQ_WEIGHTS
         if (SAL) {
-          for (int gsel = 0; gsel < groups; ++gsel) {
-            if (gsel) {
+          for (int gsel = 0; gsel < (kNarrow ? 1 : groups); ++gsel) {
+            if (!kNarrow && gsel) {
               // further groups of 16 salient channels (salient fractions above 1/8)
               const uint4 k0 = lds128<0>(stage + lane16), k1 = lds128<512>(stage + lane16);
               const uint4 k2 = lds128<(kSub > 1 ? 1024 : 0)>(stage + lane16), k3 = lds128<(kSub > 1 ? 1536 : 512)>(stage + lane16);
@@ -1336,9 +1567,18 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
             // dequantised tensor holds it.  The two codes of an accumulator are separated exactly:
             // adding 1.5 * 2^23 rounds to the integer part (the fraction stays within 1/4), the rest
             // is the second code over 512.
-            const float2 sc0 = *(const float2*)(wssc + gsel * 16 + 2 * j);
-            const float2 sc1 = *(const float2*)(wssc + gsel * 16 + 8 + 2 * j);
-            const uint2 qb = *(const uint2*)(wqsal + (gsel * 32 + lane) * 8);
+            float2 sc0, sc1;
+            uint2 qb;
+            if constexpr (kNarrow) {
+              const uint4 ra = lds128<0>(rec_it), rb = lds128<64>(rec_it);
+              sc0 = make_float2(__uint_as_float(ra.x), __uint_as_float(ra.z));
+              sc1 = make_float2(__uint_as_float(rb.x), __uint_as_float(rb.z));
+              qb = qsal;
+            } else {
+              sc0 = *(const float2*)(wssc + gsel * 16 + 2 * j);
+              sc1 = *(const float2*)(wssc + gsel * 16 + 8 + 2 * j);
+              qb = *(const uint2*)(wqsal + (gsel * 32 + lane) * 8);
+            }
 #pragma unroll
             for (int u = 0; u < kSub; ++u) {
               float hi[4], lo[4];
@@ -1355,6 +1595,12 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
             }
           }
         }
+      }
+      if (kDirect) {
+        beta[0] = fmaf(-8.f * alpha[0], wsum[0], dsum[0]);
+        beta[1] = fmaf(-8.f * alpha[1], wsum[1], dsum[1]);
+        bm[0] = beta[0] - m_run[0];
+        bm[1] = beta[1] - m_run[1];
       }
       // s2[u][k]: sub-slice u; k = 0,1 -> token r (+16u), heads 2j, 2j+1; k = 2,3 -> token r+8 (+16u)
       float s2[2][4];
@@ -1866,7 +2112,7 @@ using namespace inq;
 // device, not to the process: a process that drives several GPUs (or several host threads) gets
 // one record per device ordinal, filled under a mutex on first use.
 constexpr int kMaxDevices = 64;
-constexpr int kKernelVariants = 36;   // 16 general, 4 whole-slice, 2 coded values, 6 4-bit values, 4 2-bit values in one or four groups, 4 of 16-token slices with more than 16 salient channels
+constexpr int kKernelVariants = 38;   // 16 general, 4 whole-slice, 2 coded values, 6 4-bit values, 4 2-bit values in one or four groups, 4 of 16-token slices with more than 16 salient channels, 2 of whole 16-token pages
 struct DeviceState {
   int sm_count = 0;
   bool raised[kKernelVariants] = {};
@@ -2026,7 +2272,9 @@ extern "C" int inq_decode_attention(const inq_decode_args_t* a, inq_stream_t str
       decode_kernel<0, __half, true, 2, true, 0, 4>, decode_kernel<0, __nv_bfloat16, true, 2, true, 0, 4>,
       // 16-token slices with more than 16 salient channels
       decode_kernel<0, __half, true, 1, false, 0, 2, true>, decode_kernel<0, __nv_bfloat16, true, 1, false, 0, 2, true>,
-      decode_kernel<1, __half, true, 1, false, 0, 2, true>, decode_kernel<1, __nv_bfloat16, true, 1, false, 0, 2, true>};
+      decode_kernel<1, __half, true, 1, false, 0, 2, true>, decode_kernel<1, __nv_bfloat16, true, 1, false, 0, 2, true>,
+      // pages of exactly 16 tokens, 16 salient channels
+      decode_kernel<1, __half, true, 1, true>, decode_kernel<1, __nv_bfloat16, true, 1, true>};
   const bool fast = a->n_pad == 16 && a->block_tokens % 32 == 0 && a->block_tokens >= 64;
   const int vk = a->value_kind, vg = a->value_groups;
   if (vk < 0 || vk > 2 || (vk == 2 && vg != 1 && vg != 2 && vg != 4) || (vk == 0 && vg != 0 && vg != 1 && vg != 2 && vg != 4))
@@ -2042,6 +2290,7 @@ extern "C" int inq_decode_attention(const inq_decode_args_t* a, inq_stream_t str
                   : vk == 2 ? 22 + (vg == 1 ? 0 : vg == 2 ? 2 : 4) + (a->dtype == INQ_F16 ? 0 : 1)
                   : vk ? 20 + (a->dtype == INQ_F16 ? 0 : 1)
                   : fast ? 16 + a->layout * 2 + (a->dtype == INQ_F16 ? 0 : 1)
+                  : a->n_pad == 16 && a->block_tokens == 16 && a->layout == 1 ? 36 + (a->dtype == INQ_F16 ? 0 : 1)
                   : sub == 1 && groups > 1 ? 32 + a->layout * 2 + (a->dtype == INQ_F16 ? 0 : 1)
                          : (sub == 1 ? 8 : 0) + a->layout * 4 + (a->dtype == INQ_F16 ? 0 : 2) + (groups > 0 ? 1 : 0);
   const kernel_t kernel = kernels[which];

@@ -177,3 +177,36 @@ def test_out_of_range_page_ids_are_skipped_and_reported():
     assert torch.isfinite(out.float()).all()
     assert N.take_status(torch.device("cuda", 0), N.STATUS_BAD_INDEX) == N.STATUS_BAD_INDEX
     assert N.take_status(torch.device("cuda", 0)) == 0
+
+
+@pytest.mark.parametrize("block,pages", [(16, 1), (16, 2), (16, 3), (16, 4), (16, 61), (64, 1), (64, 2), (64, 3), (64, 9), (256, 3)])
+def test_pages_asked_for_ahead(block, pages):
+    """Every page count around the depth of the ring and of the page ids read ahead, against the oracle; an id
+    outside the pool at any place is page 0 in its stead, bit for bit, and is reported."""
+    from inquant import _native as N
+    from inquant.triton_attention import SharedDecodeWorkspace
+    from inquant_vllm.kernels import paged_decode
+    from inquant_vllm.layout import PageLayout, pack_pages
+    heads, q_heads = 2, 14
+    layout, workspace = PageLayout(block, heads), SharedDecodeWorkspace()
+    kt, vt = _pages_input(block + pages, heads, pages, block)
+    pool = torch.cat((torch.zeros((1, layout.page_bytes), dtype=torch.uint8, device="cuda"),
+                      pack_pages(to_device(kt), to_device(vt), layout).view(pages, -1).flip(0)))
+    pool[0] = pool[pages]
+    ids = torch.arange(pages, 0, -1, device="cuda", dtype=torch.int32)
+    dense = torch.zeros((2, heads, block + 4, 128), dtype=torch.bfloat16, device="cuda")
+    q32 = workloads.make_query(9, q_heads)
+    q = to_device(q32).view(1, q_heads, 128)
+
+    def decode(table):
+        return paged_decode(q, pool, table, dense, pages, 0, 0, layout, workspace, 128 ** -0.5).clone()
+    kr, vr = oracle.unpack_pages(oracle.pack_pages(kt, vt, block, heads), block, heads)
+    expected = oracle.attention_decode(q32, *(x.transpose(1, 0, 2, 3).reshape(heads, -1, 128) for x in (kr, vr)), 128 ** -0.5)
+    attention_close(to_numpy(decode(ids).float()).reshape(q_heads, 128), expected)
+    for place in sorted({0, 1, 2, pages // 2, pages - 1} & set(range(pages))):
+        outside, inside = ids.clone(), ids.clone()
+        outside[place], inside[place] = pages + 1 + place, 0
+        good = decode(inside)
+        assert N.take_status(torch.device("cuda", 0), N.STATUS_BAD_INDEX) == 0
+        assert torch.equal(decode(outside), good)
+        assert N.take_status(torch.device("cuda", 0), N.STATUS_BAD_INDEX) == N.STATUS_BAD_INDEX
