@@ -479,6 +479,33 @@ typedef struct {
 } inq_seal_args_t;
 int inq_seal_blocks(const inq_seal_args_t* args /* host */, int32_t* status, inq_stream_t stream);
 
+/* ---------------------------------------------------------------- a layer's dense history in one call
+ * Dequantises runs of sealed blocks (a run: the [n_blocks, heads, ...] output arena of one encoder
+ * launch, or one block) one behind the other into `out_key` / `out_value` from token `position` on,
+ * and copies up to six dense row ranges (sink, tail, new states; as in inq_seal_blocks, rows of 256
+ * bytes), in one launch for up to eight runs.  128 channels, 16-bit output with a token stride of 128
+ * elements and the head stride given (elements, a multiple of 8), descriptors of 8 bits, at most 64
+ * salient channels.  Sources and destinations must not overlap.  All arguments are checked before the
+ * first launch.
+ * Replaces: cache.py:328-345 (materialize: one dequantize per block, cat) and the cat of cache.py:190. */
+typedef struct {
+  const void* key_payload; const void* key_scales;          /* u8 [n, heads, tokens, 64] (4-byte aligned), f32 [n, heads, 128] */
+  const void* key_salient; const void* key_donors; const void* key_padding;   /* u8, u8, f32 [n, heads, count] */
+  const void* value_payload; const void* value_scales;      /* value_kind 1: as the key's */
+  const void* value_offsets;                                /* value_kind 0: f16 [n, heads, tokens, 128 / group], like the scales */
+  const void* value_salient; const void* value_donors; const void* value_padding;   /* value_kind 1: [n, heads, value_count] */
+  int64_t n_blocks;
+} inq_restore_run_t;
+typedef struct {
+  const inq_restore_run_t* runs /* host */; int32_t n_runs;
+  int32_t heads, block_tokens, count;
+  int32_t value_kind;                                       /* 0: affine codes of value_bits, 1: coded like the keys */
+  int32_t value_bits, value_group, value_count;
+  void* out_key; void* out_value; int64_t stride_h, position;
+  inq_row_copy_t copies[6]; int32_t n_copies, out_dtype;
+} inq_restore_args_t;
+int inq_restore_history(const inq_restore_args_t* args /* host */, inq_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

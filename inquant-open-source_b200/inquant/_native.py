@@ -107,6 +107,19 @@ class SealArgs(ctypes.Structure):
                 ("n_copies", c_int32), ("heads", c_int32), ("row_bytes", c_int32), ("reserved", c_int32)]
 
 
+class RestoreRun(ctypes.Structure):
+    _fields_ = [("key_payload", c_void_p), ("key_scales", c_void_p), ("key_salient", c_void_p), ("key_donors", c_void_p),
+                ("key_padding", c_void_p), ("value_payload", c_void_p), ("value_scales", c_void_p), ("value_offsets", c_void_p),
+                ("value_salient", c_void_p), ("value_donors", c_void_p), ("value_padding", c_void_p), ("n_blocks", c_int64)]
+
+
+class RestoreArgs(ctypes.Structure):
+    _fields_ = [("runs", c_void_p), ("n_runs", c_int32), ("heads", c_int32), ("block_tokens", c_int32), ("count", c_int32),
+                ("value_kind", c_int32), ("value_bits", c_int32), ("value_group", c_int32), ("value_count", c_int32),
+                ("out_key", c_void_p), ("out_value", c_void_p), ("stride_h", c_int64), ("position", c_int64),
+                ("copies", RowCopy * 6), ("n_copies", c_int32), ("out_dtype", c_int32)]
+
+
 class GenericDecodeArgs(ctypes.Structure):
     _fields_ = [("q", c_void_p), ("out", c_void_p), ("q_stride_h", c_int64), ("table", c_void_p),
                 ("key_roles", c_void_p), ("value_roles", c_void_p),
@@ -182,7 +195,7 @@ EXPORTS = (
     "inq_last_error", "inq_version", "inq_k4_encode", "inq_select_donors", "inq_k4_statistics",
     "inq_k4_dequantize", "inq_k4_dequantize_strided", "inq_v_encode", "inq_v_dequantize", "inq_v_dequantize_strided",
     "inq_build_roles", "inq_write_codec_pages",
-    "inq_decode_attention", "inq_decode_attention_noalloc", "inq_decode_units", "inq_merge_partials", "inq_decode_workspace_floats", "inq_decode_launch_shape", "inq_append_token", "inq_append_token_batch", "inq_seal_blocks",
+    "inq_decode_attention", "inq_decode_attention_noalloc", "inq_decode_units", "inq_merge_partials", "inq_decode_workspace_floats", "inq_decode_launch_shape", "inq_append_token", "inq_append_token_batch", "inq_seal_blocks", "inq_restore_history",
     "inq_prefill_attention", "inq_decode_generic", "inq_decode_generic_workspace_floats",
     "inq_prefill_workspace_bytes",
     "inq_exchange_merge", "inq_exchange_inbox_bytes", "inq_decode_exchange_inbox_bytes", "inq_restore_blocks_table", "inq_peer_buffer_create", "inq_peer_buffer_open",
@@ -217,6 +230,7 @@ SIGNATURES = {
     "inq_append_token": [_P, _P],
     "inq_append_token_batch": [_P, _I, _P, _P],
     "inq_seal_blocks": [_P, _P, _P],
+    "inq_restore_history": [_P, _P],
 }
 
 

@@ -86,6 +86,18 @@ class _Layer:
     append_args: tuple | None = None                # launch structure of the one-token append, per tail buffer pair
 
     sink_views: tuple | None = None                 # (count, key view, value view) handed out last
+    runs: list = field(default_factory=list)        # what sealed the blocks: (last block, keys' owner, values' owner, blocks)
+
+    def block_runs(self):
+        """The sealed blocks as runs of one encoder launch each, ``(keys' owner, values' owner, blocks)``:
+        an owner is the arena of such a launch, or a block of its own.  None when the lists no longer are
+        what the seals appended."""
+        end = 0
+        for last, _, _, count in self.runs:
+            end += count
+            if end > len(self.key_blocks) or self.key_blocks[end - 1] is not last:
+                return None
+        return self.runs if end == len(self.key_blocks) == len(self.value_blocks) else None
 
     def _sink_pair(self):
         """The sink views for the current count: the same two tensor objects until the count changes
@@ -193,6 +205,87 @@ def _dequantize_arena_into(arena, out: torch.Tensor, position: int) -> bool:
     return True
 
 
+def _row_copy(entry, source: torch.Tensor, first: int, target: torch.Tensor, start: int, tokens: int) -> None:
+    """Fill one ``inq_row_copy_t``: ``tokens`` rows of ``source`` [1, H, tokens, C] from ``first`` on to ``target`` from ``start`` on."""
+    _, source_h, source_t, _ = source.stride()
+    _, target_h, target_t, _ = target.stride()
+    size = source.element_size()
+    entry.src = source.data_ptr() + first * source_t * size
+    entry.dst = target.data_ptr() + start * target_t * size
+    entry.src_stride_h, entry.src_stride_t = source_h * size, source_t * size
+    entry.dst_stride_h, entry.dst_stride_t = target_h * size, target_t * size
+    entry.tokens = tokens
+
+
+def restore_history(layer: _Layer, out_key: torch.Tensor, out_value: torch.Tensor, new_key=None, new_value=None) -> bool:
+    """The layer's whole history -- sink, sealed blocks, tail -- into ``out_key`` / ``out_value`` [1, H, tokens, 128]
+    from token 0 on, and the rows of ``new_key`` / ``new_value`` behind it, by one launch for up to eight runs of
+    blocks (C ABI ``inq_restore_history``).  False, with nothing launched, when that launch does not serve the
+    layouts."""
+    from .value_codec import PackedValues
+    _, heads, _, channels = layer.shape
+    dtype = layer.dtype
+    if channels != 128 or dtype not in (torch.float16, torch.bfloat16) or out_key.dtype != dtype or out_value.dtype != dtype:
+        return False
+    strides = out_key.stride()
+    if strides[3] != 1 or strides[2] != channels or strides[1] % 8 or out_value.stride() != strides \
+            or out_key.data_ptr() % 16 or out_value.data_ptr() % 16:
+        return False
+    dense = [t for t in (layer.sink_key, layer.sink_value, layer.residual_key, layer.residual_value, new_key, new_value) if t is not None]
+    for tensor in dense:
+        if tensor.dtype != dtype or tensor.stride(3) != 1 or not N.dense_rows_aligned(tensor):
+            return False
+    runs = layer.block_runs()
+    if runs is None:
+        return False
+    args = N.RestoreArgs()
+    args.heads, args.out_dtype = heads, N.DTYPE_CODE[dtype]
+    args.out_key, args.out_value, args.stride_h = out_key.data_ptr(), out_value.data_ptr(), strides[1]
+    args.position = layer.sink_count
+    position = layer.sink_count
+    if runs:
+        first_key, first_value = runs[0][1], runs[0][2]
+        block_tokens, count = first_key.shape[2], first_key.salient_channels.shape[-1]
+        coded = not isinstance(first_value, PackedValues)
+        args.block_tokens, args.count = block_tokens, count
+        if coded:
+            args.value_kind, args.value_count = 1, first_value.salient_channels.shape[-1]
+        else:
+            args.value_bits, args.value_group = first_value.bits, first_value.group_size
+        if count > 64 or (coded and args.value_count > 64):
+            return False
+        records = (N.RestoreRun * len(runs))()
+        for record, (_, keys, values, blocks) in zip(records, runs):
+            fields = [keys.payload, keys.scales, keys.salient_channels, keys.donor_channels, keys.padding, values.payload, values.scales]
+            names = ["key_payload", "key_scales", "key_salient", "key_donors", "key_padding", "value_payload", "value_scales"]
+            if coded:
+                fields += [values.salient_channels, values.donor_channels, values.padding]
+                names += ["value_salient", "value_donors", "value_padding"]
+            else:
+                fields.append(values.offsets)
+                names.append("value_offsets")
+            for name, tensor in zip(names, fields):
+                if not tensor.is_contiguous() or tensor.dtype == torch.int32:
+                    return False
+                setattr(record, name, tensor.data_ptr() or None)
+            record.n_blocks = blocks
+            position += blocks * block_tokens
+        args.runs, args.n_runs = N.ctypes.cast(records, N.c_void_p), len(runs)
+    copies = []
+    if layer.sink_count:
+        copies += [(layer.sink_key, out_key, 0, layer.sink_count), (layer.sink_value, out_value, 0, layer.sink_count)]
+    if layer.tail_count:
+        copies += [(layer.residual_key, out_key, position, layer.tail_count), (layer.residual_value, out_value, position, layer.tail_count)]
+    if new_key is not None:
+        position += layer.tail_count
+        copies += [(new_key, out_key, position, new_key.shape[2]), (new_value, out_value, position, new_key.shape[2])]
+    for entry, (source, target, start, tokens) in zip(args.copies, copies):
+        _row_copy(entry, source, 0, target, start, tokens)
+    args.n_copies = len(copies)
+    N.check(N.library().inq_restore_history(N.ctypes.byref(args), N.stream_pointer(out_key.device)), "inq_restore_history")
+    return True
+
+
 def restore_blocks(blocks, out: torch.Tensor, position: int) -> int:
     """Dequantise ``blocks`` into ``out`` [1, H, tokens, C] from token ``position`` on; returns the
     position after the last block.  Blocks sealed by one call share an encoder arena: each arena is
@@ -292,14 +385,14 @@ class InQuantCache(_HFCache):
         """Reference ``cache.py:179-200``: a fresh prefill returns its inputs unchanged; later
         calls return dequantised history followed by the new states, then seal."""
         layer = self._validate_update(key_states, value_states, layer_idx, cache_kwargs)
+        history = None
         if layer is None:
             layer = _Layer(tuple(key_states.shape), key_states.dtype, key_states.device)
             full_key, full_value = key_states, value_states
         else:
-            old_key, old_value = self.materialize(layer_idx)
-            full_key = torch.cat((old_key, key_states), dim=2)
-            full_value = torch.cat((old_value, value_states), dim=2)
-        self._append(layer, key_states, value_states)
+            full_key, full_value = self._history(layer, key_states, value_states)
+            history = full_key, full_value
+        self._append(layer, key_states, value_states, history=history)
         self._layers[layer_idx] = layer
         self.record_peak(layer_idx)
         if layer_idx == 0:
@@ -310,12 +403,17 @@ class InQuantCache(_HFCache):
     def extend(self, key_states, value_states, layer_idx, cache_kwargs=None) -> None:
         """``update`` without its return value: the new states are appended and full blocks sealed
         exactly as ``update`` does (reference ``cache.py:179-200``), but the dense history is
-        neither built nor returned.  Not in the reference; used by ``inquant.prefill``, which keeps
-        its own dense history across the chunks of a prompt."""
+        neither built nor returned.  Not in the reference; used by ``inquant.prefill``, which builds
+        the dense history itself."""
+        self._extend(key_states, value_states, layer_idx, cache_kwargs)
+
+    def _extend(self, key_states, value_states, layer_idx, cache_kwargs, history=None) -> None:
+        """``history``: the dense pair [1, H, tokens, C] that the caller has built and that ends with the new
+        states; the rows to seal are then read from it instead of being put together again."""
         layer = self._validate_update(key_states, value_states, layer_idx, cache_kwargs)
         if layer is None:
             layer = _Layer(tuple(key_states.shape), key_states.dtype, key_states.device)
-        self._append(layer, key_states, value_states)
+        self._append(layer, key_states, value_states, history=history)
         self._layers[layer_idx] = layer
         self.record_peak(layer_idx)
         if layer_idx == 0:
@@ -460,14 +558,7 @@ class InQuantCache(_HFCache):
         for source, first, target, start, count in copies():
             if not count:
                 continue
-            entry = seal.copies[n]
-            _, source_h, source_t, _ = source.stride()
-            _, target_h, target_t, _ = target.stride()
-            entry.src = source.data_ptr() + first * source_t * 2
-            entry.dst = target.data_ptr() + start * target_t * 2
-            entry.src_stride_h, entry.src_stride_t = source_h * 2, source_t * 2
-            entry.dst_stride_h, entry.dst_stride_t = target_h * 2, target_t * 2
-            entry.tokens = count
+            _row_copy(seal.copies[n], source, first, target, start, count)
             n += 1
         seal.n_copies = n
         if cfg.value_bits is None:
@@ -529,9 +620,10 @@ class InQuantCache(_HFCache):
         N.check(N.library().inq_append_token(cached[3], N.stream_pointer(layer.device)), "inq_append_token")
         return True
 
-    def _append(self, layer: _Layer, keys, values, want_tail: bool = False):
+    def _append(self, layer: _Layer, keys, values, want_tail: bool = False, history=None):
         """Reference ``cache.py:271-306``.  Returns the (old tail + new tokens) pair when
-        ``want_tail`` is set."""
+        ``want_tail`` is set.  ``history`` is the layer's dense key and value history that ends with the
+        new tokens, where the caller has built it."""
         cfg = self.config
         new_tokens = keys.shape[2]
         take_sink = min(cfg.sink_tokens - layer.sink_count, new_tokens)
@@ -574,6 +666,10 @@ class InQuantCache(_HFCache):
         elif want_tail:
             tail = ((keys, values) if not layer.tail_count else
                     (torch.cat((layer.residual_key, keys), dim=2), torch.cat((layer.residual_value, values), dim=2)))
+        if pending_key is None and history is not None:
+            # tail and new tokens lie side by side at the end of the history
+            first = history[0].shape[2] - pending_count
+            pending_key, pending_value = history[0][:, :, first:], history[1][:, :, first:]
         if pending_key is None:
             pending_key, pending_value = keys[:, :, take_sink:], values[:, :, take_sink:]
             if layer.tail_count:
@@ -643,10 +739,20 @@ class InQuantCache(_HFCache):
         layer.tail_key_buffer, layer.tail_value_buffer, layer.tail_count = tail_key_buffer, tail_value_buffer, remainder
         layer.key_blocks.extend(new_keys)
         layer.value_blocks.extend(new_values)
+        if blocks:
+            self._record_run(layer, new_keys, new_values)
         if cfg.track_peak_bytes:
             layer.packed_nbytes += sum(block.nbytes for block in new_keys + new_values)
         layer.seq_length += new_tokens
         return tail
+
+    @staticmethod
+    def _record_run(layer: _Layer, new_keys, new_values) -> None:
+        owners = [getattr(new[0], "_arena", (new[0], 0))[0] for new in (new_keys, new_values)]
+        if len(new_keys) == len(new_values) and all(owner.shape[0] == len(new_keys) for owner in owners):
+            layer.runs.append((new_keys[-1], *owners, len(new_keys)))
+        else:   # sealed block by block
+            layer.runs.extend((k, k, v, 1) for k, v in zip(new_keys, new_values))
 
     def record_peak(self, layer_idx):
         """Live persistent bytes in O(1) per layer update (reference ``cache.py:308-326``)."""
@@ -670,26 +776,29 @@ class InQuantCache(_HFCache):
         self._flush_pending()
         if layer_idx not in self._layers:
             raise KeyError(f"No cached layer {layer_idx}")
-        layer = self._layers[layer_idx]
+        return self._history(self._layers[layer_idx])
 
-        def restore(sink, blocks, tail):
-            _, heads, _, channels = layer.shape
-            sink_tokens = 0 if sink is None else sink.shape[2]
-            tail_tokens = 0 if tail is None else tail.shape[2]
-            packed_tokens = sum(block.shape[2] for block in blocks)
-            out = torch.empty((1, heads, sink_tokens + packed_tokens + tail_tokens, channels),
-                              dtype=layer.dtype, device=layer.device)
+    def _history(self, layer: _Layer, new_key=None, new_value=None):
+        """Dense keys and values of the layer, followed by the new states where there are any."""
+        _, heads, _, channels = layer.shape
+        new_tokens = 0 if new_key is None else new_key.shape[2]
+        sink_tokens = layer.sink_count
+        tail_tokens = 0 if layer.tail_key_buffer is None else layer.tail_count
+        packed_tokens = len(layer.key_blocks) * self.config.block_size
+        full = [torch.empty((1, heads, sink_tokens + packed_tokens + tail_tokens + new_tokens, channels),
+                            dtype=layer.dtype, device=layer.device) for _ in range(2)]
+        if restore_history(layer, *full, new_key, new_value):
+            return tuple(full)
+        for out, sink, blocks, tail, new in ((full[0], layer.sink_key, layer.key_blocks, layer.residual_key, new_key),
+                                             (full[1], layer.sink_value, layer.value_blocks, layer.residual_value, new_value)):
             if sink_tokens:
                 out[:, :, :sink_tokens].copy_(sink)
             position = restore_blocks(blocks, out, sink_tokens)
             if tail_tokens:
-                out[:, :, position:].copy_(tail)
-            return out
-
-        return (
-            restore(layer.sink_key, layer.key_blocks, layer.residual_key),
-            restore(layer.sink_value, layer.value_blocks, layer.residual_value),
-        )
+                out[:, :, position:position + tail_tokens].copy_(tail)
+            if new_tokens:
+                out[:, :, position + tail_tokens:].copy_(new)
+        return tuple(full)
 
     # ------------------------------------------------------------------ accounting
     @property

@@ -112,3 +112,35 @@ def test_seal_entry_point_refuses_bad_row_copies_before_any_launch():
     assert lib.inq_seal_blocks(ctypes.byref(args), status, None) == N.ERR_ARGUMENT
     # nothing to encode and nothing to copy is a valid call that launches nothing
     assert lib.inq_seal_blocks(ctypes.byref(N.SealArgs()), status, None) == N.OK
+
+
+def test_restore_structs_match_the_header_and_bad_arguments_are_refused_before_any_launch(tmp_path):
+    import subprocess
+    from inquant import _native as N
+    source = tmp_path / "sizes.c"
+    source.write_text(f'#include <stdio.h>\n#include <stddef.h>\n#include "{HEADER}"\nint main(void) {{\n'
+                      '  printf("%zu %zu %zu", sizeof(inq_restore_run_t), sizeof(inq_restore_args_t), offsetof(inq_restore_args_t, n_copies));\n'
+                      '  return 0;\n}\n')
+    subprocess.run(["gcc", "-std=c11", str(source), "-o", str(tmp_path / "sizes")], check=True)
+    got = [int(x) for x in subprocess.run([str(tmp_path / "sizes")], check=True, capture_output=True, text=True).stdout.split()]
+    assert got == [ctypes.sizeof(N.RestoreRun), ctypes.sizeof(N.RestoreArgs), N.RestoreArgs.n_copies.offset]
+    lib = N.library()
+
+    def call(**changes):
+        run = N.RestoreRun(*[4096] * 11, 1)
+        args = N.RestoreArgs(ctypes.addressof(run), 1, 4, 64, 16, 0, 2, 64, 0, 4096, 4096, 1024, 0)
+        args.out_dtype = N.BF16
+        for name, value in changes.items():
+            setattr(run if hasattr(run, name) else args, name, value)
+        return lib.inq_restore_history(ctypes.byref(args), None)
+
+    assert lib.inq_restore_history(None, None) == N.ERR_ARGUMENT
+    assert call(out_dtype=N.F32) == N.ERR_UNSUPPORTED
+    for bad in ({"n_runs": -1}, {"runs": None}, {"n_copies": 7}, {"heads": 0}, {"block_tokens": 0}, {"count": 65}, {"value_bits": 3},
+                {"value_group": 48}, {"value_kind": 2}, {"out_key": 4104}, {"stride_h": 1028}, {"position": -1}, {"n_blocks": 0},
+                {"key_payload": 4098}, {"value_offsets": None}, {"key_donors": None}, {"value_kind": 1, "value_count": 2, "value_padding": None}):
+        assert call(**bad) == N.ERR_ARGUMENT, bad
+    # nothing to restore and nothing to copy is a valid call that launches nothing
+    args = N.RestoreArgs()
+    args.out_dtype = N.BF16
+    assert lib.inq_restore_history(ctypes.byref(args), None) == N.OK

@@ -292,3 +292,35 @@ def test_32k_shape_and_persistent_bytes():
     out, _ = cache.update(tail, tail, 0)
     assert tuple(out.shape) == (1, 4, 32771, 128) and cache.get_seq_length() == 32771
     assert cache.nbytes < cache.bf16_nbytes * 0.3
+
+
+@pytest.mark.parametrize("value_bits,group", [(2, 64), (2, 32), (2, 128), (4, 32), (4, 64), (4, 128), (None, 64)])
+@pytest.mark.parametrize("block,dtype,fraction", [(256, "bfloat16", 0.125), (64, "float16", 0.125), (16, "bfloat16", 0.5),
+                                                  (40, "float16", 0.25), (104, "bfloat16", 0.0)])
+def test_dense_history_equals_its_parts(value_bits, group, block, dtype, fraction):
+    """The one launch that rebuilds a layer -- runs of one and of several blocks, more than a launch takes, blocks
+    that are not whole steps of 16 or parts of 64 tokens -- against every block's own dequantised tensor, and
+    ``update``'s result (the new states behind it) against both."""
+    from inquant.cache import CacheConfig, InQuantCache
+    from inquant.codec import CodecConfig
+    heads, sink, residual = 2, 4, 8
+    config = CacheConfig(CodecConfig(donor_policy="min_error", salient_fraction=fraction), block_size=block, residual_length=residual,
+                         sink_tokens=sink, value_bits=value_bits, value_group_size=group, validate_positions=False)
+    cache = InQuantCache(config)
+    gen = torch.Generator(device="cuda").manual_seed(block)
+    for step, tokens in enumerate([3, 5 * block + 40, 2 * block, *([block] * 9), 7]):
+        k, v = (torch.randn((1, heads, tokens, 128), generator=gen, device="cuda").to(getattr(torch, dtype)) for _ in range(2))
+        if step % 2:      # rows of another stride
+            k, v = (x.transpose(1, 2).contiguous().transpose(1, 2) for x in (k, v))
+        if step:
+            layer = cache._layers[0]
+            parts = [[*(t for t in (sink_t,) if t is not None), *(b.dequantize() for b in blocks), tail] for sink_t, blocks, tail in
+                     ((layer.sink_key, layer.key_blocks, layer.residual_key), (layer.sink_value, layer.value_blocks, layer.residual_value))]
+            expected = [torch.cat(p, dim=2) for p in parts]
+            assert all(torch.equal(a, b) for a, b in zip(cache.materialize(0), expected))
+            before = layer.block_runs()
+            assert before is not None
+        full = cache.update(k, v, 0)
+        if step:
+            assert all(torch.equal(a, torch.cat((b, c), dim=2)) for a, b, c in zip(full, expected, (k, v)))
+    assert len(cache._layers[0].runs) > 8
