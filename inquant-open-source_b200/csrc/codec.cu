@@ -6,6 +6,7 @@
 // divisions.  The only fused operations are the explicit fma() calls of the division-by-
 // integer below, which is proven to return the correctly rounded quotient.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -13,7 +14,16 @@ namespace inq {
 
 constexpr int kMaxChannels = 1024;
 constexpr int kMaxWords = kMaxChannels / 32;
-constexpr int kRcpTable = 512;  // tokens per row for which 1/(t+1) is tabulated in shared memory
+constexpr int kRcpTable = 512;  // tokens per row for which 1/(t+1) is tabulated
+struct InverseTable {
+  double of[kRcpTable];
+};
+constexpr InverseTable make_inverse_table() {
+  InverseTable table{};
+  for (int t = 0; t < kRcpTable; ++t) table.of[t] = 1.0 / (double)(t + 1);   // correctly rounded
+  return table;
+}
+static __device__ const InverseTable kInverse = make_inverse_table();
 
 // ------------------------------------------------------------------------------------------
 // Sampled statistics in the summation order of the reference's CPU reduction: samples are
@@ -447,6 +457,10 @@ __global__ void __launch_bounds__(kMaxThreads) k4_encode_kernel(K4Params p) {
 //   * x / s uses a correctly rounded reciprocal and two fused corrections, which returns the
 //     IEEE quotient (Markstein); scales below 2^-100 keep the plain division;
 //   * the sets of channels are masks in registers.
+// A launch of few rows lasts as long as one CTA, one of many is bound by issue; us per launch in graphs of 20, with
+// the float64 chain walked by every channel, all-pairs ranks, settled donor choices and a branch per slot before,
+// with what the comments below describe now: 12 rows of 256 tokens 21.5 -> 13.5, 496 rows 39.9 -> 24.2, 47 x 8
+// token-major rows 41.0 -> 23.5, 187 x 8 of 64 tokens 42.2 -> 27.1, 400 of 16 tokens 11.2 -> 8.4.
 struct Mask128 {
   unsigned long long lo, hi;
   __device__ __forceinline__ int below(int pos) const {   // largest member < pos, or -1
@@ -492,19 +506,95 @@ __device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_g
 template <int N>
 __device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Channels with a larger key than `mine`, or the same one and a lower number than c (128 keys).
-__device__ __forceinline__ int rank_of(const unsigned* keys, unsigned mine, int c) {
+// Channels (of 128, one per thread) with a larger key than `mine`, or the same one and a lower number than c.
+// Keys are at most 0x7fffffff; `keys` holds those of the thread's own warp at least, `sorted` is scratch for 128.
+// The warp's own keys are compared one by one, which sorts them; the other three sorted lists are searched by
+// halves.  (Comparing with all 128 keys takes twice the instructions.)  Contains a CTA barrier between the two.
+__device__ __forceinline__ int rank_of(const unsigned* keys, unsigned* sorted, unsigned mine, int c) {
+  const int warp = c >> 5, lane = c & 31, own = lane >> 2;
   int rank = 0;
-  const int own = c >> 2;
-#pragma unroll 8
-  for (int o4 = 0; o4 < 32; ++o4) {
-    const uint4 k = *(const uint4*)(keys + 4 * o4);
+#pragma unroll
+  for (int o4 = 0; o4 < 8; ++o4) {
+    const uint4 k = *(const uint4*)(keys + 32 * warp + 4 * o4);
     const unsigned limit = mine + (o4 < own ? 0u : 1u);
     rank += (k.x >= limit) + (k.y >= limit) + (k.z >= limit) + (k.w >= limit);
   }
 #pragma unroll
-  for (int e = 0; e < 3; ++e) rank += e < (c & 3) && keys[4 * own + e] == mine;
+  for (int e = 0; e < 3; ++e) rank += e < (lane & 3) && keys[32 * warp + 4 * own + e] == mine;
+  sorted[32 * warp + rank] = mine;   // descending
+  __syncthreads();
+  const unsigned* list[3];
+  unsigned limit[3];
+  int ahead[3] = {0, 0, 0};
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int other = (warp + 1 + d) & 3;
+    list[d] = sorted + 32 * other;
+    limit[d] = mine + (other < warp ? 0u : 1u);
+  }
+#pragma unroll
+  for (int step = 16; step; step >>= 1)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) ahead[d] += list[d][ahead[d] + step - 1] >= limit[d] ? step : 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) rank += ahead[d] + (list[d][ahead[d]] >= limit[d]);
   return rank;
+}
+
+// Welford's update in float64, sequential over tokens (the reference's var_mean), of one channel.
+template <typename T>
+__device__ __noinline__ void welford(const T* column, long long step, int tokens, const double* inverse, double& mean_out, double& m2_out) {
+  double mean = 0.0, m2 = 0.0, n = 0.0;
+  for (int t = 0; t < tokens; ++t) {
+    const double x = (double)to_float<T>(column[t * step]);
+    const double delta = x - mean;
+    n = n + 1.0;
+    mean = mean + divide_by_count(delta, n, inverse[t]);
+    m2 = m2 + delta * (x - mean);
+  }
+  mean_out = mean;
+  m2_out = m2;
+}
+
+// What the encoder needs of Welford's chain is one float32 number, the error of the channel as a donor:
+// (float)(m2 / tokens) + ((float)mean - sampled mean)^2.  Plain float64 sums S1 of x and S2 of x * x lie close enough
+// to the chain that its rounding is nearly always decided: the chain's five dependent operations a token (68 cycles
+// of a warp alone, 25 of its issue) become two additions that depend on nothing but their own sums.  Every
+// rounding on the way is monotone, so the chain's number lies between those that the ends of intervals give which
+// hold the chain's mean and m2.  Where the two differ -- by a unit in the last place -- the chain is walked only if
+// that could decide which channels are among the least.
+//
+// With u = 2^-53, n tokens of at most M, V = sum (x - mean)^2 and S2 = sum x^2, and first-order terms (a margin of a
+// tenth stands for the others):
+//   chain, mean:   mean_k = mean_{k-1} (1 - 1/k) + x/k + r_k, k |r_k| <= u (2 |x - mean_{k-1}| + k |mean_k|), and the error
+//                  of mean_k is at most 1/k times the sum of these.  sum (x_k - mean_{k-1}) (x_k - mean_k) = V with
+//                  x_k - mean_k = (x_k - mean_{k-1}) (1 - 1/k), so the first parts add up to 2 (M + sqrt(2 k S2)); |mean_k| <=
+//                  sqrt(S2 / k), so the second to 2/3 (k + 1)^1.5 sqrt(S2).  For any k up to n the error is at most
+//                  E = u (2 M + sqrt(S2) (4.9 + 0.67 sqrt(n))).
+//   chain, m2:     a summand is off by |x - mean_{k-1}| E + |x - mean_k| E + E^2 + 3 u |summand|; the absolute values add
+//                  up to sqrt(2 n V) and sqrt(n V) (the first summand is exactly 0), and the additions give
+//                  n u V:  2.42 E sqrt(n V) + n E^2 + (n + 3) u V.
+//   plain sums:    in four interleaved parts:  S1 is off by u (n/4 + 3) sum |x|, S2 by u (n/4 + 4) S2, and with
+//                  sum |x| <= sqrt(n S2):  S2 - S1^2 / n is off by u (n/4 + 4) S2 + 2 u (n/4 + 3) S2 + 4 u S2.
+// `inverse` is 1 / (double)n, correctly rounded.
+__device__ __forceinline__ void plain_donor_error(double s1, double s2, int tokens, double inverse, float absmax, float sampled_mean,
+                                                  float& low, float& high) {
+  const double n = (double)tokens;
+  const double mean = s1 * inverse, v = s2 - s1 * mean;
+  const float nf = (float)tokens, u = 1.110223e-16f;
+  const float s2f = (float)s2 * 1.0001f, vf = fmaxf((float)v, 0.f) * 1.0001f + u * (0.75f * nf + 14.f) * s2f;   // no less than V
+  const float e = u * (2.f * absmax + sqrtf(s2f) * (4.9f + 0.67f * sqrtf(nf)));
+  const float mean_bound = 1.1f * (e + u * (0.25f * nf + 5.f) * absmax);
+  const float m2_bound = 1.1f * (2.42f * e * sqrtf(nf * vf) + nf * e * e + (nf + 3.f) * u * vf + (0.75f * nf + 14.f) * u * s2f);
+  const float d0 = (float)(mean - (double)mean_bound) - sampled_mean, d1 = (float)(mean + (double)mean_bound) - sampled_mean;
+  const float near = d0 * d1 > 0.f ? fminf(fabsf(d0), fabsf(d1)) : 0.f, far = fmaxf(fabsf(d0), fabsf(d1));
+  low = fmaxf((float)((v - (double)m2_bound) / n) + near * near, 0.f);
+  high = (float)((v + (double)m2_bound) / n) + far * far;
+  // (the bounds are computed in float32: a channel whose squares leave its range may be anything)
+  if (!(absmax > 1e-12f && absmax < 1e15f)) {
+    low = 0.f;
+    high = absmax == 0.f ? 0.f : INFINITY;
+  }
 }
 
 // REGULAR: tokens % 8 == 0 and sample_stride == 8.
@@ -521,14 +611,18 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
   constexpr int kRowBytes = C * (int)sizeof(T);
   constexpr int kGroupBytes = kGroupTokens * kRowBytes;
   constexpr int kWarpStage = kGroupBytes / 4;   // a warp's share of a stage
-  __shared__ __align__(16) unsigned char s_ring[STAGED ? kRing * kGroupBytes : 16];
+  // STAGED: the ring; else two pairs of rows per warp
+  __shared__ __align__(16) unsigned char s_ring[STAGED ? kRing * kGroupBytes : 4 * 4 * kRowBytes];
   __shared__ __align__(16) float s_sal[C];      // read four at a time, like s_key
   __shared__ float s_mean[C], s_scale[C], s_rcp[C];
   __shared__ __align__(16) unsigned s_key[C];
+  __shared__ unsigned s_sorted[C];
   __shared__ unsigned char s_kind[C], s_from[C], s_plain[C];
+  __shared__ signed char s_role[C];
   __shared__ int s_src[64], s_don[64];
-  __shared__ unsigned s_sel[4], s_avail[4];
-  __shared__ double s_inv[kRcpTable];
+  __shared__ unsigned s_sel[4], s_avail[4], s_range[2];
+  __shared__ uint2 s_pool[32];                  // {channel, saliency bits} of the least-error channels, ascending
+  __shared__ __align__(16) uint4 s_seek[32];    // per source: pool entries below it, its run of sources, itself
   const int tokens = p.in.tokens, count = p.count;
   const bool want_error = p.min_error != 0;
   const long long outer = blockIdx.x / p.in.n_inner, inner = blockIdx.x % p.in.n_inner;
@@ -539,17 +633,15 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
   }
   const T* row = (const T*)p.in.x + outer * p.in.s_outer + inner * p.in.s_inner;
   const int c = threadIdx.x;
-  if (want_error)
-    for (int t = c; t < tokens; t += C) s_inv[t] = 1.0 / (double)(t + 1);
   if (c < 4) s_sel[c] = s_avail[c] = 0u;
-  __syncthreads();
+  s_role[c] = -1;
 
-  // ---- statistics: one thread per channel, sequential over tokens
+  // ---- statistics: one thread per channel
   unsigned top_bits = 0u;
   CascadePair cascade;
   const int samples = (tokens + p.sample_stride - 1) / p.sample_stride;
   cascade.init(samples);
-  double mean = 0.0, m2 = 0.0, count_d = 0.0;
+  double s1[4] = {0.0, 0.0, 0.0, 0.0}, s2[4] = {0.0, 0.0, 0.0, 0.0};   // of x and of x * x, see plain_donor_error
   int next_sample = 0;
   {
     const T* column = row + c;
@@ -591,7 +683,6 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
       issue(0);
       issue(1);
       issue(2);
-      const double* inv = s_inv;
       for (int g = 0; g < n_groups; ++g) {
         stage_wait<kRing - 2>();
         __syncwarp();   // group g has landed for every lane; the stage of group g - 1 is free
@@ -609,13 +700,10 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
             top_bits = max(top_bits, __float_as_uint(x) & 0x7fffffffu);
             if (want_error) {
               const double xd = (double)x;
-              const double delta = xd - mean;
-              count_d = count_d + 1.0;
-              mean = mean + divide_by_count(delta, count_d, inv[u]);
-              m2 = m2 + delta * (xd - mean);
+              s1[u & 3] = s1[u & 3] + xd;
+              s2[u & 3] = fma(xd, xd, s2[u & 3]);
             }
           }
-          inv += kUnroll;
         }
       }
       (void)step;
@@ -624,7 +712,6 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
       const T* cursor = column;
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) ahead[u] = cursor[u * step];
-      const double* inv = s_inv;
       for (int base = 0; base < tokens; base += kUnroll) {
         float v[kUnroll];
 #pragma unroll
@@ -641,13 +728,10 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
           top_bits = max(top_bits, __float_as_uint(x) & 0x7fffffffu);
           if (want_error) {
             const double xd = (double)x;
-            const double delta = xd - mean;
-            count_d = count_d + 1.0;
-            mean = mean + divide_by_count(delta, count_d, inv[u]);
-            m2 = m2 + delta * (xd - mean);
+            s1[u & 3] = s1[u & 3] + xd;
+            s2[u & 3] = fma(xd, xd, s2[u & 3]);
           }
         }
-        inv += kUnroll;
       }
     } else {
 #pragma unroll
@@ -673,10 +757,8 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
           }
           if (want_error) {
             const double xd = (double)x;
-            const double delta = xd - mean;
-            count_d = count_d + 1.0;
-            mean = mean + divide_by_count(delta, count_d, s_inv[t]);
-            m2 = m2 + delta * (xd - mean);
+            s1[u & 3] = s1[u & 3] + xd;
+            s2[u & 3] = fma(xd, xd, s2[u & 3]);
           }
         }
       }
@@ -686,52 +768,100 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
   float abs_total, sum_total;
   cascade.finish(abs_total, sum_total);
   const float saliency = abs_total / (float)samples, sampled_mean = sum_total / (float)samples;
-  float donor_error = 0.f;
-  if (want_error) {
-    const float variance = (float)(m2 / (double)tokens);
-    const float diff = (float)mean - sampled_mean;
-    donor_error = variance + diff * diff;
-  }
   if (top_bits >= 0x7f800000u) atomicOr(p.status, INQ_STATUS_NONFINITE);
   const float absmax = __uint_as_float(top_bits);
+  float error_low = 0.f, error_high = 0.f;   // hold the channel's error as a donor
+  if (want_error)
+    plain_donor_error((s1[0] + s1[1]) + (s1[2] + s1[3]), (s2[0] + s2[1]) + (s2[2] + s2[3]), tokens, kInverse.of[tokens - 1], absmax,
+                      sampled_mean, error_low, error_high);
   s_sal[c] = saliency;
   s_mean[c] = sampled_mean;
-  __syncthreads();
+  __syncwarp();
 
   // ---- top-`count` channels by saliency (ties: lower channel), optional least-error pool
   bool selected = false;
   if (count > 0) {
-    const unsigned mine = __float_as_uint(saliency);
-    const int rank = rank_of((const unsigned*)s_sal, mine, c);
-    selected = rank < count;
+    selected = rank_of((const unsigned*)s_sal, s_sorted, __float_as_uint(saliency), c) < count;
     if (selected) atomicOr(&s_sel[c >> 5], 1u << (c & 31));
-    s_key[c] = selected ? 0x7f800000u : __float_as_uint(donor_error);
     if (!want_error && !selected) atomicOr(&s_avail[c >> 5], 1u << (c & 31));
   }
-  __syncthreads();
-  if (selected) {   // position in the ascending list of sources
-    int position = __popc(s_sel[c >> 5] & ((1u << (c & 31)) - 1u));
-    for (int w = 0; w < (c >> 5); ++w) position += __popc(s_sel[w]);
-    s_src[position] = c;
-  }
-  if (want_error && count > 0 && !selected) {
-    const unsigned mine = s_key[c];
-    // channels with a smaller error, or the same one and a lower number
-    int rank = 0;
-    const int own = c >> 2;
-#pragma unroll 8
-    for (int o4 = 0; o4 < C / 4; ++o4) {
-      const uint4 k = *(const uint4*)(s_key + 4 * o4);
-      const unsigned limit = mine + (o4 < own ? 1u : 0u);
-      rank += (k.x < limit) + (k.y < limit) + (k.z < limit) + (k.w < limit);
+  bool open = __syncthreads_or(want_error && !(error_low == error_high));   // a channel's error is not known to the last bit
+  // position of this channel in a set of channels
+  auto place = [&](const unsigned* set) {
+    int position = __popc(set[c >> 5] & ((1u << (c & 31)) - 1u));
+    for (int w = 0; w < (c >> 5); ++w) position += __popc(set[w]);
+    return position;
+  };
+  if (selected) s_src[place(s_sel)] = c;   // the ascending list of sources
+  if (want_error && count > 0) {
+    bool near;
+    while (true) {
+      // channels with a smaller error, or the same one and a lower number (descending: the smaller the error, the
+      // larger the key; a selected channel comes last)
+      s_key[c] = 0x7fffffffu - (selected ? 0x7f800000u : __float_as_uint(error_high));
+      __syncwarp();
+      near = rank_of(s_key, s_sorted, s_key[c], c) < count && !selected;
+      if (!open) break;
+      // the same channels whatever the open errors are, if the largest taken lies below the smallest left
+      if (c == 0) {
+        s_range[0] = 0u;
+        s_range[1] = 0x7f800000u;
+      }
+      __syncthreads();
+      if (near) atomicMax(&s_range[0], __float_as_uint(error_high));
+      else if (!selected) atomicMin(&s_range[1], __float_as_uint(error_low));
+      __syncthreads();
+      if (s_range[0] < s_range[1]) break;
+      double mean, m2;
+      welford<T>(row + c, p.in.s_token, tokens, kInverse.of, mean, m2);
+      const float variance = (float)(m2 / (double)tokens);
+      const float diff = (float)mean - sampled_mean;
+      error_high = variance + diff * diff;
+      open = false;
+      __syncthreads();
     }
-#pragma unroll
-    for (int e = 0; e < 3; ++e) rank += e < (c & 3) && s_key[4 * own + e] == mine;
-    if (rank < count) atomicOr(&s_avail[c >> 5], 1u << (c & 31));
+    if (near) atomicOr(&s_avail[c >> 5], 1u << (c & 31));
+    __syncthreads();
+    if (near && count <= 32) s_pool[place(s_avail) & 31] = make_uint2((unsigned)c, __float_as_uint(saliency));
   }
   __syncthreads();
-  if (c < 32 && count > 0) {
-    // Donors are taken by the sources in ascending order, each from what the earlier ones left.  One lane per
+  if (c < 32 && count > 0 && count <= 32 && want_error) {
+    // Donors are taken by the sources in ascending order, each from what the earlier ones left.  With least-error
+    // donors there are just as many of them as sources, most sources meet a donor that is gone, and one after
+    // the other is the order of things: the pool's entries are bits of one word, a source finds its two neighbours
+    // by two bit scans and one look-up.  (For 16 sources 3200 to 4500 cycles; settling choices made ahead, as below,
+    // 5200 to 8700.)
+    const Mask128 others{~((unsigned long long)s_sel[0] | ((unsigned long long)s_sel[1] << 32)),
+                         ~((unsigned long long)s_sel[2] | ((unsigned long long)s_sel[3] << 32))};
+    if (c < count) {
+      const int source = s_src[c];
+      int below = 0;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) below += __popc(s_avail[w] & bits_below(source - 32 * w));
+      s_seek[c] = make_uint4(bits_below(below), (unsigned)(others.below(source) + 1), (unsigned)(others.above(source) - 1), (unsigned)source);
+    }
+    __syncwarp();
+    unsigned free_ = bits_below(count);
+    uint4 next = s_seek[0];
+    for (int i = 0; i < count; ++i) {
+      const uint4 seek = next;
+      if (i + 1 < count) next = s_seek[i + 1];
+      const unsigned b = free_ & seek.x, h = free_ & ~seek.x;
+      const int at_low = 31 - __clz(b), at_high = __ffs(h) - 1;      // -1 where there is none
+      const uint2 e_low = s_pool[max(at_low, 0)], e_high = s_pool[max(at_high, 0)];
+      const int low = (int)e_low.x, high = (int)e_high.x, left = (int)seek.y, right = (int)seek.z, source = (int)seek.w;
+      // one next to the source itself wins over any other, else the nearer one; of two the less salient, then the lower
+      const bool has_low = b != 0u, has_high = h != 0u;
+      const int d_low = has_low ? left - low : C, d_high = has_high ? high - right : C;
+      const bool by_low = has_low && low == source - 1, by_high = has_high && high == source + 1, beside = by_low || by_high;
+      const bool take_low = beside ? by_low : has_low && d_low <= d_high, take_high = beside ? by_high : has_high && d_high <= d_low;
+      const bool lower = __uint_as_float(e_low.y) <= __uint_as_float(e_high.y);
+      const bool chosen_low = take_low && (lower || !take_high);
+      free_ &= ~(1u << ((chosen_low ? at_low : at_high) & 31));
+      if (c == i) s_don[i] = chosen_low ? low : take_high ? high : 0;   // (one is free for every source)
+    }
+  } else if (c < 32 && count > 0) {
+    // Any channel that is not a source may be a donor (or there are more than a word's bits of them).  One lane per
     // source: all choose at once, then the choices are settled one by one (a shuffle, a vote), and only when the
     // donor just taken was the choice of a later source do the later ones choose again -- a donor that is gone
     // but was not a source's choice changes neither which of its candidates is nearer nor the tie between
@@ -795,6 +925,8 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
     const int source = s_src[c], donor = s_don[c];
     s_kind[donor] = 2;
     s_from[donor] = (unsigned char)source;
+    s_role[source] = (signed char)donor;
+    s_role[donor] = (signed char)(-2 - c);
     ((float*)p.padding.at(slot, inner))[c] = s_mean[donor];
     if (p.salient.base) {
       ((unsigned char*)p.salient.at(slot, inner))[c] = (unsigned char)source;
@@ -803,11 +935,7 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
   }
   __syncthreads();
   if (p.roles.base) {
-    int role = -1;
-    for (int i = 0; i < count; ++i) {
-      if (s_src[i] == c) role = s_don[i];
-      if (s_don[i] == c) role = -2 - i;
-    }
+    const int role = s_role[c];
     if (p.role_bytes == 1)
       ((signed char*)p.roles.at(slot, inner))[c] = (signed char)role;
     else
@@ -816,55 +944,41 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
   // ---- packing: a thread owns 8 fixed slots (4 payload bytes) and strides over tokens
   unsigned char* payload = (unsigned char*)p.payload.at(slot, inner);
   const int chunk = c & 15, t0 = c >> 4;
-  // per slot: divisor, clamp limit, bias and which nibble of the code is stored -- a normal slot
-  // keeps clamp(q, +-7) + 8, a salient slot the high nibble of clamp(q, +-127) + 128, a donor slot
-  // the low nibble of its source's code; all three are (code >> shift) & 15.  Adding the bias and
-  // 1.5 * 2^23 rounds the quotient as rint does (the limits are whole and the bias is even, so neither
-  // the clamp nor the sum moves a tie) and leaves the code in the low bits; a rotation brings its nibble
-  // to the slot's place.
-  float scale[8], rcp[8], limit[8], bias[8];
-  int rotate[8], from[8], kind[8];
-  bool any_plain = false, any_remote = false;
+  // per slot: divisor, bias and which nibble of the code is stored -- a normal slot keeps q + 8, a salient slot
+  // the high nibble of q + 128, a donor slot the low nibble of its source's code; all three are
+  // (code >> shift) & 15.  q needs no clamp: a scale is the channel's largest magnitude over 7 (or 127) rounded, or
+  // larger, so the quotient is at most that whole number and a few units in its last place and rounds to it.
+  // Adding the bias and 1.5 * 2^23 rounds the quotient as rint does (the bias is even, so the sum moves no tie)
+  // and leaves the code in the low bits; a rotation brings its nibble to the slot's place.
+  float scale[8], rcp[8], bias[8];
+  int rotate[8], from[8];
+  bool any_plain = false;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int ch = chunk * 8 + j;
-    kind[j] = s_kind[ch];
+    const int kind = s_kind[ch];
     from[j] = s_from[ch];
     const int src_ch = from[j];       // a donor slot divides its source's value by its source's scale
     scale[j] = s_scale[src_ch];
     rcp[j] = s_rcp[src_ch];
     any_plain |= s_plain[src_ch] != 0;
-    limit[j] = kind[j] ? 127.f : 7.f;
-    bias[j] = 12582912.f + (kind[j] ? 128.f : 8.f);
-    rotate[j] = 4 * j - (kind[j] == 1 ? 4 : 0);
-    any_remote |= (from[j] != ch);
+    bias[j] = 12582912.f + (kind ? 128.f : 8.f);
+    rotate[j] = 4 * j - (kind == 1 ? 4 : 0);
   }
-  auto pack_row = [&](const uint4* own, const T* trow) {   // this thread's 8 channels of a token, the token's row
-    const T* hv = (const T*)own;
-    float v[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = to_float<T>(hv[j]);
-    if (any_remote) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (kind[j] == 2) v[j] = to_float<T>(trow[from[j]]);
-    }
-    float q[8];
-    if (any_plain) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) q[j] = v[j] / scale[j];
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) q[j] = exact_quotient(v[j], scale[j], rcp[j], false);
-    }
+  // A token's row in shared memory: every slot fetches its value by itself, the donor slots from their sources.
+  // (256 tokens of a CTA alone on its SM 7900 cycles; with a 16-byte load of the own channels, a branch per slot
+  // for the others and the clamps 12500.)
+  auto pack_row = [&](const T* trow, auto plain) {
     unsigned word = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const unsigned code = __float_as_uint(fminf(fmaxf(q[j], -limit[j]), limit[j]) + bias[j]);
+      const float v = to_float<T>(trow[from[j]]);
+      const unsigned code = __float_as_uint(exact_quotient(v, scale[j], rcp[j], decltype(plain)::value) + bias[j]);
       word |= __funnelshift_l(code, code, rotate[j]) & (15u << (4 * j));
     }
     return word;
   };
+  any_plain = __any_sync(0xffffffffu, any_plain);
   if constexpr (STAGED) {
     const int n_groups = tokens / kGroupTokens;
     const int warp_id = c >> 5, lane_id = c & 31;
@@ -890,35 +1004,39 @@ __global__ void __launch_bounds__(128, STAGED ? 5 : 7) k4_encode128_kernel(K4Par
       for (int i = 0; i < kGroupTokens / 8; ++i) {
         const int tl = t0 + 8 * i;   // t0 = 2 * warp + lane / 16
         const T* trow = (const T*)(tile + (2 * i + (lane_id >> 4)) * kRowBytes);
-        const uint4 cur = *(const uint4*)(trow + chunk * 8);
-        const unsigned word = pack_row(&cur, trow);
+        const unsigned word = any_plain ? pack_row(trow, std::true_type()) : pack_row(trow, std::false_type());
         *(unsigned*)(payload + (long long)(g * kGroupTokens + tl) * 64 + chunk * 4) = word;
       }
     }
     stage_wait<0>();
     return;
   }
+  // rows from global memory: a warp passes two tokens at a time through rows of its own in shared memory
   constexpr int kVec = sizeof(T) == 2 ? 1 : 2;   // 16-byte vectors per 8 elements
+  T* const lane_row = (T*)s_ring + (c >> 5) * 4 * C + ((c >> 4) & 1) * C;
   uint4 next[kVec];
   if (t0 < tokens) {
 #pragma unroll
     for (int q = 0; q < kVec; ++q) next[q] = ((const uint4*)(row + (long long)t0 * p.in.s_token + chunk * 8))[q];
   }
   const long long pack_step = 8 * p.in.s_token;
-  const T* src = row + (long long)t0 * p.in.s_token - pack_step;
-  unsigned char* dst = payload + (long long)t0 * 64 + chunk * 4 - 512;
-  for (int t = t0; t < tokens; t += 8) {
+  const T* src = row + (long long)t0 * p.in.s_token;
+  unsigned char* dst = payload + (long long)t0 * 64 + chunk * 4;
+  int turn = 0;
+  for (int t = t0 & ~1; t < tokens; t += 8) {   // (whole warps walk; the upper half has no token where the last pair is one)
+    T* const trow = lane_row + turn;
+    turn ^= 2 * C;
+#pragma unroll
+    for (int q = 0; q < kVec; ++q) ((uint4*)(trow + chunk * 8))[q] = next[q];
+    __syncwarp();
     src += pack_step;
-    dst += 512;
-    uint4 cur[kVec];
+    if (t + (t0 & 1) + 8 < tokens) {
 #pragma unroll
-    for (int q = 0; q < kVec; ++q) cur[q] = next[q];
-    if (t + 8 < tokens) {
-#pragma unroll
-      for (int q = 0; q < kVec; ++q) next[q] = ((const uint4*)(src + pack_step + chunk * 8))[q];
+      for (int q = 0; q < kVec; ++q) next[q] = ((const uint4*)(src + chunk * 8))[q];
     }
-    const unsigned word = pack_row(cur, src);
-    *(unsigned*)dst = word;
+    const unsigned word = any_plain ? pack_row(trow, std::true_type()) : pack_row(trow, std::false_type());
+    if (t + (t0 & 1) < tokens) *(unsigned*)dst = word;
+    dst += 512;
   }
 }
 

@@ -293,3 +293,46 @@ def test_value_codec_rejects_unrepresentable_parameters_and_blocks_match():
         for name, tensor in block.tensors.items():
             assert torch.equal(tensor, expected.tensors[name])
         assert block.nbytes == expected.nbytes and block.shape == (1, 3, 32, 128)
+
+
+def _hard_rows(kind, tokens, dtype, rng):
+    """[rows, 1, tokens, 128] whose donor errors lie on top of one another or at the edge of a number's range."""
+    x = rng.standard_normal((6, 1, tokens, 128)).astype(np.float32)
+    if kind == "permuted":      # every channel the same values in another order, the sampled tokens alike
+        base = rng.standard_normal(tokens).astype(np.float32)
+        others = np.array([t for t in range(tokens) if t % 8])
+        for row in x[:, 0]:
+            row[:] = base[:, None]
+            for c in range(128):
+                row[others, c] = base[rng.permutation(others)]
+        x[:, 0, ::8, :16] *= 4     # and sixteen salient ones
+    elif kind == "same":
+        x[:] = x[..., :1]
+    elif kind == "constant":
+        x[..., 20:100] = rng.standard_normal((6, 1, 1, 80)).astype(np.float32)
+    elif kind == "offset":      # spread far below the mean
+        x = x * np.float32(2.0 ** -6) + np.float32(3.0) * rng.standard_normal((6, 1, 1, 128)).astype(np.float32)
+    elif kind == "spike":
+        x *= np.float32(2.0 ** -8)
+        x[..., 5, :] = 50 * rng.standard_normal((6, 1, 128)).astype(np.float32)
+    elif kind == "range" and dtype != "float16":
+        x *= np.float32(10.0) ** rng.integers(-30, 16, (6, 1, 1, 128)).astype(np.float32)
+        x[2:4] *= np.float32(1e-8)
+        x[4, ..., 30:60] = 0
+        x[5] *= np.float32(1e18) / np.abs(x[5]).max()
+    return oracle.round_to_dtype(x, dtype)
+
+
+@pytest.mark.parametrize("kind", ["permuted", "same", "constant", "offset", "spike", "range"])
+@pytest.mark.parametrize("tokens", [16, 40, 64, 256, 512])
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16", "float32"])
+def test_k4_least_errors_where_plain_sums_cannot_tell_them_apart(kind, tokens, dtype):
+    CodecConfig, quantize, _ = _codec()
+    x32 = _hard_rows(kind, tokens, dtype, np.random.default_rng(tokens))
+    x = to_device(x32, dtype)
+    for fraction in (0.125, 0.3):
+        ref = oracle.quantize_k4(x32, dtype, 8, fraction, "min_error")
+        for source in (x, x.permute(1, 2, 0, 3).contiguous().permute(2, 0, 1, 3)):
+            packed = quantize(source, CodecConfig(salient_fraction=fraction, donor_policy="min_error"))
+            for field, tensor in packed.tensors.items():
+                assert_same_bytes(tensor, ref.fields()[field], f"{field} f={fraction}")
