@@ -2091,8 +2091,10 @@ extern "C" int inq_restore_history(const inq_restore_args_t* a, inq_stream_t str
     }
     p.position = position;
     p.row_ctas = blocks * a->heads * p.parts;
-    if (p.row_ctas + vectors) launch_restore<false>(p, kind, a->out_dtype == INQ_F16, vectors, stream);
-    INQ_CUDA_CHECK(cudaGetLastError());
+    if (p.row_ctas + vectors) {
+      launch_restore<false>(p, kind, a->out_dtype == INQ_F16, vectors, stream);
+      INQ_CUDA_CHECK(cudaGetLastError());
+    }
     position += blocks * p.tokens;
     vectors = 0;
     p.n_copies = 0;
