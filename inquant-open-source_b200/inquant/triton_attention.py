@@ -91,6 +91,12 @@ def _stacked_field(blocks, name: str) -> torch.Tensor:
     return (pieces[0] if len(pieces) == 1 else torch.cat(pieces, dim=0)).contiguous()
 
 
+def _aligned_copy(tensor: torch.Tensor) -> torch.Tensor:
+    """Contiguous copy in storage of its own: rows that are contiguous already, but do not start on 16 bytes,
+    come back unchanged from ``contiguous`` and the kernels read rows as 16-byte vectors."""
+    return tensor.clone(memory_format=torch.contiguous_format)
+
+
 class PackedDecodeState:
     """Reusable descriptors for immutable blocks; exact tails are per-call inputs
     (reference ``triton_attention.py:211-388``)."""
@@ -324,9 +330,9 @@ class PackedDecodeState:
                 raise ValueError("All inputs must share their KV head count")
             given = (key, value)
             if not N.dense_rows_aligned(key):
-                key = key.contiguous()
+                key = _aligned_copy(key)
             if not N.dense_rows_aligned(value):
-                value = value.contiguous()
+                value = _aligned_copy(value)
             if name == "sink" and self._kv_heads is not None:
                 self._checked_sink = (*given, query.dtype, query.device, key, value)
             dense.append((key, value, key.shape[2]))
@@ -363,7 +369,7 @@ class PackedDecodeState:
                 self._workspace = torch.empty(workspace_shape, dtype=torch.float32, device=query.device)
             workspace_address = self._workspace.data_ptr()
         if query.data_ptr() % 16 or query.stride(1) % 8:     # rows of a head: 16-byte aligned (unit channel stride was checked)
-            query = query.contiguous()
+            query = _aligned_copy(query)
         output = torch.empty(query.shape, dtype=query.dtype, device=query.device)
         if self._tables is None:
             self._tables = torch.empty((0, 6), dtype=torch.int64, device=query.device)

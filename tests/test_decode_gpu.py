@@ -444,3 +444,22 @@ def test_general_kernel_dense_only_fp32():
                         residual_key=to_device(k, "float32"), residual_value=to_device(v, "float32"))
     attention_close(to_numpy(out).reshape(6, 128), oracle.attention_decode(q, k[0], v[0], 128 ** -0.5),
                     max_abs=1e-4, cosine=0.999999)
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+def test_contiguous_rows_that_do_not_start_on_16_bytes(dtype):
+    """Query, sink and tail one element into their storage: copied, as rows of other strides are."""
+    CodecConfig, quantize, quantize_values, PackedDecodeState, _, _ = _mods()
+
+    def off(x):
+        buffer = torch.empty(x.numel() + 1, dtype=x.dtype, device="cuda")
+        buffer[1:] = x.reshape(-1)
+        return buffer[1:].view(x.shape)
+    k, sink, tail, q = (_random(40 + i, s, dtype) for i, s in enumerate(((1, 2, 128, 128), (1, 2, 4, 128), (1, 2, 21, 128), (1, 14, 1, 128))))
+    state = PackedDecodeState([quantize(to_device(k, dtype), CodecConfig(donor_policy="min_error"))], [quantize_values(to_device(k, dtype))])
+    query, dense = to_device(q, dtype), [to_device(x, dtype) for x in (sink, sink, tail, tail)]
+    names = ("sink_key", "sink_value", "residual_key", "residual_value")
+    expected = state.decode(query, **dict(zip(names, dense)))
+    assert off(query).is_contiguous() and off(query).data_ptr() % 16
+    assert torch.equal(state.decode(off(query), **dict(zip(names, dense))), expected)
+    assert torch.equal(state.decode(query, **dict(zip(names, map(off, dense)))), expected)
