@@ -1,7 +1,8 @@
-"""Builds libinquant_b200.so in-tree with nvcc for sm_100a (cross-compiles without a GPU)."""
+"""Builds libinquant_b200.so and inquant/_host.so in-tree with nvcc for sm_100a (cross-compiles without a GPU)."""
 from __future__ import annotations
 
 import os
+import shutil
 import subprocess
 import sys
 
@@ -22,6 +23,25 @@ SOURCES = {
     "exchange.cu": [],
     "pages.cu": [],
 }
+
+
+HOST = os.path.join(HERE, "inquant", "_host.so")   # CPython extension: host side of the per-layer calls
+
+
+def build_host(force: bool = False) -> str:
+    """Builds inquant/_host.so against the installed PyTorch."""
+    src = os.path.join(CSRC, "host.cpp")
+    if force or _stale(HOST, [src, __file__, os.path.join(os.path.dirname(HERE), "include", "inquant_b200.h")]):
+        import sysconfig
+        import torch
+        root = os.path.dirname(torch.__file__)
+        cuda = os.path.dirname(os.path.dirname(os.path.realpath(shutil.which(os.environ.get("NVCC", "nvcc")) or "/usr/local/cuda/bin/nvcc")))
+        includes = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                    sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+        subprocess.run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC",
+                        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{i}" for i in includes), src, "-o", HOST,
+                        f"-L{os.path.join(root, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"], check=True)
+    return HOST
 
 
 def _stale(target: str, deps: list[str]) -> bool:
@@ -55,6 +75,7 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
         raise subprocess.CalledProcessError(1, failed[0])
     if force or _stale(LIB, objects):
         subprocess.run([nvcc, *ARCH, "-shared", "-o", LIB, *objects, "-cudart", "static"], check=True)
+    build_host(force)
     return LIB
 
 

@@ -190,6 +190,24 @@ def library() -> ctypes.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """Native host side of the per-layer calls (``csrc/host.cpp``), bound to this process's library."""
+    global _host
+    if _host is None:
+        try:
+            from . import _host as module
+        except ImportError as exc:
+            raise ImportError("inquant/_host.so is missing or was built for another PyTorch: build it with "
+                              "`python inquant-open-source_b200/build.py`") from exc
+        lib = library()
+        module.bind(*(ctypes.cast(f, c_void_p).value for f in (lib.inq_decode_attention, lib.inq_append_token)), torch.Tensor)
+        _host = module
+    return _host
+
+
 # Every symbol declared in include/inquant_b200.h.
 EXPORTS = (
     "inq_last_error", "inq_version", "inq_k4_encode", "inq_select_donors", "inq_k4_statistics",
@@ -349,10 +367,11 @@ def make_input(x: torch.Tensor, page_ids: torch.Tensor | None = None, num_slots:
 _counters: dict[tuple, torch.Tensor] = {}
 
 
-def decode_counters(device: torch.device, count: int) -> torch.Tensor:
+def decode_counters(device: torch.device, count: int, handle: int | None = None) -> torch.Tensor:
     """Zero-initialised arrival counters of the fused split-KV merge, one array per
-    (device, stream); the kernel leaves them zero, so they are reused launch after launch."""
-    key = (device, stream_handle(device))
+    (device, stream); the kernel leaves them zero, so they are reused launch after launch.  ``handle``
+    is the current stream's, when the caller has it."""
+    key = (device, stream_handle(device) if handle is None else handle)
     tensor = _counters.get(key)
     if tensor is None or tensor.numel() < count + 1:   # one more: the launch-wide arrival counter of a fused append
         tensor = torch.zeros(max(count + 1, 1024), dtype=torch.int32, device=device)

@@ -83,8 +83,6 @@ class _Layer:
     value_blocks: list = field(default_factory=list)
     packed_nbytes: int = 0
     retired_tail: tuple | None = None               # the tail buffers replaced by the last seal
-    append_args: tuple | None = None                # launch structure of the one-token append, per tail buffer pair
-
     sink_views: tuple | None = None                 # (count, key view, value view) handed out last
     runs: list = field(default_factory=list)        # what sealed the blocks: (last block, keys' owner, values' owner, blocks)
 
@@ -457,11 +455,49 @@ class InQuantCache(_HFCache):
                     raise ValueError("Only contiguous append positions are supported; reset before a new request")
         return layer
 
-    @torch.no_grad()
     def append_for_attention(self, key_states, value_states, layer_idx, cache_kwargs=None) -> PackedAttentionView:
         """Append one token without materialising history (reference ``cache.py:242-269``).
         The snapshot holds the blocks sealed BEFORE this append and a tail that ends with the
         new token; blocks sealed by this append are used from the next step on."""
+        self._flush_pending()
+        if not cache_kwargs and type(layer_idx) is int:
+            view = self._append_native(key_states, value_states, layer_idx)
+            if view is not None:
+                return view
+        with torch.no_grad():
+            return self._append_checked(key_states, value_states, layer_idx, cache_kwargs)
+
+    def _append_native(self, key_states, value_states, layer_idx):
+        """One token into the tail with nothing to seal, checked and launched in native code; None, with nothing
+        changed, for any other call."""
+        layer, cfg = self._layers.get(layer_idx), self.config
+        if layer is None or layer.tail_key_buffer is None:
+            return None
+        count, take_sink = layer.tail_count, layer.sink_count < cfg.sink_tokens
+        if count + 1 - take_sink - cfg.residual_length >= cfg.block_size or count >= self._tail_capacity() \
+                or (take_sink and layer.sink_key_buffer is None):
+            return None
+        old_sink = (layer.sink_key, layer.sink_value)
+        done = N.host().append_token(key_states, value_states, layer.tail_key_buffer, layer.tail_value_buffer,
+                                     layer.sink_key_buffer if take_sink else None, layer.sink_value_buffer if take_sink else None,
+                                     count, layer.sink_count if take_sink else -1, N.status_word(layer.device).data_ptr())
+        if done is not True:
+            if done is not None:
+                N.check(done, "inq_append_token")
+            return None
+        layer.sink_count += take_sink
+        layer.tail_count += 1 - take_sink
+        layer.seq_length += 1
+        view = PackedAttentionView(tuple(layer.key_blocks), tuple(layer.value_blocks), *old_sink,
+                                   layer.tail_key_buffer.narrow(2, 0, count + 1), layer.tail_value_buffer.narrow(2, 0, count + 1),
+                                   layer.seq_length)
+        if cfg.track_peak_bytes:
+            self.record_peak(layer_idx)
+        if layer_idx == 0:
+            self._seen_tokens = layer.seq_length
+        return view
+
+    def _append_checked(self, key_states, value_states, layer_idx, cache_kwargs) -> PackedAttentionView:
         layer = self._validate_update(key_states, value_states, layer_idx, cache_kwargs)
         if key_states.shape[2] != 1 or layer is None:
             raise ValueError("append_for_attention requires one new token after an existing prefill")
@@ -597,19 +633,14 @@ class InQuantCache(_HFCache):
         if (keys.stride(1) * es) % 16 or keys.stride(1) != values.stride(1):
             return False
         tk, tv = layer.tail_key_buffer, layer.tail_value_buffer
-        cached = layer.append_args
-        if cached is None or cached[0] != tk.data_ptr() or cached[1] != tv.data_ptr():
-            # what only changes when the tail buffers are replaced (a seal) is filled once
-            if tk.data_ptr() % 16 or tv.data_ptr() % 16 or tk.stride(-1) != 1 or tv.stride(-1) != 1:
-                return False
-            args = N.AppendArgs()
-            args.tail_key, args.tail_value = tk.data_ptr(), tv.data_ptr()
-            args.tail_stride_h, args.tail_stride_t = tk.stride(1) * es, tk.stride(2) * es
-            args.tail_capacity = tk.shape[2]
-            args.heads, args.row_bytes = layer.shape[1], row_bytes
-            args.status = N.status_word(layer.device).data_ptr()
-            cached = layer.append_args = (tk.data_ptr(), tv.data_ptr(), args, N.ctypes.byref(args))
-        args = cached[2]
+        if tk.data_ptr() % 16 or tv.data_ptr() % 16 or tk.stride(-1) != 1 or tv.stride(-1) != 1:
+            return False
+        args = N.AppendArgs()
+        args.tail_key, args.tail_value = tk.data_ptr(), tv.data_ptr()
+        args.tail_stride_h, args.tail_stride_t = tk.stride(1) * es, tk.stride(2) * es
+        args.tail_capacity = tk.shape[2]
+        args.heads, args.row_bytes = layer.shape[1], row_bytes
+        args.status = N.status_word(layer.device).data_ptr()
         args.key, args.value, args.src_stride_h = keys.data_ptr(), values.data_ptr(), keys.stride(1) * es
         args.tail_position = layer.tail_count
         args.sink_position = sink_position
@@ -617,7 +648,7 @@ class InQuantCache(_HFCache):
             sk, sv = layer.sink_key_buffer, layer.sink_value_buffer
             args.sink_key, args.sink_value = sk.data_ptr(), sv.data_ptr()
             args.sink_stride_h, args.sink_stride_t = sk.stride(1) * es, sk.stride(2) * es
-        N.check(N.library().inq_append_token(cached[3], N.stream_pointer(layer.device)), "inq_append_token")
+        N.check(N.library().inq_append_token(N.ctypes.byref(args), N.stream_pointer(layer.device)), "inq_append_token")
         return True
 
     def _append(self, layer: _Layer, keys, values, want_tail: bool = False, history=None):

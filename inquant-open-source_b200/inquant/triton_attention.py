@@ -121,13 +121,10 @@ class PackedDecodeState:
         self._value_salient = 0
         self._inquant_values = False
         self._preset = True
+        self._kind = None            # streaming_value_kind() of the blocks there are
         self._capacity = 0
         self._stream_identity = None
         self._record_counts = {}
-        self._checked_sink = None    # sink tensors that passed decode()'s checks, with the dtype and device they passed against
-        self._seq_struct = N.DecodeSeq()
-        self._args_struct = N.DecodeArgs()
-        self._args_struct.seq_host = N.ctypes.pointer(self._seq_struct)
         self.extend(key_blocks, value_blocks)
 
     def extend(self, key_blocks, value_blocks):
@@ -258,6 +255,7 @@ class PackedDecodeState:
         if self._inquant_values:
             self._write_maps(self._value_map[old_count:count], new_values, self._value_salient)
         self.key_blocks, self.value_blocks = tuple(key_blocks), tuple(value_blocks)
+        self._kind = self.streaming_value_kind()
 
     def _write_maps(self, result, blocks, count):
         """Roles: donor channel 0..127 for a salient channel, -1 normal, -2-i for the i-th donor
@@ -294,8 +292,56 @@ class PackedDecodeState:
             return 0, 128 // self._value_group
         return None
 
-    @torch.no_grad()
     def decode(self, query, *, sink_key=None, sink_value=None, residual_key=None, residual_value=None, scale=None):
+        # the ordinary call -- streaming kernel, 16-bit rows that are 16-byte vectors -- is checked and launched
+        # in native code; whatever it does not serve takes the checks and the errors below
+        if self._kind is not None and type(query) is torch.Tensor and query.device == self._device and query.ndim == 4:
+            output = self._decode_native(query, sink_key, sink_value, residual_key, residual_value, scale)
+            if output is not None:
+                return output
+        with torch.no_grad():
+            return self._decode_checked(query, sink_key, sink_value, residual_key, residual_value, scale)
+
+    def _decode_native(self, query, sink_key, sink_value, residual_key, residual_value, scale):
+        if scale is None:
+            scale = 128 ** -0.5
+        elif not math.isfinite(scale) or scale <= 0:
+            return None
+        device, kv_heads, n_blocks = self._device, self._kv_heads, len(self.key_blocks)
+        identity = N.stream_identity(device)
+        if identity != self._stream_identity:
+            return None
+        pairs = kv_heads * ((query.shape[1] // kv_heads + 7) // 8)
+        if not pairs:
+            return None
+        records = self._records(pairs, n_blocks)
+        if self._workspace_pool is not None:
+            workspace = self._workspace_pool.acquire_address(records * N.RECORD_FLOATS, device, identity)
+        else:
+            workspace = self._own_workspace(records, device)
+        kind, groups = self._kind
+        output = N.host().decode(query, sink_key, sink_value, residual_key, residual_value, scale, kv_heads, n_blocks,
+                                 self._packed_tokens, self._salient, kind, groups, self._tables.data_ptr(), self._key_map.data_ptr(),
+                                 self._value_map.data_ptr() if kind == 1 else 0, workspace, records * N.RECORD_FLOATS,
+                                 N.decode_counters(device, pairs, identity[1]).data_ptr(), N.status_word(device).data_ptr())
+        if type(output) is int:
+            N.check(output, "inq_decode_attention")
+        return output
+
+    def _records(self, pairs: int, n_blocks: int) -> int:
+        records = self._record_counts.get((pairs, n_blocks))
+        if records is None:
+            records = workspace_floats(pairs, pairs * pair_units(n_blocks, self._packed_tokens)) // N.RECORD_FLOATS
+            self._record_counts = {(pairs, n_blocks): records}     # one entry: the count changes when a block is sealed
+        return records
+
+    def _own_workspace(self, records: int, device) -> int:
+        shape = (records, N.RECORD_FLOATS)
+        if self._workspace is None or self._workspace.shape != shape or self._workspace.device != device:
+            self._workspace = torch.empty(shape, dtype=torch.float32, device=device)
+        return self._workspace.data_ptr()
+
+    def _decode_checked(self, query, sink_key, sink_value, residual_key, residual_value, scale):
         if query.ndim != 4 or query.shape[0] != 1 or query.shape[1] < 1 or query.shape[-2:] != (1, 128):
             raise ValueError("query must have shape [1, query_heads, 1, 128]")
         if query.device.type != "cuda" or query.dtype not in (torch.float16, torch.bfloat16, torch.float32):
@@ -306,18 +352,11 @@ class PackedDecodeState:
             raise ValueError("query and packed blocks must share a device")
         kv_heads = self._kv_heads
         dense = []
-        checked = self._checked_sink
         for name, key, value in (("sink", sink_key, sink_value), ("residual", residual_key, residual_value)):
             if (key is None) != (value is None):
                 raise ValueError(f"{name} key/value must both be provided")
             if key is None:
                 dense.append((None, None, 0))
-                continue
-            if name == "sink" and checked is not None and key is checked[0] and value is checked[1] \
-                    and query.dtype == checked[2] and query.device == checked[3]:
-                # the very tensors (a cache hands out the same sink views step after step) that passed
-                # the checks below on an earlier call, against a query of the same dtype and device
-                dense.append((checked[4], checked[5], checked[4].shape[2]))
                 continue
             if key.ndim != 4 or key.shape != value.shape or key.shape[0] != 1 or key.shape[-1] != 128:
                 raise ValueError(f"{name} K/V must have matching [1, KV_heads, tokens, 128] shapes")
@@ -328,13 +367,10 @@ class PackedDecodeState:
             kv_heads = key.shape[1] if kv_heads is None else kv_heads
             if key.shape[1] != kv_heads:
                 raise ValueError("All inputs must share their KV head count")
-            given = (key, value)
             if not N.dense_rows_aligned(key):
                 key = _aligned_copy(key)
             if not N.dense_rows_aligned(value):
                 value = _aligned_copy(value)
-            if name == "sink" and self._kv_heads is not None:
-                self._checked_sink = (*given, query.dtype, query.device, key, value)
             dense.append((key, value, key.shape[2]))
         if kv_heads is None or query.shape[1] % kv_heads:
             raise ValueError("query_heads must be divisible by the nonempty KV head count")
@@ -356,18 +392,12 @@ class PackedDecodeState:
                                         residual_key, residual_value, residual_t, scale)
         tiles = (q_per_kv + 7) // 8
         pairs = kv_heads * tiles
-        records = self._record_counts.get((pairs, n_blocks))
-        if records is None:
-            records = workspace_floats(pairs, pairs * pair_units(n_blocks, self._packed_tokens)) // N.RECORD_FLOATS
-            self._record_counts = {(pairs, n_blocks): records}     # one entry: the count changes when a block is sealed
-        workspace_shape = (records, N.RECORD_FLOATS)
+        records = self._records(pairs, n_blocks)
         workspace_floats_needed = records * N.RECORD_FLOATS
         if self._workspace_pool is not None:
             workspace_address = self._workspace_pool.acquire_address(workspace_floats_needed, query.device, identity)
         else:
-            if self._workspace is None or self._workspace.shape != workspace_shape or self._workspace.device != query.device:
-                self._workspace = torch.empty(workspace_shape, dtype=torch.float32, device=query.device)
-            workspace_address = self._workspace.data_ptr()
+            workspace_address = self._own_workspace(records, query.device)
         if query.data_ptr() % 16 or query.stride(1) % 8:     # rows of a head: 16-byte aligned (unit channel stride was checked)
             query = _aligned_copy(query)
         output = torch.empty(query.shape, dtype=query.dtype, device=query.device)
@@ -376,7 +406,7 @@ class PackedDecodeState:
             self._key_map = torch.empty((0, kv_heads, 128), dtype=torch.int8, device=query.device)
             self._value_map = torch.empty((0,), dtype=torch.int8, device=query.device)
             self._device = query.device
-        seq = self._seq_struct        # reused from call to call: every field a call may leave unset is reset below
+        seq = N.DecodeSeq()
         seq.query, seq.output, seq.query_head_stride = query.data_ptr(), output.data_ptr(), query.stride(1)
         seq.table = self._tables.data_ptr() if n_blocks else None
         seq.roles = self._key_map.data_ptr() if n_blocks else None
@@ -385,17 +415,13 @@ class PackedDecodeState:
             seq.sink_key, seq.sink_value = sink_key.data_ptr(), sink_value.data_ptr()
             seq.sink_key_stride_h, seq.sink_key_stride_t = sink_key.stride(1), sink_key.stride(2)
             seq.sink_value_stride_h, seq.sink_value_stride_t = sink_value.stride(1), sink_value.stride(2)
-        else:
-            seq.sink_key = seq.sink_value = None
         if residual_t:
             seq.tail_key, seq.tail_value = residual_key.data_ptr(), residual_value.data_ptr()
             seq.tail_key_stride_h, seq.tail_key_stride_t = residual_key.stride(1), residual_key.stride(2)
             seq.tail_value_stride_h, seq.tail_value_stride_t = residual_value.stride(1), residual_value.stride(2)
-        else:
-            seq.tail_key = seq.tail_value = None
         seq.n_blocks, seq.sink_tokens, seq.tail_tokens = n_blocks, sink_t, residual_t
-        args = self._args_struct
-        args.n_seq = 1
+        args = N.DecodeArgs()
+        args.n_seq, args.seq_host = 1, N.ctypes.pointer(seq)
         args.kv_heads, args.q_per_kv = kv_heads, q_per_kv
         args.block_tokens, args.n_pad = self._packed_tokens, self._salient
         args.layout, args.dtype, args.scale = 0, N.DTYPE_CODE[query.dtype], scale

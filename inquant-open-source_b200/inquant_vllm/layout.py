@@ -2,6 +2,7 @@
 (reference ``inquant_vllm/layout.py``).  Sealing runs the fused sm_100a encoders with the
 physical pages as their destination; nothing is staged."""
 from dataclasses import dataclass
+from functools import cached_property
 import math
 
 import torch
@@ -25,7 +26,7 @@ class PageLayout:
         if self.block_size not in (16, 32, 64, 128, 256) or self.dim != 128 or self.heads < 1:
             raise ValueError("Expected block_size 64/128/256, head_dim 128, positive KV heads")
 
-    @property
+    @cached_property
     def fields(self):
         b, h, d = self.block_size, self.heads, self.dim
         return (
@@ -38,7 +39,7 @@ class PageLayout:
             ("value_offsets", torch.float16, (h, b, d // 64)),
         )
 
-    @property
+    @cached_property
     def offsets(self):
         offset, result = 0, {}
         for name, dtype, shape in self.fields:
@@ -46,9 +47,20 @@ class PageLayout:
             offset += math.prod(shape) * dtype.itemsize
         return result
 
-    @property
+    @cached_property
     def page_bytes(self):
         return self.heads * (104 * self.block_size + 832)
+
+    @cached_property
+    def kernel_offsets(self):
+        """Offsets of the fields the decode kernel reads besides the key payload, in the order it takes them."""
+        o = self.offsets
+        return (o["key_scales"], o["key_map"], o["key_padding"], o["value_payload"], o["value_scales"], o["value_offsets"])
+
+    @cached_property
+    def _placed(self):
+        """Offset and bytes per head of every field."""
+        return {name: (self.offsets[name], math.prod(shape[1:]) * dtype.itemsize) for name, dtype, shape in self.fields}
 
     def views(self, pages):
         if pages.dtype != torch.uint8 or pages.ndim != 2 or pages.shape[1] != self.page_bytes:
@@ -62,11 +74,8 @@ class PageLayout:
 
     def field(self, pool: torch.Tensor, name: str) -> N.Field:
         """Destination descriptor of one field inside a page pool (C ABI ``inq_field_t``)."""
-        for fname, dtype, shape in self.fields:
-            if fname == name:
-                inner = math.prod(shape[1:]) * dtype.itemsize
-                return N.Field(pool.data_ptr() + self.offsets[name], self.page_bytes, inner)
-        raise KeyError(name)
+        offset, inner = self._placed[name]
+        return N.Field(pool.data_ptr() + offset, self.page_bytes, inner)
 
 
 def _check_pages(keys, values, layout):

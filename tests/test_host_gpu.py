@@ -1,0 +1,103 @@
+"""The native host side of the per-layer calls against the Python code behind it: what it serves gives the same
+bits, and what it does not serve takes the general path.  A tensor subclass is never served."""
+import pytest
+import torch
+
+import workloads
+
+pytestmark = pytest.mark.gpu
+
+
+class Wrapped(torch.Tensor):
+    pass
+
+
+def _rows(seed, heads, tokens, dtype, form):
+    """[1, heads, tokens, 128]: contiguous, token-major, a slice of a longer buffer, rows that are not 16-byte aligned."""
+    x = workloads.make_kv_torch(seed, heads, max(tokens, 1), "cuda", 128)[0].to(dtype)[:, :, :tokens]
+    if form == "token-major":
+        return x.transpose(1, 2).contiguous().transpose(1, 2)
+    if form == "slice":
+        buffer = torch.zeros((1, heads, tokens + 9, 128), dtype=dtype, device="cuda")
+        buffer[:, :, 5:5 + tokens] = x
+        return buffer[:, :, 5:5 + tokens]
+    if form == "unaligned":
+        buffer = torch.zeros(heads * tokens * 128 + 1, dtype=dtype, device="cuda")
+        buffer[1:] = x.reshape(-1)
+        return buffer[1:].view(1, heads, tokens, 128)
+    return x
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("form", ["contiguous", "token-major", "slice", "unaligned"])
+@pytest.mark.parametrize("value_bits,group,block", [(2, 64, 64), (None, 64, 64), (4, 32, 128), (2, 64, 48)])
+def test_decode_and_append_are_those_of_the_general_path(dtype, form, value_bits, group, block):
+    from inquant import _native as N
+    from inquant.cache import CacheConfig, InQuantCache
+    from inquant.codec import CodecConfig
+    from inquant.triton_attention import PackedDecodeState
+    heads, q_heads = 2, 14
+    config = CacheConfig(CodecConfig(donor_policy="min_error"), block_size=block, residual_length=40, sink_tokens=4, value_bits=value_bits,
+                         value_group_size=group, validate_positions=False)
+    caches = [InQuantCache(config) for _ in range(2)]
+    prompt = [_rows(s, heads, 3 + 2 * block, dtype, "contiguous") for s in (1, 2)]
+    states = [None, None]
+    for step in range(block // 2 + 60):
+        new = [_rows(10 * step + s, heads, 1, dtype, form) for s in (3, 4)]
+        query = _rows(10 * step + 5, q_heads, 1, dtype, form)
+        results = []
+        for i, cache in enumerate(caches):
+            if not step:
+                cache.update(prompt[0][:, :, :3], prompt[1][:, :, :3], 0)     # the sink is still filling
+                cache.append_for_attention(*(x[:, :, 3:4] if not i else x[:, :, 3:4].as_subclass(Wrapped) for x in prompt), 0)
+                cache.update(prompt[0][:, :, 4:], prompt[1][:, :, 4:], 0)
+            as_given = (lambda x: x) if not i else (lambda x: x.as_subclass(Wrapped))
+            view = cache.append_for_attention(*(as_given(x) for x in new), 0)
+            if states[i] is None:
+                states[i] = PackedDecodeState(view.key_blocks, view.value_blocks)
+            elif len(states[i].key_blocks) != len(view.key_blocks):
+                states[i].extend(view.key_blocks, view.value_blocks)
+            dense = (view.sink_key, view.sink_value, view.residual_key, view.residual_value)
+            out = states[i].decode(as_given(query), sink_key=dense[0], sink_value=dense[1], residual_key=dense[2], residual_value=dense[3])
+            results.append((*(t.as_subclass(torch.Tensor) for t in (*dense, out)), view.seq_length, len(view.key_blocks)))
+        assert all(torch.equal(a, b) if isinstance(a, torch.Tensor) else a == b for a, b in zip(*results)), step
+    assert N.take_status(torch.device("cuda", 0)) == 0
+
+
+@pytest.mark.parametrize("block,pages,tail,sink", [(16, 5, 7, 4), (64, 0, 3, 3), (64, 3, 0, 4), (256, 2, 100, 0)])
+def test_paged_decode_is_that_of_the_general_path(block, pages, tail, sink):
+    from inquant.triton_attention import SharedDecodeWorkspace
+    from inquant_vllm.kernels import paged_decode
+    from inquant_vllm.layout import PageLayout, pack_pages
+    heads, q_heads = 4, 28
+    layout, workspace = PageLayout(block, heads), SharedDecodeWorkspace()
+    pool = torch.zeros((pages + 1, layout.page_bytes), dtype=torch.uint8, device="cuda")
+    if pages:
+        k, v = (x[0].view(heads, pages, block, 128).transpose(0, 1) for x in workloads.make_kv_torch(6, heads, pages * block, "cuda", 128))
+        pool[:pages] = pack_pages(k.to(torch.bfloat16), v.to(torch.bfloat16), layout).view(pages, -1)
+    dense = torch.randn((2, heads, block + 4, 128), device="cuda").to(torch.bfloat16)
+    ids = torch.randperm(pages, device="cuda")
+    query = torch.randn((1, q_heads, 128), device="cuda").to(torch.bfloat16)
+    given = torch.empty_like(query)
+    outputs = [paged_decode(q, pool, i, dense, pages, tail, sink, layout, workspace, 128 ** -0.5, output=o)
+               for q, i, o in ((query, ids.int(), None), (query, ids.int(), given), (query, ids, None), (query.as_subclass(Wrapped), ids.int(), None))]
+    assert outputs[1] is given
+    assert all(torch.equal(o.as_subclass(torch.Tensor), outputs[0]) for o in outputs)
+
+
+def test_calls_outside_the_native_path_keep_their_errors():
+    from inquant.triton_attention import PackedDecodeState
+    from inquant.codec import CodecConfig, quantize
+    from inquant.value_codec import quantize_values
+    k = _rows(1, 2, 64, torch.bfloat16, "contiguous")
+    state = PackedDecodeState([quantize(k, CodecConfig(donor_policy="min_error"))], [quantize_values(k)])
+    q, tail = _rows(2, 4, 1, torch.bfloat16, "contiguous"), _rows(3, 2, 5, torch.bfloat16, "contiguous")
+    state.decode(q, residual_key=tail, residual_value=tail)
+    for query, args, error in ((q[:, :3], {}, "divisible"), (q[:, :1], {}, "divisible"), (q, {"scale": -1.0}, "positive and finite"), (q, {"scale": float("nan")}, "positive and finite"),
+                               (q, {"residual_key": tail}, "both be provided"), (q, {"residual_key": tail, "residual_value": tail[:, :, 1:]}, "matching"),
+                               (q, {"residual_key": tail.half(), "residual_value": tail.half()}, "match query dtype"),
+                               (q, {"sink_key": tail[:, :1], "sink_value": tail[:, :1]}, "KV head count"), (q[0], {}, "query must have shape")):
+        with pytest.raises(ValueError, match=error):
+            state.decode(query, **args)
+    with torch.cuda.stream(torch.cuda.Stream()), pytest.raises(RuntimeError, match="one CUDA stream"):
+        state.decode(q)
