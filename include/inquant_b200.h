@@ -265,7 +265,7 @@ typedef struct {
    * memory.  NULL is allowed when every sequence holds `uniform_blocks` blocks (with
    * seq_host the count is taken from the descriptor). */
   const int64_t* pair_starts;
-  int64_t total_units;      /* pair_starts[n_pairs]; ignored without pair_starts */
+  int64_t total_units;      /* pair_starts[n_pairs], below 2^31 less 88 per pair (4 TB of blocks); ignored without pair_starts */
   int32_t uniform_blocks;
   float* partials;          /* scratch, contents undefined on entry and exit */
   int64_t partials_floats;  /* its size: at least inq_decode_workspace_floats(n_pairs, total_units) */

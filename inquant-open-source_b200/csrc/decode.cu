@@ -123,8 +123,8 @@ struct DecodeParams {
   SeqDesc one;
   int n_seq, H, G, T, n_pad;
   int n_ctas, n_pairs;
-  long long per_cta, total_units, uniform_units;   // flat work decomposition (total_units counts the ramp units too)
-  long long ramp_units;                            // list positions every pair is charged for its fixed costs
+  int per_cta, total_units, uniform_units;         // flat work decomposition (total_units counts the ramp units too)
+  int ramp_units;                                  // list positions every pair is charged for its fixed costs
   const long long* pair_starts;                    // [n_pairs + 1] or nullptr when every pair has uniform_units
   float scale_log2e;
   long long page_bytes;
@@ -226,6 +226,13 @@ __device__ __forceinline__ unsigned hmul2_bits(unsigned a, unsigned b) {
   unsigned d;
   asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
+}
+// Counts an arrival for the whole GPU: everything the CTA did before the barrier ahead of it is visible to whoever
+// sees the count, and the other way round (one instruction in place of a fence of all threads and an addition).
+__device__ __forceinline__ int arrive_count(int* counter) {
+  int old;
+  asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
+  return old;
 }
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 // D = A*B with a zero accumulator (first step of a chain: nothing to keep live or to clear)
@@ -569,28 +576,36 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   // fixed cost a CTA pays per pair it touches (query staging, first copies, dense slices, record,
   // merge), so a CTA whose range crosses into the next pair is given fewer slices.  A CTA that
   // reaches only the ramp of a pair leaves that pair alone.
-  const long long R = P.ramp_units;
-  const long long c_begin = (long long)blockIdx.x * P.per_cta;
-  const long long c_end = min(c_begin + P.per_cta, P.total_units);
-  long long pos = c_begin;
+  // (the host refuses lists of 2^31 positions and more)
+  const int R = P.ramp_units, per_cta = P.per_cta;
+  const int c_begin = (int)blockIdx.x * per_cta;
+  const int c_end = min(c_begin + per_cta, P.total_units);
+  int pos = c_begin;
   int pair;
   if (P.pair_starts) {
-    int lo = 0, hi = P.n_pairs - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (P.pair_starts[mid] + mid * R <= pos) lo = mid; else hi = mid - 1;
+    // the last pair that starts at or before the range: every lane probes one place, so two rounds of loads
+    // find one of a thousand
+    pair = 0;
+    for (int n = P.n_pairs; n > 1;) {
+      const int step = (n + 31) >> 5, at = lane * step;
+      const bool before = at < n && (int)__ldg(P.pair_starts + pair + min(at, n - 1)) + (pair + at) * R <= pos;
+      const int k = 31 - __clz(__ballot_sync(0xffffffffu, before || lane == 0));
+      pair += k * step;
+      n = min(step, n - k * step);
     }
-    pair = lo;
   } else {
-    pair = (int)(pos / (P.uniform_units + R));
+    pair = pos / (P.uniform_units + R);
   }
+  bool arrived = false;   // this CTA has counted itself for the launch-wide advance below
+  int order = 0;          // the count it met
+  __shared__ int s_tail;
   for (; pos < c_end; ++pair) {
-  const long long pair_lo = (P.pair_starts ? P.pair_starts[pair] : (long long)pair * P.uniform_units) + (pair + 1) * R;   // first slice
-  const long long pair_hi = (P.pair_starts ? P.pair_starts[pair + 1] : (long long)(pair + 1) * P.uniform_units) + (pair + 1) * R;
-  const long long seg_lo = max(pos, pair_lo) - pair_lo, seg_hi = min(c_end, pair_hi) - pair_lo;
+  const int pair_lo = (P.pair_starts ? (int)__ldg(P.pair_starts + pair) : pair * P.uniform_units) + (pair + 1) * R;   // first slice
+  const int pair_hi = (P.pair_starts ? (int)__ldg(P.pair_starts + pair + 1) : (pair + 1) * P.uniform_units) + (pair + 1) * R;
+  const int seg_lo = max(pos, pair_lo) - pair_lo, seg_hi = min(c_end, pair_hi) - pair_lo;
   pos = min(c_end, pair_hi);
   if (seg_hi <= seg_lo) continue;   // only ramp positions of this pair fall into the range
-  const int first_cta = (int)(pair_lo / P.per_cta), last_cta = (int)((pair_hi - 1) / P.per_cta);
+  const int first_cta = pair_lo / per_cta, last_cta = (pair_hi - 1) / per_cta;
   const int n_cta_pair = last_cta - first_cta + 1;
   const int seq = pair / (P.H * gtiles);
   const int h = (pair / gtiles) % P.H, gt = pair % gtiles;
@@ -617,12 +632,193 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   const int n_blocks = SEQ(n_blocks);
   const int sink_tokens = SEQ(sink_tokens);
   const int* const tail_dev = SEQ(tail_tokens_dev);
-  const int tail_tokens = tail_dev ? *tail_dev : SEQ(tail_tokens);
+  // (one thread reads it, so that the CTA has read it once its threads have met)
+  if (threadIdx.x == 0) s_tail = tail_dev ? *tail_dev : SEQ(tail_tokens);
   const int g_valid = min(8, P.G - gt * 8);
   const long long q_head0 = (long long)h * P.G + gt * 8;
   const QT* qptr = (const QT*)SEQ(q);
   const long long q_stride = SEQ(q_stride_h);
 
+  // packed slices are cut evenly over all warps of this (sequence, KV head); the few dense
+  // slices are dealt round-robin so that no warp ends with a long exposed-latency tail
+  const int n_workers = n_cta_pair * kWarps, worker = ((int)blockIdx.x - first_cta) * kWarps + warp;
+  const int n_packed = n_blocks * spb;
+  const int pa = min(n_packed, seg_lo + (seg_hi - seg_lo) * warp / kWarps);
+  const int pb = min(n_packed, seg_lo + (seg_hi - seg_lo) * (warp + 1) / kWarps);
+  const int n_my = max(0, pb - pa);
+  int pf_block = (int)(pa / spb), pf_slice = (int)(pa % spb);   // prefetch cursor
+  auto locate = [&](int b) {
+    return locate_block<MODE, VK, VG>(P, d_table + (long long)b * 6, d_roles, d_pool, MODE == 1 ? d_pages[b] : 0, d_pool_pages, b, h, d_vroles);
+  };
+  BlockPtrs pf_ptrs = {};
+  if (n_my > 0 && !(FAST && SUB == 1)) pf_ptrs = locate(pf_block);
+  auto page_base = [&](int id) {
+    if (d_pool_pages > 0 && (unsigned)id >= (unsigned)d_pool_pages) {   // as in locate_block
+      atomicOr(P.status, INQ_STATUS_BAD_INDEX);
+      id = 0;
+    }
+    return d_pool + (long long)id * P.page_bytes;
+  };
+  int to_issue = n_my, issue_stage = 0;
+  int meta_block = -1;        // block whose metadata is staged (or in flight) in wmeta
+  int folded_block = -2;      // last block whose weights were derived from wmeta
+  auto stage_meta = [&](const BlockPtrs& bp, unsigned char* dst, int slot = 0) {
+    cp_async16(dst + lane * 16, bp.ks + lane * 16);
+    if (lane < (MODE == 0 ? 8 : 16)) cp_async16(dst + 512 + lane * 16, bp.kr + lane * 16);
+    for (int i = lane; i < n_pad; i += 32) cp_async4(dst + 768 + i * 4, bp.kpad + i * 4);
+    if (VK == 1) {
+      unsigned char* const vdst = wvmeta + slot * kValueMeta;
+      cp_async16(vdst + lane * 16, bp.vs + lane * 16);
+      if (lane < 8) cp_async16(vdst + 512 + lane * 16, bp.vr + lane * 16);
+      if (lane < 16) cp_async4(vdst + 640 + lane * 4, bp.vo + lane * 4);
+    }
+  };
+  // FAST: this lane's source pointers of the next slice to request (K rows, V rows, V scale and
+  // offset pairs), the shared-memory address of the stage it goes to, slices left in its block
+  const unsigned char* fk = pf_ptrs.kp + pf_slice * 2048 + lane * 16;
+  const unsigned char* fv = pf_ptrs.vp + pf_slice * (VK ? 2048 : 1024) + lane * 16;
+  constexpr int kParamLane = VK != 1 && VG == 4 ? 8 : 4;   // bytes of a parameter array one lane copies per slice
+  const unsigned char* fs = pf_ptrs.vs + pf_slice * (kStageP / 2) + lane * kParamLane;
+  const unsigned char* fo = pf_ptrs.vo + pf_slice * (kStageP / 2) + lane * kParamLane;
+  const unsigned ring_lo = smem_addr(ring), ring_hi = ring_lo + kRing * kStageBytes;
+  unsigned issue_addr = ring_lo;
+  int pf_left = spb - pf_slice;
+  // value rows in a stage.  2-bit values: 32 B per token, the halves of tokens 4..7 (mod 8) swapped.
+  // Coded values: 64 B per token like the keys, the 16-byte chunks XORed with (token / 2) % 4 so that
+  // the later ldmatrix reads of eight tokens' chunks fall into distinct banks.
+  const unsigned fast_v_dst = VK ? (unsigned)(kStageK + (lane >> 2) * 64 + (((lane & 3) ^ ((lane >> 3) & 3)) << 4))
+                                 : (unsigned)(kStageK + (((lane >> 1) * 2 + ((lane & 1) ^ ((lane >> 3) & 1))) << 4));
+  // Whole-slice path: where the next block lies is asked for one block ahead, its table row by a copy into
+  // slot block % 2 (which lands with the slice requested next) or its page id by a load into a register,
+  // so that a request that enters a block waits for neither.
+  int next_page = 0;
+  auto request_row = [&](int b) {
+    if (MODE == 0) {
+      if (lane < 6) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(wrow + (b & 1) * 8 + lane)), "l"(d_table + (long long)b * 6 + lane));
+    } else {
+      next_page = d_pages[b];
+    }
+  };
+  int page_after = 0;     // 16-token pages: the id after the next
+  if (FAST && SUB == 1) {
+    if (n_my > 0) next_page = d_pages[pf_block];
+    if (n_my > 1) page_after = d_pages[pf_block + 1];
+  } else if (FAST && n_my > 0) {
+    stage_meta(pf_ptrs, wmeta + (pf_block & 1) * 1024, pf_block & 1);   // the first block's metadata rides with its first slice
+    if (to_issue > pf_left) request_row(pf_block + 1);
+  }
+  // FAST with 16-token slices (paged layout): where this lane's copies start inside a page
+  const int page_k = h * 1024 + lane * 16, page_v = P.off_vp + h * 512 + lane * 16;
+  const int page_p = (lane < 16 ? P.off_vs : P.off_vo) + h * 64 + (lane & 15) * 4;
+  const int page_s = P.off_ks + h * 512 + lane * 16, page_r = P.off_km + h * 256 + (lane & 15) * 16, page_c = P.off_kp + h * 64 + (lane & 15) * 4;
+  auto issue = [&](bool ahead) {   // ahead: one of the requests before the loop
+    if (FAST && SUB == 1) {
+      if (to_issue > 0) {
+        const unsigned char* const page = page_base(next_page);
+        const unsigned dk = issue_addr + lane * 16, dv = issue_addr + fast_v_dst;
+        const unsigned dm = issue_addr + kMetaOffset;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dm + lane * 16), "l"(page + page_s));
+        if (lane < 16) {
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dm + 512 + lane * 16), "l"(page + page_r));
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dm + 768 + lane * 4), "l"(page + page_c));
+        }
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dk), "l"(page + page_k));
+        asm volatile("cp.async.cg.shared.global [%0+512], [%1+512], 16;" ::"r"(dk), "l"(page + page_k));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dv), "l"(page + page_v));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(issue_addr + kStageK + kStageV + lane * 4), "l"(page + page_p));
+        --to_issue;
+        issue_addr += kStageBytes;
+        if (issue_addr == ring_hi) issue_addr = ring_lo;
+        // ids are read two requests ahead
+        ++pf_block;
+        next_page = page_after;
+        if (to_issue > 1) page_after = d_pages[pf_block + 1];
+      }
+      cp_async_commit();
+      return;
+    }
+    if (FAST) {
+      if (to_issue > 0) {
+        const unsigned dk = issue_addr + lane * 16, dv = issue_addr + fast_v_dst;
+        const unsigned dp = issue_addr + kStageK + kStageV + lane * (VK != 1 && VG == 4 ? 8 : 4);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dk), "l"(fk));
+        asm volatile("cp.async.cg.shared.global [%0+512], [%1+512], 16;" ::"r"(dk), "l"(fk));
+        asm volatile("cp.async.cg.shared.global [%0+1024], [%1+1024], 16;" ::"r"(dk), "l"(fk));
+        asm volatile("cp.async.cg.shared.global [%0+1536], [%1+1536], 16;" ::"r"(dk), "l"(fk));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dv), "l"(fv));
+        asm volatile("cp.async.cg.shared.global [%0+512], [%1+512], 16;" ::"r"(dv), "l"(fv));
+        if (VK) {
+          asm volatile("cp.async.cg.shared.global [%0+1024], [%1+1024], 16;" ::"r"(dv), "l"(fv));
+          asm volatile("cp.async.cg.shared.global [%0+1536], [%1+1536], 16;" ::"r"(dv), "l"(fv));
+        }
+        if (VK != 1 && VG == 4) {
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dp), "l"(fs));
+          asm volatile("cp.async.ca.shared.global [%0+256], [%1], 8;" ::"r"(dp), "l"(fo));
+        } else if (VK != 1 && VG == 1) {
+          if (lane < 16) {
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dp), "l"(fs));
+            asm volatile("cp.async.ca.shared.global [%0+64], [%1], 4;" ::"r"(dp), "l"(fo));
+          }
+        } else if (VK != 1) {
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dp), "l"(fs));
+          asm volatile("cp.async.ca.shared.global [%0+128], [%1], 4;" ::"r"(dp), "l"(fo));
+        }
+        fk += 2048; fv += VK ? 2048 : 1024; fs += kStageP / 2; fo += kStageP / 2;
+        --to_issue;
+        issue_addr += kStageBytes;
+        if (issue_addr == ring_hi) issue_addr = ring_lo;
+        if (--pf_left == 0) {
+          pf_left = spb;
+          ++pf_block;
+          if (to_issue > 0) {
+            // the cursor enters a new block: its rows, and its metadata at once into slot block % 2.
+            // The cursor runs at most three slices ahead of the slice being consumed and a block has
+            // at least two, so the slot's previous block lies behind the consumed one or is the
+            // consumed one, whose fold precedes this request (see issue_late).
+            // Its row was requested a block ago, at least two requests back, so the wait at the top of this
+            // iteration covered it; the two requests ahead of the loop had no such wait.
+            pf_ptrs = ahead ? locate(pf_block)
+                            : locate_block<MODE, VK, VG>(P, wrow + (pf_block & 1) * 8, d_roles, d_pool, next_page, d_pool_pages, pf_block, h, d_vroles);
+            if (to_issue > spb) request_row(pf_block + 1);
+            fk = pf_ptrs.kp + lane * 16; fv = pf_ptrs.vp + lane * 16; fs = pf_ptrs.vs + lane * kParamLane; fo = pf_ptrs.vo + lane * kParamLane;
+            stage_meta(pf_ptrs, wmeta + (pf_block & 1) * 1024, pf_block & 1);
+          }
+        }
+      }
+      cp_async_commit();
+      return;
+    }
+    if (to_issue > 0) {
+      unsigned char* const stage_ptr = ring + issue_stage * kStageBytes;
+      if (kMetaInStage) {
+        // every slice is a whole block: its metadata travels in the slice's own stage
+        stage_meta(pf_ptrs, stage_ptr + kMetaOffset);
+      } else {
+        // a new block's metadata rides in the same group as its first slice, provided the
+        // staging area is no longer needed by an earlier block
+        const bool first_of_block = to_issue == n_my || pf_slice == 0;
+        if (first_of_block && (meta_block < 0 || folded_block == meta_block)) {
+          stage_meta(pf_ptrs, wmeta);
+          meta_block = pf_block;
+        }
+      }
+      stage_slice<kSub>(stage_ptr, pf_ptrs.kp, pf_ptrs.vp, pf_ptrs.vs, pf_ptrs.vo, pf_slice * kSliceTokens, T, lane);
+      --to_issue;
+      if (++issue_stage == kRing) issue_stage = 0;
+      if (++pf_slice == spb) {
+        pf_slice = 0;
+        ++pf_block;
+        if (to_issue > 0) pf_ptrs = locate(pf_block);
+      }
+    }
+    cp_async_commit();
+  };
+  // The first slices are requested ahead of everything else: their way through the look-up and memory is the longest
+  // chain of a short range, and staging the query hides in it.
+  if (n_my > 0) {
+#pragma unroll
+    for (int s = 0; s < kRing - 1; ++s) issue(true);
+  }
   // the merge of the previous pair may have used this scratch: start from an empty selection
   // matrix and an empty list of written cells
   for (int v = lane; v < groups * 128; v += 32) ((uint4*)wsel)[v] = make_uint4(0u, 0u, 0u, 0u);
@@ -678,13 +874,14 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
     if ((threadIdx.x & 15) == 0) qinv[g] = P.scale_log2e * __uint_as_float((unsigned)(127 + ex - 12) << 23);
   }
   __syncthreads();
-  const long long n_packed = (long long)n_blocks * spb;
+  const int tail_tokens = s_tail;
+  // The last pair of the range: this CTA has read its last tail length.  It counts itself now, so that the way to
+  // memory and back lies beside the work and not behind it (an exchange reads its step number at the end).
+  if (P.fused_append && !P.exchange && pos >= c_end) {
+    if (threadIdx.x == 0) order = arrive_count(P.counters + P.n_pairs);
+    arrived = true;
+  }
   const int sink_slices = (sink_tokens + 15) >> 4, tail_slices = (tail_tokens + 15) >> 4;
-  // packed slices are cut evenly over all warps of this (sequence, KV head); the few dense
-  // slices are dealt round-robin so that no warp ends with a long exposed-latency tail
-  const int n_workers = n_cta_pair * kWarps, worker = ((int)blockIdx.x - first_cta) * kWarps + warp;
-  const long long pa = min(n_packed, seg_lo + (seg_hi - seg_lo) * warp / kWarps);
-  const long long pb = min(n_packed, seg_lo + (seg_hi - seg_lo) * (warp + 1) / kWarps);
   // with a fused append the step's new token is one more dense slice: it is read from the caller's
   // rows (tail_tokens counts the tokens before it) and stored behind the tail for the next steps
   const bool has_new = P.fused_append && SEQ(new_k) != nullptr;
@@ -840,172 +1037,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   };
 
   // ---------------------------------------------------------------- packed history
-  if (pb > pa) {
-    const int n_my = (int)(pb - pa);
-    int pf_block = (int)(pa / spb), pf_slice = (int)(pa % spb);   // prefetch cursor
-    auto locate = [&](int b) {
-      return locate_block<MODE, VK, VG>(P, d_table + (long long)b * 6, d_roles, d_pool, MODE == 1 ? d_pages[b] : 0, d_pool_pages, b, h, d_vroles);
-    };
-    BlockPtrs pf_ptrs = {};
-    if (!(FAST && SUB == 1)) pf_ptrs = locate(pf_block);
-    auto page_base = [&](int id) {
-      if (d_pool_pages > 0 && (unsigned)id >= (unsigned)d_pool_pages) {   // as in locate_block
-        atomicOr(P.status, INQ_STATUS_BAD_INDEX);
-        id = 0;
-      }
-      return d_pool + (long long)id * P.page_bytes;
-    };
-    int to_issue = n_my, issue_stage = 0;
-    int meta_block = -1;        // block whose metadata is staged (or in flight) in wmeta
-    int folded_block = -2;      // last block whose weights were derived from wmeta
-    auto stage_meta = [&](const BlockPtrs& bp, unsigned char* dst, int slot = 0) {
-      cp_async16(dst + lane * 16, bp.ks + lane * 16);
-      if (lane < (MODE == 0 ? 8 : 16)) cp_async16(dst + 512 + lane * 16, bp.kr + lane * 16);
-      for (int i = lane; i < n_pad; i += 32) cp_async4(dst + 768 + i * 4, bp.kpad + i * 4);
-      if (VK == 1) {
-        unsigned char* const vdst = wvmeta + slot * kValueMeta;
-        cp_async16(vdst + lane * 16, bp.vs + lane * 16);
-        if (lane < 8) cp_async16(vdst + 512 + lane * 16, bp.vr + lane * 16);
-        if (lane < 16) cp_async4(vdst + 640 + lane * 4, bp.vo + lane * 4);
-      }
-    };
-    // FAST: this lane's source pointers of the next slice to request (K rows, V rows, V scale and
-    // offset pairs), the shared-memory address of the stage it goes to, slices left in its block
-    const unsigned char* fk = pf_ptrs.kp + pf_slice * 2048 + lane * 16;
-    const unsigned char* fv = pf_ptrs.vp + pf_slice * (VK ? 2048 : 1024) + lane * 16;
-    constexpr int kParamLane = VK != 1 && VG == 4 ? 8 : 4;   // bytes of a parameter array one lane copies per slice
-    const unsigned char* fs = pf_ptrs.vs + pf_slice * (kStageP / 2) + lane * kParamLane;
-    const unsigned char* fo = pf_ptrs.vo + pf_slice * (kStageP / 2) + lane * kParamLane;
-    const unsigned ring_lo = smem_addr(ring), ring_hi = ring_lo + kRing * kStageBytes;
-    unsigned issue_addr = ring_lo;
-    int pf_left = spb - pf_slice;
-    // value rows in a stage.  2-bit values: 32 B per token, the halves of tokens 4..7 (mod 8) swapped.
-    // Coded values: 64 B per token like the keys, the 16-byte chunks XORed with (token / 2) % 4 so that
-    // the later ldmatrix reads of eight tokens' chunks fall into distinct banks.
-    const unsigned fast_v_dst = VK ? (unsigned)(kStageK + (lane >> 2) * 64 + (((lane & 3) ^ ((lane >> 3) & 3)) << 4))
-                                   : (unsigned)(kStageK + (((lane >> 1) * 2 + ((lane & 1) ^ ((lane >> 3) & 1))) << 4));
-    // Whole-slice path: where the next block lies is asked for one block ahead, its table row by a copy into
-    // slot block % 2 (which lands with the slice requested next) or its page id by a load into a register,
-    // so that a request that enters a block waits for neither.
-    int next_page = 0;
-    auto request_row = [&](int b) {
-      if (MODE == 0) {
-        if (lane < 6) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(wrow + (b & 1) * 8 + lane)), "l"(d_table + (long long)b * 6 + lane));
-      } else {
-        next_page = d_pages[b];
-      }
-    };
-    if (FAST && SUB == 1) {
-      next_page = d_pages[pf_block];
-    } else if (FAST) {
-      stage_meta(pf_ptrs, wmeta + (pf_block & 1) * 1024, pf_block & 1);   // the first block's metadata rides with its first slice
-      if (to_issue > pf_left) request_row(pf_block + 1);
-    }
-    // FAST with 16-token slices (paged layout): where this lane's copies start inside a page
-    const int page_k = h * 1024 + lane * 16, page_v = P.off_vp + h * 512 + lane * 16;
-    const int page_p = (lane < 16 ? P.off_vs : P.off_vo) + h * 64 + (lane & 15) * 4;
-    const int page_s = P.off_ks + h * 512 + lane * 16, page_r = P.off_km + h * 256 + (lane & 15) * 16, page_c = P.off_kp + h * 64 + (lane & 15) * 4;
-    auto issue = [&](bool ahead) {   // ahead: one of the requests before the loop
-      if (FAST && SUB == 1) {
-        if (to_issue > 0) {
-          const unsigned char* const page = page_base(next_page);
-          const unsigned dk = issue_addr + lane * 16, dv = issue_addr + fast_v_dst;
-          const unsigned dm = issue_addr + kMetaOffset;
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dm + lane * 16), "l"(page + page_s));
-          if (lane < 16) {
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dm + 512 + lane * 16), "l"(page + page_r));
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dm + 768 + lane * 4), "l"(page + page_c));
-          }
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dk), "l"(page + page_k));
-          asm volatile("cp.async.cg.shared.global [%0+512], [%1+512], 16;" ::"r"(dk), "l"(page + page_k));
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dv), "l"(page + page_v));
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(issue_addr + kStageK + kStageV + lane * 4), "l"(page + page_p));
-          --to_issue;
-          issue_addr += kStageBytes;
-          if (issue_addr == ring_hi) issue_addr = ring_lo;
-          if (to_issue > 0) next_page = d_pages[++pf_block];   // needed by the next request only
-        }
-        cp_async_commit();
-        return;
-      }
-      if (FAST) {
-        if (to_issue > 0) {
-          const unsigned dk = issue_addr + lane * 16, dv = issue_addr + fast_v_dst;
-          const unsigned dp = issue_addr + kStageK + kStageV + lane * (VK != 1 && VG == 4 ? 8 : 4);
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dk), "l"(fk));
-          asm volatile("cp.async.cg.shared.global [%0+512], [%1+512], 16;" ::"r"(dk), "l"(fk));
-          asm volatile("cp.async.cg.shared.global [%0+1024], [%1+1024], 16;" ::"r"(dk), "l"(fk));
-          asm volatile("cp.async.cg.shared.global [%0+1536], [%1+1536], 16;" ::"r"(dk), "l"(fk));
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dv), "l"(fv));
-          asm volatile("cp.async.cg.shared.global [%0+512], [%1+512], 16;" ::"r"(dv), "l"(fv));
-          if (VK) {
-            asm volatile("cp.async.cg.shared.global [%0+1024], [%1+1024], 16;" ::"r"(dv), "l"(fv));
-            asm volatile("cp.async.cg.shared.global [%0+1536], [%1+1536], 16;" ::"r"(dv), "l"(fv));
-          }
-          if (VK != 1 && VG == 4) {
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dp), "l"(fs));
-            asm volatile("cp.async.ca.shared.global [%0+256], [%1], 8;" ::"r"(dp), "l"(fo));
-          } else if (VK != 1 && VG == 1) {
-            if (lane < 16) {
-              asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dp), "l"(fs));
-              asm volatile("cp.async.ca.shared.global [%0+64], [%1], 4;" ::"r"(dp), "l"(fo));
-            }
-          } else if (VK != 1) {
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dp), "l"(fs));
-            asm volatile("cp.async.ca.shared.global [%0+128], [%1], 4;" ::"r"(dp), "l"(fo));
-          }
-          fk += 2048; fv += VK ? 2048 : 1024; fs += kStageP / 2; fo += kStageP / 2;
-          --to_issue;
-          issue_addr += kStageBytes;
-          if (issue_addr == ring_hi) issue_addr = ring_lo;
-          if (--pf_left == 0) {
-            pf_left = spb;
-            ++pf_block;
-            if (to_issue > 0) {
-              // the cursor enters a new block: its rows, and its metadata at once into slot block % 2.
-              // The cursor runs at most three slices ahead of the slice being consumed and a block has
-              // at least two, so the slot's previous block lies behind the consumed one or is the
-              // consumed one, whose fold precedes this request (see issue_late).
-              // Its row was requested a block ago, at least two requests back, so the wait at the top of this
-              // iteration covered it; the two requests ahead of the loop had no such wait.
-              pf_ptrs = ahead ? locate(pf_block)
-                              : locate_block<MODE, VK, VG>(P, wrow + (pf_block & 1) * 8, d_roles, d_pool, next_page, d_pool_pages, pf_block, h, d_vroles);
-              if (to_issue > spb) request_row(pf_block + 1);
-              fk = pf_ptrs.kp + lane * 16; fv = pf_ptrs.vp + lane * 16; fs = pf_ptrs.vs + lane * kParamLane; fo = pf_ptrs.vo + lane * kParamLane;
-              stage_meta(pf_ptrs, wmeta + (pf_block & 1) * 1024, pf_block & 1);
-            }
-          }
-        }
-        cp_async_commit();
-        return;
-      }
-      if (to_issue > 0) {
-        unsigned char* const stage_ptr = ring + issue_stage * kStageBytes;
-        if (kMetaInStage) {
-          // every slice is a whole block: its metadata travels in the slice's own stage
-          stage_meta(pf_ptrs, stage_ptr + kMetaOffset);
-        } else {
-          // a new block's metadata rides in the same group as its first slice, provided the
-          // staging area is no longer needed by an earlier block
-          const bool first_of_block = to_issue == n_my || pf_slice == 0;
-          if (first_of_block && (meta_block < 0 || folded_block == meta_block)) {
-            stage_meta(pf_ptrs, wmeta);
-            meta_block = pf_block;
-          }
-        }
-        stage_slice<kSub>(stage_ptr, pf_ptrs.kp, pf_ptrs.vp, pf_ptrs.vs, pf_ptrs.vo, pf_slice * kSliceTokens, T, lane);
-        --to_issue;
-        if (++issue_stage == kRing) issue_stage = 0;
-        if (++pf_slice == spb) {
-          pf_slice = 0;
-          ++pf_block;
-          if (to_issue > 0) pf_ptrs = locate(pf_block);
-        }
-      }
-      cp_async_commit();
-    };
-#pragma unroll
-    for (int s = 0; s < kRing - 1; ++s) issue(true);
+  if (n_my > 0) {
     // the dense slices of this warp hide behind the DRAM latency of the first packed slices;
     // their contribution is brought into the packed loop's per-row units (powers of two)
     dense_part();
@@ -1957,20 +1989,20 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
     }
   }
   // ---------------------------------------------------------------- last CTA merges
-  __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
-    const int old = atomicAdd(P.counters + pair, 1);
-    s_is_last = (old == n_cta_pair - 1);
+    s_is_last = n_cta_pair == 1 || arrive_count(P.counters + pair) == n_cta_pair - 1;
     if (s_is_last) P.counters[pair] = 0;   // scratch is left zeroed for the next launch
   }
   __syncthreads();
   if (s_is_last) {
-  __threadfence();
     // A sequence decoded alone is cut into a hundred parts per pair, so this merge is written for
-    // many loads in flight: (m, l) of every (query head, part) are staged first, the weights
-    // come from shared memory, and each thread then sums 8 channels of one head over the parts
-    // with 16 vector loads outstanding.
+    // many loads in flight: (m, l) of every (query head, part) are staged first, and each thread then sums 8
+    // channels of one head over the parts, eight at a time; past the end the last part is fetched once more and
+    // weighted 0 (one by one, the four parts beyond eight of a pair of twelve were four trips to memory).
+    // Requesting the first eight together with (m, l) would save another, but the registers they stand in
+    // make the slice loop spill.
+    const int g = threadIdx.x >> 4, c8 = (threadIdx.x & 15) * 8;   // kThreads = 128: 8 heads x 16 threads
     float* mw = (float*)warp_base;                 // [8][np] running maxima, then weights
     const int np = n_cta_pair;
     float* lw = mw + 8 * np;                       // [8][np] partial normalisers
@@ -1978,6 +2010,14 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
     float* mtop = norm + 8;
     const float* base = P.partials + ((long long)first_cta + pair) * kRecordFloats;
     float* const partial = SEQ(partial_out);
+    auto fetch = [&](float4 (&a)[8], float4 (&b)[8], int p0) {   // (past the end the last part once more, weighted 0)
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float4* const at = (const float4*)(base + (long long)min(p0 + u, np - 1) * kRecordFloats + g * kRecordStride + c8);
+        a[u] = __ldcg(at);
+        b[u] = __ldcg(at + 1);
+      }
+    };
 #pragma unroll 4
     for (int i = threadIdx.x; i < 8 * np; i += kThreads) {
       const int g = i & 7, p = i >> 3;
@@ -1988,6 +2028,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
       }
     }
     __syncthreads();
+#pragma unroll 1
     for (int g = warp; g < g_valid; g += kWarps) {
       float top = kNegBig;
       for (int p = lane; p < np; p += 32) top = fmaxf(top, mw[g * np + p]);
@@ -2007,35 +2048,25 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
       }
     }
     __syncthreads();
-    const int g = threadIdx.x >> 4, c8 = (threadIdx.x & 15) * 8;   // kThreads = 128: 8 heads x 16 threads
     float4 ex_a = make_float4(0.f, 0.f, 0.f, 0.f), ex_b = ex_a;
     if (g < g_valid) {
       float o[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) o[k] = 0.f;
-      const float* rec = base + g * kRecordStride + c8;
       const float* wg = mw + g * np;
-      int p = 0;
-      for (; p + 8 <= np; p += 8) {
+      auto add = [&](const float4 (&a)[8], const float4 (&b)[8], int p0) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const float wt = p0 + u < np ? wg[p0 + u] : 0.f;
+          o[0] = fmaf(a[u].x, wt, o[0]); o[1] = fmaf(a[u].y, wt, o[1]); o[2] = fmaf(a[u].z, wt, o[2]); o[3] = fmaf(a[u].w, wt, o[3]);
+          o[4] = fmaf(b[u].x, wt, o[4]); o[5] = fmaf(b[u].y, wt, o[5]); o[6] = fmaf(b[u].z, wt, o[6]); o[7] = fmaf(b[u].w, wt, o[7]);
+        }
+      };
+#pragma unroll 1
+      for (int p0 = 0; p0 < np; p0 += 8) {
         float4 va[8], vb[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          va[u] = __ldcg((const float4*)(rec + (long long)(p + u) * kRecordFloats));
-          vb[u] = __ldcg((const float4*)(rec + (long long)(p + u) * kRecordFloats) + 1);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const float wt = wg[p + u];
-          o[0] = fmaf(va[u].x, wt, o[0]); o[1] = fmaf(va[u].y, wt, o[1]); o[2] = fmaf(va[u].z, wt, o[2]); o[3] = fmaf(va[u].w, wt, o[3]);
-          o[4] = fmaf(vb[u].x, wt, o[4]); o[5] = fmaf(vb[u].y, wt, o[5]); o[6] = fmaf(vb[u].z, wt, o[6]); o[7] = fmaf(vb[u].w, wt, o[7]);
-        }
-      }
-      for (; p < np; ++p) {
-        const float4 va = __ldcg((const float4*)(rec + (long long)p * kRecordFloats));
-        const float4 vb = __ldcg((const float4*)(rec + (long long)p * kRecordFloats) + 1);
-        const float wt = wg[p];
-        o[0] = fmaf(va.x, wt, o[0]); o[1] = fmaf(va.y, wt, o[1]); o[2] = fmaf(va.z, wt, o[2]); o[3] = fmaf(va.w, wt, o[3]);
-        o[4] = fmaf(vb.x, wt, o[4]); o[5] = fmaf(vb.y, wt, o[5]); o[6] = fmaf(vb.z, wt, o[6]); o[7] = fmaf(vb.w, wt, o[7]);
+        fetch(va, vb, p0);
+        add(va, vb, p0);
       }
       if (P.exchange) {
         // handed to the exchange below (every thread of the CTA takes part in it)
@@ -2073,9 +2104,8 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
     __shared__ int s_grid_last;
     __syncthreads();
     if (threadIdx.x == 0) {
-      __threadfence();
-      const int old = atomicAdd(P.counters + P.n_pairs, 1);
-      s_grid_last = old == (int)gridDim.x - 1;
+      if (!arrived) order = arrive_count(P.counters + P.n_pairs);
+      s_grid_last = order == (int)gridDim.x - 1;
       if (s_grid_last) P.counters[P.n_pairs] = 0;
     }
     __syncthreads();
@@ -2182,6 +2212,26 @@ static Plan make_plan(long long total_units, int n_pairs, long long uniform_unit
   p.total = total_units + ramp * n_pairs;
   p.per_cta = (p.total + n - 1) / n;
   p.n_ctas = (int)((p.total + p.per_cta - 1) / p.per_cta);
+  // Pairs of equal length, few slices each: a range that crosses into the next pair visits two, and the second
+  // visit is as long as the ramp charge says, which a short range cannot make up for with fewer slices.  So every
+  // pair gets ranges of its own where these are no longer than a shared range with the full charge: whole
+  // slices per warp, the positions left over at the pair's start (its first CTA has the dense slices to do).
+  // us per launch in graphs of 20, shared ranges / ranges of their own: one layer of 8 heads, pages of 64, 1000 /
+  // 3000 / 8000 tokens 13.3 / 10.4, 14.7 / 10.4, 17.2 / 14.1; one layer of 4 heads, 4096 tokens 16.4 / 12.8; 28
+  // layers of 1999 tokens 23.8 / 20.5, of 4096 28.9 / 28.0.  From 8192 tokens in 28 layers on the rule keeps shared
+  // ranges.
+  const long long most = std::min(slots / n_pairs, 64ll);   // ranges of a pair
+  if (uniform_units > 0 && most > 0) {
+    long long per = std::max((uniform_units + most - 1) / most, 2ll * kWarps);
+    per = (per + kWarps - 1) / kWarps * kWarps;
+    if (per * n <= (uniform_units + kRampUnits) * n_pairs) {
+      const long long parts = (uniform_units + per - 1) / per;
+      p.per_cta = per;
+      p.ramp_units = parts * per - uniform_units;
+      p.total = parts * per * n_pairs;
+      p.n_ctas = (int)(parts * n_pairs);
+    }
+  }
   return p;
 }
 
@@ -2201,8 +2251,9 @@ extern "C" int64_t inq_decode_units(int32_t n_blocks, int32_t block_tokens) {
 }
 
 extern "C" int64_t inq_decode_workspace_floats(int32_t n_pairs, int64_t total_units) {
-  const Plan p = make_plan(total_units > n_pairs ? total_units : n_pairs, n_pairs, 0, 8);
-  return ((int64_t)p.n_ctas + n_pairs) * kRecordFloats;
+  // (pairs of equal length may have one range more each than an even cut of the whole list)
+  const long long most = std::min<long long>(8ll * sm_count(), std::max<long long>(total_units / 8, 1));
+  return ((int64_t)most + 2 * n_pairs) * kRecordFloats;
 }
 
 extern "C" int inq_decode_launch_shape(int32_t n_pairs, int64_t total_units, int32_t block_tokens, int32_t n_pad, int32_t value_kind,
@@ -2317,6 +2368,7 @@ extern "C" int inq_decode_attention(const inq_decode_args_t* a, inq_stream_t str
     }
     resident = d.per_sm[which][groups];
   }
+  if (total + (kRampUnits + 64) * n_pairs >= (1ll << 31) - 65536) return INQ_ERR_UNSUPPORTED;   // 32-bit list positions (4 TB of blocks)
   const Plan plan = make_plan(total, (int)n_pairs, uniform, resident);
   if (((long long)plan.n_ctas + n_pairs) * kRecordFloats > a->partials_floats) return INQ_ERR_CAPACITY;
   const int shared = launch_smem(scratch, shared_limit, plan.n_ctas);
@@ -2331,10 +2383,10 @@ extern "C" int inq_decode_attention(const inq_decode_args_t* a, inq_stream_t str
   P.n_pad = a->n_pad;
   P.n_ctas = plan.n_ctas;
   P.n_pairs = plan.n_pairs;
-  P.per_cta = plan.per_cta;
-  P.total_units = plan.total;
-  P.uniform_units = plan.uniform_units;
-  P.ramp_units = plan.ramp_units;
+  P.per_cta = (int)plan.per_cta;
+  P.total_units = (int)plan.total;
+  P.uniform_units = (int)plan.uniform_units;
+  P.ramp_units = (int)plan.ramp_units;
   P.pair_starts = (const long long*)a->pair_starts;
   P.scale_log2e = a->scale * 1.4426950408889634f;
   P.page_bytes = a->page_bytes;

@@ -136,6 +136,9 @@ class DecodeBatch:
         # prefix sums of the work units of every (sequence, KV head, head tile) pair
         units = [int(N.library().inq_decode_units(self._blocks_of(s), self.block_tokens))
                  for s in sequences for _ in range(self.kv_heads * tiles)]
+        # sequences of one length need no list: the kernel divides, and short pairs get ranges of their own
+        blocks = {self._blocks_of(s) for s in sequences}
+        self.uniform_blocks = blocks.pop() if len(blocks) == 1 else None
         starts = torch.tensor([0] + units, dtype=torch.int64).cumsum(0)
         self.total_units = int(starts[-1])
         self.pair_starts = starts.to(self.device)
@@ -254,6 +257,8 @@ class DecodeBatch:
             from inquant_vllm.kernels import page_offsets_array
             args.page_bytes, args.page_offsets = self.layout.page_bytes, page_offsets_array(self.layout)
         args.pair_starts, args.total_units = self.pair_starts.data_ptr(), self.total_units
+        if self.uniform_blocks is not None:
+            args.pair_starts, args.uniform_blocks = None, self.uniform_blocks
         args.partials, args.partials_floats = self.partials.data_ptr(), self.partials.numel()
         args.counters = self.counters.data_ptr()
         args.status = N.status_word(self.device).data_ptr()

@@ -193,3 +193,46 @@ def test_a_long_request_beside_short_ones_at_one_kv_head(fraction):
         p = torch.softmax(batch.queries[i].double() @ k.T * 128 ** -0.5, -1)
         attention_close(to_numpy(out[i].float()), to_numpy(p @ v))
     assert N.take_status(batch.device) == 0
+
+
+@pytest.mark.parametrize("layers,heads,q_heads,tokens", [(1, 1, 1, 45), (1, 2, 16, 130), (1, 4, 28, 1100), (1, 8, 32, 6000), (3, 2, 14, 700), (28, 4, 28, 500),
+                                                         (150, 1, 8, 300), (120, 4, 28, 200)])
+def test_sequences_of_one_length_with_ranges_of_their_own(layers, heads, q_heads, tokens):
+    """Short pairs of equal length get whole ranges each, longer ones share: the same batch with the list of pair
+    starts always shares.  Both against one another (an output differs by the merge's order and the lagging
+    maxima: an fp16 rounding of the probabilities here and there) and each sequence decoded by itself."""
+    from inquant.batched import DecodeBatch, SequenceState
+    caches = [_cache(tokens, i, heads=heads)[0] for i in range(min(layers, 6))]
+    batch = DecodeBatch([SequenceState.from_cache_layer(caches[i % len(caches)], 0) for i in range(layers)], q_heads, torch.bfloat16)
+    assert batch.uniform_blocks is not None
+    batch.queries.copy_(torch.randn(batch.queries.shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(tokens)))
+    own = batch.attend().clone()
+    batch.uniform_blocks = None
+    batch._prepare_launch_arguments()
+    shared = batch.attend().clone()
+    for i in range(0, layers, max(1, layers // 5)):
+        s = batch.sequences[i]
+        alone = s.decode_state.decode(batch.queries[i][None, :, None], sink_key=s.sink_key, sink_value=s.sink_value,
+                                      residual_key=s.tail_key_buffer[:, :, :s.tail_count], residual_value=s.tail_value_buffer[:, :, :s.tail_count])
+        for out in (own[i], shared[i]):
+            attention_close(to_numpy(out.float()), to_numpy(alone.float()).reshape(q_heads, 128), max_abs=1e-2)
+    attention_close(to_numpy(own.float()).reshape(-1, 128), to_numpy(shared.float()).reshape(-1, 128), max_abs=1e-2)
+
+
+@pytest.mark.parametrize("sequences", [3, 17, 33, 260])
+def test_ranges_find_their_pair_among_many_of_uneven_length(sequences):
+    from inquant.batched import DecodeBatch, SequenceState
+    caches = [_cache(n, n, heads=2)[0] for n in (40, 170, 400, 1500)]
+    order = torch.randint(0, 4, (sequences,), generator=torch.Generator().manual_seed(sequences)).tolist()
+    batch = DecodeBatch([SequenceState.from_cache_layer(caches[k], 0) for k in order], 20, torch.bfloat16)   # two tiles of query heads
+    assert batch.uniform_blocks is None
+    batch.queries.copy_(torch.randn((1, 20, 128), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).expand(sequences, -1, -1))
+    out = batch.attend()
+    for k in range(4):
+        rows = [i for i, o in enumerate(order) if o == k]
+        if rows:
+            s = batch.sequences[rows[0]]
+            alone = s.decode_state.decode(batch.queries[0][None, :, None], sink_key=s.sink_key, sink_value=s.sink_value,
+                                          residual_key=s.tail_key_buffer[:, :, :s.tail_count], residual_value=s.tail_value_buffer[:, :, :s.tail_count])
+            for i in rows:
+                attention_close(to_numpy(out[i].float()), to_numpy(alone.float()).reshape(20, 128), max_abs=1e-2)
