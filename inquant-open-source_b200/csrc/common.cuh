@@ -20,6 +20,30 @@ int fail_cuda(cudaError_t err, const char* where);
     if (inq_err__ != cudaSuccess) return inq::fail_cuda(inq_err__, #expr); \
   } while (0)
 
+// A launch that may be set up while the launch before it in the stream still runs: its CTAs take the places that
+// fall free and stand in follow_stream() until everything before is complete and visible.  Every thread of such a
+// kernel calls it before its first access to global memory and before anything that CTAs of different launches
+// compete for while they run (tensor memory): a launch that has yet to take what a waiting one holds would never
+// end.  For the same reason allow_next(), after which the launch behind this one may be set up, comes after the
+// allocation.  Only for kernels of one CTA per SM or of CTAs too small to matter: CTAs set up early go to the SMs
+// that fall free first and stay there (the decode kernel, one layer of 16384 tokens, 19.1 -> 23.9 us).
+template <typename... P, typename... A>
+inline cudaError_t launch_following(void (*kernel)(P...), dim3 grid, dim3 block, size_t shared, cudaStream_t stream, const A&... args) {
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = shared;
+  config.stream = stream;
+  config.attrs = &early;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, args...);
+}
+__device__ __forceinline__ void follow_stream() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <typename T>
 __device__ __forceinline__ float to_float(T v);
 template <>

@@ -216,3 +216,39 @@ def test_prefill_history_without_a_dense_copy_rebuilds_from_the_packed_cache():
     assert 0 < history.nbytes <= 2 * heads * 1024 * 128 * 2     # one pair for both layers, grown geometrically
     history.release()
     assert history.nbytes == 0
+
+
+@pytest.mark.parametrize("q_heads,kv_heads,q_tokens,kv_tokens", [(4, 2, 96, 96), (28, 4, 256, 2048), (28, 4, 1100, 1100)])   # one item per head, cut items with a merge, several rounds
+@pytest.mark.parametrize("captured", [False, True])
+def test_launches_in_a_row_read_what_the_one_before_wrote(q_heads, kv_heads, q_tokens, kv_tokens, captured):
+    """A launch is set up while the one before it runs: every pass reads the output of the pass before it as its
+    queries, inputs that a copy has just written, and writes over inputs that the pass before it read."""
+    from inquant.prefill import prefill_attention
+    gen = torch.Generator(device="cuda").manual_seed(q_tokens)
+    start, k0, v0 = (torch.randn((1, h, t, 128), device="cuda", generator=gen).to(torch.bfloat16)
+                     for h, t in ((q_heads, q_tokens), (kv_heads, kv_tokens), (kv_heads, kv_tokens)))
+    q, k, v = torch.empty_like(start), torch.empty_like(k0), torch.empty_like(v0)
+
+    def chain(settle):
+        q.copy_(start), k.copy_(k0), v.copy_(v0)
+        for i in range(6):
+            settle()
+            out = prefill_attention(q, k, v)
+            settle()
+            prefill_attention(out, k, v, out=q)      # writes what the pass before it read
+            settle()
+            if i % 2:
+                k.mul_(-1.0)
+                settle()
+        return q
+
+    expected = chain(torch.cuda.synchronize).clone()
+    if captured:
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            chain(lambda: None)
+        graph.replay()
+    else:
+        chain(lambda: None)
+    torch.cuda.synchronize()
+    assert torch.isfinite(expected.float()).all() and torch.equal(q, expected)
