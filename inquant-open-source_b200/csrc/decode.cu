@@ -214,6 +214,15 @@ __device__ __forceinline__ unsigned lds32(unsigned addr) {
   asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(addr), "n"(OFF));
   return v;
 }
+__device__ __forceinline__ unsigned lds16(unsigned addr) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ unsigned clamp_s16x2(unsigned x, unsigned lo, unsigned hi) {
+  asm("min.s16x2 %0, %0, %1;\n\tmax.s16x2 %0, %0, %2;" : "+r"(x) : "r"(hi), "r"(lo));
+  return x;
+}
 // four transposed 8x8 b16 matrices: register i of lane (r, j) holds elements (2j, r) and (2j+1, r) of matrix i
 template <int OFF>
 __device__ __forceinline__ uint4 ldsm4_trans(unsigned addr) {
@@ -521,12 +530,18 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   // 32-token slice of 256-token blocks 985 of 2993 cycles, per 16-token page 5000 of 6700.  Straight-line, with the
   // look-up one block ahead, they are 630 and 1740, and a launch takes (us, before -> after, L2 warm) 129 -> 120
   // (28 layers x 4 heads x 32768 tokens), 93.5 -> 86.5 (16384 tokens, values coded like the keys), 3084 -> 2668
-  // (16 requests x 32 layers x 8 heads, pages of 64) and 7272 -> 4201 (pages of 16).
+  // (16 requests x 32 layers x 8 heads, pages of 64) and 7272 -> 4201 (pages of 16).  The kernel runs at the power cap
+  // and close to the ALU's issue rate (280 of the 608 instructions per 16-token page): roles clamped two at a time, one
+  // fused add and minimum per channel for its record, the selection cell from a table and query addresses ready in the
+  // records took (us) 114.9 -> 112.4 (28 layers x 32768), 2639 -> 2624 and 4112 -> 3927.
   constexpr bool kNarrow = FAST || (SUB == 1 && !WIDE);
   // every slice is a block of its own: its weights are multiplied out where the score MMAs read them
   constexpr bool kDirect = SUB == 1 && kNarrow;
   constexpr bool kMetaInStage = SliceCfg<SUB, VK, VG>::kStageMeta > 0;   // host guarantees one slice per block
   constexpr int kMetaOffset = kStageK + kStageV + kStageP;
+  // staged metadata: K scales 512 B | role map 256 B | with kNarrow a zero, which stands for a role that is asked for
+  // in vain (16 B) | padding
+  constexpr int kMetaPad = kNarrow ? 784 : 768;
   extern __shared__ __align__(16) unsigned char smem[];
   float* qs = (float*)smem;                                             // 8 heads x 4 chunks x kQChunk
   // kNarrow: the staged query times 2^-12 in the model dtype, 8 heads x kQRow, in the place of qs
@@ -546,8 +561,8 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   // are being derived the same 2 KB hold the per-channel slot weights and additive constants
   unsigned char* wW = wb;
   float* wssc = (float*)(wb + (kDirect ? 0 : 2048));                                    // scale of salient channel i
-  // kNarrow: record i = {scale, source channel | donor slot << 8} of salient channel i; record 16 takes
-  // what the regular channels write
+  // kNarrow: record 15 - i = {scale, 2 x source channel | 2 x donor slot << 16} of salient channel i; record 16
+  // takes what the regular channels write
   uint2* wrec = (uint2*)wssc;
   unsigned char* wsrc = (unsigned char*)(wssc + 64);                    // channel of salient i
   unsigned char* wdon = wsrc + 64;                                      // its donor slot
@@ -568,6 +583,12 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   float* wvx = (float*)(wvkind + 32 * 16);                              // [16 list entries][8 heads] low-nibble sums
   unsigned char* ring = (unsigned char*)wcell + groups * 64 + (VK == 1 ? kValueScratch : 0);
   __shared__ int s_is_last;
+  // kNarrow: where a channel's nibble stands in the selection matrix (byte offset within column 0)
+  __shared__ unsigned short s_cell[kNarrow && SAL ? kThreads : 1];
+  if (kNarrow && SAL) {
+    const int jj = threadIdx.x >> 5, u = threadIdx.x & 31;
+    s_cell[threadIdx.x] = (unsigned short)(((2 * (u >> 3) + ((u >> 1) & 1)) * 32 + jj) * 8 + (u & 1) * 4 + ((u >> 2) & 1) * 2);
+  }
 
   // Flat decomposition: the packed slices of all (sequence, KV head, head tile) pairs form one
   // list that is cut into gridDim.x equal ranges; a CTA walks its range pair by pair.
@@ -665,7 +686,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   auto stage_meta = [&](const BlockPtrs& bp, unsigned char* dst, int slot = 0) {
     cp_async16(dst + lane * 16, bp.ks + lane * 16);
     if (lane < (MODE == 0 ? 8 : 16)) cp_async16(dst + 512 + lane * 16, bp.kr + lane * 16);
-    for (int i = lane; i < n_pad; i += 32) cp_async4(dst + 768 + i * 4, bp.kpad + i * 4);
+    for (int i = lane; i < n_pad; i += 32) cp_async4(dst + kMetaPad + i * 4, bp.kpad + i * 4);
     if (VK == 1) {
       unsigned char* const vdst = wvmeta + slot * kValueMeta;
       cp_async16(vdst + lane * 16, bp.vs + lane * 16);
@@ -720,7 +741,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dm + lane * 16), "l"(page + page_s));
         if (lane < 16) {
           asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dm + 512 + lane * 16), "l"(page + page_r));
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dm + 768 + lane * 4), "l"(page + page_c));
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dm + kMetaPad + lane * 4), "l"(page + page_c));
         }
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dk), "l"(page + page_k));
         asm volatile("cp.async.cg.shared.global [%0+512], [%1+512], 16;" ::"r"(dk), "l"(page + page_k));
@@ -822,6 +843,8 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   // the merge of the previous pair may have used this scratch: start from an empty selection
   // matrix and an empty list of written cells
   for (int v = lane; v < groups * 128; v += 32) ((uint4*)wsel)[v] = make_uint4(0u, 0u, 0u, 0u);
+  if (kNarrow && lane < (kMetaInStage ? kRing : 2))
+    *(int*)((kMetaInStage ? ring + lane * kStageBytes + kMetaOffset : wmeta + lane * 1024) + (MODE == 0 ? 640 : 768)) = 0;
   for (int v = lane; v < 64; v += 32) wssc[v] = 0.f;   // scales of unused salient slots must be finite
   if (!kNarrow)
     for (int v = lane; v < groups * 32; v += 32) wcell[v] = 0;
@@ -1197,30 +1220,38 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
         const float2 sa = *(const float2*)(meta + c0 * 4), sb = *(const float2*)(meta + c0 * 4 + 16);
         const float scv[4] = {sa.x, sa.y, sb.x, sb.y};
         int role[4], partner[4];
+        bool bad;
         if (MODE == 0) {
           const int ra = *(const short*)(roles8 + c0), rb = *(const short*)(roles8 + c0 + 4);
-          role[0] = (int)(signed char)ra; role[1] = ra >> 8; role[2] = (int)(signed char)rb; role[3] = rb >> 8;
+          const int word[4] = {(int)(signed char)ra, ra >> 8, (int)(signed char)rb, rb >> 8};
+          bad = false;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            role[i] = max(word[i], -1 - n_pad);
+            bad |= role[i] != word[i];
+          }
         } else {
-          const int ra = *(const int*)(roles16 + c0), rb = *(const int*)(roles16 + c0 + 4);
-          role[0] = (int)(short)ra; role[1] = ra >> 16; role[2] = (int)(short)rb; role[3] = rb >> 16;
+          const unsigned ra = *(const unsigned*)(roles16 + c0), rb = *(const unsigned*)(roles16 + c0 + 4);
+          const unsigned least = (unsigned)(-1 - n_pad) * 0x10001u + 0x10000u;   // -1 - n_pad in both halves
+          const unsigned fa = clamp_s16x2(ra, least, 0x007f007fu), fb = clamp_s16x2(rb, least, 0x007f007fu);
+          bad = fa != ra || fb != rb;
+          role[0] = (int)(short)fa; role[1] = (int)fa >> 16; role[2] = (int)(short)fb; role[3] = (int)fb >> 16;
         }
         float pad[4] = {0.f, 0.f, 0.f, 0.f};   // padding list entries 2j, 2j+1, 2j+8, 2j+9
         if (SAL) {
-          const float2 pa2 = *(const float2*)(meta + 768 + 8 * j), pb2 = *(const float2*)(meta + 800 + 8 * j);
+          const float2 pa2 = *(const float2*)(meta + kMetaPad + 8 * j), pb2 = *(const float2*)(meta + kMetaPad + 32 + 8 * j);
           pad[0] = pa2.x; pad[1] = pa2.y; pad[2] = pb2.x; pad[3] = pb2.y;
           if (!FAST) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) pad[k] = 2 * j + (k & 1) + 8 * (k >> 1) < n_pad ? pad[k] : 0.f;
           }
         }
-        bool bad = false;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const bool wrong = role[i] > 127 || role[i] < -1 - n_pad;
-          bad |= wrong;
-          role[i] = wrong ? -1 : role[i];
-          // a salient channel's role is its donor slot, whose own role tells the index in the lists
-          partner[i] = MODE == 0 ? (int)roles8[max(role[i], 0)] : (int)roles16[max(role[i], 0)];
+          // a salient channel's role is its donor slot, whose own role tells the index in the lists; the others
+          // read a zero behind the map
+          const int at = (int)min((unsigned)role[i], 128u);
+          partner[i] = MODE == 0 ? (int)roles8[at] : (int)roles16[at];
         }
         // the block's scales are brought into [0, 2) by a power of two
         unsigned top = __float_as_uint(fmaxf(fmaxf(fabsf(scv[0]), fabsf(scv[1])), fmaxf(fabsf(scv[2]), fabsf(scv[3]))));
@@ -1232,16 +1263,14 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
         for (int i = 0; i < 4; ++i) {
           // a regular channel; the odd channel of a byte is its high nibble: 16 times the code as an fp16
           // subnormal.  Salient channels are rebuilt exactly below, donor slots hold their low nibbles
-          fv[i] = role[i] == -1 ? scv[i] * ((i & 1) ? 0.0625f * down : down) : 0.f;
+          const float scaled = scv[i] * down;
+          fv[i] = role[i] == -1 ? ((i & 1) ? scaled * 0.0625f : scaled) : 0.f;
           if (SAL) {
-            const bool salient = role[i] >= 0;
-            const int idx = -partner[i] - 2;
-            const bool listed = salient && (unsigned)idx < (unsigned)n_pad;
-            bad |= salient && !listed;
-            // the scale in the units of the score accumulator (see below); the second code of a gather column
-            // carries a factor 1/512
-            wrec[listed ? idx : 16] = make_uint2(__float_as_uint(scv[i] * (down * ((idx & 8) ? 0.125f : (1.f / 4096.f)))),
-                                                 (unsigned)(c0 + (i & 1) + 4 * (i >> 1)) | ((unsigned)role[i] << 8));
+            // list entry idx is the donor's role -2 - idx: it stands in record 15 - idx, everything else in record 16
+            const unsigned at = __viaddmin_u32((unsigned)partner[i], 17u, 16u);
+            bad |= role[i] >= 0 && at == 16u;
+            // channel | donor slot as byte offsets into a row of the 16-bit query
+            wrec[at] = make_uint2(__float_as_uint(scaled), (unsigned)(2 * (c0 + (i & 1) + 4 * (i >> 1))) + ((unsigned)role[i] << 17));
           } else {
             bad |= role[i] >= 0;
           }
@@ -1257,16 +1286,17 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
           // every entry and every partial sum is exact.  One cell per lane: the source (even lane) or the
           // donor slot (odd lane) of salient lane / 2.
           {
-            const unsigned m = wrec[lane >> 1].y;
-            const int idx = lane >> 1, which = lane & 1;
-            const int c = (which ? m >> 8 : m) & 127;
-            const int jj = c >> 5, u = c & 31;
-            const int ks = 2 * (u >> 3) + ((u >> 1) & 1), half = u & 1, e = (u >> 2) & 1;
+            const uint2 m = wrec[lane >> 1];
+            const int idx = 15 - (lane >> 1), which = lane & 1;
+            const int at = s_cell[((m.y >> (16 * which)) & 0xfeu) >> 1];
+            // the scale in the units of the score accumulator (see below); the second code of a gather column
+            // carries a factor 1/512
+            if (!which) ((float*)wrec)[lane] = __uint_as_float(m.x) * ((idx & 8) ? 0.125f : (1.f / 4096.f));
             // fp16 bits of 32768 (source), 2048 (donor), each divided by 16 for the high nibble of a
-            // byte and by 512 for the second salient channel of the column
+            // byte (odd channels) and by 512 for the second salient channel of the column
             if (FAST || idx < n_pad) {
-              my_cell = (ks * 32 + (((idx & 7) << 2) | jj)) * 8 + half * 4 + e * 2;
-              *(unsigned short*)(wsel + my_cell) = (unsigned short)(0x7800 - (which + half) * 0x1000 - ((idx >> 3) & 1) * 0x2400);
+              my_cell = at + ((idx & 7) << 5);
+              *(unsigned short*)(wsel + my_cell) = (unsigned short)(0x7800 - which * 0x1000 - ((idx >> 3) & 1) * 0x2400 - ((at & 4) << 10));
             }
           }
           // B fragments of the salient step (query at the salient channels) and of the donors' step (query at
@@ -1274,14 +1304,15 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
           // score accumulator, whose unit is alpha = qinv * 2^(24 + ex_f): the staged query times 2^-12 and
           // the salient value times 2^-(12 + ex_f) give exactly that unit, and both factors are powers of
           // two, so the rounding to the model dtype is the reference's
-          const uint4 ra = *(const uint4*)(wrec + 2 * j), rb = *(const uint4*)(wrec + 2 * j + 8);
-          const unsigned short* const qrow = (const unsigned short*)(q16 + r * kQRow);
-          const unsigned m4[4] = {ra.y, ra.w, rb.y, rb.w};
+          const uint4 ra = *(const uint4*)(wrec + 14 - 2 * j), rb = *(const uint4*)(wrec + 6 - 2 * j);
+          const unsigned qrow = smem_addr(q16 + r * kQRow) * 0x10001u;   // (the query lies in the first 64 KB)
+          const unsigned m4[4] = {ra.w, ra.y, rb.w, rb.y};
           unsigned qa[4], qd[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            qa[k] = qrow[m4[k] & 127];
-            qd[k] = qrow[(m4[k] >> 8) & 127];
+            const unsigned at = m4[k] + qrow;
+            qa[k] = lds16(at & 0xffffu);
+            qd[k] = lds16(at >> 16);
           }
           qsal = make_uint2(__byte_perm(qa[0], qa[1], 0x5410u), __byte_perm(qa[2], qa[3], 0x5410u));
           // the donors' constant values (the reference stores the sampled mean as the donor channel's own
@@ -1503,7 +1534,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
       }
 
       const unsigned stage = launder(FAST ? consume_addr : ring_addr + stage_index * kStageBytes);
-      const unsigned ww_it = launder(ww_addr), sel_it = launder(sel_addr), rec_it = launder(smem_addr(wrec) + 16 * j);
+      const unsigned ww_it = launder(ww_addr), sel_it = launder(sel_addr), rec_it = launder(smem_addr(wrec) + 16 * (3 - j));
       if (FAST) {
         consume_addr += kStageBytes;
         if (consume_addr == ring_hi) consume_addr = ring_lo;
@@ -1602,9 +1633,9 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
             float2 sc0, sc1;
             uint2 qb;
             if constexpr (kNarrow) {
-              const uint4 ra = lds128<0>(rec_it), rb = lds128<64>(rec_it);
-              sc0 = make_float2(__uint_as_float(ra.x), __uint_as_float(ra.z));
-              sc1 = make_float2(__uint_as_float(rb.x), __uint_as_float(rb.z));
+              const uint4 ra = lds128<64>(rec_it), rb = lds128<0>(rec_it);
+              sc0 = make_float2(__uint_as_float(ra.z), __uint_as_float(ra.x));
+              sc1 = make_float2(__uint_as_float(rb.z), __uint_as_float(rb.x));
               qb = qsal;
             } else {
               sc0 = *(const float2*)(wssc + gsel * 16 + 2 * j);

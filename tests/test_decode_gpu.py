@@ -463,3 +463,19 @@ def test_contiguous_rows_that_do_not_start_on_16_bytes(dtype):
     assert off(query).is_contiguous() and off(query).data_ptr() % 16
     assert torch.equal(state.decode(off(query), **dict(zip(names, dense))), expected)
     assert torch.equal(state.decode(query, **dict(zip(names, map(off, dense)))), expected)
+
+
+@pytest.mark.parametrize("block", [5, 16])
+@pytest.mark.parametrize("fraction", [1 / 128, 0.0625, 0.125])       # 1, 8 and 16 salient channels: part of the list, all of it
+def test_short_lists_of_salient_channels_in_short_blocks(block, fraction):
+    CodecConfig, quantize, quantize_values, PackedDecodeState, _, _ = _mods()
+    cfg = CodecConfig(salient_fraction=fraction, donor_policy="neighbors")
+    # outliers at both ends of the head, so that sources and donors reach channels 0 and 127
+    gain = np.where((np.arange(128) < 3) | (np.arange(128) > 124), 12, 1).astype(np.float32)
+    ks = [oracle.round_to_dtype(_random(70 + i, (1, 2, block, 128), "bfloat16") * gain, "bfloat16") for i in range(4)]
+    vs = [_random(80 + i, (1, 2, block, 128), "bfloat16") for i in range(4)]
+    state = PackedDecodeState([quantize(to_device(k, "bfloat16"), cfg) for k in ks], [quantize_values(to_device(v, "bfloat16")) for v in vs])
+    q = _random(5, (14, 128), "bfloat16")
+    actual = state.decode(to_device(q, "bfloat16").view(1, 14, 1, 128))
+    ok = [oracle.dequantize_k4(oracle.quantize_k4(k, "bfloat16", 8, fraction, "neighbors"))[0] for k in ks]
+    _check(actual, _expected(q, ok, [oracle.dequantize_values(oracle.quantize_values(v, "bfloat16"))[0] for v in vs]))

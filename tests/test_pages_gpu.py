@@ -210,3 +210,36 @@ def test_pages_asked_for_ahead(block, pages):
         assert N.take_status(torch.device("cuda", 0), N.STATUS_BAD_INDEX) == 0
         assert torch.equal(decode(outside), good)
         assert N.take_status(torch.device("cuda", 0), N.STATUS_BAD_INDEX) == N.STATUS_BAD_INDEX
+
+
+@pytest.mark.parametrize("block", [16, 64, 256])
+def test_wrong_words_in_a_role_map_are_reported_and_stay_with_their_head(block):
+    """A role outside its range, and a salient channel whose slot belongs to no donor: the call reports it, and what
+    the other KV heads of the page give is the same bit for bit."""
+    from inquant import _native as N
+    from inquant.triton_attention import SharedDecodeWorkspace
+    from inquant_vllm.kernels import paged_decode
+    from inquant_vllm.layout import PageLayout, pack_pages
+    heads, q_heads, pages = 3, 21, 3
+    layout, workspace = PageLayout(block, heads), SharedDecodeWorkspace()
+    kt, vt = _pages_input(block, heads, pages, block)
+    pool = pack_pages(to_device(kt), to_device(vt), layout).view(pages, -1)
+    roles = layout.views(pool)["key_map"][1, 1]
+    ids = torch.arange(pages, device="cuda", dtype=torch.int32)
+    dense = torch.zeros((2, heads, block + 4, 128), dtype=torch.bfloat16, device="cuda")
+    q = to_device(workloads.make_query(9, q_heads)).view(1, q_heads, 128)
+
+    def decode():
+        return paged_decode(q, pool, ids, dense, pages, 0, 0, layout, workspace, 128 ** -0.5).clone()
+    good = decode()
+    words = roles.cpu()
+    assert N.take_status(torch.device("cuda", 0), N.STATUS_BAD_INDEX) == 0
+    regular, salient = int((words == -1).nonzero()[-1]), int((words >= 0).nonzero()[0])
+    for channel, word in ((regular, 128), (regular, -18), (regular, 32767), (regular, -32768), (regular, regular), (salient, regular), (salient, salient)):
+        roles[channel] = word
+        out = decode()
+        roles[channel] = int(words[channel])
+        assert N.take_status(torch.device("cuda", 0), N.STATUS_BAD_INDEX) == N.STATUS_BAD_INDEX, (channel, word)
+        others = [h for h in range(q_heads) if h // 7 != 1]
+        assert torch.equal(out.view(q_heads, -1)[others], good.view(q_heads, -1)[others])
+    assert torch.equal(decode(), good) and N.take_status(torch.device("cuda", 0), N.STATUS_BAD_INDEX) == 0
