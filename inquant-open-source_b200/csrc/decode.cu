@@ -78,7 +78,7 @@ constexpr int kRecordFloats = 8 * kRecordStride;    // one partial record (8 que
 constexpr int kQChunk = 36;                         // padded 32-float chunk of the staged query
 constexpr int kQFragBytes = 8 * 32 * 8;              // the staged query as fp16 B fragments of the 8 K steps
 constexpr int kQRow = 136;                          // padded row of the query staged in the model dtype (at most 16 salient channels)
-static_assert(8 * kQRow * 2 <= 8 * 4 * kQChunk * 4 && kQRow % 8 == 0, "the 16-bit query takes the place of the fp32 one");
+static_assert(2 * 8 * kQRow * 2 <= 8 * 4 * kQChunk * 4 && kQRow % 8 == 0, "the two 16-bit queries take the place of the fp32 one");
 constexpr int kQBytes = 8 * 4 * kQChunk * 4 + 64 + kQFragBytes;   // staged query, two factors per head, fragments
 constexpr float kNegBig = -1.0e30f;
 constexpr float kRescaleSlack = 4.f;   // the running reference maximum may lag the true one by 2^4
@@ -214,10 +214,16 @@ __device__ __forceinline__ unsigned lds32(unsigned addr) {
   asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(addr), "n"(OFF));
   return v;
 }
+template <int OFF = 0>
 __device__ __forceinline__ unsigned lds16(unsigned addr) {
   unsigned short v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+  asm volatile("ld.shared.u16 %0, [%1+%2];" : "=h"(v) : "r"(addr), "n"(OFF));
   return v;
+}
+template <typename QT>
+__device__ __forceinline__ float qt_bits_to_float(unsigned bits) {
+  const unsigned short b = (unsigned short)bits;
+  return to_float<QT>(*(const QT*)&b);
 }
 __device__ __forceinline__ unsigned clamp_s16x2(unsigned x, unsigned lo, unsigned hi) {
   asm("min.s16x2 %0, %0, %1;\n\tmax.s16x2 %0, %0, %2;" : "+r"(x) : "r"(hi), "r"(lo));
@@ -544,7 +550,8 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   constexpr int kMetaPad = kNarrow ? 784 : 768;
   extern __shared__ __align__(16) unsigned char smem[];
   float* qs = (float*)smem;                                             // 8 heads x 4 chunks x kQChunk
-  // kNarrow: the staged query times 2^-12 in the model dtype, 8 heads x kQRow, in the place of qs
+  // kNarrow: the staged query times 2^-12 in the model dtype, 8 heads x kQRow, in the place of qs; behind it the
+  // query as it was given, which the donors' constants meet in fp32
   QT* q16 = (QT*)smem;
   float* qinv = qs + 8 * 4 * kQChunk;   // per head: softmax scale * log2(e) * 2^(exponent of max|q| - 12)
   // the staged query once more as fp16 pairs in B-fragment order: entry [K step][lane (head r, chunk j)]
@@ -889,6 +896,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
       w.z = pack_qt2<QT>(v[4] * (1.f / 4096.f), v[5] * (1.f / 4096.f));
       w.w = pack_qt2<QT>(v[6] * (1.f / 4096.f), v[7] * (1.f / 4096.f));
       *(uint4*)(q16 + g * kQRow + c0) = w;
+      *(uint4*)(q16 + (8 + g) * kQRow + c0) = raw;
     } else {
       float* const dst = qs + (g * 4 + (c0 >> 5)) * kQChunk + (c0 & 31);
       *(float4*)dst = make_float4(v[0], v[1], v[2], v[3]);
@@ -1203,7 +1211,7 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
       const bool issue_late = FAST ? SUB == 2 && it == 0 : (!kMetaInStage && spb < 3 && need_weights);
       if (!issue_late) issue(false);
 
-      float wsum[4] = {0.f, 0.f, 0.f, 0.f}, dsum[4] = {0.f, 0.f, 0.f, 0.f};
+      float wsum[4] = {0.f, 0.f, 0.f, 0.f}, dsum[2] = {0.f, 0.f};
       unsigned ff_it = 0u, qf_it = 0u;   // kDirect: channel weights and query of this block's fragments
       if (kNarrow && (kDirect || need_weights)) {
         // ---- fold this block's descriptor, scales and padding into the query: no branches, so that the
@@ -1299,26 +1307,31 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
               *(unsigned short*)(wsel + my_cell) = (unsigned short)(0x7800 - which * 0x1000 - ((idx >> 3) & 1) * 0x2400 - ((at & 4) << 10));
             }
           }
-          // B fragments of the salient step (query at the salient channels) and of the donors' step (query at
-          // the donor slots): entries 2j, 2j+1 | 2j+8, 2j+9 of head r.  The salient step adds straight into the
-          // score accumulator, whose unit is alpha = qinv * 2^(24 + ex_f): the staged query times 2^-12 and
-          // the salient value times 2^-(12 + ex_f) give exactly that unit, and both factors are powers of
-          // two, so the rounding to the model dtype is the reference's
+          // B fragments of the salient step (query at the salient channels): entries 2j, 2j+1 | 2j+8, 2j+9 of head
+          // r.  The step adds straight into the score accumulator, whose unit is alpha = qinv * 2^(24 + ex_f): the
+          // staged query times 2^-12 and the salient value times 2^-(12 + ex_f) give exactly that unit, and both
+          // factors are powers of two, so the rounding to the model dtype is the reference's
           const uint4 ra = *(const uint4*)(wrec + 14 - 2 * j), rb = *(const uint4*)(wrec + 6 - 2 * j);
           const unsigned qrow = smem_addr(q16 + r * kQRow) * 0x10001u;   // (the query lies in the first 64 KB)
           const unsigned m4[4] = {ra.w, ra.y, rb.w, rb.y};
-          unsigned qa[4], qd[4];
+          unsigned qa[4];
+          float dterm[2];   // entries 2j and 2j+8, 2j+1 and 2j+9
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const unsigned at = m4[k] + qrow;
             qa[k] = lds16(at & 0xffffu);
-            qd[k] = lds16(at >> 16);
+            // the donors' constant values (the reference stores the sampled mean as the donor channel's own value
+            // and rounds it to the model dtype) times the query as it was given, in fp32: staged in the model dtype,
+            // fp16 components far below a head's largest one would lose bits
+            const float qd = qt_bits_to_float<QT>(lds16<8 * kQRow * 2>(at >> 16)), constant = to_float<QT>(from_float<QT>(pad[k]));
+            dterm[k & 1] = k < 2 ? qd * constant : fmaf(qd, constant, dterm[k & 1]);
           }
           qsal = make_uint2(__byte_perm(qa[0], qa[1], 0x5410u), __byte_perm(qa[2], qa[3], 0x5410u));
-          // the donors' constant values (the reference stores the sampled mean as the donor channel's own
-          // value and rounds it to the model dtype) times the query, the same in all 16 rows
-          const unsigned p_lo = pack_qt2<QT>(pad[0], pad[1]), p_hi = pack_qt2<QT>(pad[2], pad[3]);
-          mma_qt<QT>(dsum, p_lo, p_lo, p_hi, p_hi, __byte_perm(qd[0], qd[1], 0x5410u), __byte_perm(qd[2], qd[3], 0x5410u));
+          float donors = dterm[0] + dterm[1];   // of head r, summed over the row; this lane's columns are heads 2j, 2j+1
+          donors += __shfl_xor_sync(0xffffffffu, donors, 1);
+          donors += __shfl_xor_sync(0xffffffffu, donors, 2);
+          dsum[0] = __shfl_sync(0xffffffffu, donors, 8 * j);
+          dsum[1] = __shfl_sync(0xffffffffu, donors, 8 * j + 4);
         }
         // The B fragments of the eight K steps are the staged query (fp16 pairs in fragment order) times the
         // block's channel weights, one HMUL2 per register; the same fragments against an A operand of ones
@@ -1348,8 +1361,8 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
           const float up = __uint_as_float((unsigned)(127 + 24 + ex_f) << 23);
           alpha[0] = qf.x * up;
           alpha[1] = qf.y * up;
-          dsum[0] *= qf.x * 4096.f;
-          dsum[1] *= qf.y * 4096.f;
+          dsum[0] *= P.scale_log2e;
+          dsum[1] *= P.scale_log2e;
         }
         if (!kDirect) {
           beta[0] = fmaf(-8.f * alpha[0], wsum[0], dsum[0]);

@@ -479,3 +479,35 @@ def test_short_lists_of_salient_channels_in_short_blocks(block, fraction):
     actual = state.decode(to_device(q, "bfloat16").view(1, 14, 1, 128))
     ok = [oracle.dequantize_k4(oracle.quantize_k4(k, "bfloat16", 8, fraction, "neighbors"))[0] for k in ks]
     _check(actual, _expected(q, ok, [oracle.dequantize_values(oracle.quantize_values(v, "bfloat16"))[0] for v in vs]))
+
+
+@pytest.mark.parametrize("block", [16, 64])
+def test_donor_constants_meet_the_query_in_32_bits(block):
+    """fp16 query components 2^-16 of a head's largest one, at the donor slots only, against constants of 4000 whose
+    products nearly cancel: staged beside the largest component in fp16 they would keep 9 of 11 bits, which moves the two
+    blocks' scores by 1e-2 and more.  With exact products and fp32 sums what is left is the rounding of the probabilities
+    and of the output to fp16, 2^-11 each of values in [-1, 1]."""
+    CodecConfig, quantize, quantize_values, PackedDecodeState, _, _ = _mods()
+    rng, heads = np.random.default_rng(77), 7
+    keys = [quantize(to_device(_random(60 + i, (1, 1, block, 128), "float16"), "float16"), CodecConfig(donor_policy="min_error")) for i in range(2)]
+    for name in ("salient_channels", "donor_channels"):
+        getattr(keys[1], name).copy_(getattr(keys[0], name))
+    taken = keys[0].salient_channels.flatten().tolist() + keys[0].donor_channels.flatten().tolist()
+    largest = next(c for c in range(128) if c not in taken)
+    donors = keys[0].donor_channels.flatten().long().cpu().numpy()
+    small = (0.03125 * (1 + rng.integers(1, 1024, (heads, 16)) / 1024)).astype(np.float16)
+    small[1:] = small[0] * rng.choice([0.5, 1.0, 2.0], (heads - 1, 1)).astype(np.float16)      # (heads whose products cancel alike)
+    query = np.zeros((heads, 128), np.float32)
+    query[:, donors], query[:, largest] = small, 2048.0
+    constants = np.full(16, 4000.0, np.float32)
+    constants[1::2] = np.float16(-4000.0 * small[0, ::2].astype(np.float64) / small[0, 1::2])
+    values = []
+    for sign, key in zip((1.0, -1.0), keys):
+        key.scales[..., largest] = 1e-30                 # the largest component adds nothing
+        key.padding.copy_(torch.from_numpy(sign * constants).cuda())
+        values.append(quantize_values(torch.full((1, 1, block, 128), sign, dtype=torch.float16, device="cuda")))
+    out = PackedDecodeState(keys, values).decode(to_device(query, "float16").view(1, heads, 1, 128))
+    dense = [to_numpy(torch.cat([b.dequantize() for b in blocks], dim=2)[0]).astype(np.float64) for blocks in (keys, values)]
+    expected = oracle.attention_decode(query, *dense, 128 ** -0.5)
+    error = np.abs(to_numpy(out).reshape(heads, 128) - expected).max()
+    assert error < 2 * 2 ** -11, error
