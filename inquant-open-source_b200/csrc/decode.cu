@@ -1340,19 +1340,15 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
         qf_it = launder(smem_addr(qfrag) + lane * 8);
         ff_it = launder(smem_addr(wfrag) + j * 8);
         if (!kDirect) {
-          float wsum2[4] = {0.f, 0.f, 0.f, 0.f};   // two chains
-#define INQ_FOLD(KS, SUM)                                                                                  \
+#define INQ_FOLD(KS)                                                                                       \
   {                                                                                                        \
     const uint2 qq = lds64<(KS) * 256>(qf_it), ff2 = lds64<(KS) * 32>(ff_it);                              \
     const uint2 ww = make_uint2(hmul2_bits(qq.x, ff2.x), hmul2_bits(qq.y, ff2.y));                         \
     *(uint2*)(wW + ((KS) * 32 + lane) * 8) = ww;                                                           \
-    mma_f16(SUM, 0x00010001u, 0x00010001u, 0x00100010u, 0x00100010u, ww.x, ww.y);                          \
+    mma_f16(wsum, 0x00010001u, 0x00010001u, 0x00100010u, 0x00100010u, ww.x, ww.y);                         \
   }
-          INQ_FOLD(0, wsum) INQ_FOLD(1, wsum2) INQ_FOLD(2, wsum) INQ_FOLD(3, wsum2)
-          INQ_FOLD(4, wsum) INQ_FOLD(5, wsum2) INQ_FOLD(6, wsum) INQ_FOLD(7, wsum2)
+          INQ_FOLD(0) INQ_FOLD(1) INQ_FOLD(2) INQ_FOLD(3) INQ_FOLD(4) INQ_FOLD(5) INQ_FOLD(6) INQ_FOLD(7)
 #undef INQ_FOLD
-          wsum[0] += wsum2[0];
-          wsum[1] += wsum2[1];
         }
         // raw score -> base-2 score: undo 2^-24 (subnormal nibbles), the scale exponent and the query
         // factor; score columns of this thread are query heads 2j and 2j+1
