@@ -2038,8 +2038,9 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   if (s_is_last) {
     // A sequence decoded alone is cut into a hundred parts per pair, so this merge is written for
     // many loads in flight: (m, l) of every (query head, part) are staged first, and each thread then sums 8
-    // channels of one head over the parts, eight at a time; past the end the last part is fetched once more and
-    // weighted 0 (one by one, the four parts beyond eight of a pair of twelve were four trips to memory).
+    // channels of one head over the parts, eight at a time, the loads of all eight before the first sum (one by one,
+    // the four parts beyond eight of a pair of twelve were four trips to memory).  Past the end nothing is added, not
+    // even with weight 0: a part may hold infinities.
     // Requesting the first eight together with (m, l) would save another, but the registers they stand in
     // make the slice loop spill.
     const int g = threadIdx.x >> 4, c8 = (threadIdx.x & 15) * 8;   // kThreads = 128: 8 heads x 16 threads
@@ -2050,12 +2051,15 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
     float* mtop = norm + 8;
     const float* base = P.partials + ((long long)first_cta + pair) * kRecordFloats;
     float* const partial = SEQ(partial_out);
-    auto fetch = [&](float4 (&a)[8], float4 (&b)[8], int p0) {   // (past the end the last part once more, weighted 0)
+    auto fetch = [&](float4 (&a)[8], float4 (&b)[8], int p0) {
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        const float4* const at = (const float4*)(base + (long long)min(p0 + u, np - 1) * kRecordFloats + g * kRecordStride + c8);
-        a[u] = __ldcg(at);
-        b[u] = __ldcg(at + 1);
+        a[u] = b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p0 + u < np) {
+          const float4* const at = (const float4*)(base + (long long)(p0 + u) * kRecordFloats + g * kRecordStride + c8);
+          a[u] = __ldcg(at);
+          b[u] = __ldcg(at + 1);
+        }
       }
     };
 #pragma unroll 4

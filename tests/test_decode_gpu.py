@@ -511,3 +511,28 @@ def test_donor_constants_meet_the_query_in_32_bits(block):
     expected = oracle.attention_decode(query, *dense, 128 ** -0.5)
     error = np.abs(to_numpy(out).reshape(heads, 128) - expected).max()
     assert error < 2 * 2 ** -11, error
+
+
+@pytest.mark.parametrize("blocks", [0, 1, 3, 9])
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+def test_an_infinite_value_gives_an_infinite_output(blocks, dtype):
+    """Every whole slice of the tail holds an infinity in one channel, so that every part of a pair may bring one to the
+    merge, whose parts are not a multiple of eight."""
+    CodecConfig, quantize, quantize_values, PackedDecodeState, _, _ = _mods()
+    heads, tail = 2, 16 * 40
+    k, v = _random(80, (1, heads, 64 * max(blocks, 1), 128), dtype), _random(81, (1, heads, 64 * max(blocks, 1), 128), dtype)
+    pieces = [slice(64 * i, 64 * i + 64) for i in range(blocks)]
+    keys = [quantize(to_device(k[:, :, p], dtype), CodecConfig(donor_policy="min_error")) for p in pieces]
+    values = [quantize_values(to_device(v[:, :, p], dtype)) for p in pieces]
+    tail_k, tail_v = _random(82, (1, heads, tail, 128), dtype), _random(83, (1, heads, tail, 128), dtype)
+    dense = [to_device(x, dtype) for x in (tail_k, tail_v)]
+    query = to_device(_random(84, (14, 128), dtype), dtype).view(1, 14, 1, 128)
+
+    def run():
+        return PackedDecodeState(keys, values).decode(query, residual_key=dense[0], residual_value=dense[1]).reshape(14, 128)
+    finite = run()
+    dense[1][:, :, ::16, 5] = float("inf")
+    out = run()
+    assert torch.isfinite(finite).all() and (out[:, 5] == float("inf")).all()
+    out[:, 5] = finite[:, 5]
+    assert torch.equal(out, finite)
