@@ -18,7 +18,9 @@ Only batch-one, append-only inference on CUDA tensors is supported.
 """
 from __future__ import annotations
 
+import itertools
 import math
+import operator
 from dataclasses import dataclass, field
 from typing import Any, Iterator
 
@@ -84,18 +86,17 @@ class _Layer:
     packed_nbytes: int = 0
     retired_tail: tuple | None = None               # the tail buffers replaced by the last seal
     sink_views: tuple | None = None                 # (count, key view, value view) handed out last
-    runs: list = field(default_factory=list)        # what sealed the blocks: (last block, keys' owner, values' owner, blocks)
+    runs: list = field(default_factory=list)        # what sealed the blocks: (key blocks, value blocks, keys' owner, values' owner)
 
     def block_runs(self):
-        """The sealed blocks as runs of one encoder launch each, ``(keys' owner, values' owner, blocks)``:
-        an owner is the arena of such a launch, or a block of its own.  None when the lists no longer are
-        what the seals appended."""
-        end = 0
-        for last, _, _, count in self.runs:
-            end += count
-            if end > len(self.key_blocks) or self.key_blocks[end - 1] is not last:
+        """The sealed blocks as runs of one encoder launch each, ``(key blocks, value blocks, keys' owner, values'
+        owner)``: an owner is the arena of such a launch, or a block of its own.  None when any block is not the one
+        that a seal appended at its place."""
+        for blocks, side in ((self.key_blocks, 0), (self.value_blocks, 1)):
+            if len(blocks) != sum(len(run[side]) for run in self.runs) \
+                    or not all(map(operator.is_, blocks, itertools.chain.from_iterable(run[side] for run in self.runs))):
                 return None
-        return self.runs if end == len(self.key_blocks) == len(self.value_blocks) else None
+        return self.runs
 
     def _sink_pair(self):
         """The sink views for the current count: the same two tensor objects until the count changes
@@ -215,11 +216,11 @@ def _row_copy(entry, source: torch.Tensor, first: int, target: torch.Tensor, sta
     entry.tokens = tokens
 
 
-def restore_history(layer: _Layer, out_key: torch.Tensor, out_value: torch.Tensor, new_key=None, new_value=None) -> bool:
-    """The layer's whole history -- sink, sealed blocks, tail -- into ``out_key`` / ``out_value`` [1, H, tokens, 128]
-    from token 0 on, and the rows of ``new_key`` / ``new_value`` behind it, by one launch for up to eight runs of
-    blocks (C ABI ``inq_restore_history``).  False, with nothing launched, when that launch does not serve the
-    layouts."""
+def restore_history(layer: _Layer, runs, out_key: torch.Tensor, out_value: torch.Tensor, new_key=None, new_value=None) -> bool:
+    """The layer's whole history -- sink, sealed blocks (``runs``: ``layer.block_runs()``), tail -- into ``out_key`` /
+    ``out_value`` [1, H, tokens, 128] from token 0 on, and the rows of ``new_key`` / ``new_value`` behind it, by one
+    launch for up to eight runs of blocks (C ABI ``inq_restore_history``).  False, with nothing launched, when that
+    launch does not serve the layouts."""
     from .value_codec import PackedValues
     _, heads, _, channels = layer.shape
     dtype = layer.dtype
@@ -233,7 +234,6 @@ def restore_history(layer: _Layer, out_key: torch.Tensor, out_value: torch.Tenso
     for tensor in dense:
         if tensor.dtype != dtype or tensor.stride(3) != 1 or not N.dense_rows_aligned(tensor):
             return False
-    runs = layer.block_runs()
     if runs is None:
         return False
     args = N.RestoreArgs()
@@ -242,7 +242,7 @@ def restore_history(layer: _Layer, out_key: torch.Tensor, out_value: torch.Tenso
     args.position = layer.sink_count
     position = layer.sink_count
     if runs:
-        first_key, first_value = runs[0][1], runs[0][2]
+        first_key, first_value = runs[0][2:]
         block_tokens, count = first_key.shape[2], first_key.salient_channels.shape[-1]
         coded = not isinstance(first_value, PackedValues)
         args.block_tokens, args.count = block_tokens, count
@@ -253,7 +253,7 @@ def restore_history(layer: _Layer, out_key: torch.Tensor, out_value: torch.Tenso
         if count > 64 or (coded and args.value_count > 64):
             return False
         records = (N.RestoreRun * len(runs))()
-        for record, (_, keys, values, blocks) in zip(records, runs):
+        for record, (sealed, _, keys, values) in zip(records, runs):
             fields = [keys.payload, keys.scales, keys.salient_channels, keys.donor_channels, keys.padding, values.payload, values.scales]
             names = ["key_payload", "key_scales", "key_salient", "key_donors", "key_padding", "value_payload", "value_scales"]
             if coded:
@@ -266,8 +266,8 @@ def restore_history(layer: _Layer, out_key: torch.Tensor, out_value: torch.Tenso
                 if not tensor.is_contiguous() or tensor.dtype == torch.int32:
                     return False
                 setattr(record, name, tensor.data_ptr() or None)
-            record.n_blocks = blocks
-            position += blocks * block_tokens
+            record.n_blocks = len(sealed)
+            position += len(sealed) * block_tokens
         args.runs, args.n_runs = N.ctypes.cast(records, N.c_void_p), len(runs)
     copies = []
     if layer.sink_count:
@@ -781,9 +781,9 @@ class InQuantCache(_HFCache):
     def _record_run(layer: _Layer, new_keys, new_values) -> None:
         owners = [getattr(new[0], "_arena", (new[0], 0))[0] for new in (new_keys, new_values)]
         if len(new_keys) == len(new_values) and all(owner.shape[0] == len(new_keys) for owner in owners):
-            layer.runs.append((new_keys[-1], *owners, len(new_keys)))
+            layer.runs.append((tuple(new_keys), tuple(new_values), *owners))
         else:   # sealed block by block
-            layer.runs.extend((k, k, v, 1) for k, v in zip(new_keys, new_values))
+            layer.runs.extend(((k,), (v,), k, v) for k, v in zip(new_keys, new_values))
 
     def record_peak(self, layer_idx):
         """Live persistent bytes in O(1) per layer update (reference ``cache.py:308-326``)."""
@@ -815,10 +815,14 @@ class InQuantCache(_HFCache):
         new_tokens = 0 if new_key is None else new_key.shape[2]
         sink_tokens = layer.sink_count
         tail_tokens = 0 if layer.tail_key_buffer is None else layer.tail_count
-        packed_tokens = len(layer.key_blocks) * self.config.block_size
+        runs = layer.block_runs()
+        if runs is None:
+            packed = [sum(block.shape[2] for block in blocks) for blocks in (layer.key_blocks, layer.value_blocks)]
+        else:
+            packed = [sum(len(run[0]) * run[2].shape[2] for run in runs)] * 2
         full = [torch.empty((1, heads, sink_tokens + packed_tokens + tail_tokens + new_tokens, channels),
-                            dtype=layer.dtype, device=layer.device) for _ in range(2)]
-        if restore_history(layer, *full, new_key, new_value):
+                            dtype=layer.dtype, device=layer.device) for packed_tokens in packed]
+        if restore_history(layer, runs, *full, new_key, new_value):
             return tuple(full)
         for out, sink, blocks, tail, new in ((full[0], layer.sink_key, layer.key_blocks, layer.residual_key, new_key),
                                              (full[1], layer.sink_value, layer.value_blocks, layer.residual_value, new_value)):

@@ -186,7 +186,7 @@ class PrefillHistory:
         layer = cache._layers.get(layer_idx)
         if layer is None:
             layer = _Layer(tuple(key.shape), key.dtype, key.device)     # no history yet: the chunk's rows alone
-        if not restore_history(layer, scratch[0], scratch[1], key, value):
+        if not restore_history(layer, layer.block_runs(), scratch[0], scratch[1], key, value):
             for out, sink, blocks, tail, new in ((scratch[0], layer.sink_key, layer.key_blocks, layer.residual_key, key),
                                                  (scratch[1], layer.sink_value, layer.value_blocks, layer.residual_value, value)):
                 position = 0 if sink is None else sink.shape[2]

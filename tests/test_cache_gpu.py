@@ -324,3 +324,21 @@ def test_dense_history_equals_its_parts(value_bits, group, block, dtype, fractio
         if step:
             assert all(torch.equal(a, torch.cat((b, c), dim=2)) for a, b, c in zip(full, expected, (k, v)))
     assert len(cache._layers[0].runs) > 8
+
+
+@pytest.mark.parametrize("side,index", [("key_blocks", 1), ("key_blocks", 4), ("value_blocks", 2), ("value_blocks", 4)])
+def test_history_holds_the_blocks_that_stand_in_the_layers_lists(side, index):
+    """A block put in another's place, inside a run of one encoder launch or at its end, on either side."""
+    from inquant.value_codec import quantize_values
+    CacheConfig, InQuantCache, CodecConfig, quantize = _mods()
+    codec = CodecConfig(donor_policy="min_error")
+    cache = InQuantCache(CacheConfig(codec, block_size=32, residual_length=8, sink_tokens=4, value_bits=2))
+    cache.update(*(to_device(_randn(s, (1, 2, 4 + 5 * 32 + 11, 128))) for s in (50, 51)), 0)
+    layer, other = cache._layers[0], to_device(_randn(52, (1, 2, 32, 128)))
+    assert len(layer.key_blocks) == 5
+    getattr(layer, side)[index] = quantize(other, codec) if side == "key_blocks" else quantize_values(other)
+    expected = [torch.cat([sink, *(b.dequantize() for b in blocks), tail], dim=2) for sink, blocks, tail in
+                ((layer.sink_key, layer.key_blocks, layer.residual_key), (layer.sink_value, layer.value_blocks, layer.residual_value))]
+    assert all(torch.equal(a, b) for a, b in zip(cache.materialize(0), expected))
+    new = [to_device(_randn(s, (1, 2, 3, 128))) for s in (53, 54)]
+    assert all(torch.equal(a, torch.cat((b, c), dim=2)) for a, b, c in zip(cache.update(*new, 0), expected, new))
