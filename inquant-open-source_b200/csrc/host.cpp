@@ -217,6 +217,7 @@ PyObject* paged_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (q->dim() != 3 || q->size(0) != 1 || q->size(2) != 128 || q->scalar_type() != at::kBFloat16 || !q->is_contiguous() || !aligned(*q)) return none();
     if (q->size(1) % heads || q->size(1) / heads < 1 || q->size(1) / heads > 16) return none();
     if (blocks->scalar_type() != at::kInt || dense->scalar_type() != q->scalar_type() || !dense->is_contiguous()) return none();
+    if (!aligned(*dense) || !aligned(*cache)) return none();
     if (dense->dim() != 4 || dense->size(0) != 2 || dense->size(1) != heads || dense->size(2) != block + 4 || dense->size(3) != 128) return none();
     if (pages * block + tail == 0 && !sink) return none();
     at::Tensor out;

@@ -163,6 +163,8 @@ class DecodeBatch:
         for i, s in enumerate(self.sequences):
             if s.layout != self.layout or s.dense.dtype != self.dtype or not s.dense.is_contiguous():
                 raise ValueError("all paged sequences must share the layout and hold contiguous dense tensors of the batch dtype")
+            if s.dense.data_ptr() % 16 or s.pool.data_ptr() % 16:
+                raise ValueError("dense rows and pages must start on 16 bytes")
             table = s.page_table if s.page_table.dtype == torch.int32 else s.page_table.to(torch.int32)
             s.page_table = table
             fill_paged_sequence(seqs[i], self.queries[i], self.outputs[i], s.pool, table, s.dense, s.num_pages,

@@ -91,7 +91,7 @@ def _stacked_field(blocks, name: str) -> torch.Tensor:
     return (pieces[0] if len(pieces) == 1 else torch.cat(pieces, dim=0)).contiguous()
 
 
-def _aligned_copy(tensor: torch.Tensor) -> torch.Tensor:
+def aligned_copy(tensor: torch.Tensor) -> torch.Tensor:
     """Contiguous copy in storage of its own: rows that are contiguous already, but do not start on 16 bytes,
     come back unchanged from ``contiguous`` and the kernels read rows as 16-byte vectors."""
     return tensor.clone(memory_format=torch.contiguous_format)
@@ -368,9 +368,9 @@ class PackedDecodeState:
             if key.shape[1] != kv_heads:
                 raise ValueError("All inputs must share their KV head count")
             if not N.dense_rows_aligned(key):
-                key = _aligned_copy(key)
+                key = aligned_copy(key)
             if not N.dense_rows_aligned(value):
-                value = _aligned_copy(value)
+                value = aligned_copy(value)
             dense.append((key, value, key.shape[2]))
         if kv_heads is None or query.shape[1] % kv_heads:
             raise ValueError("query_heads must be divisible by the nonempty KV head count")
@@ -399,7 +399,7 @@ class PackedDecodeState:
         else:
             workspace_address = self._own_workspace(records, query.device)
         if query.data_ptr() % 16 or query.stride(1) % 8:     # rows of a head: 16-byte aligned (unit channel stride was checked)
-            query = _aligned_copy(query)
+            query = aligned_copy(query)
         output = torch.empty(query.shape, dtype=query.dtype, device=query.device)
         if self._tables is None:
             self._tables = torch.empty((0, 6), dtype=torch.int64, device=query.device)

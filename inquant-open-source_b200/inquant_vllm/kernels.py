@@ -6,7 +6,7 @@ import ctypes
 import torch
 
 from inquant import _native as N
-from inquant.triton_attention import pair_units, workspace_floats
+from inquant.triton_attention import aligned_copy, pair_units, workspace_floats
 
 
 def fill_paged_sequence(seq, query, output, cache, blocks, dense, num_pages, tail_tokens, sink_tokens, layout):
@@ -53,12 +53,16 @@ def paged_decode(query, cache, blocks, dense, num_pages, tail_tokens, sink_token
     if hq % hkv or hq // hkv > 16:
         raise ValueError("Expected 1..16 query heads per KV head")
     N.require_cuda(query, "paged_decode")
-    if not query.is_contiguous():
-        query = query.contiguous()
+    if cache.data_ptr() % 16:
+        raise ValueError("cache pages must start on 16 bytes")
+    if not query.is_contiguous() or query.data_ptr() % 16:     # rows are read as 16-byte vectors
+        query = aligned_copy(query)
     if blocks.dtype != torch.int32:
         blocks = blocks.to(torch.int32)
     if dense.dtype != query.dtype or tuple(dense.shape) != (2, hkv, layout.block_size + 4, 128) or not dense.is_contiguous():
         raise ValueError("dense must be a contiguous [2, KV_heads, block_size + 4, 128] tensor of the query dtype")
+    if dense.data_ptr() % 16:
+        dense = aligned_copy(dense)
     if not (num_pages * layout.block_size + tail_tokens) and not sink_tokens:
         raise ValueError("Attention requires at least one key/value token")
     q_per_kv = hq // hkv

@@ -101,3 +101,25 @@ def test_calls_outside_the_native_path_keep_their_errors():
             state.decode(query, **args)
     with torch.cuda.stream(torch.cuda.Stream()), pytest.raises(RuntimeError, match="one CUDA stream"):
         state.decode(q)
+
+
+def test_paged_decode_copies_rows_that_do_not_start_on_16_bytes():
+    from inquant.triton_attention import SharedDecodeWorkspace
+    from inquant_vllm.kernels import paged_decode
+    from inquant_vllm.layout import PageLayout, pack_pages
+    heads, q_heads, block = 2, 14, 64
+    layout, workspace = PageLayout(block, heads), SharedDecodeWorkspace()
+    k, v = (x[0].view(heads, 3, block, 128).transpose(0, 1) for x in workloads.make_kv_torch(7, heads, 3 * block, "cuda", 128))
+    pool = pack_pages(k.to(torch.bfloat16), v.to(torch.bfloat16), layout).view(3, -1)
+    dense = torch.randn((2, heads, block + 4, 128), device="cuda").to(torch.bfloat16)
+    ids, query = torch.arange(3, device="cuda", dtype=torch.int32), torch.randn((1, q_heads, 128), device="cuda").to(torch.bfloat16)
+
+    def off(x):
+        buffer = torch.empty(x.numel() + 1, dtype=x.dtype, device="cuda")
+        buffer[1:] = x.reshape(-1)
+        return buffer[1:].view(x.shape)
+    expected, of_query, of_dense = (paged_decode(q, pool, ids, d, 3, 9, 4, layout, workspace, 128 ** -0.5)
+                                    for q, d in ((query, dense), (off(query), dense), (query, off(dense))))
+    assert torch.equal(of_query, expected) and torch.equal(of_dense, expected)
+    with pytest.raises(ValueError, match="start on 16 bytes"):
+        paged_decode(query, off(pool), ids, dense, 3, 9, 4, layout, workspace, 128 ** -0.5)
