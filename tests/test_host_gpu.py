@@ -1,5 +1,7 @@
 """The native host side of the per-layer calls against the Python code behind it: what it serves gives the same
 bits, and what it does not serve takes the general path.  A tensor subclass is never served."""
+from types import SimpleNamespace
+
 import pytest
 import torch
 
@@ -26,6 +28,23 @@ def _rows(seed, heads, tokens, dtype, form):
         buffer[1:] = x.reshape(-1)
         return buffer[1:].view(1, heads, tokens, 128)
     return x
+
+
+@pytest.fixture
+def served(monkeypatch):
+    """Per native call, in order: True when it served the call, False when it left it to the Python code."""
+    from inquant import _native as N
+    host, calls = N.host(), {"append_token": [], "decode": [], "paged_decode": []}
+
+    def counted(name):
+        def call(*args):
+            result = getattr(host, name)(*args)
+            calls[name].append(result is not None)
+            return result
+        return call
+    module = SimpleNamespace(**{name: counted(name) for name in calls})
+    monkeypatch.setattr(N, "host", lambda: module)
+    return calls
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
@@ -123,3 +142,31 @@ def test_paged_decode_copies_rows_that_do_not_start_on_16_bytes():
     assert torch.equal(of_query, expected) and torch.equal(of_dense, expected)
     with pytest.raises(ValueError, match="start on 16 bytes"):
         paged_decode(query, off(pool), ids, dense, 3, 9, 4, layout, workspace, 128 ** -0.5)
+
+
+@pytest.mark.parametrize("validate", [False, True])
+def test_append_with_the_keywords_of_an_attention_module_is_native(served, validate):
+    """The form in which a patched model's attention appends: angles and the position beside the states."""
+    from inquant.cache import CacheConfig, InQuantCache
+    from inquant.codec import CodecConfig
+    config = CacheConfig(CodecConfig(donor_policy="min_error"), block_size=16, residual_length=8, sink_tokens=4, value_bits=2,
+                         validate_positions=validate)
+    prompt, angles = [_rows(s, 2, 30, torch.bfloat16, "contiguous") for s in (1, 2)], torch.zeros(4, device="cuda")
+    caches = [InQuantCache(config) for _ in range(2)]
+    for cache in caches:
+        cache.update(*prompt, 0)
+    for step in range(20):      # two seals among them, by tokens that complete a tail in place
+        new = [_rows(10 * step + s, 2, 1, torch.bfloat16, "token-major") for s in (3, 4)]
+        position = torch.tensor([30 + step], device="cuda")
+        views = [cache.append_for_attention(*new, 0, kwargs) for cache, kwargs in
+                 zip(caches, (None, {"sin": angles, "cos": angles, "cache_position": position}))]
+        assert all(torch.equal(getattr(views[0], n), getattr(views[1], n)) for n in ("sink_key", "sink_value", "residual_key", "residual_value"))
+        assert views[0].seq_length == views[1].seq_length == 31 + step
+    assert len(served["append_token"]) == 40 and all(served["append_token"])
+    wrong = {"cache_position": torch.tensor([3], device="cuda")}
+    if validate:
+        with pytest.raises(ValueError, match="contiguous append positions"):
+            caches[1].append_for_attention(*new, 0, wrong)
+        assert len(served["append_token"]) == 40 and caches[1].get_seq_length(0) == 50
+    with pytest.raises(ValueError, match="1D integer tensor"):
+        caches[1].append_for_attention(*new, 0, {"cache_position": 50})
