@@ -1452,7 +1452,7 @@ struct RestoreParams {
   const long long* table;             // instead of runs: 6 pointers per block and an int8 role map
   const signed char* roles;
   int n_runs, heads, tokens, parts;   // parts: CTAs per (block, head) row
-  int count, value_count, value_bits, value_group;
+  int count, value_count, value_group;
   void* out_k;
   void* out_v;
   long long stride_h, position, row_ctas;   // strides in elements; row_ctas: CTAs that decode
@@ -1472,7 +1472,6 @@ struct CodedRow {
   const float* scales;
   const unsigned char* salient;
   const unsigned char* donors;
-  const signed char* roles;
   const float* padding;
   int count;
 
@@ -1997,7 +1996,6 @@ extern "C" int inq_restore_blocks_table(const int64_t* table, const int8_t* role
   p.tokens = tokens;
   p.parts = (tokens + kRestoreTokens - 1) / kRestoreTokens;
   p.count = count;
-  p.value_bits = 2;
   p.value_group = 64;
   p.out_k = out_key;
   p.out_v = out_value;
@@ -2051,7 +2049,6 @@ extern "C" int inq_restore_history(const inq_restore_args_t* a, inq_stream_t str
     p.parts = (a->block_tokens + kRestoreTokens - 1) / kRestoreTokens;
     p.count = a->count;
     p.value_count = a->value_count;
-    p.value_bits = a->value_bits;
     p.value_group = a->value_group;
     p.out_k = a->out_key;
     p.out_v = a->out_value;

@@ -216,11 +216,12 @@ def _row_copy(entry, source: torch.Tensor, first: int, target: torch.Tensor, sta
     entry.tokens = tokens
 
 
-def restore_history(layer: _Layer, runs, out_key: torch.Tensor, out_value: torch.Tensor, new_key=None, new_value=None) -> bool:
+def restore_history(layer: _Layer, runs, out_key: torch.Tensor, out_value: torch.Tensor, new_key=None, new_value=None,
+                    restored_tokens: int = 0) -> bool:
     """The layer's whole history -- sink, sealed blocks (``runs``: ``layer.block_runs()``), tail -- into ``out_key`` /
     ``out_value`` [1, H, tokens, 128] from token 0 on, and the rows of ``new_key`` / ``new_value`` behind it, by one
-    launch for up to eight runs of blocks (C ABI ``inq_restore_history``).  False, with nothing launched, when that
-    launch does not serve the layouts."""
+    launch for up to eight runs of blocks (C ABI ``inq_restore_history``).  A caller that restores the blocks itself
+    gives no runs but their tokens.  False, with nothing launched, when that launch does not serve the layouts."""
     from .value_codec import PackedValues
     _, heads, _, channels = layer.shape
     dtype = layer.dtype
@@ -240,7 +241,7 @@ def restore_history(layer: _Layer, runs, out_key: torch.Tensor, out_value: torch
     args.heads, args.out_dtype = heads, N.DTYPE_CODE[dtype]
     args.out_key, args.out_value, args.stride_h = out_key.data_ptr(), out_value.data_ptr(), strides[1]
     args.position = layer.sink_count
-    position = layer.sink_count
+    position = layer.sink_count + restored_tokens
     if runs:
         first_key, first_value = runs[0][2:]
         block_tokens, count = first_key.shape[2], first_key.salient_channels.shape[-1]

@@ -61,6 +61,13 @@ def prefill_attention(query: torch.Tensor, key: torch.Tensor, value: torch.Tenso
     return out
 
 
+# More runs of blocks than this (every seal is one, of one block during decode) are restored through decode descriptors:
+# a record per run takes 4 us of host time and every eight records a launch, descriptors 250 us and more once and 40 us
+# per chunk.  us per chunk of 256 tokens behind 12 / 24 / 39 / 64 / 128 / 512 runs of one 256-token block each, records:
+# 264 / 305 / 338 / 413 / 698 / 2320; descriptors: 283 / 249 / 282 / 261 / 325 / 709.
+_TABLE_RUNS = 32
+
+
 class PrefillHistory:
     """Dense copy of what the next chunk of a prompt attends to, kept across chunks.
 
@@ -84,8 +91,9 @@ class PrefillHistory:
     dense cache the packed one exists to avoid.  ``persistent=False`` (the default) therefore keeps
     NO per-layer copy: one scratch pair serves every layer, and a layer's history is rebuilt into it
     from the packed cache for each of its chunks (sink and tail copied, every sealed block
-    dequantised and the chunk's rows put behind them by ONE launch,
-    ``inq_restore_history``: a few per cent of the chunk's attention time).  That is
+    dequantised and the chunk's rows put behind them by one launch for every eight seals that the
+    layer has seen, ``inq_restore_history``, and by two in all from 33 seals on,
+    ``inq_restore_blocks_table``: a few per cent of the chunk's attention time).  That is
     the reference's own semantics (``update`` materialises per call) at 2 * H * tokens * C elements
     in total (71 MB for the same prompt).  ``persistent=True`` keeps the per-layer copies and
     dequantises every block once.  ``release`` frees either.  Tensors grow geometrically unless
@@ -99,9 +107,11 @@ class PrefillHistory:
         self.persistent = bool(persistent)
         self._layers: dict[int, list] = {}    # layer -> [key, value, tokens, restored blocks]
         self._scratch: list = [None, None, 0, 0]   # the shared pair of the non-persistent mode
+        self._descriptors: dict[int, object] = {}  # layer -> decode descriptors of its blocks, for histories of many runs
 
     def release(self) -> None:
         self._layers.clear()
+        self._descriptors.clear()
         self._scratch = [None, None, 0, 0]
 
     def check(self) -> None:
@@ -170,6 +180,33 @@ class PrefillHistory:
         state[2] = seen + tokens
         return out
 
+    def _restore_from_table(self, layer_idx, layer, key, value) -> bool:
+        """A history of many runs into the scratch pair: every sealed block by ONE launch, addressed through the layer's
+        decode descriptors (kept here and extended by the blocks that were sealed since), the dense rows by another.
+        False, with nothing launched, for layouts that these do not serve."""
+        from .cache import restore_history
+        from .triton_attention import PackedDecodeState
+        out_key, out_value = self._scratch[:2]
+        blocks, state, values = len(layer.key_blocks), self._descriptors.get(layer_idx), layer.runs[0][3]
+        if (getattr(values, "bits", 0), getattr(values, "group_size", 0)) != (2, 64):
+            return False
+        try:
+            if state is None or len(state.key_blocks) > blocks:
+                state = self._descriptors[layer_idx] = PackedDecodeState(layer.key_blocks, layer.value_blocks)
+            else:
+                state.extend(layer.key_blocks, layer.value_blocks)
+        except (ValueError, RuntimeError):
+            self._descriptors.pop(layer_idx, None)
+            return False
+        tokens = state._packed_tokens
+        if not state._preset or state._salient > 64 or layer.sink_count + blocks * tokens + layer.tail_count != layer.seq_length \
+                or not restore_history(layer, (), out_key, out_value, key, value, blocks * tokens):
+            return False
+        rc = N.library().inq_restore_blocks_table(state._tables.data_ptr(), state._key_map.data_ptr(), blocks, out_key.shape[1], tokens,
+                                                  state._salient, out_key.data_ptr(), out_value.data_ptr(), out_key.stride(1),
+                                                  layer.sink_count, N.DTYPE_CODE[out_key.dtype], N.stream_pointer(out_key.device))
+        N.check(rc, "inq_restore_blocks_table")
+        return True
 
     def _chunk_from_packed(self, query, key, value, layer_idx, scale, cache_kwargs) -> torch.Tensor:
         """One chunk with the layer's history rebuilt from the packed cache into the shared scratch."""
@@ -186,7 +223,8 @@ class PrefillHistory:
         layer = cache._layers.get(layer_idx)
         if layer is None:
             layer = _Layer(tuple(key.shape), key.dtype, key.device)     # no history yet: the chunk's rows alone
-        if not restore_history(layer, layer.block_runs(), scratch[0], scratch[1], key, value):
+        if not (len(layer.runs) > _TABLE_RUNS and self._restore_from_table(layer_idx, layer, key, value)) \
+                and not restore_history(layer, layer.block_runs(), scratch[0], scratch[1], key, value):
             for out, sink, blocks, tail, new in ((scratch[0], layer.sink_key, layer.key_blocks, layer.residual_key, key),
                                                  (scratch[1], layer.sink_value, layer.value_blocks, layer.residual_value, value)):
                 position = 0 if sink is None else sink.shape[2]

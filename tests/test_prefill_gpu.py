@@ -252,3 +252,81 @@ def test_launches_in_a_row_read_what_the_one_before_wrote(q_heads, kv_heads, q_t
         chain(lambda: None)
     torch.cuda.synchronize()
     assert torch.isfinite(expected.float()).all() and torch.equal(q, expected)
+
+
+@pytest.fixture
+def restores(monkeypatch):
+    """Calls of the two restore entry points: the runs given to one, the blocks given to the other."""
+    from inquant import _native as N
+    lib, calls = N.library(), []
+    history, table = lib.inq_restore_history, lib.inq_restore_blocks_table
+
+    def of_runs(args, stream):
+        calls.append(("runs", args._obj.n_runs))
+        return history(args, stream)
+
+    def of_blocks(*args):
+        calls.append(("blocks", args[2]))
+        return table(*args)
+    monkeypatch.setattr(lib, "inq_restore_history", of_runs)
+    monkeypatch.setattr(lib, "inq_restore_blocks_table", of_blocks)
+    return calls
+
+
+@pytest.mark.parametrize("seals", [32, 33, 70])
+def test_history_of_many_seals_is_restored_by_two_launches(restores, seals):
+    """A layer sealed block by block: up to 32 runs travel as records, more are addressed through decode descriptors."""
+    from inquant.cache import CacheConfig, InQuantCache
+    from inquant.codec import CodecConfig
+    from inquant.prefill import PrefillHistory
+    gen, heads = torch.Generator(device="cuda").manual_seed(seals), 2
+    cache = InQuantCache(CacheConfig(CodecConfig(donor_policy="min_error"), block_size=16, residual_length=8, sink_tokens=4, value_bits=2))
+
+    def states(tokens, n=heads):
+        return torch.randn((1, n, tokens, 128), device="cuda", generator=gen).bfloat16()
+    cache.update(states(12), states(12), 0)
+    for _ in range(seals):
+        cache.extend(states(16), states(16), 0)
+    assert len(cache._layers[0].runs) == seals
+    history = PrefillHistory(cache)
+    for tokens, kept in ((3, seals), (16, seals), (5, seals + 1)):       # the second chunk seals a block more
+        del restores[:]
+        history.chunk(states(tokens, 4), states(tokens), states(tokens), 0)
+        assert restores == ([("runs", kept)] if kept <= 32 else [("runs", 0), ("blocks", kept)])
+    history.check()
+    history.release()
+    assert not history._descriptors
+
+
+@pytest.mark.parametrize("block,fraction", [(256, 0.125), (64, 0.0), (40, 0.25), (16, 0.5), (104, 0.125)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_blocks_restored_through_descriptors_equal_their_own_tensors(restores, monkeypatch, block, fraction, dtype):
+    """Blocks that are not whole steps of 16 or parts of 64 tokens, no, 16, 32 and 64 salient channels, blocks of one
+    and of several to an encoder launch, beside the dense rows; a layer that was reset starts anew."""
+    import inquant.prefill as prefill
+    from inquant.cache import CacheConfig, InQuantCache
+    from inquant.codec import CodecConfig
+    monkeypatch.setattr(prefill, "_TABLE_RUNS", 1)
+    gen, heads = torch.Generator(device="cuda").manual_seed(block), 3
+    cache = InQuantCache(CacheConfig(CodecConfig(donor_policy="min_error", salient_fraction=fraction), block_size=block,
+                                     residual_length=8, sink_tokens=4, value_bits=2))
+    history = prefill.PrefillHistory(cache)
+
+    def states(tokens, n=heads):
+        return torch.randn((1, n, tokens, 128), device="cuda", generator=gen).to(dtype)
+    for _ in range(2):
+        for step, tokens in enumerate((20, 3 * block, 1, block + 3, 2 * block, 7, block)):
+            key, value = states(tokens), states(tokens)
+            layer = cache._layers.get(0)
+            expected = (key, value) if layer is None else [
+                torch.cat([sink, *(b.dequantize() for b in blocks), tail, new], dim=2) for sink, blocks, tail, new in
+                ((layer.sink_key, layer.key_blocks, layer.residual_key, key), (layer.sink_value, layer.value_blocks, layer.residual_value, value))]
+            by_table = layer is not None and len(layer.runs) > 1
+            del restores[:]
+            out = history.chunk(states(tokens, 6), key, value, 0)
+            assert ("blocks" in dict(restores)) == by_table and torch.isfinite(out.float()).all()
+            for scratch, rows in zip(history._scratch, expected):
+                assert torch.equal(scratch[:, :, :rows.shape[2]], rows), (step, tokens)
+        assert by_table
+        cache.reset()
+    history.check()
