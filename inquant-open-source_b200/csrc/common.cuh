@@ -39,14 +39,7 @@ inline cudaError_t launch_following(void (*kernel)(P...), dim3 grid, dim3 block,
   config.stream = stream;
   config.attrs = &early;
   config.numAttrs = 1;
-  cudaError_t err = cudaLaunchKernelEx(&config, kernel, args...);
-  if (err != cudaSuccess) {
-    // a runtime without extended launches: an ordinary one, whose error, if it has one too, is the caller's
-    (void)cudaGetLastError();
-    kernel<<<grid, block, shared, stream>>>(args...);
-    err = cudaGetLastError();
-  }
-  return err;
+  return cudaLaunchKernelEx(&config, kernel, args...);
 }
 __device__ __forceinline__ void follow_stream() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -14,6 +14,7 @@ RUNTIME = r"""
 #include <string.h>
 extern "C" {
 int fake_registers = 168, fake_failures = 0, fake_launches = 0;
+int fake_refusals = 0;   // of launches
 static int encode(...) { return 0; }
 void** __cudaRegisterFatBinary(void*) { static void* handle; return &handle; }
 void __cudaRegisterFatBinaryEnd(void**) {}
@@ -45,6 +46,11 @@ cudaError_t cudaGetDriverEntryPoint(const char*, void** p, unsigned long long, c
 }
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t) { ++fake_launches; return cudaSuccess; }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**) {
+  if (fake_refusals > 0) { --fake_refusals; return cudaErrorUnknown; }
+  ++fake_launches;
+  return cudaSuccess;
+}
 }
 """
 
@@ -89,3 +95,10 @@ def test_a_kernel_with_too_few_registers_is_not_launched(library):
     ctypes.c_int.in_dll(library, "fake_registers").value = 160
     assert _call(library, N.BF16) == N.ERR_UNSUPPORTED
     assert ctypes.c_int.in_dll(library, "fake_launches").value == 0
+
+
+def test_a_refused_launch_is_reported_and_not_repeated(library):
+    ctypes.c_int.in_dll(library, "fake_refusals").value = 1
+    assert _call(library, N.BF16) == N.ERR_CUDA
+    assert b"refused by the test" in library.inq_last_error() and ctypes.c_int.in_dll(library, "fake_launches").value == 0
+    assert _call(library, N.BF16) == N.OK and ctypes.c_int.in_dll(library, "fake_launches").value == 1
