@@ -2,7 +2,9 @@
 from __future__ import annotations
 
 import ctypes
+import importlib
 import os
+import warnings
 from ctypes import c_int32, c_int64, c_void_p
 
 import torch
@@ -190,21 +192,25 @@ def library() -> ctypes.CDLL:
     return _lib
 
 
-_host = None
+_host, _host_sought = None, False
 
 
 def host():
-    """Native host side of the per-layer calls (``csrc/host.cpp``), bound to this process's library."""
-    global _host
-    if _host is None:
+    """Native host side of the per-layer calls (``csrc/host.cpp``), bound to this process's library.  None, after a
+    warning, when it is missing or does not load: the Python code behind these calls then fills the same launches, at
+    8 to 25 us more per call."""
+    global _host, _host_sought
+    if not _host_sought:
         try:
-            from . import _host as module
+            module = importlib.import_module("._host", __package__)
+            lib = library()
+            module.bind(*(ctypes.cast(f, c_void_p).value for f in (lib.inq_decode_attention, lib.inq_append_token)), torch.Tensor)
+            _host = module
         except ImportError as exc:
-            raise ImportError("inquant/_host.so is missing or was built for another PyTorch: build it with "
-                              "`python inquant-open-source_b200/build.py`") from exc
-        lib = library()
-        module.bind(*(ctypes.cast(f, c_void_p).value for f in (lib.inq_decode_attention, lib.inq_append_token)), torch.Tensor)
-        _host = module
+            library()   # that one has no way round
+            warnings.warn(f"inquant/_host.so does not load ({exc}): decode and append take their slower Python form until "
+                          "`python inquant-open-source_b200/build.py` has run", RuntimeWarning, stacklevel=3)
+        _host_sought = True
     return _host
 
 

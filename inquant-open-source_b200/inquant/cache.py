@@ -623,9 +623,12 @@ class InQuantCache(_HFCache):
     def _write_token_native(layer: _Layer, keys, values, sink_position: int) -> bool:
         """One token into the tail (and the sink) in native code; False, with nothing launched, when that does not serve
         the tensors."""
+        host = N.host()
+        if host is None:
+            return False
         sink = (layer.sink_key_buffer, layer.sink_value_buffer) if sink_position >= 0 else (None, None)
-        done = N.host().append_token(keys, values, layer.tail_key_buffer, layer.tail_value_buffer, *sink,
-                                     layer.tail_count, sink_position, N.status_word(layer.device).data_ptr())
+        done = host.append_token(keys, values, layer.tail_key_buffer, layer.tail_value_buffer, *sink,
+                                 layer.tail_count, sink_position, N.status_word(layer.device).data_ptr())
         if done is not True and done is not None:
             N.check(done, "inq_append_token")
         return done is True

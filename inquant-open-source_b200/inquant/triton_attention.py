@@ -308,8 +308,8 @@ class PackedDecodeState:
         elif not math.isfinite(scale) or scale <= 0:
             return None
         device, kv_heads, n_blocks = self._device, self._kv_heads, len(self.key_blocks)
-        identity = N.stream_identity(device)
-        if identity != self._stream_identity:
+        identity, host = N.stream_identity(device), N.host()
+        if host is None or identity != self._stream_identity:
             return None
         pairs = kv_heads * ((query.shape[1] // kv_heads + 7) // 8)
         if not pairs:
@@ -320,10 +320,10 @@ class PackedDecodeState:
         else:
             workspace = self._own_workspace(records, device)
         kind, groups = self._kind
-        output = N.host().decode(query, sink_key, sink_value, residual_key, residual_value, scale, kv_heads, n_blocks,
-                                 self._packed_tokens, self._salient, kind, groups, self._tables.data_ptr(), self._key_map.data_ptr(),
-                                 self._value_map.data_ptr() if kind == 1 else 0, workspace, records * N.RECORD_FLOATS,
-                                 N.decode_counters(device, pairs, identity[1]).data_ptr(), N.status_word(device).data_ptr())
+        output = host.decode(query, sink_key, sink_value, residual_key, residual_value, scale, kv_heads, n_blocks,
+                             self._packed_tokens, self._salient, kind, groups, self._tables.data_ptr(), self._key_map.data_ptr(),
+                             self._value_map.data_ptr() if kind == 1 else 0, workspace, records * N.RECORD_FLOATS,
+                             N.decode_counters(device, pairs, identity[1]).data_ptr(), N.status_word(device).data_ptr())
         if type(output) is int:
             N.check(output, "inq_decode_attention")
         return output

@@ -36,13 +36,15 @@ def page_offsets_array(layout):
 def paged_decode(query, cache, blocks, dense, num_pages, tail_tokens, sink_tokens, layout, workspace, scale, output=None):
     # the ordinary call is checked and launched in native code; the rest takes the checks and errors below
     hkv, device = layout.heads, query.device
-    if type(query) is torch.Tensor and device.type == "cuda" and query.ndim == 3 and query.shape[1] >= hkv:
+    ordinary = type(query) is torch.Tensor and device.type == "cuda" and query.ndim == 3 and query.shape[1] >= hkv
+    host = N.host() if ordinary else None
+    if host is not None:
         pairs = hkv * ((query.shape[1] // hkv + 7) // 8)
         floats = workspace_floats(pairs, pairs * pair_units(num_pages, layout.block_size))
         identity = N.stream_identity(device)
-        result = N.host().paged_decode(query, cache, blocks, dense, output, num_pages, tail_tokens, sink_tokens, hkv, layout.block_size,
-                                       layout.page_bytes, layout.kernel_offsets, scale, workspace.acquire_address(floats, device, identity),
-                                       floats, N.decode_counters(device, pairs, identity[1]).data_ptr(), N.status_word(device).data_ptr())
+        result = host.paged_decode(query, cache, blocks, dense, output, num_pages, tail_tokens, sink_tokens, hkv, layout.block_size,
+                                   layout.page_bytes, layout.kernel_offsets, scale, workspace.acquire_address(floats, device, identity),
+                                   floats, N.decode_counters(device, pairs, identity[1]).data_ptr(), N.status_word(device).data_ptr())
         if type(result) is int:
             N.check(result, "inq_decode_attention")
         if result is not None:

@@ -1,5 +1,6 @@
 """The native host side of the per-layer calls against the Python code behind it: what it serves gives the same
 bits, and what it does not serve takes the general path.  A tensor subclass is never served."""
+import sys
 from types import SimpleNamespace
 
 import pytest
@@ -170,3 +171,33 @@ def test_append_with_the_keywords_of_an_attention_module_is_native(served, valid
         assert len(served["append_token"]) == 40 and caches[1].get_seq_length(0) == 50
     with pytest.raises(ValueError, match="1D integer tensor"):
         caches[1].append_for_attention(*new, 0, {"cache_position": 50})
+
+
+def test_calls_without_the_native_host_side_give_the_same(monkeypatch):
+    """An extension that does not load leaves every call to the Python code."""
+    from inquant import _native as N
+    from inquant.cache import CacheConfig, InQuantCache
+    from inquant.codec import CodecConfig
+    from inquant.triton_attention import PackedDecodeState, SharedDecodeWorkspace
+    from inquant_vllm.kernels import paged_decode
+    from inquant_vllm.layout import PageLayout
+    config = CacheConfig(CodecConfig(donor_policy="min_error"), block_size=64, residual_length=8, sink_tokens=4, value_bits=2)
+    layout, dense = PageLayout(64, 2), torch.randn((2, 2, 68, 128), device="cuda").to(torch.bfloat16)
+    prompt, query = [_rows(s, 2, 150, torch.bfloat16, "contiguous") for s in (1, 2)], _rows(3, 8, 1, torch.bfloat16, "contiguous")
+    new, pool = [_rows(s, 2, 1, torch.bfloat16, "contiguous") for s in (4, 5)], torch.zeros((1, layout.page_bytes), dtype=torch.uint8, device="cuda")
+
+    def run():
+        cache = InQuantCache(config)
+        cache.update(*prompt, 0)
+        view = cache.append_for_attention(*new, 0)
+        state = PackedDecodeState(view.key_blocks, view.value_blocks)
+        return (view.residual_key, state.decode(query, residual_key=view.residual_key, residual_value=view.residual_value),
+                paged_decode(query[:, :, 0], pool, torch.zeros(1, dtype=torch.int32, device="cuda"), dense, 0, 9, 4, layout,
+                             SharedDecodeWorkspace(), 128 ** -0.5))
+    expected = run()
+    monkeypatch.setattr(N, "_host", None)
+    monkeypatch.setattr(N, "_host_sought", False, raising=False)
+    monkeypatch.setitem(sys.modules, "inquant._host", None)        # an import of it raises ImportError
+    with pytest.warns(RuntimeWarning, match="slower Python form"):
+        without = run()
+    assert all(torch.equal(a, b) for a, b in zip(expected, without))
