@@ -29,18 +29,28 @@ HOST = os.path.join(HERE, "inquant", "_host.so")   # CPython extension: host sid
 
 
 def build_host(force: bool = False) -> str:
-    """Builds inquant/_host.so against the installed PyTorch."""
-    src = os.path.join(CSRC, "host.cpp")
+    """Builds inquant/_host.so against the installed PyTorch, anew for another PyTorch or Python."""
+    import sysconfig
+    if HERE not in sys.path:
+        sys.path.insert(0, HERE)
+    import torch
+    from inquant._native import host_built_for
+    src, stamp, built_for = os.path.join(CSRC, "host.cpp"), os.path.join(HERE, "build", "host.stamp"), host_built_for()
+    try:
+        with open(stamp) as file:
+            force = force or file.read() != built_for
+    except OSError:
+        force = True
     if force or _stale(HOST, [src, __file__, os.path.join(os.path.dirname(HERE), "include", "inquant_b200.h")]):
-        import sysconfig
-        import torch
         root = os.path.dirname(torch.__file__)
         cuda = os.path.dirname(os.path.dirname(os.path.realpath(shutil.which(os.environ.get("NVCC", "nvcc")) or "/usr/local/cuda/bin/nvcc")))
         includes = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
                     sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
         subprocess.run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC",
-                        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{i}" for i in includes), src, "-o", HOST,
+                        f'-DINQ_BUILT_FOR="{built_for}"', f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{i}" for i in includes), src, "-o", HOST,
                         f"-L{os.path.join(root, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"], check=True)
+        with open(stamp, "w") as file:
+            file.write(built_for)
     return HOST
 
 

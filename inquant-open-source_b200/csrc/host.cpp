@@ -280,4 +280,12 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host(void) {
+  PyObject* const created = PyModule_Create(&module);
+  // the PyTorch and the Python this was compiled against, compared before the first use
+  if (created && PyModule_AddStringConstant(created, "built_for", INQ_BUILT_FOR) < 0) {
+    Py_DECREF(created);
+    return nullptr;
+  }
+  return created;
+}

@@ -4,6 +4,7 @@ from __future__ import annotations
 import ctypes
 import importlib
 import os
+import sys
 import warnings
 from ctypes import c_int32, c_int64, c_void_p
 
@@ -195,21 +196,30 @@ def library() -> ctypes.CDLL:
 _host, _host_sought = None, False
 
 
+def host_built_for() -> str:
+    """What an extension against PyTorch's C++ interface depends on besides its source; the build compiles this text
+    into the native host side."""
+    return f"PyTorch {torch.__version__}, {sys.implementation.cache_tag}, C++11 ABI {int(torch._C._GLIBCXX_USE_CXX11_ABI)}"
+
+
 def host():
     """Native host side of the per-layer calls (``csrc/host.cpp``), bound to this process's library.  None, after a
-    warning, when it is missing or does not load: the Python code behind these calls then fills the same launches, at
-    8 to 25 us more per call."""
+    warning, when it is missing, does not load or was built for another PyTorch or Python (which may load and misread
+    tensors): the Python code behind these calls then fills the same launches, at 8 to 25 us more per call."""
     global _host, _host_sought
     if not _host_sought:
+        lib = library()   # that one has no way round
         try:
             module = importlib.import_module("._host", __package__)
-            lib = library()
+            found = getattr(module, "built_for", "an unknown PyTorch")
+        except ImportError as exc:
+            module, found = None, f"nothing that loads here ({exc})"
+        if found == host_built_for():
             module.bind(*(ctypes.cast(f, c_void_p).value for f in (lib.inq_decode_attention, lib.inq_append_token)), torch.Tensor)
             _host = module
-        except ImportError as exc:
-            library()   # that one has no way round
-            warnings.warn(f"inquant/_host.so does not load ({exc}): decode and append take their slower Python form until "
-                          "`python inquant-open-source_b200/build.py` has run", RuntimeWarning, stacklevel=3)
+        else:
+            warnings.warn(f"inquant/_host.so is built for {found}, not for {host_built_for()}: decode and append take their slower "
+                          "Python form until `python inquant-open-source_b200/build.py` has run", RuntimeWarning, stacklevel=3)
         _host_sought = True
     return _host
 
