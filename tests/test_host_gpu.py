@@ -201,3 +201,37 @@ def test_calls_without_the_native_host_side_give_the_same(monkeypatch):
     with pytest.warns(RuntimeWarning, match="slower Python form"):
         without = run()
     assert all(torch.equal(a, b) for a, b in zip(expected, without))
+
+
+def test_ordinary_tensors_are_served_and_no_others(served):
+    """Which form each call took: without this, both arms of a comparison could be the Python code."""
+    from inquant.cache import CacheConfig, InQuantCache
+    from inquant.codec import CodecConfig
+    from inquant.triton_attention import PackedDecodeState, SharedDecodeWorkspace
+    from inquant_vllm.kernels import paged_decode
+    from inquant_vllm.layout import PageLayout
+    config = CacheConfig(CodecConfig(donor_policy="min_error"), block_size=64, residual_length=8, sink_tokens=4, value_bits=2)
+    cache = InQuantCache(config)
+    cache.update(*(_rows(s, 2, 150, torch.bfloat16, "contiguous") for s in (1, 2)), 0)
+    forms = {"contiguous": True, "token-major": True, "slice": True, "unaligned": False}
+    for form in forms:
+        view = cache.append_for_attention(*(_rows(s, 2, 1, torch.bfloat16, form) for s in (3, 4)), 0)
+    cache.append_for_attention(*(_rows(s, 2, 1, torch.bfloat16, "contiguous").as_subclass(Wrapped) for s in (3, 4)), 0)
+    # (what the plain call does not serve is offered again behind its checks)
+    assert served["append_token"] == [True, True, True, False, False, False, False]
+    state = PackedDecodeState(view.key_blocks, view.value_blocks)
+    dense = {"residual_key": view.residual_key, "residual_value": view.residual_value}
+    for form in forms:
+        state.decode(_rows(5, 8, 1, torch.bfloat16, form), **dense)
+    assert served["decode"] == list(forms.values())
+    state.decode(_rows(5, 8, 1, torch.float32, "contiguous"), **{n: t.float() for n, t in dense.items()})
+    assert served["decode"] == [*forms.values(), False]
+    state.decode(_rows(5, 8, 1, torch.bfloat16, "contiguous").as_subclass(Wrapped), **dense)
+    assert len(served["decode"]) == 5          # (not even asked)
+    layout, workspace = PageLayout(64, 2), SharedDecodeWorkspace()
+    pool, ids = torch.zeros((2, layout.page_bytes), dtype=torch.uint8, device="cuda"), torch.zeros(2, dtype=torch.int32, device="cuda")
+    rows, query = torch.randn((2, 2, 68, 128), device="cuda").to(torch.bfloat16), _rows(6, 8, 1, torch.bfloat16, "contiguous")[:, :, 0]
+    unaligned = _rows(6, 8, 1, torch.bfloat16, "unaligned")[:, :, 0]
+    for q, i in ((query, ids), (unaligned, ids), (query, ids.long())):
+        paged_decode(q, pool, i, rows, 0, 5, 4, layout, workspace, 128 ** -0.5)
+    assert served["paged_decode"] == [True, False, False]
