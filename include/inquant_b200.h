@@ -422,7 +422,9 @@ int64_t inq_decode_workspace_floats(int32_t n_pairs, int64_t total_units);
 /* The launch that inq_decode_attention makes for such a batch with `ctas_per_sm` resident CTAs per SM (it
  * asks the runtime for that number): the list of total_units + n_pairs * ramp_units positions is cut into
  * n_ctas ranges of per_cta, and shared_bytes of dynamic shared memory hold the merge of a pair that is
- * cut into up to merge_parts parts.  INQ_ERR_CAPACITY as the launch itself would answer.  Host only. */
+ * cut into up to merge_parts parts.  INQ_ERR_CAPACITY as the launch itself would answer.  Host only.
+ * inq_decode_launch_shape answers for launches with `pair_starts`; launches without, whose pairs all hold
+ * pair_units units, may give every pair ranges of its own: those are inq_decode_launch_shape_uniform's. */
 typedef struct {
   int32_t n_ctas, shared_bytes;
   int64_t per_cta, ramp_units;
@@ -430,6 +432,8 @@ typedef struct {
 } inq_decode_shape_t;
 int inq_decode_launch_shape(int32_t n_pairs, int64_t total_units, int32_t block_tokens, int32_t n_pad, int32_t value_kind,
                             int32_t value_groups, int32_t ctas_per_sm, inq_decode_shape_t* shape);
+int inq_decode_launch_shape_uniform(int32_t n_pairs, int64_t pair_units, int32_t block_tokens, int32_t n_pad, int32_t value_kind,
+                                    int32_t value_groups, int32_t ctas_per_sm, inq_decode_shape_t* shape);
 
 /* ---------------------------------------------------------------- incremental append
  * Writes the key and value rows of ONE new token (all KV heads) at `tail_position` of the

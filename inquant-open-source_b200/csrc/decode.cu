@@ -2300,12 +2300,12 @@ extern "C" int64_t inq_decode_workspace_floats(int32_t n_pairs, int64_t total_un
   return ((int64_t)most + 2 * n_pairs) * kRecordFloats;
 }
 
-extern "C" int inq_decode_launch_shape(int32_t n_pairs, int64_t total_units, int32_t block_tokens, int32_t n_pad, int32_t value_kind,
-                                       int32_t value_groups, int32_t ctas_per_sm, inq_decode_shape_t* shape) {
+static int launch_shape(int n_pairs, long long total_units, long long uniform_units, int block_tokens, int n_pad, int value_kind,
+                        int value_groups, int ctas_per_sm, inq_decode_shape_t* shape) {
   if (!shape || n_pairs < 1 || total_units < n_pairs || block_tokens < 1 || n_pad < 0 || n_pad > 64 || ctas_per_sm < 1)
     return INQ_ERR_ARGUMENT;
   const int sub = block_tokens <= 16 ? 1 : 2, groups = (n_pad + 15) / 16;
-  const Plan plan = make_plan(total_units, n_pairs, 0, ctas_per_sm);
+  const Plan plan = make_plan(total_units, n_pairs, uniform_units, ctas_per_sm);
   const int shared = launch_smem(smem_bytes(groups, sub, value_kind, value_groups), smem_bytes(value_kind ? 1 : 4, sub, value_kind, value_groups),
                                  plan.n_ctas);
   if (shared < 0) return INQ_ERR_CAPACITY;
@@ -2316,6 +2316,17 @@ extern "C" int inq_decode_launch_shape(int32_t n_pairs, int64_t total_units, int
   shape->merge_parts = (int32_t)((shared - merge_bytes(0)) / (merge_bytes(1) - merge_bytes(0)));
   shape->reserved = 0;
   return INQ_OK;
+}
+
+extern "C" int inq_decode_launch_shape(int32_t n_pairs, int64_t total_units, int32_t block_tokens, int32_t n_pad, int32_t value_kind,
+                                       int32_t value_groups, int32_t ctas_per_sm, inq_decode_shape_t* shape) {
+  return launch_shape(n_pairs, total_units, 0, block_tokens, n_pad, value_kind, value_groups, ctas_per_sm, shape);
+}
+
+extern "C" int inq_decode_launch_shape_uniform(int32_t n_pairs, int64_t pair_units, int32_t block_tokens, int32_t n_pad, int32_t value_kind,
+                                               int32_t value_groups, int32_t ctas_per_sm, inq_decode_shape_t* shape) {
+  if (pair_units < 1 || pair_units >= (1ll << 31)) return INQ_ERR_ARGUMENT;
+  return launch_shape(n_pairs, (long long)n_pairs * pair_units, pair_units, block_tokens, n_pad, value_kind, value_groups, ctas_per_sm, shape);
 }
 
 extern "C" int inq_decode_attention(const inq_decode_args_t* a, inq_stream_t stream_) {

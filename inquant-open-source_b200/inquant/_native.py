@@ -229,7 +229,7 @@ EXPORTS = (
     "inq_last_error", "inq_version", "inq_k4_encode", "inq_select_donors", "inq_k4_statistics",
     "inq_k4_dequantize", "inq_k4_dequantize_strided", "inq_v_encode", "inq_v_dequantize", "inq_v_dequantize_strided",
     "inq_build_roles", "inq_write_codec_pages",
-    "inq_decode_attention", "inq_decode_attention_noalloc", "inq_decode_units", "inq_merge_partials", "inq_decode_workspace_floats", "inq_decode_launch_shape", "inq_append_token", "inq_append_token_batch", "inq_seal_blocks", "inq_restore_history",
+    "inq_decode_attention", "inq_decode_attention_noalloc", "inq_decode_units", "inq_merge_partials", "inq_decode_workspace_floats", "inq_decode_launch_shape", "inq_decode_launch_shape_uniform", "inq_append_token", "inq_append_token_batch", "inq_seal_blocks", "inq_restore_history",
     "inq_prefill_attention", "inq_decode_generic", "inq_decode_generic_workspace_floats",
     "inq_prefill_workspace_bytes",
     "inq_exchange_merge", "inq_exchange_inbox_bytes", "inq_decode_exchange_inbox_bytes", "inq_restore_blocks_table", "inq_peer_buffer_create", "inq_peer_buffer_open",
@@ -251,6 +251,7 @@ SIGNATURES = {
     "inq_restore_blocks_table": [_P, _P, _I, _I, _I, _I, _P, _P, _L, _L, _I, _P],
     "inq_decode_attention": [_P, _P],
     "inq_decode_launch_shape": [_I, _L, _I, _I, _I, _I, _I, _P],
+    "inq_decode_launch_shape_uniform": [_I, _L, _I, _I, _I, _I, _I, _P],
     "inq_write_codec_pages": [_P, _P],
     "inq_decode_attention_noalloc": [_P, _P],
     "inq_merge_partials": [_P, _I, _L, _P, _I, _P],

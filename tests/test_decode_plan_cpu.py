@@ -81,3 +81,44 @@ def test_launch_shape_refuses_what_no_launch_could_have():
     assert lib.inq_decode_launch_shape(1, 1, 16, 0, 0, 2, 4, None) == N.ERR_ARGUMENT
     for bad in ((0, 1, 16, 0, 0, 2, 4), (2, 1, 16, 0, 0, 2, 4), (1, 1, 0, 0, 0, 2, 4), (1, 1, 16, 65, 0, 2, 4), (1, 1, 16, 0, 0, 2, 0)):
         assert lib.inq_decode_launch_shape(*bad, ctypes.byref(shape)) == N.ERR_ARGUMENT
+
+
+@pytest.mark.parametrize("block_tokens,n_pad", [(16, 16), (64, 16), (256, 16), (16, 48), (40, 0)])
+def test_pairs_of_equal_length_are_covered_once_by_resident_ranges(block_tokens, n_pad):
+    """The launch without a list of starts, walked as the kernel walks it: every slice of every pair in one range, each
+    part with a record of its own inside the workspace, no more parts than the merge's scratch holds."""
+    lib, shape = N.library(), N.DecodeShape()
+    own = 0
+    for ctas_per_sm in (1, 2, 3, 4):
+        for pairs in (1, 2, 8, 16, 28 * 4, 32 * 8, 444, 445, 1000):
+            for units in (1, 2, 7, 8, 9, 31, 40, 63, 64, 65, 128, 250, 512, 1000, 4096):
+                if pairs * units > 200000:
+                    continue
+                assert lib.inq_decode_launch_shape_uniform(pairs, units, block_tokens, n_pad, 0, 2, ctas_per_sm, ctypes.byref(shape)) == N.OK
+                ramp, per, total = shape.ramp_units, shape.per_cta, pairs * (units + shape.ramp_units)
+                assert shape.n_ctas <= 148 * ctas_per_sm and (shape.n_ctas - 1) * per < total <= shape.n_ctas * per
+                own += ramp + units == per * -(-units // per) and pairs > 1
+                workspace = lib.inq_decode_workspace_floats(pairs, pairs * units) // N.RECORD_FLOATS
+                ends, parts, records = [0] * pairs, [0] * pairs, set()
+                for cta in range(shape.n_ctas):
+                    pos, stop = cta * per, min((cta + 1) * per, total)
+                    pair = pos // (units + ramp)
+                    while pos < stop:
+                        first = pair * (units + ramp) + ramp                 # the pair's first slice
+                        lo, hi = max(pos, first) - first, min(stop, first + units) - first
+                        pos = min(stop, first + units)
+                        if hi > lo:
+                            assert lo == ends[pair] and cta - first // per == parts[pair]
+                            ends[pair], parts[pair] = hi, parts[pair] + 1
+                            records.add(cta + pair)
+                        pair += 1
+                assert ends == [units] * pairs and len(records) == sum(parts) and max(records) < workspace
+                assert parts == [(first + units - 1) // per - first // per + 1 for first in (p * (units + ramp) + ramp for p in range(pairs))]
+                assert max(parts) <= shape.merge_parts
+    assert own > 20      # ranges of their own are among them
+
+
+def test_uniform_launch_shape_refuses_what_no_launch_could_have():
+    lib, shape = N.library(), N.DecodeShape()
+    for bad in ((0, 1, 16, 0, 0, 2, 4), (2, 0, 16, 0, 0, 2, 4), (1, 1, 0, 0, 0, 2, 4), (1, 1, 16, 65, 0, 2, 4), (1, 1, 16, 0, 0, 2, 0)):
+        assert lib.inq_decode_launch_shape_uniform(*bad, ctypes.byref(shape)) == N.ERR_ARGUMENT
