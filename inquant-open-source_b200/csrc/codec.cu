@@ -1429,6 +1429,7 @@ __global__ void __launch_bounds__(256) v_dequantize128_kernel(const unsigned cha
 // of 32768 tokens in chunks of 2048 on one layer 9.82 -> 8.68 ms.
 constexpr int kRestoreTokens = 64;
 constexpr int kRestoreRuns = 8;     // runs of one launch
+constexpr long long kRestoreCtas = 1ll << 30;   // fewer of one launch decode
 
 // the blocks of one encoder launch: contiguous fields [block][head]...
 struct RestoreRun {
@@ -2038,15 +2039,16 @@ extern "C" int inq_restore_history(const inq_restore_args_t* a, inq_stream_t str
     if (a->value_kind == 0 ? (a->value_bits != 2 && a->value_bits != 4) || (a->value_group != 32 && a->value_group != 64 && a->value_group != 128)
                            : a->value_kind != 1)
       return INQ_ERR_ARGUMENT;
+    p.parts = (a->block_tokens + kRestoreTokens - 1) / kRestoreTokens;
     for (int r = 0; r < a->n_runs; ++r) {
       const inq_restore_run_t& run = a->runs[r];
       if (run.n_blocks < 1 || run.n_blocks >= (1ll << 31) || !run.key_payload || !run.key_scales || !run.value_payload || !run.value_scales) return INQ_ERR_ARGUMENT;
       if (a->count && (!run.key_salient || !run.key_donors || !run.key_padding)) return INQ_ERR_ARGUMENT;
       if (a->value_kind == 0 ? !run.value_offsets : a->value_count && (!run.value_salient || !run.value_donors || !run.value_padding)) return INQ_ERR_ARGUMENT;
       if (((uintptr_t)run.key_payload | (uintptr_t)run.value_payload) % 4) return INQ_ERR_ARGUMENT;   // words of 8 nibbles or 2-bit codes
+      if (run.n_blocks > (kRestoreCtas - 1) / ((long long)a->heads * p.parts)) return INQ_ERR_UNSUPPORTED;   // a run is part of one launch
     }
     p.tokens = a->block_tokens;
-    p.parts = (a->block_tokens + kRestoreTokens - 1) / kRestoreTokens;
     p.count = a->count;
     p.value_count = a->value_count;
     p.value_group = a->value_group;
@@ -2065,10 +2067,7 @@ extern "C" int inq_restore_history(const inq_restore_args_t* a, inq_stream_t str
     long long blocks = 0;
     while (next < a->n_runs && p.n_runs < kRestoreRuns) {
       const inq_restore_run_t& run = a->runs[next];
-      if ((blocks + run.n_blocks) * a->heads * p.parts >= (1ll << 30)) {
-        if (!p.n_runs) return INQ_ERR_UNSUPPORTED;
-        break;
-      }
+      if (p.n_runs && (blocks + run.n_blocks) * a->heads * p.parts >= kRestoreCtas) break;
       RestoreRun& out = p.run[p.n_runs];
       out.key_payload = (const unsigned char*)run.key_payload;
       out.key_scales = (const float*)run.key_scales;

@@ -144,3 +144,12 @@ def test_restore_structs_match_the_header_and_bad_arguments_are_refused_before_a
     args = N.RestoreArgs()
     args.out_dtype = N.BF16
     assert lib.inq_restore_history(ctypes.byref(args), None) == N.OK
+
+
+def test_a_run_too_large_for_a_launch_is_refused_before_the_runs_ahead_of_it_are_launched():
+    from inquant import _native as N
+    for sizes in ((1, 1 << 28), (1 << 28, 1), (*[1] * 9, 1 << 30), (1, (1 << 31) - 1)):
+        runs = (N.RestoreRun * len(sizes))(*(N.RestoreRun(*[4096] * 11, n) for n in sizes))
+        args = N.RestoreArgs(ctypes.addressof(runs), len(sizes), 4, 64, 16, 0, 2, 64, 0, 4096, 4096, 1024, 0)
+        args.out_dtype = N.BF16
+        assert N.library().inq_restore_history(ctypes.byref(args), None) == N.ERR_UNSUPPORTED, sizes
