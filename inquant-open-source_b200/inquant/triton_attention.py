@@ -315,8 +315,10 @@ class PackedDecodeState:
         if not pairs:
             return None
         records = self._records(pairs, n_blocks)
-        if self._workspace_pool is not None:
-            workspace = self._workspace_pool.acquire_address(records * N.RECORD_FLOATS, device, identity)
+        pool, bound = self._workspace_pool, None
+        if pool is not None:
+            bound = pool._stream_identity
+            workspace = pool.acquire_address(records * N.RECORD_FLOATS, device, identity)
         else:
             workspace = self._own_workspace(records, device)
         kind, groups = self._kind
@@ -326,6 +328,8 @@ class PackedDecodeState:
                              N.decode_counters(device, pairs, identity[1]).data_ptr(), N.status_word(device).data_ptr())
         if type(output) is int:
             N.check(output, "inq_decode_attention")
+        if output is None and pool is not None:
+            pool._stream_identity = bound       # nothing was launched: the call has tied the pool to no stream
         return output
 
     def _records(self, pairs: int, n_blocks: int) -> int:

@@ -41,7 +41,7 @@ def paged_decode(query, cache, blocks, dense, num_pages, tail_tokens, sink_token
     if host is not None:
         pairs = hkv * ((query.shape[1] // hkv + 7) // 8)
         floats = workspace_floats(pairs, pairs * pair_units(num_pages, layout.block_size))
-        identity = N.stream_identity(device)
+        identity, bound = N.stream_identity(device), workspace._stream_identity
         result = host.paged_decode(query, cache, blocks, dense, output, num_pages, tail_tokens, sink_tokens, hkv, layout.block_size,
                                    layout.page_bytes, layout.kernel_offsets, scale, workspace.acquire_address(floats, device, identity),
                                    floats, N.decode_counters(device, pairs, identity[1]).data_ptr(), N.status_word(device).data_ptr())
@@ -49,6 +49,7 @@ def paged_decode(query, cache, blocks, dense, num_pages, tail_tokens, sink_token
             N.check(result, "inq_decode_attention")
         if result is not None:
             return result
+        workspace._stream_identity = bound      # nothing was launched: the call has tied the workspace to no stream
     if query.shape[0] != 1 or query.shape[-1] != 128 or query.dtype != torch.bfloat16:
         raise ValueError("Paged decode expects one BF16 query [1, heads, 128]")
     hq, hkv = query.shape[1], layout.heads

@@ -235,3 +235,33 @@ def test_ordinary_tensors_are_served_and_no_others(served):
     for q, i in ((query, ids), (unaligned, ids), (query, ids.long())):
         paged_decode(q, pool, i, rows, 0, 5, 4, layout, workspace, 128 ** -0.5)
     assert served["paged_decode"] == [True, False, False]
+
+
+def test_a_refused_call_ties_a_shared_workspace_to_no_stream():
+    from inquant.codec import CodecConfig, quantize
+    from inquant.triton_attention import PackedDecodeState, SharedDecodeWorkspace
+    from inquant.value_codec import quantize_values
+    from inquant_vllm.kernels import paged_decode
+    from inquant_vllm.layout import PageLayout
+    side = torch.cuda.Stream()
+    k, q = _rows(1, 2, 64, torch.bfloat16, "contiguous"), _rows(2, 8, 1, torch.bfloat16, "contiguous")
+    blocks = [quantize(k, CodecConfig(donor_policy="min_error"))], [quantize_values(k)]
+    pool = SharedDecodeWorkspace()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side), pytest.raises(ValueError, match="match query dtype"):
+        PackedDecodeState(*blocks, workspace_pool=pool).decode(q, residual_key=k.half(), residual_value=k.half())
+    torch.cuda.synchronize()
+    PackedDecodeState(*blocks, workspace_pool=pool).decode(q, residual_key=k, residual_value=k)
+    layout, workspace = PageLayout(64, 2), SharedDecodeWorkspace()
+    pages, ids = torch.zeros((1, layout.page_bytes), dtype=torch.uint8, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    dense = torch.randn((2, 2, 68, 128), device="cuda").to(torch.bfloat16)
+
+    def paged(query):
+        return paged_decode(query[:, :, 0], pages, ids, dense, 0, 9, 4, layout, workspace, 128 ** -0.5)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side), pytest.raises(ValueError, match="one BF16 query"):
+        paged(q.half())
+    paged(q)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side), pytest.raises(RuntimeError, match="one CUDA stream"):     # a served call ties it, as before
+        paged(q)
