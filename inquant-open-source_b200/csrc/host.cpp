@@ -271,10 +271,22 @@ PyObject* paged_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   });
 }
 
+// same_objects(list, list) -> whether both hold the same objects in the same order
+PyObject* same_objects(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 2) return PyErr_Format(PyExc_TypeError, "same_objects takes 2 arguments");
+  if (!PyList_Check(args[0]) || !PyList_Check(args[1])) Py_RETURN_FALSE;
+  const Py_ssize_t count = PyList_GET_SIZE(args[0]);
+  if (count != PyList_GET_SIZE(args[1])) Py_RETURN_FALSE;
+  for (Py_ssize_t i = 0; i < count; ++i)
+    if (PyList_GET_ITEM(args[0], i) != PyList_GET_ITEM(args[1], i)) Py_RETURN_FALSE;
+  Py_RETURN_TRUE;
+}
+
 PyMethodDef methods[] = {{"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(bind)), METH_FASTCALL, nullptr},
                          {"append_token", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(append_token)), METH_FASTCALL, nullptr},
                          {"decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(decode)), METH_FASTCALL, nullptr},
                          {"paged_decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(paged_decode)), METH_FASTCALL, nullptr},
+                         {"same_objects", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(same_objects)), METH_FASTCALL, nullptr},
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

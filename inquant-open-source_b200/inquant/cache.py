@@ -18,9 +18,7 @@ Only batch-one, append-only inference on CUDA tensors is supported.
 """
 from __future__ import annotations
 
-import itertools
 import math
-import operator
 from dataclasses import dataclass, field
 from typing import Any, Iterator
 
@@ -86,17 +84,25 @@ class _Layer:
     packed_nbytes: int = 0
     retired_tail: tuple | None = None               # the tail buffers replaced by the last seal
     sink_views: tuple | None = None                 # (count, key view, value view) handed out last
-    runs: list = field(default_factory=list)        # what sealed the blocks: (key blocks, value blocks, keys' owner, values' owner)
+    sealed_blocks: tuple = field(default_factory=lambda: ([], []))   # the key and value blocks as the seals appended them
+    runs: list = field(default_factory=list)        # blocks of each of these seals
 
     def block_runs(self):
-        """The sealed blocks as runs of one encoder launch each, ``(key blocks, value blocks, keys' owner, values'
-        owner)``: an owner is the arena of such a launch, or a block of its own.  None when any block is not the one
-        that a seal appended at its place."""
-        for blocks, side in ((self.key_blocks, 0), (self.value_blocks, 1)):
-            if len(blocks) != sum(len(run[side]) for run in self.runs) \
-                    or not all(map(operator.is_, blocks, itertools.chain.from_iterable(run[side] for run in self.runs))):
-                return None
-        return self.runs
+        """The sealed blocks as runs of one encoder launch each, ``(blocks, keys' owner, values' owner)``: an owner is
+        the arena of such a launch, or a block of its own.  None when any block is not the one that a seal appended at
+        its place."""
+        keys, values = self.sealed_blocks
+        if not (N.same_objects(self.key_blocks, keys) and N.same_objects(self.value_blocks, values)):
+            return None
+        runs, at = [], 0
+        for count in self.runs:
+            owners = [getattr(side[at], "_arena", None) for side in (keys, values)] if count > 1 else (None, None)
+            if count > 1 and all(owner is not None and owner[0].shape[0] == count for owner in owners):
+                runs.append((count, owners[0][0], owners[1][0]))
+            else:   # a block of its own, or several
+                runs.extend((1, *pair) for pair in zip(keys[at:at + count], values[at:at + count]))
+            at += count
+        return runs
 
     def _sink_pair(self):
         """The sink views for the current count: the same two tensor objects until the count changes
@@ -205,14 +211,14 @@ def _dequantize_arena_into(arena, out: torch.Tensor, position: int) -> bool:
 
 
 def _row_copy(entry, source: torch.Tensor, first: int, target: torch.Tensor, start: int, tokens: int) -> None:
-    """Fill one ``inq_row_copy_t``: ``tokens`` rows of ``source`` [1, H, tokens, C] from ``first`` on to ``target`` from ``start`` on."""
+    """Fill one ``inq_row_copy_t``: ``tokens`` rows of ``source`` [1, H, tokens, C], 16-bit, from ``first`` on to ``target``
+    from ``start`` on."""
     _, source_h, source_t, _ = source.stride()
     _, target_h, target_t, _ = target.stride()
-    size = source.element_size()
-    entry.src = source.data_ptr() + first * source_t * size
-    entry.dst = target.data_ptr() + start * target_t * size
-    entry.src_stride_h, entry.src_stride_t = source_h * size, source_t * size
-    entry.dst_stride_h, entry.dst_stride_t = target_h * size, target_t * size
+    entry.src = source.data_ptr() + first * source_t * 2
+    entry.dst = target.data_ptr() + start * target_t * 2
+    entry.src_stride_h, entry.src_stride_t = source_h * 2, source_t * 2
+    entry.dst_stride_h, entry.dst_stride_t = target_h * 2, target_t * 2
     entry.tokens = tokens
 
 
@@ -243,7 +249,7 @@ def restore_history(layer: _Layer, runs, out_key: torch.Tensor, out_value: torch
     args.position = layer.sink_count
     position = layer.sink_count + restored_tokens
     if runs:
-        first_key, first_value = runs[0][2:]
+        first_key, first_value = runs[0][1:]
         block_tokens, count = first_key.shape[2], first_key.salient_channels.shape[-1]
         coded = not isinstance(first_value, PackedValues)
         args.block_tokens, args.count = block_tokens, count
@@ -254,7 +260,7 @@ def restore_history(layer: _Layer, runs, out_key: torch.Tensor, out_value: torch
         if count > 64 or (coded and args.value_count > 64):
             return False
         records = (N.RestoreRun * len(runs))()
-        for record, (sealed, _, keys, values) in zip(records, runs):
+        for record, (blocks, keys, values) in zip(records, runs):
             fields = [keys.payload, keys.scales, keys.salient_channels, keys.donor_channels, keys.padding, values.payload, values.scales]
             names = ["key_payload", "key_scales", "key_salient", "key_donors", "key_padding", "value_payload", "value_scales"]
             if coded:
@@ -267,8 +273,8 @@ def restore_history(layer: _Layer, runs, out_key: torch.Tensor, out_value: torch
                 if not tensor.is_contiguous() or tensor.dtype == torch.int32:
                     return False
                 setattr(record, name, tensor.data_ptr() or None)
-            record.n_blocks = len(sealed)
-            position += len(sealed) * block_tokens
+            record.n_blocks = blocks
+            position += blocks * block_tokens
         args.runs, args.n_runs = N.ctypes.cast(records, N.c_void_p), len(runs)
     copies = []
     if layer.sink_count:
@@ -784,19 +790,13 @@ class InQuantCache(_HFCache):
         layer.key_blocks.extend(new_keys)
         layer.value_blocks.extend(new_values)
         if blocks:
-            self._record_run(layer, new_keys, new_values)
+            layer.sealed_blocks[0].extend(new_keys)
+            layer.sealed_blocks[1].extend(new_values)
+            layer.runs.append(blocks)
         if cfg.track_peak_bytes:
             layer.packed_nbytes += sum(block.nbytes for block in new_keys + new_values)
         layer.seq_length += new_tokens
         return tail
-
-    @staticmethod
-    def _record_run(layer: _Layer, new_keys, new_values) -> None:
-        owners = [getattr(new[0], "_arena", (new[0], 0))[0] for new in (new_keys, new_values)]
-        if len(new_keys) == len(new_values) and all(owner.shape[0] == len(new_keys) for owner in owners):
-            layer.runs.append((tuple(new_keys), tuple(new_values), *owners))
-        else:   # sealed block by block
-            layer.runs.extend(((k,), (v,), k, v) for k, v in zip(new_keys, new_values))
 
     def record_peak(self, layer_idx):
         """Live persistent bytes in O(1) per layer update (reference ``cache.py:308-326``)."""
@@ -832,7 +832,7 @@ class InQuantCache(_HFCache):
         if runs is None:
             packed = [sum(block.shape[2] for block in blocks) for blocks in (layer.key_blocks, layer.value_blocks)]
         else:
-            packed = [sum(len(run[0]) * run[2].shape[2] for run in runs)] * 2
+            packed = [sum(blocks * owner.shape[2] for blocks, owner, _ in runs)] * 2
         full = [torch.empty((1, heads, sink_tokens + packed_tokens + tail_tokens + new_tokens, channels),
                             dtype=layer.dtype, device=layer.device) for packed_tokens in packed]
         if restore_history(layer, runs, *full, new_key, new_value):

@@ -187,7 +187,7 @@ class PrefillHistory:
         from .cache import restore_history
         from .triton_attention import PackedDecodeState
         out_key, out_value = self._scratch[:2]
-        blocks, state, values = len(layer.key_blocks), self._descriptors.get(layer_idx), layer.runs[0][3]
+        blocks, state, values = len(layer.key_blocks), self._descriptors.get(layer_idx), layer.value_blocks[0]
         if (getattr(values, "bits", 0), getattr(values, "group_size", 0)) != (2, 64):
             return False
         try:

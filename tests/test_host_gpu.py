@@ -43,7 +43,7 @@ def served(monkeypatch):
             calls[name].append(result is not None)
             return result
         return call
-    module = SimpleNamespace(**{name: counted(name) for name in calls})
+    module = SimpleNamespace(same_objects=host.same_objects, **{name: counted(name) for name in calls})
     monkeypatch.setattr(N, "host", lambda: module)
     return calls
 

@@ -59,3 +59,14 @@ def test_the_module_is_built_anew_for_another_pytorch(unsought, tmp_path):
         unsought.setattr(N, "host_built_for", lambda: f"PyTorch {version}")
         build.build_host()
         assert len(commands) == runs and f'-DINQ_BUILT_FOR="PyTorch {version}"' in commands[-1]
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_lists_of_the_same_objects(unsought, native):
+    if not native:
+        unsought.setattr(N, "_host_sought", True)
+    assert (N.host() is not None) == native
+    a, b = object(), object()
+    for x, y, same in (([], [], True), ([a], [], False), ([a, b], [a, b], True), ([a, b], [b, a], False), ([a, a], [a, b], False),
+                       ([1000.5], [float("1000.5")], False)):       # equal, but another object
+        assert N.same_objects(x, y) is same
