@@ -62,8 +62,8 @@ struct SliceCfg {
 constexpr int kPlanSliceTokens = 32;                // the unit of the flat work list (equal for both SUB when a block has <= 16 tokens)
 constexpr int kCtasPerSm = 3;                       // register budget: 168 per thread
 // Blocks of at most 16 tokens: every slice pays for a whole block's fold, a chain of dependent steps, and a
-// fourth CTA per SM (128 registers per thread) hides more of it than 168 registers save.  With more than 16
-// salient channels (WIDE) the larger scratch holds three CTAs at most, so these keep 168 registers, and two
+// fourth CTA per SM (128 registers per thread; 12 bytes are spilled, 4 of them read back) hides more of it than 168
+// registers save.  With more than 16 salient channels (WIDE) the larger scratch holds three CTAs at most, so these keep 168 registers, and two
 // ring stages, whose space is what lets the third CTA in at 33 to 48 channels: 28 layers of 8192 tokens at
 // 32 / 48 / 64 salient channels 139.3 / 159.7 / 215.0 us (with 128 registers 145.4 / 169.9 / 227.4, with 168
 // and three stages 139.3 / 200.7 / 215.0).
@@ -537,9 +537,10 @@ __global__ void __launch_bounds__(kThreads, VK ? 2 : SUB == 1 && !WIDE ? kCtasSm
   // look-up one block ahead, they are 630 and 1740, and a launch takes (us, before -> after, L2 warm) 129 -> 120
   // (28 layers x 4 heads x 32768 tokens), 93.5 -> 86.5 (16384 tokens, values coded like the keys), 3084 -> 2668
   // (16 requests x 32 layers x 8 heads, pages of 64) and 7272 -> 4201 (pages of 16).  The kernel runs at the power cap
-  // and close to the ALU's issue rate (280 of the 608 instructions per 16-token page): roles clamped two at a time, one
-  // fused add and minimum per channel for its record, the selection cell from a table and query addresses ready in the
-  // records took (us) 114.9 -> 112.4 (28 layers x 32768), 2639 -> 2624 and 4112 -> 3927.
+  // and close to the ALU's issue rate (a fold was 280 of the 608 instructions per 16-token page): roles clamped two at a
+  // time, one fused add and minimum per channel for its record, the selection cell from a table and query addresses
+  // ready in the records took (us) 114.9 -> 112.4 (28 layers x 32768), 2639 -> 2624 and 4112 -> 3927.  What the donors'
+  // constants add is summed in fp32 (pages of 16 4137 -> 4156 us against a matrix instruction on 16-bit operands).
   constexpr bool kNarrow = FAST || (SUB == 1 && !WIDE);
   // every slice is a block of its own: its weights are multiplied out where the score MMAs read them
   constexpr bool kDirect = SUB == 1 && kNarrow;
@@ -2227,9 +2228,10 @@ struct Plan {
 
 static int spb_of(int block_tokens) { return (block_tokens + kPlanSliceTokens - 1) / kPlanSliceTokens; }
 
-// List positions charged per pair for its fixed costs, in slices: a visit of a pair costs a CTA
-// 11-14 us (measured with the phase stamps) against ~0.45 us per 32-token slice of a 256-token
-// block; 12..36 all beat 0 on the 28-layer, 32768-token step (157.8 us at 24 against 163.1).
+// List positions charged per pair for its fixed costs (query staging, first copies, dense slices, record, merge), in
+// slices.  us at a charge of 0 / 6 / 12 / 18 / 24 / 32 / 48: 28 layers x 32768 tokens 127.6 / 126.4 / 126.0 / 125.2 / 124.4 /
+// 124.2 / 124.9; x 16384, coded values 85.6 / 85.3 / 83.5 / 83.0 / 82.8 / 82.6 / 82.5; 16 requests x 32 layers, pages of 64
+// 2828 / 2809 / 2766 / 2753 / 2749 / 2747 / 2750; pages of 16 4162 / 4157 / 4148 / 4156 / 4166 / 4156 / 4161 (no difference).
 constexpr long long kRampUnits = 24;
 
 static Plan make_plan(long long total_units, int n_pairs, long long uniform_units, int ctas_per_sm) {

@@ -176,9 +176,11 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const PrefillPar
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  // set up beside the end of the launch before it (one CTA per SM: there is no place to be had too early).  us back
-  // to back, before / after: 1500 x 1500 of 32 heads 32.9 / 30.4, 4096 x 4096 155 / 144, 2048 x 2048 of 28 37.9 / 36.7,
-  // 300 x 4000 in cuts with a merge 58.9 / 56.0
+  // Set up beside the end of the launch before it (one CTA per SM: there is no place to be had too early).  us per call,
+  // ordinary launches / these.  Calls in a row: 700 x 700 of 32 heads 18.9 / 16.0, 1500 x 1500 29.2 / 27.2, 4096 x 4096 129 /
+  // 126, 2048 x 2048 of 28 42 / 39, 512 x 8000 in cuts with a merge 91 / 86.  With another kernel between two calls only what
+  // the launch itself takes is hidden: of 16 MB 25.1 / 23.0, 35.4 / 33.4, 146 / 147, 45.5 / 42.2, 93 / 90; of 4 KB no difference,
+  // nor in graphs with either (in a row there 16.2 / 15.4, 27.0 / 26.0, 136 / 137, 36.4 / 35.4, 82.3 / 81.5).
   follow_stream();
   if (warp == 8) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
