@@ -64,7 +64,7 @@ def prefill_attention(query: torch.Tensor, key: torch.Tensor, value: torch.Tenso
 # More runs of blocks than this (every seal is one, of one block during decode) are restored through decode descriptors:
 # a record per run takes 4 us of host time and every eight records a launch, descriptors 250 us and more once and 40 us
 # per chunk.  us per chunk of 256 tokens behind 12 / 24 / 39 / 64 / 128 / 512 runs of one 256-token block each, records:
-# 264 / 305 / 338 / 413 / 698 / 2320; descriptors: 283 / 249 / 282 / 261 / 325 / 709.
+# 264 / 305 / 338 / 413 / 698 / 2320; descriptors: 283 / 249 / 282 / 259 / 301 / 640.
 _TABLE_RUNS = 32
 
 
